@@ -142,10 +142,10 @@ int modlin_block_inverse_device(uint64_t p, const uint64_t *d_P, size_t ldp, uin
 
 /* ---- Linear complexity (src/fp.rs:257-308) ------------------------------ */
 
-#define MODLIN_LC_AUTO 0      /* block kernel for short, cluster for long, grid beyond the cluster */
+#define MODLIN_LC_AUTO 0      /* block kernel for short sequences, grid from about 1000 on */
 #define MODLIN_LC_BLOCK 1     /* one CTA runs the whole sequence (plain form) */
-#define MODLIN_LC_GRID 2      /* persistent cooperative kernel, one grid barrier per step */
-#define MODLIN_LC_CLUSTER 3   /* one 16-CTA thread-block cluster, one cluster barrier per step
+#define MODLIN_LC_GRID 2      /* persistent cooperative kernel, one CTA per SM */
+#define MODLIN_LC_CLUSTER 3   /* the grid kernel on one 16-CTA thread-block cluster
                                  (n <= 409600; MODLIN_EINVAL_N beyond) */
 
 typedef struct {
@@ -169,7 +169,7 @@ int modlin_linear_complexity_device(uint64_t p, const uint64_t *d_s, size_t n,
  * the linear complexity of the device sequence d_s[0..n) is written to the
  * device slot *d_lc_out, asynchronously on `stream`, without any allocation
  * (n = 0 writes 0). The Berlekamp-Massey scratch lives in shared memory when
- * it fits (n <= 8533), else in a fixed 6 MiB device array, so n <= 262144
+ * it fits (200 KiB), else in a fixed 4 MiB device array, so n <= 262144
  * (MODLIN_EINVAL_N beyond). All calls share that array: calls that overlap on
  * the GPU race, so order them (e.g. one stream). The first call on a device
  * is a set-up that loads the library's device code for this entry point and

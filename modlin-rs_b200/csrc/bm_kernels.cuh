@@ -1,4 +1,4 @@
-// Berlekamp-Massey launchers (host side).
+// Linear-complexity launchers (host side).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -17,6 +17,19 @@ struct BmJob {
   int64_t slot;       // output index
 };
 
+// 64-bit words of the two residual arrays of an n-residue sequence, stored as
+// S (32-bit entries for p < 2^31).
+template <class S>
+MODLIN_HD int64_t bm_words(int64_t n) {
+  return (2 * (n + 64) * (int64_t)sizeof(S) + 7) / 8;
+}
+int64_t bm_smem_words(uint64_t p, int64_t n);  // for the storage type of p
+int64_t bm_workspace_words(int64_t n);         // for any p
+
+constexpr int64_t kBmMaxN = int64_t(1) << 30;  // longest sequence of the one-CTA kernels (32-bit indices)
+
+// threads: a multiple of 32 from 128 to 512. gws: workspace of
+// bm_smem_words(p, n) words when that is more than smem_words.
 cudaError_t launch_bm_block(const BmJob& job, uint64_t* gws, int64_t smem_words, int threads, int64_t* d_out,
                             cudaStream_t st);
 cudaError_t launch_bm_batch(const BmJob* d_jobs, int64_t count, unsigned long long* d_next, uint64_t* gws,
@@ -27,20 +40,18 @@ int bm_batch_max_blocks_per_sm(int threads, int64_t smem_words);
 // loaded module would otherwise be loaded, and its memory allocated, at the
 // first launch).
 cudaError_t bm_block_prepare();
-// spin: cycles a CTA waits at a grid barrier before it gives up and sets the
-// error word; skip_cta (>= 0, tests only): that CTA skips its arrival at the
-// first step barrier, so the waits expire.
-cudaError_t launch_bm_grid(const FieldParams& fp, const uint64_t* s, int64_t n, int ctas, int threads, uint64_t* b0,
-                           uint64_t* b1, void* gs, long long spin, int skip_cta, int64_t* d_out, cudaStream_t st,
-                           int* ctas_used);
-// One long sequence on one thread-block cluster of R = 16 CTAs (8 where 16
-// cannot be launched and the slices fit); b0, b1: n-word global workspaces.
-// bm_cluster_size gives R for n (0: too long for the cluster's shared memory).
-constexpr int64_t kBmClusterSliceBytes = 200 * 1024;
-int bm_cluster_size(int64_t n);
-cudaError_t launch_bm_cluster(const FieldParams& fp, const uint64_t* s, int64_t n, int R, uint64_t* b0, uint64_t* b1,
+
+// One long sequence on up to `ctas` CTAs (cooperative launch; at least two),
+// or on one thread-block cluster of 16 CTAs (8 where 16 cannot be launched).
+// ws: bm_long_bytes(n) bytes. spin: cycles a CTA waits before it gives up and
+// sets the error word (at bm_long_err_offset() in ws); skip_cta (>= 0, tests
+// only): that CTA does not signal, so the waits expire.
+size_t bm_long_bytes(int64_t n);
+int bm_long_err_offset();
+cudaError_t launch_bm_long(const FieldParams& fp, const uint64_t* s, int64_t n, int ctas, int num_sms, void* ws,
+                           long long spin, int skip_cta, int64_t* d_out, cudaStream_t st);
+cudaError_t launch_bm_cluster(const FieldParams& fp, const uint64_t* s, int64_t n, void* ws, long long spin,
                               int64_t* d_out, cudaStream_t st);
-size_t grid_sync_bytes();
-int grid_sync_err_offset();
+constexpr int64_t kBmClusterMaxN = 409600;
 
 }  // namespace modlin

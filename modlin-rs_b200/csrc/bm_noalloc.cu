@@ -4,20 +4,19 @@
 // hands every byte of device memory to its own pool allocator, or a loop that
 // must not pay the implicit device synchronisation of cudaMalloc/cudaFree.
 // modlin_linear_complexity_device_noalloc serves them: it runs the
-// one-CTA-per-sequence Berlekamp-Massey kernel (bm_block_kernel) with its
-// scratch — the c, b and t polynomials — in dynamic shared memory when they
-// fit (3n words within 200 KiB, n <= 8533), else in a fixed file-scope
-// device array, never in a workspace from cudaMalloc. The caller passes the
+// one-CTA-per-sequence kernel (bm_block_kernel) with its scratch — the two
+// residual arrays — in dynamic shared memory when they fit (200 KiB), else in
+// a fixed file-scope device array, never in a workspace from cudaMalloc. The caller passes the
 // sequence and the result slot, both in device memory.
 //
 // Limits and sharing:
-//  * at most kNoAllocMaxN residues per call (the array holds 3 * kNoAllocMaxN
-//    words = 6 MiB, which every GPU that loads the library keeps until exit);
+//  * at most kNoAllocMaxN residues per call (the array holds two arrays of
+//    kNoAllocMaxN words, 4 MiB, which every GPU that loads the library keeps
+//    until exit);
 //  * every call uses the same array, so calls that overlap on the GPU race:
 //    issue them on one stream (or otherwise order them);
-//  * the array keeps the previous call's contents; the kernel initialises c
-//    and b itself, and t is written before it is read, so nothing needs
-//    clearing between calls;
+//  * the array keeps the previous call's contents; the kernel initialises
+//    both residuals itself, so nothing needs clearing between calls;
 //  * the first call on a device is the set-up: with that device current it
 //    looks up the array's device address (cudaGetSymbolAddress) and caches
 //    it, and it loads the modules of the array and of the kernel, which the
@@ -39,9 +38,9 @@
 namespace modlin {
 
 constexpr int64_t kNoAllocMaxN = int64_t(1) << 18;
-constexpr int64_t kNoAllocSmemWords = (200 * 1024) / 8;  // shared memory used when 3n words fit
+constexpr int64_t kNoAllocSmemWords = (200 * 1024) / 8;  // shared memory used when the residuals fit
 
-static __device__ __align__(256) uint64_t g_noalloc_scratch[3 * kNoAllocMaxN];
+static __device__ __align__(256) uint64_t g_noalloc_scratch[2 * (kNoAllocMaxN + 64)];
 
 static std::mutex g_noalloc_mu;
 static uint64_t* g_noalloc_addr[64];  // device address of the array, per device
@@ -80,7 +79,7 @@ extern "C" int modlin_linear_complexity_device_noalloc(uint64_t p, const uint64_
   const int rc = noalloc_scratch(&scratch);
   if (rc != MODLIN_OK) return rc;
   const BmJob job{fp.p, fp.mu_lo, fp.mu_hi, fp.safe_batch, d_s, (int64_t)n, 0};
-  const cudaError_t e = launch_bm_block(job, scratch, kNoAllocSmemWords, n >= 4096 ? 1024 : 256, d_lc_out,
+  const cudaError_t e = launch_bm_block(job, scratch, kNoAllocSmemWords, n >= 1024 ? 512 : 256, d_lc_out,
                                         static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? MODLIN_OK : MODLIN_ECUDA;
 }

@@ -64,15 +64,19 @@ struct Tune {
   bool measured = false;
   int tc_cross[4] = {512, 512, 512, 512};           // 1, 2, 4, 8 limbs
   int two_panel_min = 256;
-  int bm_threads[4] = {256, 256, 1024, 1024};       // n < 1024, < 4096, < 16384, longer
-  int bm_cluster_min = 16384;
+  int bm_threads[4] = {256, 512, 512, 512};         // n < 1024, < 4096, < 16384, longer
+  int bm_long_min = 1024;                           // one CTA below, many from here on
+  int bm_cluster_min = 4096;                        // from here on one cluster beats one CTA (not a rule of AUTO)
   int bm_batch_threads[3] = {128, 256, 512};        // longest < 512, < 2048, longer
   // Shared memory per batch CTA (KiB), by the same classes: a sequence whose
-  // c, b, t (24 bytes per entry) do not fit runs from the CTA's global
-  // workspace; smaller caps put more CTAs on an SM.
+  // residuals (16 bytes an entry, 8 for p < 2^31) do not fit runs from the
+  // CTA's global workspace; smaller caps put more CTAs on an SM.
   int bm_batch_smem_kib[3] = {200, 200, 200};
   int batch_tc_min = 1 << 30;  // batched rank: sides on the tensor-core kernel (off until measured faster)
 };
+
+// MODLIN_LC_GRID refuses more CTAs than this per SM (it runs on one per SM).
+constexpr int kBmGridMaxPerSm = 8;
 
 static int limb_class(uint64_t p) {
   const int bits = 64 - __builtin_clzll(p - 1);
@@ -101,7 +105,7 @@ struct Ctx {
   PanelState* h_ps = nullptr;
   int2* h_moves = nullptr;
   // linear-complexity workspaces
-  DevBuf seq, bmws, bmout, bmsync, bmjobs, bmnext;
+  DevBuf seq, bmws, bmout, bmjobs, bmnext;
   DevBuf gena, genjobs;  // planted-generator coefficients and jobs
   DevBuf jump;           // jump-ahead scratch of the long planted generator
   DevBuf batchm, rbjobs, rbout;  // batched rank: matrix arena, jobs, ranks
@@ -600,54 +604,41 @@ static int lc_device_locked(Ctx* C, uint64_t p, const uint64_t* d_s, size_t n, c
   }
   int kernel = opts ? opts->kernel : MODLIN_LC_AUTO;
   if (kernel == MODLIN_LC_AUTO)
-    kernel = (int64_t)n < C->tune.bm_cluster_min ? MODLIN_LC_BLOCK
-             : (bm_cluster_size((int64_t)n) ? MODLIN_LC_CLUSTER : MODLIN_LC_GRID);
-  if (kernel == MODLIN_LC_CLUSTER) {
-    const int R = bm_cluster_size((int64_t)n);
-    if (!R) return MODLIN_EINVAL_N;
-    CK(C->bmout.ensure(sizeof(int64_t) * 4));
-    CK(C->bmws.ensure((size_t)2 * n * 8));
-    uint64_t* b0 = C->bmws.as<uint64_t>();
-    CK(launch_bm_cluster(fp, d_s, (int64_t)n, R, b0, b0 + n, C->bmout.as<int64_t>(), st));
+    kernel = (int64_t)n < C->tune.bm_long_min ? MODLIN_LC_BLOCK : MODLIN_LC_GRID;
+  CK(C->bmout.ensure(sizeof(int64_t) * 4));
+  int64_t* d_out = C->bmout.as<int64_t>();
+  if (kernel == MODLIN_LC_BLOCK) {
+    if ((int64_t)n > kBmMaxN) return MODLIN_EINVAL_N;
+    const int64_t smem_words = (200 * 1024) / 8;
+    const int64_t words = bm_smem_words(p, (int64_t)n);
+    if (words > smem_words) CK(C->bmws.ensure((size_t)words * 8));
+    BmJob job{fp.p, fp.mu_lo, fp.mu_hi, fp.safe_batch, d_s, (int64_t)n, 0};
+    CK(launch_bm_block(job, C->bmws.as<uint64_t>(), smem_words, C->tune.bm_threads[bm_len_class(n)], d_out, st));
     g_launches++;
-    CK(cudaMemcpyAsync(C->h_out, C->bmout.p, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(C->h_out, d_out, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     *lc_out = (size_t)C->h_out[0];
     return MODLIN_OK;
   }
-  CK(C->bmout.ensure(sizeof(int64_t) * 4));
-  int64_t* d_out = C->bmout.as<int64_t>();
-  if (kernel == MODLIN_LC_BLOCK) {
-    const int64_t smem_words = (200 * 1024) / 8;
-    if (3 * (int64_t)n > smem_words) CK(C->bmws.ensure((size_t)3 * n * 8));
-    BmJob job{fp.p, fp.mu_lo, fp.mu_hi, fp.safe_batch, d_s, (int64_t)n, 0};
-    CK(launch_bm_block(job, C->bmws.as<uint64_t>(), smem_words, C->tune.bm_threads[bm_len_class(n)], d_out, st));
-    g_launches++;
+  CK(C->bmws.ensure(bm_long_bytes((int64_t)n)));
+  // About one second of waiting at ~2 GHz before a wait is declared stuck.
+  long long spin = 2000000000LL;
+  if (kernel == MODLIN_LC_CLUSTER) {
+    if ((int64_t)n > kBmClusterMaxN) return MODLIN_EINVAL_N;
+    CK(launch_bm_cluster(fp, d_s, (int64_t)n, C->bmws.p, spin, d_out, st));
   } else {
-    int ctas = opts && opts->grid_ctas > 0 ? opts->grid_ctas : C->num_sms;
-    // Each CTA keeps its slice of c in shared memory (<= 200 KiB).
-    const int64_t min_ctas = ((int64_t)n * 8 + 200 * 1024 - 1) / (200 * 1024);
-    if (ctas < min_ctas) ctas = (int)min_ctas;
-    if ((int64_t)ctas > (int64_t)n) ctas = (int)n;
-    CK(C->bmws.ensure((size_t)2 * n * 8));
-    CK(C->bmsync.ensure(grid_sync_bytes()));
-    CK(cudaMemsetAsync(C->bmsync.p, 0, grid_sync_bytes(), st));
-    uint64_t* b0 = C->bmws.as<uint64_t>();
-    int used = 0;
-    // About one second of spinning at ~2 GHz before a wait is declared stuck.
-    long long spin = 2000000000LL;
+    const int ctas = opts && opts->grid_ctas > 0 ? opts->grid_ctas : C->num_sms;
+    if (ctas > kBmGridMaxPerSm * C->num_sms) return MODLIN_ECUDA;
     const int skip_cta = g_fault_skip_cta.exchange(-1);
     if (skip_cta >= 0) spin = g_fault_spin.load();
-    CK(launch_bm_grid(fp, d_s, (int64_t)n, ctas, 256, b0, b0 + n, C->bmsync.p, spin, skip_cta, d_out, st, &used));
-    g_launches += 2;
-    int err = 0;
-    CK(cudaMemcpyAsync(&err, C->bmsync.as<char>() + grid_sync_err_offset(), sizeof(int), cudaMemcpyDeviceToHost,
-                       st));
-    CK(cudaStreamSynchronize(st));
-    if (err) return MODLIN_ETIMEOUT;
+    CK(launch_bm_long(fp, d_s, (int64_t)n, ctas, C->num_sms, C->bmws.p, spin, skip_cta, d_out, st));
   }
+  g_launches += 2;
+  int* err = reinterpret_cast<int*>(C->h_out + 1);
   CK(cudaMemcpyAsync(C->h_out, d_out, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+  CK(cudaMemcpyAsync(err, C->bmws.as<char>() + bm_long_err_offset(), sizeof(int), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  if (*err) return MODLIN_ETIMEOUT;
   *lc_out = (size_t)C->h_out[0];
   return MODLIN_OK;
 }
@@ -727,34 +718,49 @@ static int rank_batch_locked(Ctx* C, const uint64_t* p, uint64_t* const* d_m, co
   return MODLIN_OK;
 }
 
+// Launch shape of a batch of sequences (jobs sorted longest first).
+struct BmBatchShape {
+  int threads, blocks;
+  int64_t smem_words, gws_words;  // per CTA: shared memory, global workspace
+};
+static BmBatchShape bm_batch_shape(const Ctx* C, const std::vector<BmJob>& jobs) {
+  BmBatchShape B{};
+  int64_t maxn = 1, words = 0;
+  for (const BmJob& j : jobs) {
+    maxn = std::max(maxn, j.n);
+    words = std::max(words, bm_smem_words(j.p, j.n));
+  }
+  const int c = bm_batch_class(maxn);
+  B.threads = C->tune.bm_batch_threads[c];
+  B.smem_words = std::min<int64_t>(words, (int64_t)C->tune.bm_batch_smem_kib[c] * 128);
+  B.gws_words = words > B.smem_words ? words : 0;
+  const int per_sm = std::max(1, bm_batch_max_blocks_per_sm(B.threads, B.smem_words));
+  B.blocks = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)C->num_sms * per_sm, (int64_t)jobs.size()));
+  return B;
+}
+
 static int lc_batch_locked(Ctx* C, const uint64_t* p, const uint64_t* const* d_data, const size_t* n,
                            size_t count, size_t* lcs_out, cudaStream_t st) {
   if (count == 0) return MODLIN_OK;
   std::vector<BmJob> jobs(count);
-  int64_t maxn = 0;
   for (size_t i = 0; i < count; ++i) {
     FieldParams fp;
     if (!make_field_params(p[i], &fp)) return MODLIN_EINVAL_P;
+    if ((int64_t)n[i] > kBmMaxN) return MODLIN_EINVAL_N;
     jobs[i] = BmJob{fp.p, fp.mu_lo, fp.mu_hi, fp.safe_batch, d_data[i], (int64_t)n[i], (int64_t)i};
-    maxn = std::max<int64_t>(maxn, (int64_t)n[i]);
   }
   // Longest first: the persistent CTAs then finish close together (LPT).
   std::stable_sort(jobs.begin(), jobs.end(), [](const BmJob& a, const BmJob& b) { return a.n > b.n; });
-  const int threads = C->tune.bm_batch_threads[bm_batch_class(maxn)];
-  int64_t smem_words = std::min<int64_t>(3 * maxn, (int64_t)C->tune.bm_batch_smem_kib[bm_batch_class(maxn)] * 128);
-  int per_sm = bm_batch_max_blocks_per_sm(threads, smem_words);
-  if (per_sm < 1) per_sm = 1;
-  int blocks = C->num_sms * per_sm;
-  if ((size_t)blocks > count) blocks = (int)count;
-  const int64_t gws_words = 3 * maxn > smem_words ? 3 * maxn : 0;
-  if (gws_words) CK(C->bmws.ensure((size_t)blocks * gws_words * 8));
+  const BmBatchShape B = bm_batch_shape(C, jobs);
+  if (B.gws_words) CK(C->bmws.ensure((size_t)B.blocks * B.gws_words * 8));
   CK(C->bmjobs.ensure(sizeof(BmJob) * count));
   CK(C->bmnext.ensure(sizeof(unsigned long long)));
   CK(C->bmout.ensure(sizeof(int64_t) * count));
   CK(cudaMemcpyAsync(C->bmjobs.p, jobs.data(), sizeof(BmJob) * count, cudaMemcpyHostToDevice, st));
   CK(cudaMemsetAsync(C->bmnext.p, 0, sizeof(unsigned long long), st));
   CK(launch_bm_batch(C->bmjobs.as<BmJob>(), (int64_t)count, C->bmnext.as<unsigned long long>(),
-                     C->bmws.as<uint64_t>(), gws_words, smem_words, blocks, threads, C->bmout.as<int64_t>(), st));
+                     C->bmws.as<uint64_t>(), B.gws_words, B.smem_words, B.blocks, B.threads, C->bmout.as<int64_t>(),
+                     st));
   g_launches += 2;
   std::vector<int64_t> out(count);
   CK(cudaMemcpyAsync(out.data(), C->bmout.p, sizeof(int64_t) * count, cudaMemcpyDeviceToHost, st));
@@ -817,7 +823,7 @@ static int autotune_locked(Ctx* C, std::string& rep) {
   int rc = MODLIN_OK;
   cudaStream_t st = C->stream;
   Tune T = C->tune;
-  char buf[256];
+  char buf[384];
   rep = "{";
   // 1. Plain vs tensor-core rank per limb count (uniform matrices).
   const uint64_t primes[4] = {127, 65521, 2147483647ULL, kM61};
@@ -933,10 +939,10 @@ static int autotune_locked(Ctx* C, std::string& rep) {
   FieldParams fp;
   make_field_params(kM61, &fp);
   const int64_t bm_len[4] = {768, 3072, 12288, 32768};
-  const int thr[4] = {128, 256, 512, 1024};
+  const int thr[3] = {128, 256, 512};
   TK(C->seq.ensure((size_t)65536 * 8));
   TK(C->bmout.ensure(sizeof(int64_t) * 4));
-  TK(C->bmws.ensure((size_t)3 * 65536 * 8));
+  TK(C->bmws.ensure(std::max<size_t>((size_t)bm_workspace_words(65536) * 8, bm_long_bytes(65536))));
   uint64_t* seq = C->seq.as<uint64_t>();
   const int64_t smem_words = (200 * 1024) / 8;
   rep += ", \"bm_block_ms\": {";
@@ -962,36 +968,31 @@ static int autotune_locked(Ctx* C, std::string& rep) {
       }
     }
   }
-  rep += "}, \"bm_cluster_ms\": {";
-  {
-    const std::vector<int> csz = {4096, 8192, 16384, 32768, 65536};
-    std::vector<bool> cl_wins;
+  // One CTA against many (AUTO's rule), and against one cluster (reported for
+  // callers that choose the kernel).
+  for (int which = 0; which < 2; ++which) {
+    const std::vector<int> csz = which ? std::vector<int>{4096, 8192, 16384, 32768} : std::vector<int>{512, 1024, 2048, 4096, 8192};
+    std::vector<bool> wins;
+    rep += which ? "}, \"bm_cluster_ms\": {" : "}, \"bm_long_ms\": {";
     for (int n : csz) {
       uint64_t nl = 0;
       TK(gen_uniform_device(kM61, 777 + n, seq, (uint64_t)n, st, &nl));
-      BmJob job{fp.p, fp.mu_lo, fp.mu_hi, fp.safe_batch, seq, n, 0};
-      const int tb = T.bm_threads[bm_len_class(n)];
-      const float tblk = best_ms(C, 1, [&]() -> int {
-        return launch_bm_block(job, C->bmws.as<uint64_t>(), smem_words, tb, C->bmout.as<int64_t>(), st) ==
-                       cudaSuccess
-                   ? MODLIN_OK
-                   : MODLIN_ECUDA;
-      }, &rc);
-      if (rc) return rc;
-      const float tcl = best_ms(C, 1, [&]() -> int {
-        uint64_t* b0 = C->bmws.as<uint64_t>();
-        const cudaError_t e = launch_bm_cluster(fp, seq, n, bm_cluster_size(n), b0, b0 + n, C->bmout.as<int64_t>(), st);
-        if (e != cudaSuccess) rep += std::string("\"error\": \"bm cluster n=") + std::to_string(n) + ": " +
-                                     cudaGetErrorName(e) + "\", ";
-        return e == cudaSuccess ? MODLIN_OK : MODLIN_ECUDA;
-      }, &rc);
-      if (rc) return rc;
-      cl_wins.push_back(tcl <= tblk);
-      std::snprintf(buf, sizeof buf, "%s\"n=%d\": [%.3f, %.3f]", n == csz[0] ? "" : ", ", n, finite_ms(tblk),
-                    finite_ms(tcl));
+      size_t lc = 0;
+      float t[2];
+      for (int k = 0; k < 2; ++k) {
+        const modlin_lc_opts o{k == 0 ? MODLIN_LC_BLOCK : which ? MODLIN_LC_CLUSTER : MODLIN_LC_GRID, 0, 0};
+        const int saved = C->tune.bm_threads[bm_len_class(n)];
+        C->tune.bm_threads[bm_len_class(n)] = T.bm_threads[bm_len_class(n)];
+        t[k] = best_ms(C, 2, [&]() -> int { return lc_device_locked(C, kM61, seq, n, &o, &lc, st); }, &rc);
+        C->tune.bm_threads[bm_len_class(n)] = saved;
+        if (rc) return rc;
+      }
+      wins.push_back(t[1] <= t[0]);
+      std::snprintf(buf, sizeof buf, "%s\"n=%d\": [%.3f, %.3f]", n == csz[0] ? "" : ", ", n, finite_ms(t[0]),
+                    finite_ms(t[1]));
       rep += buf;
     }
-    T.bm_cluster_min = crossover(csz, cl_wins, 1 << 30);
+    (which ? T.bm_cluster_min : T.bm_long_min) = crossover(csz, wins, 1 << 30);
   }
   rep += "}";
   // 5. BM batches: threads per CTA and the shared-memory cap per CTA by the
@@ -1019,7 +1020,7 @@ static int autotune_locked(Ctx* C, std::string& rep) {
       float best = 1e30f;
       const int saved = C->tune.bm_batch_threads[c], saved_kib = C->tune.bm_batch_smem_kib[c];
       for (int kib : {200, 96, 48, 24}) {
-        if (kib < 200 && (int64_t)kib * 1024 >= 24 * hi[c]) continue;  // the same as a larger cap
+        if (kib < 200 && (int64_t)kib * 1024 >= 8 * bm_smem_words(kM61, hi[c])) continue;  // the same as a larger cap
         for (int t : bthr) {
           C->tune.bm_batch_threads[c] = t;
           C->tune.bm_batch_smem_kib[c] = kib;
@@ -1050,10 +1051,10 @@ static int autotune_locked(Ctx* C, std::string& rep) {
   C->tune = T;
   std::snprintf(buf, sizeof buf,
                 ", \"choice\": {\"tc_crossover\": [%d, %d, %d, %d], \"two_panel_min\": %d, "
-                "\"batch_tc_min\": %d, \"bm_threads\": [%d, %d, %d, %d], \"bm_cluster_min\": %d, "
+                "\"batch_tc_min\": %d, \"bm_threads\": [%d, %d, %d, %d], \"bm_long_min\": %d, \"bm_cluster_min\": %d, "
                 "\"bm_batch_threads\": [%d, %d, %d], \"bm_batch_smem_kib\": [%d, %d, %d]}}",
                 T.tc_cross[0], T.tc_cross[1], T.tc_cross[2], T.tc_cross[3], T.two_panel_min, T.batch_tc_min,
-                T.bm_threads[0], T.bm_threads[1], T.bm_threads[2], T.bm_threads[3], T.bm_cluster_min,
+                T.bm_threads[0], T.bm_threads[1], T.bm_threads[2], T.bm_threads[3], T.bm_long_min, T.bm_cluster_min,
                 T.bm_batch_threads[0], T.bm_batch_threads[1], T.bm_batch_threads[2], T.bm_batch_smem_kib[0],
                 T.bm_batch_smem_kib[1], T.bm_batch_smem_kib[2]);
   rep += buf;
@@ -1844,25 +1845,23 @@ int modlin_lc_batch_plan_new(const uint64_t* p, const uint64_t* const* d_s, cons
   int rc = get_ctx(&C);
   if (rc) return rc;
   std::vector<BmJob> jobs;
-  int64_t maxn = 1;
   for (size_t i = 0; i < count; ++i) {
     FieldParams fp;
     if (!make_field_params(p[i], &fp)) return MODLIN_EINVAL_P;
     if (n[i] && !d_s[i]) return MODLIN_EINVAL_ARG;
     if (n[i] > (size_t)1 << 30) return MODLIN_EINVAL_N;
     jobs.push_back(BmJob{fp.p, fp.mu_lo, fp.mu_hi, fp.safe_batch, d_s[i], (int64_t)n[i], (int64_t)i});
-    maxn = std::max<int64_t>(maxn, (int64_t)n[i]);
   }
   std::stable_sort(jobs.begin(), jobs.end(), [](const BmJob& a, const BmJob& b) { return a.n > b.n; });
   std::unique_ptr<modlin_lc_batch_plan> P(new modlin_lc_batch_plan());
   P->device = C->device;
   P->count = (int64_t)count;
   P->out = d_lcs_out;
-  P->threads = C->tune.bm_batch_threads[bm_batch_class(maxn)];
-  P->smem_words = std::min<int64_t>(3 * maxn, (int64_t)C->tune.bm_batch_smem_kib[bm_batch_class(maxn)] * 128);
-  const int per_sm = std::max(1, bm_batch_max_blocks_per_sm(P->threads, P->smem_words));
-  P->blocks = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)C->num_sms * per_sm, (int64_t)count));
-  P->gws_words = 3 * maxn > P->smem_words ? 3 * maxn : 0;
+  const BmBatchShape B = bm_batch_shape(C, jobs);
+  P->threads = B.threads;
+  P->blocks = B.blocks;
+  P->smem_words = B.smem_words;
+  P->gws_words = B.gws_words;
   CK(P->jobs.ensure(std::max<size_t>(jobs.size(), 1) * sizeof(BmJob)));
   CK(P->next.ensure(sizeof(unsigned long long)));
   if (P->gws_words) CK(P->gws.ensure((size_t)P->blocks * P->gws_words * 8));
