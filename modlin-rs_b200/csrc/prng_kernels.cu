@@ -23,9 +23,10 @@
 // canonical jump-ahead start may then differ from ROOT's state in
 // representation; the host reruns it from the flagged segment's exact end.
 //
-// xoroshiro128++ (src/prng.rs:48-83): the state transition is linear over
-// GF(2) (the host computes the jump-ahead states); one thread per segment,
-// outputs staged 32 per thread in shared memory and written row by row.
+// xoroshiro128++ (src/prng.rs:48-83): the state transition T is linear over
+// GF(2), and the matrices T^(2^k) are kept on the device; one thread per
+// segment of 2^m outputs, each block of threads jumps to its segments itself,
+// and outputs are staged 16 per thread in shared memory and written in rows.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -343,44 +344,118 @@ cudaError_t mix_dispatch(const MixFill& a, uint64_t p, const FieldParams& fp, cu
 }
 
 // ---- xoroshiro128++ ----------------------------------------------------------------
-constexpr int kXoroWarps = 4;
+constexpr int kXoroThreads = 128;
+constexpr int kXoroRow = 16;              // outputs staged per thread: 128-byte rows
+constexpr int kXoroStride = kXoroRow + 2;  // 16-byte aligned rows, conflict-free 16-byte accesses
 
 __device__ __forceinline__ uint64_t rotl64(uint64_t x, int k) { return (x << k) | (x >> (64 - k)); }
 
+// acc ^= column j of a GF(2) matrix for every set bit j of the 32-bit word w.
+__device__ __forceinline__ void gf2_word(uint4& acc, uint32_t w, const uint4* col) {
+#pragma unroll 8
+  for (int j = 0; j < 32; ++j) {
+    const uint32_t m = 0u - ((w >> j) & 1u);
+    const uint4 c = col[j];
+    acc.x ^= c.x & m;
+    acc.y ^= c.y & m;
+    acc.z ^= c.z & m;
+    acc.w ^= c.w & m;
+  }
+}
+
+// Thread t runs segment t. Its state is T^(2^m t) times the starting state:
+// warp 0 applies the matrices of the bits of the block's first segment (a
+// lane holds 4 of the 128 columns), then 7 doublings fill the block's 128
+// states (about 4 % of the work of 2^11-output segments). The fill itself is
+// bound by instruction issue, about 30 an output: 2^28 outputs mod 2^61 - 1
+// take 490 us (the segments' states came from the host before: 19400).
 template <class R>
-__global__ void __launch_bounds__(kXoroWarps * 32) xoro_fill_kernel(XoroFill a, R red) {
-  __shared__ uint64_t sh[kXoroWarps][32][33];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, t0 = t - lane;
+__global__ void __launch_bounds__(kXoroThreads) xoro_fill_kernel(XoroFill a, R red) {
+  __shared__ __align__(16) uint64_t sh[kXoroThreads / 32][32 * kXoroStride];
+  __shared__ uint4 mat[128];
+  __shared__ uint4 state[kXoroThreads];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int64_t first = (int64_t)blockIdx.x * kXoroThreads, t = first + tid, t0 = t - lane;
+  const uint4* mats = reinterpret_cast<const uint4*>(a.mats);  // T^(2^k) at 128 k, by columns
+  if (w == 0) {
+    uint4 v = make_uint4((uint32_t)a.s0, (uint32_t)(a.s0 >> 32), (uint32_t)a.s1, (uint32_t)(a.s1 >> 32));
+    for (int k = 7; first >> k; ++k) {
+      if (!((first >> k) & 1)) continue;
+      const uint4* col = mats + 128 * (a.m + k) + 4 * lane;
+      const uint32_t word = lane < 8 ? v.x : lane < 16 ? v.y : lane < 24 ? v.z : v.w;
+      uint4 acc = make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t mk = 0u - ((word >> (4 * (lane & 7) + j)) & 1u);
+        const uint4 c = col[j];
+        acc.x ^= c.x & mk;
+        acc.y ^= c.y & mk;
+        acc.z ^= c.z & mk;
+        acc.w ^= c.w & mk;
+      }
+      v = make_uint4(__reduce_xor_sync(kFull, acc.x), __reduce_xor_sync(kFull, acc.y),
+                     __reduce_xor_sync(kFull, acc.z), __reduce_xor_sync(kFull, acc.w));
+    }
+    if (lane == 0) state[0] = v;
+  }
+  const int64_t segs = a.S - first;  // of this block (at least one)
+  for (int have = 1, k = 0; have < kXoroThreads && have < segs; have *= 2, ++k) {
+    __syncthreads();
+    mat[tid] = mats[128 * (a.m + k) + tid];
+    __syncthreads();
+    if (tid < have) {
+      const uint4 v = state[tid];
+      uint4 acc = make_uint4(0, 0, 0, 0);
+      gf2_word(acc, v.x, mat);
+      gf2_word(acc, v.y, mat + 32);
+      gf2_word(acc, v.z, mat + 64);
+      gf2_word(acc, v.w, mat + 96);
+      state[have + tid] = acc;
+    }
+  }
+  __syncthreads();
   if (t0 >= a.S) return;
   const bool act = t < a.S;
-  uint64_t s0 = 0, s1 = 0;
-  if (act) {
-    s0 = a.starts[2 * t];
-    s1 = a.starts[2 * t + 1];
-  }
-  const int64_t beg = t * a.L, cnt = act ? ((a.count - beg) < a.L ? (a.count - beg) : a.L) : 0;
-  const int64_t nch = (a.L + 31) / 32;
-  for (int64_t c = 0; c < nch; ++c) {
-#pragma unroll 4
-    for (int i = 0; i < 32; ++i) {
-      if (c * 32 + i < cnt) {  // src/prng.rs:75-83
-        const uint64_t r = rotl64(s0 + s1, 17) + s0;
-        const uint64_t b = s1 ^ s0;
-        s0 = rotl64(s0, 49) ^ b ^ (b << 21);
-        s1 = rotl64(b, 28);
-        sh[w][lane][i] = red(r);
+  const uint4 v = state[tid];  // of a segment past the last: unused
+  uint64_t s0 = (uint64_t)v.y << 32 | v.x, s1 = (uint64_t)v.w << 32 | v.z;
+  const int64_t L = (int64_t)1 << a.m;
+  const int64_t beg = t << a.m, cnt = act ? ((a.count - beg) < L ? (a.count - beg) : L) : 0;
+  uint64_t* row = sh[w] + lane * kXoroStride;
+  const auto next = [&]() {  // src/prng.rs:75-83
+    const uint64_t r = rotl64(s0 + s1, 17) + s0;
+    const uint64_t b = s1 ^ s0;
+    s0 = rotl64(s0, 49) ^ b ^ (b << 21);
+    s1 = rotl64(b, 28);
+    return red(r);
+  };
+  // The warp's rows are all full when its last segment is.
+  const bool full = t0 + 31 < a.S && ((t0 + 32) << a.m) <= a.count && ((uintptr_t)a.out & 15) == 0;
+  for (int64_t c = 0; c < L; c += kXoroRow) {
+    if (full) {
+#pragma unroll
+      for (int i = 0; i < kXoroRow; i += 2) {
+        const uint64_t r0 = next(), r1 = next();
+        *reinterpret_cast<ulonglong2*>(row + i) = make_ulonglong2(r0, r1);
       }
+      __syncwarp();
+      // 8 lanes write a row's 128 bytes.
+      uint64_t* dst = a.out + ((t0 + (lane >> 3)) << a.m) + c + 2 * (lane & 7);
+      const uint64_t* src = sh[w] + (lane >> 3) * kXoroStride + 2 * (lane & 7);
+#pragma unroll
+      for (int r = 0; r < 32; r += 4)
+        *reinterpret_cast<ulonglong2*>(dst + ((int64_t)r << a.m)) =
+            *reinterpret_cast<const ulonglong2*>(src + r * kXoroStride);
+      __syncwarp();
+    } else {
+      for (int i = 0; i < kXoroRow; ++i)
+        if (c + i < cnt) row[i] = next();
+      __syncwarp();
+      for (int r = lane >> 4; r < 32; r += 2) {
+        const int64_t rb = ((t0 + r) << a.m) + c + (lane & 15);
+        if (t0 + r < a.S && rb < a.count) a.out[rb] = sh[w][r * kXoroStride + (lane & 15)];
+      }
+      __syncwarp();
     }
-    __syncwarp();
-    for (int r = 0; r < 32; ++r) {
-      const int64_t tr = t0 + r;
-      if (tr >= a.S) break;
-      const int64_t rb = tr * a.L, rc = (a.count - rb) < a.L ? (a.count - rb) : a.L;
-      const int64_t off = c * 32 + lane;
-      if (off < rc) a.out[rb + off] = sh[w][r][lane];
-    }
-    __syncwarp();
   }
   if (t == a.S - 1) {
     a.ends[0] = s0;
@@ -391,8 +466,7 @@ __global__ void __launch_bounds__(kXoroWarps * 32) xoro_fill_kernel(XoroFill a, 
 template <class R>
 cudaError_t launch_xoro(const XoroFill& a, R red, cudaStream_t st) {
   if (a.S <= 0) return cudaSuccess;
-  const int64_t threads = kXoroWarps * 32;
-  xoro_fill_kernel<R><<<(unsigned)((a.S + threads - 1) / threads), (unsigned)threads, 0, st>>>(a, red);
+  xoro_fill_kernel<R><<<(unsigned)((a.S + kXoroThreads - 1) / kXoroThreads), kXoroThreads, 0, st>>>(a, red);
   return cudaGetLastError();
 }
 
@@ -671,54 +745,51 @@ void gf2_mul(const M128& A, const M128& B, M128* C) {  // C = A B
   for (int j = 0; j < 128; ++j) C->col[j] = gf2_apply(A, B.col[j]);
 }
 
-int xoro_fill_host(PrngCache& c, int num_sms, modlin_prng_impl::Xoroshiro& x, uint64_t p, const FieldParams& fp,
-                   uint64_t* d_out, uint64_t count, cudaStream_t st, uint64_t* launches) {
-  int64_t S = std::min<int64_t>(((int64_t)count + 63) / 64, (int64_t)num_sms * 256);
-  if (S < 1) S = 1;
-  const int64_t L = ((int64_t)count + S - 1) / S;
-  S = ((int64_t)count + L - 1) / L;
-  // T: one step; J = T^L.
-  M128 T, J, P, tmp;
+// The matrices T^(2^k), k < kXoroPows, on the device (built once per device).
+constexpr int kXoroPows = 48;
+
+int ensure_xoro_pows(PrngCache& c, cudaStream_t st) {
+  if (c.xoro) return MODLIN_OK;
+  std::vector<M128> P(kXoroPows);
   for (int j = 0; j < 128; ++j) {
     modlin_prng_impl::Xoroshiro u;
     u.s0 = j < 64 ? 1ULL << j : 0;
     u.s1 = j < 64 ? 0 : 1ULL << (j - 64);
     u.step();
-    T.col[j] = V128{u.s0, u.s1};
+    P[0].col[j] = V128{u.s0, u.s1};
   }
-  P = T;
-  bool have = false;
-  for (int64_t e = L; e; e >>= 1) {
-    if (e & 1) {
-      if (!have) {
-        J = P;
-        have = true;
-      } else {
-        gf2_mul(J, P, &tmp);
-        J = tmp;
-      }
-    }
-    if (e > 1) {
-      gf2_mul(P, P, &tmp);
-      P = tmp;
-    }
+  for (int k = 1; k < kXoroPows; ++k) gf2_mul(P[k - 1], P[k - 1], &P[k]);
+  uint64_t* d = nullptr;
+  PCK(cudaMalloc(&d, kXoroPows * sizeof(M128)));
+  cudaError_t e = cudaMemcpyAsync(d, P.data(), kXoroPows * sizeof(M128), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) {
+    cudaFree(d);
+    cudaGetLastError();
+    return MODLIN_ECUDA;
   }
-  std::vector<uint64_t> starts(2 * S);
-  V128 v{x.s0, x.s1};
-  for (int64_t t = 0; t < S; ++t) {
-    starts[2 * t] = v.lo;
-    starts[2 * t + 1] = v.hi;
-    if (t + 1 < S) v = gf2_apply(J, v);
-  }
-  const int rc = ensure_ws(c, (2 * S + 2) * sizeof(uint64_t));
+  c.xoro = d;
+  return MODLIN_OK;
+}
+
+int xoro_fill_host(PrngCache& c, int num_sms, modlin_prng_impl::Xoroshiro& x, uint64_t p, const FieldParams& fp,
+                   uint64_t* d_out, uint64_t count, cudaStream_t st, uint64_t* launches) {
+  // Segments of a power of two of outputs (their jumps are single cached
+  // matrices): the longest that leave 512 threads an SM, at least 64.
+  int m = 6;
+  while (m < 30 && ((int64_t)count >> (m + 1)) >= (int64_t)num_sms * 512) ++m;
+  const int64_t S = ((int64_t)count + ((int64_t)1 << m) - 1) >> m;
+  if (m + 1 + (64 - __builtin_clzll((uint64_t)S)) > kXoroPows) return MODLIN_EINVAL_N;  // 2^47 outputs
+  int rc = ensure_xoro_pows(c, st);
   if (rc) return rc;
-  uint64_t* ws = static_cast<uint64_t*>(c.ws);
-  PCK(cudaMemcpyAsync(ws, starts.data(), 2 * S * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-  XoroFill a{ws, ws + 2 * S, d_out, (int64_t)count, L, S};
+  rc = ensure_ws(c, 2 * sizeof(uint64_t));
+  if (rc) return rc;
+  uint64_t* ends = static_cast<uint64_t*>(c.ws);
+  const XoroFill a{c.xoro, ends, d_out, (int64_t)count, S, x.s0, x.s1, m};
   PCK(xoro_fill(a, p, fp, st));
   ++*launches;
   uint64_t e[2];
-  PCK(cudaMemcpyAsync(e, ws + 2 * S, sizeof(e), cudaMemcpyDeviceToHost, st));
+  PCK(cudaMemcpyAsync(e, ends, sizeof(e), cudaMemcpyDeviceToHost, st));
   PCK(cudaStreamSynchronize(st));
   x.s0 = e[0];
   x.s1 = e[1];

@@ -37,13 +37,16 @@ cudaError_t mixmax_fill(const MixFill& a, uint64_t p, const FieldParams& fp, cud
 // Warps of one launch that run at once on this device (segments per wave).
 int mixmax_resident_warps(int N, int num_sms);
 
-// xoroshiro128++: thread t of S produces outputs [t*L, min((t+1)*L, count))
-// from starts[2t], starts[2t+1] = (s0, s1); ends[0..2) = state after `count`.
+// xoroshiro128++: thread t of S produces outputs [t 2^m, min((t + 1) 2^m,
+// count)) from T^(t 2^m) (s0, s1), T the state transition; ends[0..2) = state
+// after `count`.
 struct XoroFill {
-  const uint64_t* starts;
+  const uint64_t* mats;  // T^(2^k), 128 columns of 2 words each, k ascending
   uint64_t* ends;
   uint64_t* out;
-  int64_t count, L, S;
+  int64_t count, S;
+  uint64_t s0, s1;
+  int m;
 };
 cudaError_t xoro_fill(const XoroFill& a, uint64_t p, const FieldParams& fp, cudaStream_t st);
 
@@ -53,6 +56,7 @@ cudaError_t xoro_fill(const XoroFill& a, uint64_t p, const FieldParams& fp, cuda
 struct PrngCache {
   uint64_t* pow[3] = {nullptr, nullptr, nullptr};  // MIXMAX-17, -240, -256: kPowMax matrices N x N
   int have[3] = {0, 0, 0};
+  uint64_t* xoro = nullptr;  // xoroshiro128++'s T^(2^k)
   void* ws = nullptr;
   size_t ws_bytes = 0;
 };
