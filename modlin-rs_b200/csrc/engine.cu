@@ -220,8 +220,8 @@ static int rank_impl(const RankRun& R, size_t* rank_out) {
     CK(C->tcA.ensure(tc_a_bytes(n)));
     CK(C->tcB.ensure(tc_b_bytes(n)));
   }
-  CK(C->tcerr.ensure(2 * sizeof(int)));
-  CK(cudaMemsetAsync(C->tcerr.p, 0, 2 * sizeof(int), st));
+  CK(C->tcerr.ensure(4 * sizeof(int)));
+  CK(cudaMemsetAsync(C->tcerr.p, 0, 4 * sizeof(int), st));
   uint64_t* Lbuf = C->lbuf.as<uint64_t>();
   uint64_t* Ubuf = C->ubuf.as<uint64_t>();
   uint64_t* Upanel = C->upanel.as<uint64_t>();
@@ -474,6 +474,7 @@ static int rank_impl(const RankRun& R, size_t* rank_out) {
 
   int rank = 0, col = 0;
   bool general_next = false;  // the panel at col had a singular block
+  int empty_left = 1, empty_gap = 1;  // panels without a pivot until the rest is looked at
   while (col < n && rank < n) {
     if (!general_next && width(rank, col) > 0) {
       if (int rc = run_pipeline(rank, col, general_next)) return rc;
@@ -546,6 +547,17 @@ static int rank_impl(const RankRun& R, size_t* rank_out) {
     }
     rank += pb;
     col = jend;
+    if (pb == 0 && rank < n && col < n && --empty_left == 0) {
+      // A panel without a pivot: when all that is left is zero, so are all
+      // later panels. Looked at after 1, 2, 4, ... such panels.
+      int* h_nz = reinterpret_cast<int*>(C->h_out);
+      CK(launch_any_nonzero(R.m, ld, rank, col, n, C->tcerr.as<int>() + 2, C->num_sms, st));
+      g_launches += 2;
+      CK(cudaMemcpyAsync(h_nz, C->tcerr.as<int>() + 2, sizeof(int), cudaMemcpyDeviceToHost, st));
+      CK(cudaStreamSynchronize(st));
+      if (!*h_nz) col = n;
+      empty_left = empty_gap *= 2;
+    }
     if (R.cb) R.cb(R.cb_ctx, (size_t)col, (size_t)n);
   }
   CK(cudaStreamSynchronize(st));
@@ -575,7 +587,9 @@ static int rank_device_locked(Ctx* C, uint64_t p, uint64_t* d_m, size_t n, const
   std::vector<int> pc;
   RankRun R{&fp, d_m, (int)n, opts ? opts->kernel : MODLIN_RANK_AUTO, st, C, pivot_cols_out ? &pc : nullptr,
             cb, cb_ctx, C->tune.two_panel_min};
-  const int rc = p == kM61 ? rank_impl<FpM61>(R, rank_out) : rank_impl<FpBarrett>(R, rank_out);
+  const int rc = p == kM61              ? rank_impl<FpM61>(R, rank_out)
+                 : p < (1ULL << 32) ? rank_impl<FpSmall>(R, rank_out)
+                                    : rank_impl<FpBarrett>(R, rank_out);
   if (rc != MODLIN_OK) return rc;
   if (pivot_cols_out) {
     std::sort(pc.begin(), pc.end());
@@ -1179,6 +1193,9 @@ int modlin_trailing_update_device(uint64_t p, uint64_t* d_C, size_t ldc, size_t 
     if (p == kM61)
       launch_trailing_plain<FpM61>(FpM61(fp), d_C, (int64_t)ldc, 0, (int)M, 0, (int)N, d_L, 0, d_U, (int64_t)ldu,
                                    (int)K, C->tcerr.as<int>(), st);
+    else if (p < (1ULL << 32))
+      launch_trailing_plain<FpSmall>(FpSmall(fp), d_C, (int64_t)ldc, 0, (int)M, 0, (int)N, d_L, 0, d_U, (int64_t)ldu,
+                                     (int)K, C->tcerr.as<int>(), st);
     else
       launch_trailing_plain<FpBarrett>(FpBarrett(fp), d_C, (int64_t)ldc, 0, (int)M, 0, (int)N, d_L, 0, d_U,
                                        (int64_t)ldu, (int)K, C->tcerr.as<int>(), st);
@@ -1589,6 +1606,8 @@ int modlin_panel_pivots_device(uint64_t p, const uint64_t* d_panel, size_t ld, s
   std::lock_guard<std::mutex> g(C->mu);
   cudaStream_t st = user_stream(stream);
   if (p == kM61) return panel_pivots_locked(C, FpM61(fp), d_panel, ld, rows, W, prow_out, pcol_out, pb_out, st);
+  if (p < (1ULL << 32))
+    return panel_pivots_locked(C, FpSmall(fp), d_panel, ld, rows, W, prow_out, pcol_out, pb_out, st);
   return panel_pivots_locked(C, FpBarrett(fp), d_panel, ld, rows, W, prow_out, pcol_out, pb_out, st);
 }
 
@@ -1605,6 +1624,8 @@ int modlin_block_inverse_device(uint64_t p, const uint64_t* d_P, size_t ldp, uin
   CK(C->invst.ensure(sizeof(int)));
   if (p == kM61)
     launch_block_inverse<FpM61>(FpM61(fp), d_P, (int64_t)ldp, 0, 0, d_out, C->invst.as<int>(), st, true);
+  else if (p < (1ULL << 32))
+    launch_block_inverse<FpSmall>(FpSmall(fp), d_P, (int64_t)ldp, 0, 0, d_out, C->invst.as<int>(), st, true);
   else
     launch_block_inverse<FpBarrett>(FpBarrett(fp), d_P, (int64_t)ldp, 0, 0, d_out, C->invst.as<int>(), st, true);
   g_launches++;

@@ -89,8 +89,9 @@ struct FpSmall {
   FpBarrett wide;  // reduction of u128 accumulators
   FpSmall() = default;
   MODLIN_HD explicit FpSmall(const FieldParams& f) : wide(f) {}
-  MODLIN_HD uint64_t reduce(u128 t) const { return wide.reduce(t); }
-  MODLIN_HD uint64_t reduce2(u128 t) const { return wide.reduce(t); }
+  // Sums of products of small residues seldom leave 64 bits.
+  MODLIN_HD uint64_t reduce(u128 t) const { return (uint64_t)(t >> 64) ? wide.reduce(t) : reduce64((uint64_t)t); }
+  MODLIN_HD uint64_t reduce2(u128 t) const { return reduce(t); }
   MODLIN_HD uint64_t reduce64(uint64_t x) const {
     const uint64_t q = (uint64_t)(((u128)x * wide.mu_hi) >> 64);
     uint64_t r = x - q * wide.p;

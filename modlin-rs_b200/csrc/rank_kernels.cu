@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(128) couple_kernel(F f, const uint64_t* __rest
     uint64_t tot = 0, cnt = 0;
 #pragma unroll 8
     for (int k2 = 0; k2 < k; ++k2) {
-      acc += (u128)Gs[k][k2] * Us[k2][t];
+      acc += f.prod(Gs[k][k2], Us[k2][t]);
       if (++cnt == sb) {
         tot = f.add(tot, f.reduce(acc));
         acc = 0;
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(256) trailing_plain_kernel(F f, uint64_t* __re
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int q = 0; q < 4; ++q) acc[i][q] += (u128)a[i] * b[q];
+      for (int q = 0; q < 4; ++q) acc[i][q] += f.prod(a[i], b[q]);
     if (++cnt == sb) {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
@@ -815,6 +815,32 @@ __global__ void zero_kernel(uint64_t* __restrict__ p, int64_t n, Guard g) {
 }
 
 // ---------------------------------------------------------------------------
+// any_nonzero_kernel — *flag = 1 when some entry of rows [r0, n), columns
+// [c0, n) is nonzero: a zero rest ends the rank (a matrix of recurrence rows is
+// zero after its order's pivots). A warp per 256 columns of a row; DRAM-bound,
+// and over at once when an entry is found.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) any_nonzero_kernel(const uint64_t* __restrict__ m, int64_t ld, int32_t r0,
+                                                          int32_t c0, int32_t n, int* flag) {
+  const int lane = threadIdx.x & 31;
+  const int64_t per_row = (n - c0 + 255) / 256, items = per_row * (n - r0);
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t q = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); q < items; q += warps) {
+    if (*(volatile int*)flag) return;
+    const uint64_t* row = m + (r0 + q / per_row) * ld;
+    const int64_t c = c0 + (q % per_row) * 256 + lane;
+    uint64_t v = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (c + 32 * k < n) v |= row[c + 32 * k];
+    if (__any_sync(0xffffffffu, v != 0)) {
+      if (lane == 0) atomicExch(flag, 1);
+      return;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Launch wrappers (explicit instantiation for both field policies).
 // ---------------------------------------------------------------------------
 template <class F>
@@ -892,7 +918,7 @@ void launch_block_inverse(const F& f, const uint64_t* m, int64_t ld, int r0, int
     cudaFuncSetAttribute(block_inverse_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     attr_set = true;
   }
-  const int rec = f.modulus() > (1ULL << 20);
+  const int rec = f.modulus() > (1ULL << 12);
   launch_k(block_inverse_kernel<F>, dim3(1), dim3(kInvThreads), smem, st, 1, f, m, ld, (int32_t)r0, (int32_t)col,
            Vneg, status, rec, reset_status ? 1 : 0, g);
 }
@@ -920,6 +946,14 @@ void launch_zero(uint64_t* p, int64_t n, cudaStream_t st, const Guard& g) {
   launch_k(zero_kernel, dim3((unsigned)blocks), dim3(256), 0, st, 1, p, n, g);
 }
 
+cudaError_t launch_any_nonzero(const uint64_t* m, int64_t ld, int r0, int c0, int n, int* flag, int num_sms,
+                               cudaStream_t st) {
+  const cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), st);
+  if (e != cudaSuccess) return e;
+  any_nonzero_kernel<<<num_sms * 8, 256, 0, st>>>(m, ld, r0, c0, n, flag);
+  return cudaGetLastError();
+}
+
 #define INSTANTIATE(F)                                                                                          \
   template void launch_small_gemm64<F>(const F&, const uint64_t*, int64_t, const uint64_t*, int64_t,            \
                                        const uint64_t*, int64_t, uint64_t*, int64_t, bool, cudaStream_t,        \
@@ -939,6 +973,7 @@ void launch_zero(uint64_t* p, int64_t n, cudaStream_t st, const Guard& g) {
   template int plain_blocks_per_sm<F>();
 
 INSTANTIATE(FpBarrett)
+INSTANTIATE(FpSmall)
 INSTANTIATE(FpM61)
 
 }  // namespace modlin

@@ -175,6 +175,24 @@ __device__ __forceinline__ uint64_t finish(const F& f, u128 lo, u128 hi, uint64_
   }
 }
 
+// p < 2^32: sum_d 2^(8d) a[d][c] mod p. The diagonals are below 2^26 (K <=
+// 128), so up to three of them (LIMBS <= 2) sum to less than 2^43; the seven of
+// LIMBS = 4 are split at 2^32 (r32 = 2^32 mod p).
+template <int LIMBS, int DIAG>
+__device__ __forceinline__ uint64_t finish_small(const FpSmall& f, const uint32_t (&a)[DIAG][4], int c, uint64_t r32) {
+  uint64_t lo = a[0][c];
+#pragma unroll
+  for (int d = 1; d < (DIAG < 4 ? DIAG : 4); ++d) lo += (uint64_t)a[d][c] << (8 * d);
+  if constexpr (DIAG <= 4) {
+    return f.reduce64(lo);
+  } else {
+    uint64_t hi = a[4][c];
+#pragma unroll
+    for (int d = 5; d < DIAG; ++d) hi += (uint64_t)a[d][c] << (8 * (d - 4));
+    return f.add(f.reduce64(lo), f.reduce64(f.reduce64(hi) * r32));
+  }
+}
+
 __device__ __forceinline__ uint64_t mad_wide_u32(uint32_t a, uint32_t b, uint64_t c) {
   uint64_t d;
   asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
@@ -706,38 +724,34 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     } else {
       // Fewer limbs (p < 2^32): NS >= 32 columns per subtile; direct access.
+      // All diagonals of a 4-column group are loaded from TMEM at once, and C
+      // of the next group is loaded while this one is reduced.
       int mt = (int)(g0 / S.nsub), sb = (int)(g0 - (int64_t)mt * S.nsub);
       for (int64_t g = g0; g < g1 && ok; ++g, ++it, sb = sb + 1 == S.nsub ? (++mt, 0) : sb + 1) {
         const int64_t r = (int64_t)rbeg + (int64_t)mt * 128 + row;
         const bool row_ok = r < rend;
         const int ab = it & 1;
         const uint32_t lane_addr = lane_base + ab * 256;
+        const int64_t cb = (int64_t)jend + (int64_t)sb * NS + qc * 4;
+        uint64_t* crow = m + r * ld + cb;
+        uint64_t cv[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) cv[c] = (row_ok && cb + c < cend) ? crow[c] : 0;
         ok = __all_sync(0xffffffffu, mbar_wait(acc_full + ab, (it >> 1) & 1, err));
         if (!ok) break;
         fence_after();
+#pragma unroll
         for (int q = 0; q < NS / 16; ++q) {
-          const int64_t c0 = (int64_t)jend + (int64_t)sb * NS + q * 16 + qc * 4;
-          uint64_t* crow = m + r * ld + c0;
-          uint64_t cv[4];
+          uint32_t a[SH::DIAG][4];
 #pragma unroll
-          for (int c = 0; c < 4; ++c) cv[c] = (row_ok && c0 + c < cend) ? crow[c] : 0;
-          u128 lo[4], hi[4];
+          for (int d = 0; d < SH::DIAG; ++d) tmem_ld4(lane_addr + d * NS + q * 16, a[d]);
+          uint64_t nv[4];
+          if (q + 1 < NS / 16) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) lo[c] = hi[c] = 0;
-#pragma unroll 1
-          for (int d = 0; d < SH::DIAG; ++d) {
-            uint32_t a[4];
-            tmem_ld4(lane_addr + d * NS + q * 16, a);
-            tmem_wait_ld();
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              asm volatile("" : "+r"(a[c]));
-              if (d < 8)
-                lo[c] += (u128)a[c] << (8 * d);
-              else
-                hi[c] += (u128)a[c] << (8 * (d - 8));
-            }
+            for (int c = 0; c < 4; ++c)
+              nv[c] = (row_ok && cb + 16 * (q + 1) + c < cend) ? crow[16 * (q + 1) + c] : 0;
           }
+          tmem_wait_ld();
           if (q == NS / 16 - 1) {
             fence_before();
             __syncwarp();
@@ -746,8 +760,10 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (row_ok) {
 #pragma unroll
             for (int c = 0; c < 4; ++c)
-              if (c0 + c < cend) crow[c] = f.sub(cv[c], finish(f, lo[c], hi[c], r64));
+              if (cb + 16 * q + c < cend) crow[16 * q + c] = f.sub(cv[c], finish_small<LIMBS>(f, a, c, r64));
           }
+#pragma unroll
+          for (int c = 0; c < 4; ++c) cv[c] = nv[c];
         }
       }
     }
@@ -1238,11 +1254,28 @@ cudaError_t tc_update(const FieldParams& fp, uint64_t* m, int64_t ld, int rbeg, 
       tc::update_t<FpM61, 8, 64>(FpM61(fp), m, ld, rbeg, rend, jend, cend, Aw, Bw, max_ctas, r64, err, st, g, lo);
     return cudaGetLastError();
   }
-  const FpBarrett f(fp);
-#define MODLIN_UPDATE(LL, KK) \
-  tc::update_t<FpBarrett, LL, KK>(f, m, ld, rbeg, rend, jend, cend, Aw, Bw, max_ctas, r64, err, st, g, lo)
-  MODLIN_TC_DISPATCH(MODLIN_UPDATE);
+  if (tc::limbs_of(fp.p) == 8) {
+    const FpBarrett f(fp);
+    if (K > 64)
+      tc::update_t<FpBarrett, 8, 128>(f, m, ld, rbeg, rend, jend, cend, Aw, Bw, max_ctas, r64, err, st, g, lo);
+    else
+      tc::update_t<FpBarrett, 8, 64>(f, m, ld, rbeg, rend, jend, cend, Aw, Bw, max_ctas, r64, err, st, g, lo);
+    return cudaGetLastError();
+  }
+  const FpSmall f(fp);
+  const uint64_t r32 = ((uint64_t)1 << 32) % fp.p;
+  switch (tc::limbs_of(fp.p) * 2 + (K > 64)) {
+#define MODLIN_UPDATE(LL, KK)                                                                              \
+  tc::update_t<FpSmall, LL, KK>(f, m, ld, rbeg, rend, jend, cend, Aw, Bw, max_ctas, r32, err, st, g, lo); \
+  break
+    case 2: MODLIN_UPDATE(1, 64);
+    case 3: MODLIN_UPDATE(1, 128);
+    case 4: MODLIN_UPDATE(2, 64);
+    case 5: MODLIN_UPDATE(2, 128);
+    case 8: MODLIN_UPDATE(4, 64);
+    default: MODLIN_UPDATE(4, 128);
 #undef MODLIN_UPDATE
+  }
   return cudaGetLastError();
 }
 
