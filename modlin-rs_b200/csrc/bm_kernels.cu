@@ -60,25 +60,12 @@ constexpr unsigned kAll = 0xffffffffu;
 // kFold offsets (two products each), and after kFoldHigh of those again.
 // ---------------------------------------------------------------------------
 
-// p = 2^61 - 1. S and W are two 31-bit halves, x = lo + 2^31 hi, as the two
-// 32-bit words: the four half products need no carries between them. S is
-// balanced (|lo| <= 2^30, |hi| <= 2^29 + 1), W is not (0 <= lo < 2^31,
-// 0 <= hi <= 2^30).
-struct BmM61 {
+// p = 2^61 - 1. S and W are two 31-bit halves (M61Halves); S is balanced (|lo|
+// <= 2^30, |hi| <= 2^29 + 1), so that a Dot takes more products.
+struct BmM61 : M61Halves {
   using S = uint64_t;
-  using W = uint64_t;
   using R = uint64_t;
   __device__ explicit BmM61(const FieldParams&) {}
-  static __device__ __forceinline__ int32_t lo(uint64_t x) { return (int32_t)(uint32_t)x; }
-  static __device__ __forceinline__ int32_t hi(uint64_t x) { return (int32_t)(uint32_t)(x >> 32); }
-  static __device__ __forceinline__ uint64_t words(int32_t l, int32_t h) {
-    return (uint64_t)(uint32_t)h << 32 | (uint32_t)l;
-  }
-  static __device__ __forceinline__ int64_t mad(int32_t a, int32_t b, int64_t c) {
-    int64_t d;
-    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
-    return d;
-  }
   __device__ __forceinline__ S pack(R x) const {
     const int64_t y = (int64_t)x - (x >= (1ULL << 60) ? (int64_t)kM61 : 0);  // in [-2^60, 2^60]
     const int32_t l = (int32_t)((uint32_t)y << 1) >> 1;
@@ -87,29 +74,9 @@ struct BmM61 {
   __device__ __forceinline__ W load(S x) const {
     int64_t v = ((int64_t)hi(x) << 31) + lo(x);
     if (v < 0) v += (int64_t)kM61;
-    return words((int32_t)((uint32_t)v & 0x7fffffffu), (int32_t)(v >> 31));
+    return split((uint64_t)v);
   }
-  __device__ __forceinline__ S store(W x) const {
-    uint64_t v = (uint64_t)((int64_t)hi(x) << 31) + (uint64_t)(int64_t)lo(x);
-    if (v >= kM61) v -= kM61;
-    return pack(v);
-  }
-  __device__ __forceinline__ W neg(W d) const { return words(-lo(d), -hi(d)); }
-  __device__ __forceinline__ bool zero(W d) const { return d == 0 || d == words(0x7fffffff, 0x3fffffff); }
-  // ll + 2^31 mid + 2^62 hh, |ll| < 2^62, |mid| < 2^62, |hh| < 2^60:
-  // 2^31 mid = 2^31 (mid mod 2^30) + (mid >> 30), 2^62 = 2, and 4 p makes the
-  // sum positive; it stays below 2^64.
-  __device__ __forceinline__ W comb(W bb, W a, W nd, W b) const {
-    const int64_t ll = mad(lo(nd), lo(b), mad(lo(bb), lo(a), (int64_t)(4 * kM61)));
-    const int64_t m0 = mad(hi(nd), lo(b), mad(hi(bb), lo(a), 0));
-    const int64_t m1 = mad(lo(nd), hi(b), mad(lo(bb), hi(a), 0));
-    const int64_t hh = mad(hi(nd), hi(b), mad(hi(bb), hi(a), 0));
-    const int64_t mid = m0 + m1;
-    const uint64_t x = (uint64_t)ll + (uint64_t)(hh << 1) + ((uint64_t)((uint32_t)mid & 0x3fffffffu) << 31) +
-                       (uint64_t)(mid >> 30);
-    const uint64_t y = (x & kM61) + (x >> 61);  // <= p + 7
-    return words((int32_t)((uint32_t)y & 0x7fffffffu), (int32_t)(y >> 31));
-  }
+  __device__ __forceinline__ S store(W x) const { return pack(M61Halves::value(x)); }
   __device__ __forceinline__ R add(R a, R b) const {
     const uint64_t s = a + b;
     return s >= kM61 ? s - kM61 : s;

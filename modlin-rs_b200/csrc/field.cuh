@@ -150,6 +150,51 @@ struct FpM61 {
   MODLIN_HD uint64_t modulus() const { return kM61; }
 };
 
+#ifdef __CUDACC__
+// 2^61 - 1 on two 31-bit halves, x = lo + 2^31 hi, in one 64-bit word: the
+// four half products of a multiplication need no carries between them, which
+// halves the dependent chain of a multiply-add with its reduction. W values
+// have 0 <= lo < 2^31 and 0 <= hi <= 2^30 and are at most p + 7.
+struct M61Halves {
+  using W = uint64_t;
+  static __device__ __forceinline__ int32_t lo(W x) { return (int32_t)(uint32_t)x; }
+  static __device__ __forceinline__ int32_t hi(W x) { return (int32_t)(uint32_t)(x >> 32); }
+  static __device__ __forceinline__ W words(int32_t l, int32_t h) {
+    return (uint64_t)(uint32_t)h << 32 | (uint32_t)l;
+  }
+  static __device__ __forceinline__ int64_t mad(int32_t a, int32_t b, int64_t c) {
+    int64_t d;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+    return d;
+  }
+  // y <= p + 7.
+  static __device__ __forceinline__ W split(uint64_t y) {
+    return words((int32_t)((uint32_t)y & 0x7fffffffu), (int32_t)(y >> 31));
+  }
+  // The canonical residue.
+  static __device__ __forceinline__ uint64_t value(W x) {
+    const uint64_t v = (uint64_t)((int64_t)hi(x) << 31) + (uint64_t)(int64_t)lo(x);
+    return v >= kM61 ? v - kM61 : v;
+  }
+  static __device__ __forceinline__ W neg(W d) { return words(-lo(d), -hi(d)); }
+  static __device__ __forceinline__ bool zero(W d) { return d == 0 || d == words(0x7fffffff, 0x3fffffff); }
+  // bb a + nd b, nd the neg of a W value (or, with bb = 0, a W value): ll +
+  // 2^31 mid + 2^62 hh with |ll| < 2^62, |mid| < 2^62, |hh| <= 2^60: 2^31 mid =
+  // 2^31 (mid mod 2^30) + (mid >> 30), 2^62 = 2, and 4 p makes the sum
+  // positive; it stays below 2^64.
+  static __device__ __forceinline__ W comb(W bb, W a, W nd, W b) {
+    const int64_t ll = mad(lo(nd), lo(b), mad(lo(bb), lo(a), (int64_t)(4 * kM61)));
+    const int64_t m0 = mad(hi(nd), lo(b), mad(hi(bb), lo(a), 0));
+    const int64_t m1 = mad(lo(nd), hi(b), mad(lo(bb), hi(a), 0));
+    const int64_t hh = mad(hi(nd), hi(b), mad(hi(bb), hi(a), 0));
+    const int64_t mid = m0 + m1;
+    const uint64_t x = (uint64_t)ll + (uint64_t)(hh << 1) + ((uint64_t)((uint32_t)mid & 0x3fffffffu) << 31) +
+                       (uint64_t)(mid >> 30);
+    return split((x & kM61) + (x >> 61));
+  }
+};
+#endif
+
 // a^-1 mod 2^61 - 1 (a != 0) as a^(p-2), p - 2 = 2^61 - 3 = 4 (2^59 - 1) + 1.
 // With x_k = a^(2^k - 1), x_(j+k) = x_j^(2^k) x_k builds x_59 from x_1 in 58
 // squarings and 9 multiplications; then a^(p-2) = x_59^4 a. One dependent

@@ -3,36 +3,38 @@
 // in flight at once).
 //
 // One CTA eliminates one matrix at a time, pulling jobs (largest first) from a
-// device counter. The method is the reference's blocked elimination
-// (src/fp.rs:125-255) with PANEL = 64:
-//   A. in-panel elimination: per column, the first nonzero row at or below
-//      the current rank is the pivot (src/fp.rs:151-156); the row order is a
-//      logical permutation in shared memory instead of physical swaps
-//      (src/fp.rs:158-162); each row below stores its multiplier in place of
-//      the eliminated entry (src/fp.rs:169-170) and updates the rest of the
-//      panel (src/fp.rs:171-173);
-//   B. U block: forward substitution among the panel's pivot rows
-//      (src/fp.rs:181-200), done per 64-column tile in shared memory;
-//   C. trailing update: rows below the pivots -= multipliers x U
-//      (src/fp.rs:202-248), 64x64 tiles, u128 accumulators reduced once per
-//      safe_batch products.
-// The rank is the number of pivots; every residue is exact, so the result is
-// the reference's bit for bit.
+// device counter. The row order is a logical permutation in shared memory
+// instead of physical swaps (src/fp.rs:158-162). Per 64-column panel:
+//  * Block step, when the 64 x 64 block P of the next 64 rows is invertible:
+//    its rows and columns are the panel's pivots, and the rest becomes the
+//    Schur complement: H = -X P^-1 for the panel X below P (written over X),
+//    then C += H U tile by tile. P^-1 by inv64, the products as 64 x 64 x 64
+//    limb products on the tensor cores (mma_limbs.cuh).
+//  * Otherwise (dependent columns, the last ragged panel) the reference's panel
+//    (src/fp.rs:125-255): A. in-panel elimination with the first nonzero row as
+//    pivot (src/fp.rs:151-178); B. U block by forward substitution
+//    (src/fp.rs:181-200); C. trailing update on the integer pipes
+//    (src/fp.rs:202-248), one reduction per safe_batch products.
+// When an update leaves nothing nonzero, the rank is what has been counted.
+// Every residue is exact, so the rank is the reference's.
 #include <cuda_runtime.h>
 
 #include <climits>
 
+#include "block_inv.cuh"
 #include "field.cuh"
+#include "mma_limbs.cuh"
 #include "rank_batch.cuh"
 
 namespace modlin {
 
 namespace {
 
-constexpr int kT = kRankBatchThreads;  // 256
-constexpr int kNW = kT / 32;
 constexpr int kP = 64;  // panel width
 constexpr int kG = 8;   // rows per warp in flight during the in-panel elimination
+constexpr int kStride = 80;                // bytes per row of a 64-deep limb plane
+constexpr int kPlane = kP * kStride;       // one limb plane of a 64 x 64 tile
+constexpr int kRegion = 8 * kPlane;        // 8 limb planes: 40 KiB
 
 // Lazy accumulation of products of residues: u128 sums reduced once per
 // safe_batch products in general; for p < 2^32 a product fits in 32 x 32 ->
@@ -57,29 +59,221 @@ struct Acc<FpSmall> {
   }
 };
 
+// Regions of shared memory: `a` holds the block being inverted, then the left
+// operand's planes, or LF on the panel path; `b` the inverse's scratch, then
+// the right operand's planes, or Us; `a2` (one CTA an SM) the left operand's
+// second buffer.
 struct BatchSmem {
-  uint64_t LF[kP][kP + 1];  // multipliers of a row tile, or the pivot rows' multipliers F[k][k2]
-  uint64_t Us[kP][kP];      // U block of one 64-column tile
-  uint64_t prow[kP];        // pivot row's panel segment
+  alignas(16) uint8_t b[kRegion];
+  alignas(16) uint8_t a[kRegion];
+  uint64_t prow[kP];  // pivot row's panel segment
   int pcol[kP];
-  int red[kNW];
+  int red[16];
   uint64_t inv;
   int found;
   long long job;
 };
+static_assert(sizeof(InvScratch<8>) <= kRegion && kP * kInvLd * 8 <= kRegion && kP * (kP + 1) * 8 <= kRegion, "");
 
-template <class F>
-__device__ __noinline__ int rank_one(const F& f, uint64_t* __restrict__ m, const int n, int* perm, BatchSmem& S) {
+// Diagonal sums of the 16 x 8 tile (row group rg, column group cg) of the
+// 64 x 64 product of the planes at A and B.
+template <int LIMBS>
+__device__ __forceinline__ void block_tile(uint32_t (&acc)[2 * LIMBS - 1][4], const uint8_t* A, const uint8_t* B,
+                                           int rg, int cg) {
+  mml::tile_k32<LIMBS, 2, kStride>(acc, mml::saddr(A) + rg * 16 * kStride, kPlane, mml::saddr(B) + cg * 8 * kStride,
+                                   kPlane);
+}
+
+// One block step at (r0, c0); false when P is not invertible (nothing has
+// changed but the order of the 64 rows). any: something right of and below
+// the block is nonzero afterwards.
+// Bound: 8 x 64 x 64 limb-product instructions per tile and 2^61 - 1 (8192 of
+// an SM's cycles), the epilogue and the conversions for fewer limbs.
+template <class F, int LIMBS, int kT>
+__device__ bool block_step(const F& f, uint64_t* __restrict__ m, const int n, int* perm, BatchSmem& S, uint8_t* a2,
+                           int r0, int c0, bool& any) {
+  const LimbRed<F, LIMBS> red(f);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint64_t p = f.modulus();
+  uint64_t* M = reinterpret_cast<uint64_t*>(S.a);
+  InvScratch<LIMBS>& I = *reinterpret_cast<InvScratch<LIMBS>*>(S.b);
+  for (int q = tid; q < kP * kP; q += kT) M[(q >> 6) * kInvLd + (q & 63)] = m[(int64_t)perm[r0 + (q >> 6)] * n + c0 + (q & 63)];
+  __syncthreads();
+  if (!inv64<F, LIMBS, kT>(f, red, M, I)) return false;
+  uint64_t fac[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) fac[u] = I.fac[u];
+  const int moved = tid < kP ? perm[r0 + I.order[tid]] : 0;
+  __syncthreads();
+  if (tid < kP) perm[r0 + tid] = moved;
+  // Right operand: -P^-1, plane row = column of P^-1.
+  for (int q = tid; q < kP * 16; q += kT) {
+    const int i = q & 63, k4 = 4 * (q >> 6);
+    const uint64_t fk = k4 < 32 ? (k4 < 16 ? fac[0] : fac[1]) : (k4 < 48 ? fac[2] : fac[3]);
+    uint64_t v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      v[u] = f.mul(M[(k4 + u) * kInvLd + i], fk);
+      v[u] = v[u] ? p - v[u] : 0;
+    }
+    mml::put_planes4<LIMBS>(S.b + i * kStride + k4, kPlane, v);
+  }
+  const int rb = r0 + kP, cb = c0 + kP;
+  // This warp's tiles: rows 16 rg .. +16, kTiles groups of 8 columns from cg0.
+  constexpr int kTiles = 32 / (kT / 32), kRound = kT / 16;
+  const int rg = warp & 3, cg0 = (warp >> 2) * kTiles;
+  const int g = lane >> 2, t2 = 2 * (lane & 3);
+  // Left operand: rows rt .. rt + 63 of the panel, through registers.
+  constexpr int kN = kP / kRound;
+  const auto load_rows = [&](int rt, uint64_t (&v)[kN][4]) {
+#pragma unroll
+    for (int w = 0; w < kN; ++w) {
+      const int i = (tid >> 4) + kRound * w, k4 = 4 * (tid & 15);
+      const uint64_t* src = rt + i < n ? m + (int64_t)perm[rt + i] * n + c0 + k4 : nullptr;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[w][u] = src ? src[u] : 0;
+    }
+  };
+  const auto put_rows = [&](uint8_t* dst, const uint64_t (&v)[kN][4]) {
+#pragma unroll
+    for (int w = 0; w < kN; ++w)
+      mml::put_planes4<LIMBS>(dst + ((tid >> 4) + kRound * w) * kStride + 4 * (tid & 15), kPlane, v[w]);
+  };
+  // The next tile's rows are loaded during this one's products where the
+  // registers allow; with two buffers one barrier a tile is enough.
+  constexpr bool kTwo = kT == 512, kEarly = LIMBS <= 4;
+  uint8_t* const bufs[2] = {S.a, kTwo ? a2 : S.a};
+  uint32_t acc[2 * LIMBS - 1][4];
+  uint64_t lv[kN][4];
+  if (cb < n && rb < n && kEarly) load_rows(rb, lv);
+  for (int rt = rb, k = 0; rt < n && cb < n; rt += kP, k ^= 1) {  // H over X
+    if (!kEarly) load_rows(rt, lv);
+    if (!kTwo || rt == rb) __syncthreads();  // the last product has read the buffer (or P^-1)
+    put_rows(bufs[k], lv);
+    __syncthreads();
+    if (kEarly && rt + kP < n) load_rows(rt + kP, lv);
+    const int ra = rt + 16 * rg + g, rz = ra + 8;
+    uint64_t* pa = ra < n ? m + (int64_t)perm[ra] * n + c0 : nullptr;
+    uint64_t* pz = rz < n ? m + (int64_t)perm[rz] * n + c0 : nullptr;
+#pragma unroll 1
+    for (int q = 0; q < kTiles; ++q) {
+      block_tile<LIMBS>(acc, bufs[k], S.b, rg, cg0 + q);
+      const int c = 8 * (cg0 + q) + t2;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        uint64_t* dst = e < 2 ? pa : pz;
+        const uint64_t v = red.residue(acc, e);
+        if (dst) dst[c + (e & 1)] = v;
+      }
+    }
+  }
+  // Trailing update by strips of kCols column tiles whose right operands fill
+  // region b: the left operand's load and the barriers are shared by them.
+  constexpr int kCols = LIMBS == 8 || !kTwo ? 1 : LIMBS == 4 ? 2 : 4;
+  bool nz = false;
+  for (int ct = cb; ct < n; ct += kP * kCols) {
+    __syncthreads();
+    constexpr int kRows4 = kT / 64;
+#pragma unroll 1
+    for (int s = 0; s < kCols; ++s) {
+      uint64_t uv[kN][4];
+      const int col = ct + kP * s + (tid & 63);
+#pragma unroll
+      for (int w = 0; w < kN; ++w)  // U: plane row = column
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          uv[w][u] = col < n ? m[(int64_t)perm[r0 + 4 * ((tid >> 6) + kRows4 * w) + u] * n + col] : 0;
+#pragma unroll
+      for (int w = 0; w < kN; ++w)
+        mml::put_planes4<LIMBS>(S.b + s * LIMBS * kPlane + (tid & 63) * kStride + 4 * ((tid >> 6) + kRows4 * w),
+                                kPlane, uv[w]);
+    }
+    if (kEarly) load_rows(rb, lv);
+    for (int rt = rb, k = 0; rt < n; rt += kP, k ^= 1) {
+      const int ra = rt + 16 * rg + g, rz = ra + 8;
+      uint64_t* pa = ra < n ? m + (int64_t)perm[ra] * n : nullptr;
+      uint64_t* pz = rz < n ? m + (int64_t)perm[rz] * n : nullptr;
+      // C of this warp's tiles is loaded before the left operand where
+      // registers allow, else before each tile's products (which cover it).
+      constexpr bool kAhead = LIMBS <= 4;
+      constexpr int kAll = kTiles * kCols;
+      uint64_t cv[kAhead ? kAll : 1][4];
+      const auto column = [&](int q) { return ct + kP * (q / kTiles) + 8 * (cg0 + q % kTiles) + t2; };
+      const auto load_c = [&](int q, uint64_t (&x)[4]) {
+        const int c = column(q);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const uint64_t* src = e < 2 ? pa : pz;
+          x[e] = src && c + (e & 1) < n ? src[c + (e & 1)] : 0;
+        }
+      };
+      if (kAhead) {
+#pragma unroll
+        for (int q = 0; q < kAll; ++q) load_c(q, cv[q]);
+      }
+      if (!kEarly) load_rows(rt, lv);
+      if (!kTwo && rt > rb) __syncthreads();
+      put_rows(bufs[k], lv);
+      __syncthreads();
+      if (kEarly && rt + kP < n) load_rows(rt + kP, lv);
+#pragma unroll(kAhead ? kAll : 1)
+      for (int q = 0; q < kAll; ++q) {
+        const int c = column(q);
+        uint64_t(&x)[4] = cv[kAhead ? q : 0];
+        if (!kAhead) load_c(q, x);
+        block_tile<LIMBS>(acc, bufs[k], S.b + q / kTiles * LIMBS * kPlane, rg, cg0 + q % kTiles);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          uint64_t* dst = e < 2 ? pa : pz;
+          const uint64_t v = red.plus(x[e], acc, e);
+          if (dst && c + (e & 1) < n) {
+            dst[c + (e & 1)] = v;
+            nz |= v != 0;
+          }
+        }
+      }
+    }
+  }
+  any = __syncthreads_or(nz);
+  return true;
+}
+
+template <class F, int LIMBS, int kT>
+__device__ __noinline__ int rank_one(const F& f, uint64_t* __restrict__ m, const int n, int* perm, BatchSmem& S,
+                                     uint8_t* a2) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   using A = Acc<F>;
   using AT = typename A::T;
   const uint64_t p = f.modulus();
   const uint64_t sb = A::batch(f);
+  uint64_t(*LF)[kP + 1] = reinterpret_cast<uint64_t(*)[kP + 1]>(S.a);  // multipliers of a row tile, or F[k][k2]
+  uint64_t(*Us)[kP] = reinterpret_cast<uint64_t(*)[kP]>(S.b);          // U block of one 64-column tile
   for (int i = tid; i < n; i += kT) perm[i] = i;
   __syncthreads();
   int r0 = 0;
   for (int c0 = 0; c0 < n && r0 < n; c0 += kP) {
     const int W = min(kP, n - c0);
+    if (W == kP && n - r0 >= kP) {
+      // A block without a pivot (4 / p of the invertible ones, the dependent
+      // ones always) is tried again with the next 64 rows, and once more.
+      bool any = false, step = false;
+      for (int t = 1;; ++t) {
+        step = block_step<F, LIMBS, kT>(f, m, n, perm, S, a2, r0, c0, any);
+        if (step || t == 3 || n - r0 < (t + 1) * kP) break;
+        if (tid < kP) {
+          const int o = perm[r0 + tid];
+          perm[r0 + tid] = perm[r0 + t * kP + tid];
+          perm[r0 + t * kP + tid] = o;
+        }
+        __syncthreads();
+      }
+      if (step) {
+        r0 += kP;
+        if (!any) break;
+        continue;
+      }
+      __syncthreads();
+    }
     int pb = 0;
     // ---- A. in-panel elimination ------------------------------------------
     for (int kk = 0; kk < W && r0 + pb < n; ++kk) {
@@ -95,14 +289,15 @@ __device__ __noinline__ int rank_one(const F& f, uint64_t* __restrict__ m, const
       __syncthreads();
       if (tid == 0) {
         int b = INT_MAX;
-        for (int w = 0; w < kNW; ++w) b = min(b, S.red[w]);
+        for (int w = 0; w < kT / 32; ++w) b = min(b, S.red[w]);
         S.found = b != INT_MAX;
         if (b != INT_MAX) {
           const int t = perm[r];
           perm[r] = perm[b];
           perm[b] = t;
           S.pcol[pb] = c;
-          S.inv = fp_inv_binary(m[(int64_t)perm[r] * n + c], p);
+          const uint64_t e = m[(int64_t)perm[r] * n + c];
+          S.inv = std::is_same<F, FpM61>::value ? fp_inv_m61(e) : fp_inv_binary(e, p);
         }
       }
       __syncthreads();
@@ -116,12 +311,12 @@ __device__ __noinline__ int rank_one(const F& f, uint64_t* __restrict__ m, const
       const uint64_t inv = S.inv;
       const uint64_t pv0 = lane > kk && lane < W ? S.prow[lane] : 0;
       const uint64_t pv1 = lane + 32 > kk && lane + 32 < W ? S.prow[lane + 32] : 0;
-      for (int base = r + 1 + warp; base < n; base += kNW * kG) {
+      for (int base = r + 1 + warp; base < n; base += kT / 32 * kG) {
         uint64_t* R[kG];
         uint64_t x0[kG], x1[kG];
 #pragma unroll
         for (int g = 0; g < kG; ++g) {
-          const int i = base + g * kNW;
+          const int i = base + g * (kT / 32);
           R[g] = i < n ? m + (int64_t)perm[i] * n + c0 : nullptr;
           x0[g] = R[g] && lane < W ? R[g][lane] : 0;
           x1[g] = R[g] && lane + 32 < W ? R[g][lane + 32] : 0;
@@ -141,6 +336,7 @@ __device__ __noinline__ int rank_one(const F& f, uint64_t* __restrict__ m, const
     }
     if (pb == 0) continue;
     const int jend = c0 + W;
+    bool nz = false;
     if (jend < n && r0 + pb < n) {
       // ---- B + C. per 64-column tile: U block, then the trailing rows ------
       const int tx = tid & 15, ty = tid >> 4;
@@ -148,22 +344,23 @@ __device__ __noinline__ int rank_one(const F& f, uint64_t* __restrict__ m, const
         // Pivot rows' multipliers F[k][k2] (k2 < k) and their tile of U.
         for (int idx = tid; idx < pb * pb; idx += kT) {
           const int k = idx / pb, k2 = idx - k * pb;
-          S.LF[k][k2] = k2 < k ? m[(int64_t)perm[r0 + k] * n + S.pcol[k2]] : 0;
+          LF[k][k2] = k2 < k ? m[(int64_t)perm[r0 + k] * n + S.pcol[k2]] : 0;
         }
         for (int idx = tid; idx < pb * kP; idx += kT) {
           const int k = idx >> 6, ci = idx & 63;
           const int cc = ct + ci;
-          S.Us[k][ci] = cc < n ? m[(int64_t)perm[r0 + k] * n + cc] : 0;
+          Us[k][ci] = cc < n ? m[(int64_t)perm[r0 + k] * n + cc] : 0;
         }
         __syncthreads();
         {
-          // U_k -= sum_{k2<k} F[k][k2] U_k2, four threads per column.
-          const int ci = tid >> 2, q = tid & 3;
+          // U_k -= sum_{k2<k} F[k][k2] U_k2, kQ threads per column.
+          constexpr int kQ = kT / kP;
+          const int ci = tid / kQ, q = tid % kQ;
           for (int k = 1; k < pb; ++k) {
             AT acc = 0;
             uint64_t tot = 0, cnt = 0;
-            for (int k2 = q; k2 < k; k2 += 4) {
-              acc += A::prod(f, S.LF[k][k2], S.Us[k2][ci]);
+            for (int k2 = q; k2 < k; k2 += kQ) {
+              acc += A::prod(f, LF[k][k2], Us[k2][ci]);
               if (++cnt >= sb) {
                 tot = f.add(tot, A::reduce(f, acc));
                 acc = 0;
@@ -171,9 +368,9 @@ __device__ __noinline__ int rank_one(const F& f, uint64_t* __restrict__ m, const
               }
             }
             uint64_t part = f.add(tot, A::reduce(f, acc));
-            part = f.add(part, __shfl_xor_sync(0xffffffffu, part, 1));
-            part = f.add(part, __shfl_xor_sync(0xffffffffu, part, 2));
-            if (q == 0) S.Us[k][ci] = f.sub(S.Us[k][ci], part);
+#pragma unroll
+            for (int o = 1; o < kQ; o <<= 1) part = f.add(part, __shfl_xor_sync(0xffffffffu, part, o));
+            if (q == 0) Us[k][ci] = f.sub(Us[k][ci], part);
             __syncwarp();
           }
         }
@@ -183,17 +380,18 @@ __device__ __noinline__ int rank_one(const F& f, uint64_t* __restrict__ m, const
           for (int idx = tid; idx < pb * kP; idx += kT) {
             const int ri = idx / pb, k = idx - ri * pb;
             const int rr = rt + ri;
-            S.LF[k][ri] = rr < n ? m[(int64_t)perm[rr] * n + S.pcol[k]] : 0;
+            LF[k][ri] = rr < n ? m[(int64_t)perm[rr] * n + S.pcol[k]] : 0;
           }
           __syncthreads();
+          constexpr int kI = kP / (kT / 16);  // rows per thread
           // A reduced accumulator (< p <= (p-1)^2 + 1) counts as one product,
           // so sb terms never overflow the u128.
           // The tile's C entries are loaded before the products so that
           // their latency overlaps the arithmetic.
-          uint64_t cv[4][4];
+          uint64_t cv[kI][4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int rr = rt + ty + 16 * i;
+          for (int i = 0; i < kI; ++i) {
+            const int rr = rt + ty + kT / 16 * i;
             const uint64_t* R = rr < n ? m + (int64_t)perm[rr] * n : nullptr;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -201,39 +399,42 @@ __device__ __noinline__ int rank_one(const F& f, uint64_t* __restrict__ m, const
               cv[i][q] = R && cc < n ? R[cc] : 0;
             }
           }
-          AT acc[4][4];
+          AT acc[kI][4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
+          for (int i = 0; i < kI; ++i)
 #pragma unroll
             for (int q = 0; q < 4; ++q) acc[i][q] = 0;
           uint64_t cnt = 0;
           for (int k = 0; k < pb; ++k) {
-            uint64_t a[4], b[4];
+            uint64_t a[kI], b[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = S.LF[k][ty + 16 * i];
+            for (int i = 0; i < kI; ++i) a[i] = LF[k][ty + kT / 16 * i];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) b[q] = S.Us[k][tx + 16 * q];
+            for (int q = 0; q < 4; ++q) b[q] = Us[k][tx + 16 * q];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < kI; ++i)
 #pragma unroll
               for (int q = 0; q < 4; ++q) acc[i][q] += A::prod(f, a[i], b[q]);
             if (++cnt >= sb) {
 #pragma unroll
-              for (int i = 0; i < 4; ++i)
+              for (int i = 0; i < kI; ++i)
 #pragma unroll
                 for (int q = 0; q < 4; ++q) acc[i][q] = A::reduce(f, acc[i][q]);
               cnt = 1;
             }
           }
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int rr = rt + ty + 16 * i;
+          for (int i = 0; i < kI; ++i) {
+            const int rr = rt + ty + kT / 16 * i;
             if (rr >= n) continue;
             uint64_t* R = m + (int64_t)perm[rr] * n;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               const int cc = ct + tx + 16 * q;
-              if (cc < n) R[cc] = f.sub(cv[i][q], A::reduce(f, acc[i][q]));
+              if (cc >= n) continue;
+              const uint64_t v = f.sub(cv[i][q], A::reduce(f, acc[i][q]));
+              R[cc] = v;
+              nz |= v != 0;
             }
           }
           __syncthreads();
@@ -241,15 +442,20 @@ __device__ __noinline__ int rank_one(const F& f, uint64_t* __restrict__ m, const
       }
     }
     r0 += pb;
+    if (!__syncthreads_or(nz)) break;
   }
   return r0;
 }
 
-__global__ void __launch_bounds__(kT, 2)
+// NT = 256: two CTAs an SM; 512: one.
+template <int NT>
+__global__ void __launch_bounds__(NT, 512 / NT)
     rank_batch_kernel(const RankJob* __restrict__ jobs, int64_t count, unsigned long long* next, int64_t* out) {
   extern __shared__ __align__(16) unsigned char rb_smem[];
   BatchSmem& S = *reinterpret_cast<BatchSmem*>(rb_smem);
-  int* perm = reinterpret_cast<int*>(rb_smem + sizeof(BatchSmem));
+  // One CTA an SM: the left operand's second buffer, then the row order.
+  uint8_t* a2 = rb_smem + sizeof(BatchSmem);
+  int* perm = reinterpret_cast<int*>(a2 + (NT == 512 ? kRegion : 0));
   for (;;) {
     if (threadIdx.x == 0) S.job = (long long)atomicAdd(next, 1ULL);
     __syncthreads();
@@ -259,12 +465,17 @@ __global__ void __launch_bounds__(kT, 2)
     const RankJob J = jobs[q];
     const FieldParams fp{J.p, J.mu_lo, J.mu_hi, J.safe_batch};
     int r;
-    if (J.p == kM61)
-      r = rank_one(FpM61(fp), J.m, (int)J.n, perm, S);
-    else if (J.p < (1ULL << 32))
-      r = rank_one(FpSmall(fp), J.m, (int)J.n, perm, S);
-    else
-      r = rank_one(FpBarrett(fp), J.m, (int)J.n, perm, S);
+    if (J.p == kM61) {
+      r = rank_one<FpM61, 8, NT>(FpM61(fp), J.m, (int)J.n, perm, S, a2);
+    } else if (J.p < (1ULL << 32)) {
+      const FpSmall f(fp);
+      r = J.p <= (1ULL << 8)    ? rank_one<FpSmall, 1, NT>(f, J.m, (int)J.n, perm, S, a2)
+          : J.p <= (1ULL << 16) ? rank_one<FpSmall, 2, NT>(f, J.m, (int)J.n, perm, S, a2)
+                                : rank_one<FpSmall, 4, NT>(f, J.m, (int)J.n, perm, S, a2);
+    } else {
+      const FpBarrett f(fp);
+      r = rank_one<FpBarrett, 8, NT>(f, J.m, (int)J.n, perm, S, a2);
+    }
     if (threadIdx.x == 0) out[J.slot] = r;
     __syncthreads();
   }
@@ -272,37 +483,64 @@ __global__ void __launch_bounds__(kT, 2)
 
 }  // namespace
 
-size_t rank_batch_smem_bytes(int64_t max_n) { return sizeof(BatchSmem) + (size_t)max_n * sizeof(int); }
+static size_t rank_batch_smem_bytes(int threads, int64_t max_n) {
+  return sizeof(BatchSmem) + (threads == 512 ? kRegion : 0) + (size_t)max_n * sizeof(int);
+}
 
-// The kernel's dynamic shared memory cap is set once to what the largest
-// side needs, so launches of any batch (graph-captured ones included) need no
+// The kernels' dynamic shared memory cap is set once to what the largest side
+// needs, so launches of any batch (graph-captured ones included) need no
 // attribute call.
 static cudaError_t rank_batch_attr() {
   static cudaError_t e = [] {
-    cudaError_t r = cudaFuncSetAttribute(rank_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)rank_batch_smem_bytes(kRankBatchMaxN));
+    cudaError_t r = cudaFuncSetAttribute(rank_batch_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)rank_batch_smem_bytes(256, kRankBatchMaxN));
+    if (r == cudaSuccess)
+      r = cudaFuncSetAttribute(rank_batch_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)rank_batch_smem_bytes(512, kRankBatchMaxN));
     return r;
   }();
   return e;
 }
 
-int rank_batch_blocks_per_sm(int64_t max_n) {
-  const size_t smem = rank_batch_smem_bytes(max_n);
-  if (rank_batch_attr() != cudaSuccess) return 0;
+// Threads per CTA: 512 when every matrix has an SM to itself, or the largest
+// are long enough to set the end of the batch.
+static int batch_threads(int64_t count, int64_t max_n, int num_sms) {
+  return count <= num_sms || max_n >= kRankBatchWideN ? 512 : 256;
+}
+
+RankBatchShape rank_batch_shape(int64_t count, int64_t max_n, int num_sms) {
+  RankBatchShape B{0, 0};
+  if (rank_batch_attr() != cudaSuccess) return B;
+  B.threads = batch_threads(count, max_n, num_sms);
+  const size_t smem = rank_batch_smem_bytes(B.threads, max_n);
   int nb = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rank_batch_kernel, kT, smem);
-  return nb;
+  if (B.threads == 512)
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rank_batch_kernel<512>, 512, smem);
+  else
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rank_batch_kernel<256>, 256, smem);
+  B.blocks = (int)(count < (int64_t)nb * num_sms ? count : (int64_t)nb * num_sms);
+  return B;
 }
 
 cudaError_t launch_rank_batch(const RankJob* d_jobs, int64_t count, unsigned long long* d_next, int64_t max_n,
-                              int blocks, int64_t* d_out, cudaStream_t st) {
-  const size_t smem = rank_batch_smem_bytes(max_n);
+                              const RankBatchShape& B, int64_t* d_out, cudaStream_t st) {
+  const size_t smem = rank_batch_smem_bytes(B.threads, max_n);
   cudaError_t e = rank_batch_attr();
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(d_next, 0, sizeof(unsigned long long), st);
   if (e != cudaSuccess) return e;
-  rank_batch_kernel<<<blocks, kT, smem, st>>>(d_jobs, count, d_next, d_out);
+  if (B.threads == 512)
+    rank_batch_kernel<512><<<B.blocks, 512, smem, st>>>(d_jobs, count, d_next, d_out);
+  else
+    rank_batch_kernel<256><<<B.blocks, 256, smem, st>>>(d_jobs, count, d_next, d_out);
   return cudaGetLastError();
+}
+
+// Modular multiply-adds of a limb class relative to one-limb primes, roughly:
+// the batch takes its longest jobs first.
+double rank_batch_cost(uint64_t p, int64_t n) {
+  const double w = p < (1ULL << 16) ? 1.0 : p < (1ULL << 32) ? 1.3 : p == kM61 ? 2.2 : 5.0;
+  return w * (double)n * n * (n + 200);
 }
 
 }  // namespace modlin

@@ -16,23 +16,19 @@ struct RankJob {
   int64_t slot;  // output index
 };
 
-constexpr int kRankBatchThreads = 256;
 // Largest side the batched kernel takes (its row permutation lives in shared
 // memory); larger matrices go through the single-matrix engine.
 constexpr int64_t kRankBatchMaxN = 8192;
+constexpr int64_t kRankBatchWideN = 384;
 
-// The tensor-core variant of the batched rank (one CTA per matrix, trailing
-// updates as INT8-limb GEMMs on its SM); used for the sides the autotuner
-// finds it faster on.
-size_t rank_batch_tc_smem_bytes(int64_t max_n);
-int rank_batch_tc_blocks_per_sm(int64_t max_n);
-// d_err: two device ints, zeroed by the caller; d_err[0] != 0 afterwards means
-// a bounded wait expired.
-cudaError_t launch_rank_batch_tc(const RankJob* d_jobs, int64_t count, unsigned long long* d_next, int64_t max_n,
-                                 int blocks, int64_t* d_out, int* d_err, cudaStream_t st);
-size_t rank_batch_smem_bytes(int64_t max_n);
-int rank_batch_blocks_per_sm(int64_t max_n);
+struct RankBatchShape {
+  int threads, blocks;
+};
+// Launch shape for `count` jobs of sides up to max_n; blocks 0 on an error.
+RankBatchShape rank_batch_shape(int64_t count, int64_t max_n, int num_sms);
+// Relative running time of a job.
+double rank_batch_cost(uint64_t p, int64_t n);
 cudaError_t launch_rank_batch(const RankJob* d_jobs, int64_t count, unsigned long long* d_next, int64_t max_n,
-                              int blocks, int64_t* d_out, cudaStream_t st);
+                              const RankBatchShape& shape, int64_t* d_out, cudaStream_t st);
 
 }  // namespace modlin

@@ -39,11 +39,11 @@ constexpr int kSgMaxProbs = 4;
 template <class F>
 void launch_small_gemm64_batch(const F& f, const SgProb* probs, int count, cudaStream_t st,
                                const Guard& g = Guard());
-// n words at p set to zero (a kernel, so that it chains with programmatic
-// dependent launches).
 // *flag (device) = whether rows [r0, n), columns [c0, n) of m hold a nonzero entry.
 cudaError_t launch_any_nonzero(const uint64_t* m, int64_t ld, int r0, int c0, int n, int* flag, int num_sms,
                                cudaStream_t st);
+// n words at p set to zero (a kernel, so that it chains with programmatic
+// dependent launches).
 void launch_zero(uint64_t* p, int64_t n, cudaStream_t st, const Guard& g = Guard());
 template <class F>
 void launch_window(const F& f, const uint64_t* m, int64_t ld, int n, int r0, int col, int W, int round,

@@ -49,6 +49,7 @@
 #include <type_traits>
 
 #include "field.cuh"
+#include "limb_sums.cuh"
 #include "rank_tc.cuh"
 #include "launch.cuh"
 #include "tc_ptx.cuh"
@@ -173,55 +174,6 @@ __device__ __forceinline__ uint64_t finish(const F& f, u128 lo, u128 hi, uint64_
   } else {
     return f.add(f.reduce(lo), f.mul(f.reduce(hi), r64));
   }
-}
-
-// p < 2^32: sum_d 2^(8d) a[d][c] mod p. The diagonals are below 2^26 (K <=
-// 128), so up to three of them (LIMBS <= 2) sum to less than 2^43; the seven of
-// LIMBS = 4 are split at 2^32 (r32 = 2^32 mod p).
-template <int LIMBS, int DIAG>
-__device__ __forceinline__ uint64_t finish_small(const FpSmall& f, const uint32_t (&a)[DIAG][4], int c, uint64_t r32) {
-  uint64_t lo = a[0][c];
-#pragma unroll
-  for (int d = 1; d < (DIAG < 4 ? DIAG : 4); ++d) lo += (uint64_t)a[d][c] << (8 * d);
-  if constexpr (DIAG <= 4) {
-    return f.reduce64(lo);
-  } else {
-    uint64_t hi = a[4][c];
-#pragma unroll
-    for (int d = 5; d < DIAG; ++d) hi += (uint64_t)a[d][c] << (8 * (d - 4));
-    return f.add(f.reduce64(lo), f.reduce64(f.reduce64(hi) * r32));
-  }
-}
-
-__device__ __forceinline__ uint64_t mad_wide_u32(uint32_t a, uint32_t b, uint64_t c) {
-  uint64_t d;
-  asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
-  return d;
-}
-
-// x = sum_{d<15} 2^(8d) a[d][c] mod 2^61 - 1, lazily: x < 2^62 and congruent.
-// The diagonal sums are a[d][c] <= 8 * 128 * 255^2 < 2^26 (K <= 128), and
-// 2^(8(d+8)) = 8 * 2^(8d) (mod p), so V_d = a_d + 8 a_(d+8) <= 57 * 128 * 255^2
-// < 2^29 (d < 7; V_7 = a_7). L = sum_{d<4} 2^(8d) V_d and H = sum_{d<4}
-// 2^(8d) V_(d+4) are < 2^54, and 2^32 H = 2^32 (H mod 2^29) + (H >> 29) (mod p)
-// since 2^61 = 1, so x = L + 2^32 (H mod 2^29) + (H >> 29) < 2^62.
-__device__ __forceinline__ uint64_t m61_fold15(const uint32_t (&a)[15][4], int c) {
-  uint32_t V[8];
-#pragma unroll
-  for (int d = 0; d < 7; ++d) V[d] = a[d][c] + 8u * a[d + 8][c];
-  V[7] = a[7][c];
-  const uint64_t L = mad_wide_u32(V[3], 1u << 24, mad_wide_u32(V[2], 1u << 16, mad_wide_u32(V[1], 1u << 8, V[0])));
-  const uint64_t H = mad_wide_u32(V[7], 1u << 24, mad_wide_u32(V[6], 1u << 16, mad_wide_u32(V[5], 1u << 8, V[4])));
-  return L + ((uint64_t)((uint32_t)H & 0x1FFFFFFFu) << 32) + (H >> 29);
-}
-
-// (cv - x) mod 2^61 - 1 for a canonical cv and any x < 2^62:
-// y = cv + 4p - x lies in (0, 2^64), one fold leaves y1 <= p + 7, and one
-// conditional subtraction makes it canonical.
-__device__ __forceinline__ uint64_t m61_sub_lazy(uint64_t cv, uint64_t x) {
-  const uint64_t y = cv + (4 * kM61) - x;
-  const uint64_t y1 = (y & kM61) + (y >> 61);
-  return y1 >= kM61 ? y1 - kM61 : y1;
 }
 
 // In place 8 x 8 byte transpose: afterwards byte c of t[i] is the former
@@ -723,6 +675,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       }
     } else {
+      const LimbRed<F, LIMBS> red(f);
       // Fewer limbs (p < 2^32): NS >= 32 columns per subtile; direct access.
       // All diagonals of a 4-column group are loaded from TMEM at once, and C
       // of the next group is loaded while this one is reduced.
@@ -760,7 +713,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (row_ok) {
 #pragma unroll
             for (int c = 0; c < 4; ++c)
-              if (cb + 16 * q + c < cend) crow[16 * q + c] = f.sub(cv[c], finish_small<LIMBS>(f, a, c, r64));
+              if (cb + 16 * q + c < cend) crow[16 * q + c] = f.sub(cv[c], red.residue(a, c));
           }
 #pragma unroll
           for (int c = 0; c < 4; ++c) cv[c] = nv[c];
@@ -1263,10 +1216,9 @@ cudaError_t tc_update(const FieldParams& fp, uint64_t* m, int64_t ld, int rbeg, 
     return cudaGetLastError();
   }
   const FpSmall f(fp);
-  const uint64_t r32 = ((uint64_t)1 << 32) % fp.p;
   switch (tc::limbs_of(fp.p) * 2 + (K > 64)) {
 #define MODLIN_UPDATE(LL, KK)                                                                              \
-  tc::update_t<FpSmall, LL, KK>(f, m, ld, rbeg, rend, jend, cend, Aw, Bw, max_ctas, r32, err, st, g, lo); \
+  tc::update_t<FpSmall, LL, KK>(f, m, ld, rbeg, rend, jend, cend, Aw, Bw, max_ctas, 0, err, st, g, lo); \
   break
     case 2: MODLIN_UPDATE(1, 64);
     case 3: MODLIN_UPDATE(1, 128);
