@@ -3,6 +3,7 @@
 // reference's src/fp.rs:125-255.
 #include <cuda_runtime.h>
 
+#include "block_inv.cuh"
 #include "launch.cuh"
 #include "rank_plain.cuh"
 #include "rank_kernels.cuh"
@@ -434,7 +435,7 @@ int plain_blocks_per_sm() {
 }
 
 // ---------------------------------------------------------------------------
-// gj64_inverse — one CTA of 1024 threads (16 per block row): the inverse of
+// gj64_inverse — one CTA of kInvThreads (8 per block row): the inverse of
 // the 64 x 64 block P = A[r0 .. r0+64, col .. col+64), or status = 1 when P
 // is singular. In-place fraction-free Gauss-Jordan: at
 // column c with pivot row `piv` (the first row not yet used whose entry is
@@ -458,9 +459,10 @@ __device__ void gj64_inverse(const F& f, const uint64_t* __restrict__ m, int64_t
   __shared__ int32_t pc[kPanel];
   __shared__ uint8_t nz[2][kPanel];  // nz[c & 1][j]: row j's entry in column c is nonzero
   const uint64_t p = f.modulus();
-  const int tid = threadIdx.x, j = tid >> 4, s = tid & 15;
+  constexpr int kRow = kInvThreads / kPanel;  // threads per block row
+  const int tid = threadIdx.x, j = tid / kRow, s = tid % kRow;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) M[j][s + 16 * q] = m[(int64_t)(r0 + j) * ld + col + s + 16 * q];
+  for (int q = 0; q < kPanel / kRow; ++q) M[j][s + kRow * q] = m[(int64_t)(r0 + j) * ld + col + s + kRow * q];
   if (s == 0) {
     d[j] = 0;
     sc[j] = 1;
@@ -475,7 +477,7 @@ __device__ void gj64_inverse(const F& f, const uint64_t* __restrict__ m, int64_t
     // Deferred from the previous column, after every thread has read the
     // pivot value there; only this thread reads this entry before the next
     // barrier.
-    if (j == last_piv && s == ((c - 1) & 15)) M[j][c - 1] = last_sc;
+    if (j == last_piv && s == (c - 1) % kRow) M[j][c - 1] = last_sc;
     // Every warp finds the pivot itself: the first row not yet used with a
     // nonzero entry in column c (a ballot over the 64 rows' flags, set before
     // the barrier by the thread that owns column c of each row).
@@ -497,11 +499,11 @@ __device__ void gj64_inverse(const F& f, const uint64_t* __restrict__ m, int64_t
     if (h != 0) {
       const uint64_t nh = p - h;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int k = s + 16 * q;
+      for (int q = 0; q < kPanel / kRow; ++q) {
+        const int k = s + kRow * q;
         M[j][k] = f.reduce2(f.prod(e, M[j][k]) + f.prod(nh, M[piv][k]));
       }
-      if (s == (c & 15)) M[j][c] = f.mul(nh, spiv);  // column c now holds E's column piv
+      if (s == c % kRow) M[j][c] = f.mul(nh, spiv);  // column c now holds E's column piv
       if (s == 0) {
         if ((used >> j) & 1)
           d[j] = f.mul(e, d[j]);
@@ -514,18 +516,18 @@ __device__ void gj64_inverse(const F& f, const uint64_t* __restrict__ m, int64_t
       pc[j] = c;
     }
     const int cn = c + 1;
-    if (cn < kPanel && s == (cn & 15)) nz[cn & 1][j] = M[j][cn] != 0;
+    if (cn < kPanel && s == cn % kRow) nz[cn & 1][j] = M[j][cn] != 0;
     last_piv = piv;
     last_sc = spiv;
     used |= 1ULL << piv;
     __syncthreads();
   }
-  if (j == last_piv && s == ((kPanel - 1) & 15)) M[j][kPanel - 1] = last_sc;
+  if (j == last_piv && s == (kPanel - 1) % kRow) M[j][kPanel - 1] = last_sc;
   if (tid < kPanel) dinv[tid] = fp_inv_binary(d[tid], p);
   __syncthreads();
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int i = s + 16 * q;
+  for (int q = 0; q < kPanel / kRow; ++q) {
+    const int i = s + kRow * q;
     const uint64_t v = f.mul(M[j][pc[i]], dinv[j]);
     Vneg[(int64_t)pc[j] * kPanel + i] = v ? p - v : 0;
   }
@@ -533,223 +535,54 @@ __device__ void gj64_inverse(const F& f, const uint64_t* __restrict__ m, int64_t
 
 
 // ---------------------------------------------------------------------------
-// Recursive fraction-free inverse of the 64 x 64 block (the fast path of
-// block_inverse_kernel). With P = [[A, B], [C, D]] in h x h blocks and
-// A^-1 = N1 / d1 (numerator, scalar denominator):
-//   S' = d1 D - (C N1) B  (= d1 S, S the Schur complement), S'^-1 = N2 / d2,
-//   W' = (N1 B) N2, V = N2 (C N1),
-//   P^-1 = [[d2 N1 + W' (C N1), -d1 W'], [-d1 V, d1^2 N2]] / (d1 d2).
-// Blocks of 32 recurse the same way; blocks of 16 are fraction-free
-// Gauss-Jordan on [X | I] with diagonal pivots (256 threads, two entries
-// each, one named barrier per column), after which row j reads
-// [D_j at column j | D_j X^-1 row j], and the per-row D_j are brought to
-// their product. No modular inverse until the single one of the final
-// denominator. The diagonal pivots and the leading 16- and 32-blocks and
-// their Schur complements must be nonzero / invertible (for large p all
-// fail with probability about 100/p); when one is not, the caller falls
-// back to gj64_inverse (first-nonzero pivoting over all 64 rows), so the
-// result never depends on that. Every product sum is exact (lazy u128 accumulation, one reduction
-// per safe_batch products).
+// block_inverse_kernel — one CTA: inv64 (block_inv.cuh), or on its failure (a
+// 16-column block without a pivot) the pivoting Gauss-Jordan over all 64 rows,
+// so the result never depends on the path. Output as gj64_inverse. On the
+// look-ahead chain: the latency of 64 dependent column steps (~400 cycles
+// each) and the K = 16 products between them. Measured over 2^61 - 1 28 us
+// (75 as a recursive inverse with all products on the integer pipes), mod
+// 65521 32 us (76; 347 by the pivoting Gauss-Jordan with 128-bit
+// reductions).
 // ---------------------------------------------------------------------------
-constexpr int kRecWords = 64 * 64 * 2 + 7 * 32 * 32 + 7 * 16 * 16 + 16 * 16;  // X, Out, scratch, base's I
-
-struct RecShared {
-  uint64_t pe[16];
-  int fail;
-};
-
-__device__ __forceinline__ void bar_base() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
-
-template <class F, int K>
-__device__ __forceinline__ uint64_t rec_dot(const F& f, const uint64_t* A, const uint64_t* B, int ldb) {
-  const uint64_t sb = f.safe_batch();
-  u128 acc = 0;
-  if (sb >= (uint64_t)K) {
-#pragma unroll 16
-    for (int k = 0; k < K; ++k) acc += f.prod(A[k], B[k * ldb]);
-  } else {
-    uint64_t cnt = 0;
-    for (int k = 0; k < K; ++k) {
-      acc += f.prod(A[k], B[k * ldb]);
-      if (++cnt == sb) {
-        acc = f.reduce(acc);
-        cnt = 1;
-      }
-    }
-  }
-  return f.reduce(acc);
-}
-
-// The dot product of this thread's output with K split over SPLIT adjacent
-// lanes (part = lane's share), summed across them by shuffles.
-template <class F, int K, int SPLIT>
-__device__ __forceinline__ uint64_t rec_dot_split(const F& f, const uint64_t* A, const uint64_t* B, int ldb, int part) {
-  constexpr int KP = K / SPLIT;
-  uint64_t v = rec_dot<F, KP>(f, A + part * KP, B + part * KP * ldb, ldb);
-#pragma unroll
-  for (int o = 1; o < SPLIT; o <<= 1) v = f.add(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-
-// 16 x 16 block X (clobbered) -> Out = X^-1 * delta, delta = product of the
-// rows' final diagonal entries. All threads call; threads 0..255 work.
-template <class F>
-__device__ void rec_base16(const F& f, uint64_t* X, int ldx, uint64_t* R, uint64_t* Out, int ldo, uint64_t* delta,
-                           RecShared& S) {
+template <class F, int LIMBS>
+__device__ bool inv64_block(const F& f, const uint64_t* __restrict__ m, int64_t ld, int32_t r0, int32_t col,
+                            uint64_t* __restrict__ Vneg, uint64_t* smem) {
+  const LimbRed<F, LIMBS> red(f);
   const uint64_t p = f.modulus();
-  const int tid = threadIdx.x;
-  if (tid < 256) {
-    const int j = tid >> 4, k = tid & 15, lane = tid & 31;
-    uint64_t x = X[j * ldx + k], y = j == k;
-    R[j * 16 + k] = y;
-    bar_base();
-    bool ok = true;
-#pragma unroll 1
-    for (int c = 0; c < 16; ++c) {
-      const uint64_t e = X[c * ldx + c], h = X[j * ldx + c];
-      if (e == 0) {  // the same in every thread
-        ok = false;
-        break;
-      }
-      const uint64_t xp = X[c * ldx + k], yp = R[c * 16 + k];
-      __syncwarp();  // row j's reads of X[j][c] precede its owner's write below
-      if (j != c && h != 0) {
-        const uint64_t nh = p - h;
-        x = f.reduce2(f.prod(e, x) + f.prod(nh, xp));
-        y = f.reduce2(f.prod(e, y) + f.prod(nh, yp));
-        X[j * ldx + k] = x;
-        R[j * 16 + k] = y;
-      }
-      bar_base();
-    }
-    if (!ok) {
-      if (tid == 0) S.fail = 1;
-    } else {
-      if (tid < 32) {  // pe[j] = product of the other rows' diagonal entries
-        const uint64_t xd = lane < 16 ? X[lane * ldx + lane] : 1;
-        uint64_t pre = xd, suf = xd;
-#pragma unroll
-        for (int off = 1; off < 16; off <<= 1) {
-          const uint64_t a = __shfl_up_sync(0xffffffffu, pre, off), b2 = __shfl_down_sync(0xffffffffu, suf, off);
-          if (lane >= off) pre = f.mul(pre, a);
-          if (lane + off < 16) suf = f.mul(suf, b2);
-        }
-        const uint64_t ex_pre = __shfl_up_sync(0xffffffffu, pre, 1), ex_suf = __shfl_down_sync(0xffffffffu, suf, 1);
-        const uint64_t all = __shfl_sync(0xffffffffu, pre, 15);
-        if (lane < 16) S.pe[lane] = f.mul(lane ? ex_pre : 1, lane < 15 ? ex_suf : 1);
-        if (lane == 0) *delta = all;
-      }
-      bar_base();
-      Out[j * ldo + k] = f.mul(y, S.pe[j]);
-    }
-  }
+  uint64_t* M = smem;
+  InvScratch<LIMBS>& S = *reinterpret_cast<InvScratch<LIMBS>*>(smem + kPanel * kInvLd);
+  for (int t = threadIdx.x; t < kPanel * kPanel; t += kInvThreads)
+    M[(t >> 6) * kInvLd + (t & 63)] = m[(int64_t)(r0 + (t >> 6)) * ld + col + (t & 63)];
   __syncthreads();
+  if (!inv64<F, LIMBS, kInvThreads>(f, red, M, S)) return false;
+  for (int t = threadIdx.x; t < kPanel * kPanel; t += kInvThreads) {
+    const int c = t >> 6, i = t & 63;
+    const uint64_t v = f.mul(M[c * kInvLd + i], S.fac[c >> 4]);
+    Vneg[c * kPanel + S.order[i]] = v ? p - v : 0;
+  }
+  return true;
 }
 
-// N x N block X (N = 32 or 64; its top-left h x h block is clobbered) ->
-// Out = X^-1 * delta. Scratch: 7 h x h buffers at scr, then the next level's.
-template <class F, int N>
-__device__ void rec_inverse(const F& f, uint64_t* X, int ldx, uint64_t* Out, int ldo, uint64_t* delta, uint64_t* scr,
-                            uint64_t* R, RecShared& S, uint64_t* dl) {
-  constexpr int H = N / 2, HH = H * H;
-  const uint64_t p = f.modulus();
-  uint64_t *N1 = scr, *CN = scr + HH, *NB = scr + 2 * HH, *Sp = scr + 3 * HH, *N2 = scr + 4 * HH, *Wp = scr + 5 * HH,
-           *V = scr + 6 * HH;
-  uint64_t* A = X;
-  const uint64_t *B = X + H, *C = X + H * ldx, *D = X + H * ldx + H;
-  if constexpr (H == 16)
-    rec_base16(f, A, ldx, R, N1, H, &dl[0], S);
-  else
-    rec_inverse<F, H>(f, A, ldx, N1, H, &dl[0], scr + 7 * HH, R, S, dl + 2);
-  if (S.fail) return;
-  // Small levels split each dot product over SP lanes (all threads busy).
-  constexpr int SP = H == 16 ? 2 : 1;
-  const uint64_t d1 = dl[0];
-  for (int tt = threadIdx.x; tt < SP * 2 * HH; tt += blockDim.x) {  // CN = C N1, NB = N1 B
-    const int t = tt / SP, part = tt % SP, u = t & (HH - 1), i = u / H, j = u % H;
-    const uint64_t v = t < HH ? rec_dot_split<F, H, SP>(f, C + i * ldx, N1 + j, H, part)
-                              : rec_dot_split<F, H, SP>(f, N1 + i * H, B + j, ldx, part);
-    if (part == 0) (t < HH ? CN : NB)[u] = v;
-  }
-  __syncthreads();
-  for (int tt = threadIdx.x; tt < SP * HH; tt += blockDim.x) {  // S' = d1 D - CN B
-    const int t = tt / SP, part = tt % SP, i = t / H, j = t % H;
-    const uint64_t v = rec_dot_split<F, H, SP>(f, CN + i * H, B + j, ldx, part);
-    if (part == 0) Sp[t] = f.sub(f.mul(d1, D[i * ldx + j]), v);
-  }
-  __syncthreads();
-  if constexpr (H == 16)
-    rec_base16(f, Sp, H, R, N2, H, &dl[1], S);
-  else
-    rec_inverse<F, H>(f, Sp, H, N2, H, &dl[1], scr + 7 * HH, R, S, dl + 2);
-  if (S.fail) return;
-  const uint64_t d2 = dl[1];
-  for (int tt = threadIdx.x; tt < SP * 2 * HH; tt += blockDim.x) {  // W' = NB N2, V = N2 CN
-    const int t = tt / SP, part = tt % SP, u = t & (HH - 1), i = u / H, j = u % H;
-    const uint64_t v = t < HH ? rec_dot_split<F, H, SP>(f, NB + i * H, N2 + j, H, part)
-                              : rec_dot_split<F, H, SP>(f, N2 + i * H, CN + j, H, part);
-    if (part == 0) (t < HH ? Wp : V)[u] = v;
-  }
-  __syncthreads();
-  const uint64_t d11 = f.mul(d1, d1);
-  for (int tt = threadIdx.x; tt < SP * HH; tt += blockDim.x) {  // top left: d2 N1 + W' CN
-    const int t = tt / SP, part = tt % SP, i = t / H, j = t % H;
-    const uint64_t v = rec_dot_split<F, H, SP>(f, Wp + i * H, CN + j, H, part);
-    if (part == 0) Out[i * ldo + j] = f.add(f.mul(d2, N1[t]), v);
-  }
-  for (int t = threadIdx.x + HH; t < 4 * HH; t += blockDim.x) {  // [[., -d1 W'], [-d1 V, d1^2 N2]]
-    const int q = t / HH, u = t & (HH - 1), i = u / H, j = u % H;
-    uint64_t v;
-    if (q == 3) {
-      v = f.mul(d11, N2[u]);
-    } else {
-      v = f.mul(d1, q == 1 ? Wp[u] : V[u]);
-      v = v ? p - v : 0;
-    }
-    Out[(i + (q >> 1) * H) * ldo + j + (q & 1) * H] = v;
-  }
-  if (threadIdx.x == 0) *delta = f.mul(d1, d2);
-  __syncthreads();
-}
-
-// block_inverse_kernel: the recursive path when `rec` (large p, where it
-// fails with probability about 100/p), else or on its failure the pivoting
-// Gauss-Jordan. Output as gj64_inverse.
 template <class F>
 __global__ void __launch_bounds__(kInvThreads) block_inverse_kernel(F f, const uint64_t* __restrict__ m, int64_t ld,
                                                                      int32_t r0, int32_t col,
-                                                                     uint64_t* __restrict__ Vneg, int* status, int rec,
+                                                                     uint64_t* __restrict__ Vneg, int* status,
                                                                      int reset_status, Guard g) {
   extern __shared__ __align__(16) uint64_t smem_inv[];
   pdl_wait();
   if (guard_skip(g)) return;  // an earlier step of the pipeline failed
   if (reset_status && status && threadIdx.x == 0) *status = 0;
-  if (rec) {
-    __shared__ RecShared S;
-    __shared__ uint64_t dl[5];  // level 64: d1, d2; level 32: d1, d2; the result's denominator
-    __shared__ uint64_t invd;
-    uint64_t* X = smem_inv;
-    uint64_t* Out = X + 64 * 64;
-    uint64_t* scr = Out + 64 * 64;
-    uint64_t* R = scr + 7 * 32 * 32 + 7 * 16 * 16;
-    for (int t = threadIdx.x; t < 64 * 64; t += blockDim.x)
-      X[t] = m[(int64_t)(r0 + (t >> 6)) * ld + col + (t & 63)];
-    if (threadIdx.x == 0) S.fail = 0;
-    __syncthreads();
-    rec_inverse<F, 64>(f, X, 64, Out, 64, &dl[4], scr, R, S, dl);
-    if (!S.fail) {
-      const uint64_t p = f.modulus();
-      if (threadIdx.x == 0) invd = std::is_same<F, FpM61>::value ? fp_inv_m61(dl[4]) : fp_inv_binary(dl[4], p);
-      __syncthreads();
-      const uint64_t inv = invd;
-      for (int t = threadIdx.x; t < 64 * 64; t += blockDim.x) {
-        const uint64_t v = f.mul(Out[t], inv);
-        Vneg[t] = v ? p - v : 0;
-      }
-      return;
-    }
-    __syncthreads();
+  bool ok;
+  if constexpr (std::is_same<F, FpSmall>::value) {
+    const uint64_t p = f.modulus();
+    ok = p <= (1ULL << 8)    ? inv64_block<F, 1>(f, m, ld, r0, col, Vneg, smem_inv)
+         : p <= (1ULL << 16) ? inv64_block<F, 2>(f, m, ld, r0, col, Vneg, smem_inv)
+                             : inv64_block<F, 4>(f, m, ld, r0, col, Vneg, smem_inv);
+  } else {
+    ok = inv64_block<F, 8>(f, m, ld, r0, col, Vneg, smem_inv);
   }
+  if (ok) return;
+  __syncthreads();
   gj64_inverse(f, m, ld, r0, col, Vneg, status, g, smem_inv);
 }
 
@@ -912,15 +745,14 @@ void launch_trailing_plain(const F& f, uint64_t* m, int64_t ld, int rbeg, int re
 template <class F>
 void launch_block_inverse(const F& f, const uint64_t* m, int64_t ld, int r0, int col, uint64_t* Vneg, int* status,
                           cudaStream_t st, bool reset_status, const Guard& g) {
-  const size_t smem = kRecWords * sizeof(uint64_t);  // >= the pivoting path's kPanel * (kPanel + 1) words
+  const size_t smem = kPanel * kInvLd * 8 + sizeof(InvScratch<8>);  // more than the pivoting path's kPanel * (kPanel + 1) words
   static bool attr_set = false;
   if (!attr_set) {
     cudaFuncSetAttribute(block_inverse_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     attr_set = true;
   }
-  const int rec = f.modulus() > (1ULL << 12);
   launch_k(block_inverse_kernel<F>, dim3(1), dim3(kInvThreads), smem, st, 1, f, m, ld, (int32_t)r0, (int32_t)col,
-           Vneg, status, rec, reset_status ? 1 : 0, g);
+           Vneg, status, reset_status ? 1 : 0, g);
 }
 
 template <class F>
