@@ -60,6 +60,9 @@ struct LimbRed<FpM61, 8> {
     const uint64_t x = FpM61::fold(y);
     return x >= kM61 ? x - kM61 : x;
   }
+  // T in a form that fits 64 bits, and c - T from it.
+  __device__ __forceinline__ uint64_t lazy(const uint32_t (&a)[15][4], int c) const { return m61_fold15(a, c); }
+  __device__ __forceinline__ uint64_t minus(uint64_t v, uint64_t t) const { return m61_sub_lazy(v, t); }
   __device__ __forceinline__ uint64_t residue(const uint32_t (&a)[15][4], int c) const {
     return last(m61_fold15(a, c));
   }
@@ -88,6 +91,8 @@ struct LimbRed<FpSmall, LIMBS> {
     w[1] = (uint32_t)f.reduce64(1ULL << 40);
     w[2] = (uint32_t)f.reduce64(1ULL << 48);
   }
+  __device__ __forceinline__ uint64_t lazy(const uint32_t (&a)[2 * LIMBS - 1][4], int c) const { return sum(a, c); }
+  __device__ __forceinline__ uint64_t minus(uint64_t v, uint64_t t) const { return f.reduce64(v + kp - t); }
   __device__ __forceinline__ uint64_t sum(const uint32_t (&a)[2 * LIMBS - 1][4], int c) const {
     uint64_t t = a[0][c];
 #pragma unroll

@@ -33,10 +33,10 @@
 // range of the (M tile, N subtile) space; it keeps the 128-row A tile (all
 // limb planes) resident and streams B subtiles through a ring; one CTA per SM
 // owns all 512 TMEM columns as two accumulator buffers, so the MMAs of
-// subtile s+1 run while the epilogue drains subtile s. Over 2^61 - 1 the
-// epilogue is two 8-warp groups, one per accumulator buffer, and C moves by
-// 2D TMA (128 x 16 tiles, 128-byte swizzle) through one shared buffer per
-// group; other primes use 16 warps and C staged by cp.async. Every mbarrier
+// subtile s+1 run while the epilogue drains subtile s. Over 2^61 - 1 and for p <
+// 2^32 the epilogue is two 8-warp groups, one per accumulator buffer, and C
+// moves by 2D TMA (128 x 16 tiles, 128-byte swizzle) through shared buffers of
+// the group; other primes use 16 warps and C staged by cp.async. Every mbarrier
 // wait is bounded; on expiry the kernel records an error, drains its own
 // copies and MMAs (bounded), frees TMEM and returns.
 #include <cuda.h>
@@ -82,11 +82,14 @@ struct Shape {
   static constexpr int C_BYTES = LIMBS == 8 ? CDEPTH * 128 * kCStride * 8 : 0;  // staged C tiles
   static constexpr int SMEM = A_BYTES + STAGES * B_BYTES + ZERO_BYTES + 1024 + C_BYTES;
   static_assert(SMEM <= 227 * 1024, "shared memory");
-  // p = 2^61 - 1: the epilogue stages C by TMA, one 128 x 16 tile per group.
-  static constexpr int STAGES_M61 = KK == 64 ? 8 : 2;
-  static constexpr int C_TMA_BYTES = 4 * 128 * 16 * 8;  // two 128 x 16 C tiles per epilogue group
-  static constexpr int SMEM_M61 = A_BYTES + STAGES_M61 * B_BYTES + ZERO_BYTES + 1024 + C_TMA_BYTES;
-  static_assert(SMEM_M61 <= 227 * 1024, "shared memory");
+  // Epilogue in two groups, C by TMA in 128 x 16 tiles (p = 2^61 - 1 and p <
+  // 2^32): NB tiles per group in shared memory, SL to a subtile.
+  static constexpr int SL = NS / 16;
+  static constexpr int NB = LIMBS == 8 ? 2 : 4;
+  static constexpr int STAGES_TMA = KK == 64 ? (LIMBS == 8 ? 8 : 4) : 2;
+  static constexpr int C_TMA_BYTES = 2 * NB * 128 * 16 * 8;
+  static constexpr int SMEM_TMA = A_BYTES + STAGES_TMA * B_BYTES + ZERO_BYTES + 1024 + C_TMA_BYTES;
+  static_assert(SMEM_TMA <= 227 * 1024, "shared memory");
 };
 
 struct Sched {
@@ -223,9 +226,10 @@ __global__ void __launch_bounds__(kThreads, 1)
                        const __grid_constant__ CUtensorMap cmap, int use_tma, Guard guard, LimbOut lo) {
   using SH = Shape<LIMBS, KK>;
   constexpr int NS = SH::NS;
-  // p = 2^61 - 1: two epilogue groups of 8 warps, one per accumulator buffer.
-  constexpr bool kM61Path = std::is_same<F, FpM61>::value;
-  constexpr int kStages = kM61Path ? SH::STAGES_M61 : SH::STAGES;
+  // p = 2^61 - 1 and p < 2^32: two epilogue groups of 8 warps, one per
+  // accumulator buffer.
+  constexpr bool kGrouped = !std::is_same<F, FpBarrett>::value;
+  constexpr int kStages = kGrouped ? SH::STAGES_TMA : SH::STAGES;
   constexpr int kCDepth = SH::CDEPTH;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sA = smem;                        // A_BYTES
@@ -253,10 +257,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     mbar_init(a_empty, 1);
     for (int b = 0; b < 2; ++b) {
       mbar_init(acc_full + b, 1);
-      mbar_init(acc_empty + b, kM61Path ? kEpiWarps / 2 : kEpiWarps);
+      mbar_init(acc_empty + b, kGrouped ? kEpiWarps / 2 : kEpiWarps);
     }
     mbar_init(mma_done, 1);
-    for (int q = 0; q < 4; ++q) mbar_init(bars + 40 + q, 1);  // c_full of (epilogue group, C buffer), 2^61 - 1
+    for (int q = 0; q < 2 * SH::NB; ++q) mbar_init(bars + 40 + q, 1);  // c_full of (epilogue group, C buffer)
     for (int st = 0; st < kStages; ++st) {
       mbar_init(b_full + st, 1);
       mbar_init(b_empty + st, 1);
@@ -358,55 +362,71 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_wait(mma_done, 0, err + 1);
     }
     __syncwarp();
-  } else if constexpr (kM61Path) {
-    // ---------------- epilogue, p = 2^61 - 1 ----------------------------------
+  } else if constexpr (kGrouped) {
+    // ---------------- epilogue, p = 2^61 - 1 or p < 2^32 ----------------------
     // Two groups of 8 warps: group g drains accumulator buffer g, i.e. the
     // subtiles it = g, g + 2, ... of this CTA's range, so each group has two
-    // MMA periods per subtile and the groups' phases interleave. In a group,
-    // warp w reads TMEM lanes 32*(w%4)..+32 (its 32 rows) and one half (8
-    // columns) of the 16-column subtile, so every thread owns one row x 8
-    // columns. It folds the 15 diagonal sums of each column and releases the
-    // accumulator buffer first; then C - T is formed against C.
+    // MMA periods per subtile and the groups' phases interleave. A subtile is
+    // worked through in units of 16 columns (one for 8 limbs): warp w reads
+    // TMEM lanes 32*(w%4)..+32 (its 32 rows) and one half (8 columns) of the
+    // unit, so every thread owns one row x 8 columns. It folds the diagonal
+    // sums of each column and releases the accumulator buffer after the
+    // subtile's last unit; then C - T is formed against C.
     // C moves by TMA (use_tma): the group's leader thread loads the 128 x 16
-    // C tile of its next subtile into the group's shared buffer (128-byte
+    // C tiles of its next units into the group's NB shared buffers (128-byte
     // swizzle, so the threads' row-wise accesses are conflict-free), the
-    // threads replace it in place by C - T, and the leader stores it back
-    // with one tensor copy, then loads the group's next tile. Without TMA
-    // (a row stride or column offset that is not 16-byte aligned) every
-    // thread reads and writes its 8 values directly.
+    // threads replace a tile in place by C - T, and the leader stores it back
+    // with one tensor copy. With few limbs the update is bound by these
+    // copies, so more tiles are in flight (direct row-wise accesses reached
+    // 1.5 TB/s for 16-bit primes). Without TMA (a row stride or column offset
+    // that is not 16-byte aligned) every thread reads and writes its 8 values
+    // directly.
+    constexpr int NB = SH::NB, SL = SH::SL;
+    const LimbRed<F, LIMBS> red(f);
     const int ew = warp - 2;
     const int grp = ew >> 3;          // accumulator buffer this group drains
     const int quad = warp & 3;        // TMEM lane quadrant
-    const int half = (ew >> 2) & 1;   // column half of the subtile
+    const int half = (ew >> 2) & 1;   // column half of the unit
     const int row = quad * 32 + lane;
     const bool leader = (ew & 7) == 0 && lane == 0;
     const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16) + grp * 256 + half * 8;
-    // Two C buffers per group: the tile of the group's next subtile loads
-    // while the current one is computed and stored.
-    uint64_t* cbuf0 = reinterpret_cast<uint64_t*>(sZ + SH::ZERO_BYTES + 1024) + grp * 2 * (128 * 16);
-    uint64_t* c_full0 = bars + 40 + 2 * grp;
-    const int64_t nsub = S.nsub;
-    // Subtile it = grp + 2 k of [g0, g1): (mt, sb) tracked incrementally.
-    int64_t g = g0 + grp;
-    int64_t mt = g / nsub, sb = g - mt * nsub;
-    auto advance = [&]() {
-      g += 2;
-      sb += 2;
-      while (sb >= nsub) {
-        sb -= nsub;
-        ++mt;
+    uint64_t* cbuf0 = reinterpret_cast<uint64_t*>(sZ + SH::ZERO_BYTES + 1024) + grp * NB * (128 * 16);
+    uint64_t* c_full0 = bars + 40 + NB * grp;
+    const int nsub = S.nsub, gend = (int)g1;  // (M tile, subtile) pairs fit 32 bits
+    // Units in order: slice sl of subtile it = grp + 2 k of [g0, g1), (mt, sb)
+    // tracked incrementally. Slices past cend do not exist.
+    struct Cursor {
+      int g, mt, sb, sl;
+    };
+    const auto col = [&](const Cursor& c) { return jend + c.sb * NS + c.sl * 16; };
+    const auto last_slice = [&](const Cursor& c) { return c.sl + 1 == SL || col(c) + 16 >= cend; };
+    const auto advance = [&](Cursor& c) {
+      if (!last_slice(c)) {
+        ++c.sl;
+        return;
+      }
+      c.sl = 0;
+      c.g += 2;
+      c.sb += 2;
+      while (c.sb >= nsub) {
+        c.sb -= nsub;
+        ++c.mt;
       }
     };
-    int loads = 0;  // TMA loads issued by the leader; load j goes to buffer j & 1
+    Cursor cur{(int)g0 + grp, ((int)g0 + grp) / nsub, 0, 0};
+    cur.sb = cur.g - cur.mt * nsub;
+    Cursor lc = cur;  // next unit to load (leader)
+    int loads = 0;    // TMA loads issued by the leader; load j goes to buffer j % NB
     auto tma_load = [&]() {
-      uint64_t* cf = c_full0 + (loads & 1);
+      uint64_t* cf = c_full0 + loads % NB;
       mbar_arrive_expect_tx(cf, 128 * 16 * 8);
-      tma_load_2d(cbuf0 + (loads & 1) * (128 * 16), &cmap, (int32_t)(jend + sb * NS), (int32_t)(rbeg + mt * 128), cf);
+      tma_load_2d(cbuf0 + (loads % NB) * (128 * 16), &cmap, (int32_t)col(lc), (int32_t)(rbeg + lc.mt * 128), cf);
       ++loads;
+      advance(lc);
     };
     auto load_c = [&](uint64_t (&cv)[8]) {
-      const int64_t r = (int64_t)rbeg + mt * 128 + row;
-      const int64_t c0 = (int64_t)jend + sb * NS + half * 8;
+      const int64_t r = (int64_t)rbeg + cur.mt * 128 + row;
+      const int64_t c0 = col(cur) + half * 8;
       const uint64_t* src = m + r * ld + c0;
 #pragma unroll
       for (int c = 0; c < 8; ++c) cv[c] = (r < rend && c0 + c < cend) ? __ldcs(src + c) : 0;
@@ -415,8 +435,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     const bool czero = lo.c_zero != 0;
     const bool tma = use_tma && !czero;
     auto put_limbs = [&](uint64_t (&res)[8]) {
-      const int64_t r = (int64_t)rbeg + mt * 128 + row;
-      const int64_t c0 = (int64_t)jend + sb * NS + half * 8;
+      const int64_t r = (int64_t)rbeg + cur.mt * 128 + row;
+      const int64_t c0 = col(cur) + half * 8;
       const int64_t lr = r - lo.row0;
       if (r >= rend || lr < 0) return;
 #pragma unroll
@@ -425,46 +445,40 @@ __global__ void __launch_bounds__(kThreads, 1)
       store_limbs8(lo.Aw, lo.kk, lr, (int)(c0 - jend), res);
     };
     uint64_t cv[8];
-    if (g < g1 && !czero) {
+    if (cur.g < gend && !czero) {
       if (!use_tma) {
         load_c(cv);
       } else if (leader) {
-        tma_load();  // subtile 0 into buffer 0
-        if (g + 2 < g1) {
-          advance();
-          tma_load();  // subtile 1 into buffer 1
-          g -= 2;      // back to subtile 0
-          sb -= 2;
-          while (sb < 0) {
-            sb += nsub;
-            --mt;
-          }
-        }
+        while (loads < NB && lc.g < gend) tma_load();
       }
     }
     bool ok = true;
-    for (int k = 0; g < g1; ++k) {
-      bool okw = __all_sync(0xffffffffu, mbar_wait(acc_full + grp, k & 1, err));
+    for (int u = 0, k = 0; cur.g < gend; ++u) {
+      bool okw = cur.sl > 0 || __all_sync(0xffffffffu, mbar_wait(acc_full + grp, k & 1, err));
+      const bool last = last_slice(cur);
       uint64_t x[8];
       if (okw) {
-        fence_after();
+        if (cur.sl == 0) fence_after();
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-          uint32_t a[15][4];
+          uint32_t a[SH::DIAG][4];
 #pragma unroll
-          for (int d = 0; d < 15; ++d) tmem_ld4(lane_base + d * NS + q * 4, a[d]);
+          for (int d = 0; d < SH::DIAG; ++d) tmem_ld4(lane_base + d * NS + cur.sl * 16 + q * 4, a[d]);
           tmem_wait_ld();
 #pragma unroll
-          for (int c = 0; c < 4; ++c) x[4 * q + c] = m61_fold15(a, c);
+          for (int c = 0; c < 4; ++c) x[4 * q + c] = red.lazy(a, c);
         }
-        fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(acc_empty + grp);
+        if (last) {
+          fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(acc_empty + grp);
+          ++k;
+        }
       }
       uint64_t res[8];
       if (tma) {
-        uint64_t* const cbuf = cbuf0 + (k & 1) * (128 * 16);
-        if (okw) okw = __all_sync(0xffffffffu, mbar_wait(c_full0 + (k & 1), (k >> 1) & 1, err));
+        uint64_t* const cbuf = cbuf0 + (u % NB) * (128 * 16);
+        if (okw) okw = __all_sync(0xffffffffu, mbar_wait(c_full0 + u % NB, (u / NB) & 1, err));
         if (okw) {
           // Row `row`, 16-byte chunks 4 half .. +4 of the 128-byte row; the
           // 128-byte swizzle XORs the chunk index (address bits 4-6) with
@@ -477,8 +491,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int delta = (int)((a ^ (a >> 3)) & 0x70u) - (int)(a & 0x70u);
             ulonglong2* pq = reinterpret_cast<ulonglong2*>(reinterpret_cast<uint8_t*>(lp) + delta);
             const ulonglong2 v = *pq;
-            res[2 * q] = m61_sub_lazy(v.x, x[2 * q]);
-            res[2 * q + 1] = m61_sub_lazy(v.y, x[2 * q + 1]);
+            res[2 * q] = red.minus(v.x, x[2 * q]);
+            res[2 * q + 1] = red.minus(v.y, x[2 * q + 1]);
             *pq = make_ulonglong2(res[2 * q], res[2 * q + 1]);
           }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -490,15 +504,14 @@ __global__ void __launch_bounds__(kThreads, 1)
           break;
         }
         if (leader) {
-          tma_store_2d(&cmap, (int32_t)(jend + sb * NS), (int32_t)(rbeg + mt * 128), cbuf);
+          tma_store_2d(&cmap, (int32_t)col(cur), (int32_t)(rbeg + cur.mt * 128), cbuf);
           bulk_commit();
         }
-        if (lo.Aw) put_limbs(res);
-        advance();
-        if (leader && g < g1 && loads == k + 1) {
-          // The tile after next goes to the other buffer once the store
-          // issued from it one subtile ago has read it (this subtile's store
-          // may still be reading).
+        if (LIMBS == 8 && lo.Aw) put_limbs(res);
+        advance(cur);
+        if (leader && lc.g < gend && loads < u + NB) {
+          // Unit u - 1 + NB goes to unit u - 1's buffer once its store has read
+          // it (this unit's store may still be reading).
           asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
           tma_load();
         }
@@ -507,25 +520,26 @@ __global__ void __launch_bounds__(kThreads, 1)
           ok = false;
           break;
         }
-        const int64_t r = (int64_t)rbeg + mt * 128 + row;
-        const int64_t c0 = (int64_t)jend + sb * NS + half * 8;
+        const int64_t r = (int64_t)rbeg + cur.mt * 128 + row;
+        const int64_t c0 = col(cur) + half * 8;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) res[c] = m61_sub_lazy(czero ? 0 : cv[c], x[c]);
+        for (int c = 0; c < 8; ++c) res[c] = red.minus(czero ? 0 : cv[c], x[c]);
         if (!czero && r < rend) {
           uint64_t* dst = m + r * ld + c0;
 #pragma unroll
           for (int c = 0; c < 8; ++c)
             if (c0 + c < cend) dst[c] = res[c];
         }
-        if (lo.Aw) put_limbs(res);
-        advance();
-        if (g < g1 && !czero) load_c(cv);
+        if (LIMBS == 8 && lo.Aw) put_limbs(res);
+        advance(cur);
+        if (cur.g < gend && !czero) load_c(cv);
       }
     }
     if (leader && tma) {
       bulk_wait_all0();  // stores complete
       if (!ok) {  // loads still landing: the last one into each buffer
-        for (int j = loads - 2 > 0 ? loads - 2 : 0; j < loads; ++j) mbar_wait(c_full0 + (j & 1), (j >> 1) & 1, err + 1);
+        for (int j = loads - NB > 0 ? loads - NB : 0; j < loads; ++j)
+          mbar_wait(c_full0 + j % NB, (j / NB) & 1, err + 1);
       }
     }
     if (!ok) atomicExch(err, 1);
@@ -672,51 +686,6 @@ __global__ void __launch_bounds__(kThreads, 1)
               if (gr < rend && gc < cend) m[gr * ld + gc] = slot[lr * kCStride + cc];
             }
           }
-        }
-      }
-    } else {
-      const LimbRed<F, LIMBS> red(f);
-      // Fewer limbs (p < 2^32): NS >= 32 columns per subtile; direct access.
-      // All diagonals of a 4-column group are loaded from TMEM at once, and C
-      // of the next group is loaded while this one is reduced.
-      int mt = (int)(g0 / S.nsub), sb = (int)(g0 - (int64_t)mt * S.nsub);
-      for (int64_t g = g0; g < g1 && ok; ++g, ++it, sb = sb + 1 == S.nsub ? (++mt, 0) : sb + 1) {
-        const int64_t r = (int64_t)rbeg + (int64_t)mt * 128 + row;
-        const bool row_ok = r < rend;
-        const int ab = it & 1;
-        const uint32_t lane_addr = lane_base + ab * 256;
-        const int64_t cb = (int64_t)jend + (int64_t)sb * NS + qc * 4;
-        uint64_t* crow = m + r * ld + cb;
-        uint64_t cv[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) cv[c] = (row_ok && cb + c < cend) ? crow[c] : 0;
-        ok = __all_sync(0xffffffffu, mbar_wait(acc_full + ab, (it >> 1) & 1, err));
-        if (!ok) break;
-        fence_after();
-#pragma unroll
-        for (int q = 0; q < NS / 16; ++q) {
-          uint32_t a[SH::DIAG][4];
-#pragma unroll
-          for (int d = 0; d < SH::DIAG; ++d) tmem_ld4(lane_addr + d * NS + q * 16, a[d]);
-          uint64_t nv[4];
-          if (q + 1 < NS / 16) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-              nv[c] = (row_ok && cb + 16 * (q + 1) + c < cend) ? crow[16 * (q + 1) + c] : 0;
-          }
-          tmem_wait_ld();
-          if (q == NS / 16 - 1) {
-            fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(acc_empty + ab);
-          }
-          if (row_ok) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-              if (cb + 16 * q + c < cend) crow[16 * q + c] = f.sub(cv[c], red.residue(a, c));
-          }
-#pragma unroll
-          for (int c = 0; c < 4; ++c) cv[c] = nv[c];
         }
       }
     }
@@ -1079,17 +1048,18 @@ void update_t(const F& f, uint64_t* m, int64_t ld, int rbeg, int rend, int jend,
   S.nsub = (cend - jend + SH::NS - 1) / SH::NS;
   const int64_t total = (int64_t)S.mtiles * S.nsub;
   const int grid = total < max_ctas ? (int)total : max_ctas;  // one CTA per SM: it owns all 512 TMEM columns
-  constexpr int smem = std::is_same<F, FpM61>::value ? SH::SMEM_M61 : SH::SMEM;
+  constexpr bool grouped = !std::is_same<F, FpBarrett>::value;
+  constexpr int smem = grouped ? SH::SMEM_TMA : SH::SMEM;
   static bool attr = false;
   if (!attr) {
     cudaFuncSetAttribute(trailing_tc_kernel<F, LIMBS, KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     attr = true;
   }
-  // C through TMA (p = 2^61 - 1): 16-byte aligned rows and column offset.
+  // C through TMA (the grouped epilogue): 16-byte aligned rows and column offset.
   CUtensorMap cmap;
   std::memset(&cmap, 0, sizeof cmap);
   int use_tma = 0;
-  if (std::is_same<F, FpM61>::value && !lo.c_zero && (ld & 1) == 0 && ((uintptr_t)m & 15) == 0 && (jend & 1) == 0)
+  if (grouped && !lo.c_zero && (ld & 1) == 0 && ((uintptr_t)m & 15) == 0 && (jend & 1) == 0)
     use_tma = make_c_map(&cmap, m, ld, rend, cend) ? 1 : 0;
   launch_k(trailing_tc_kernel<F, LIMBS, KK>, dim3(grid), dim3(kThreads), smem, st, 1, f, Aw, Bw, m, ld,
            (int32_t)rbeg, (int32_t)rend, (int32_t)jend, (int32_t)cend, S, r64, err, cmap, use_tma, g, lo);
