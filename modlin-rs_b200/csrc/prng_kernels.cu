@@ -30,8 +30,10 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "field.cuh"
+#include "mma_limbs.cuh"
 #include "prng_kernels.cuh"
 
 namespace modlin {
@@ -68,40 +70,64 @@ struct RedSmall {
 };
 
 // ---- C = A * B mod 2^61 - 1 ------------------------------------------------
-constexpr int kGT = 32;  // output tile kGT x kGT, 256 threads, 4 outputs each
+// 64 x 32 output tiles, K in chunks of 64 as 8-bit limb products on the tensor
+// cores (mma_limbs.cuh), each chunk's diagonals folded into one 64-bit sum. A
+// state doubling of MIXMAX-256 (2048 x 256 x 256) takes 35 us (330 with
+// 128-bit sums on the integer pipes).
+constexpr int kGM = 64, kGN = 32, kGK = 64, kGStride = 80;
+constexpr int kGemmSmem = 8 * (kGM + kGN) * kGStride;
 
 __global__ void __launch_bounds__(256) m61_gemm_kernel(const uint64_t* __restrict__ A, const uint64_t* __restrict__ B,
                                                        uint64_t* __restrict__ C, int M, int K, int N) {
-  __shared__ uint64_t As[kGT][kGT + 1], Bs[kGT][kGT + 1];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // ty 0..7
-  const int r0 = blockIdx.y * kGT, c0 = blockIdx.x * kGT;
-  u128 acc[4] = {0, 0, 0, 0};
-  for (int k0 = 0; k0 < K; k0 += kGT) {
+  extern __shared__ __align__(16) uint8_t gsm[];
+  uint8_t *pa = gsm, *pb = gsm + 8 * kGM * kGStride;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int r0 = blockIdx.y * kGM, c0 = blockIdx.x * kGN;
+  const int rg = warp & 3, cg0 = 2 * (warp >> 2);  // this warp's 16 rows and two groups of 8 columns
+  uint64_t sum[2][4] = {};
+  for (int k0 = 0; k0 < K; k0 += kGK) {
+    uint64_t va[4][4], vb[2][4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int r = ty + 8 * q;
-      As[r][tx] = (r0 + r < M && k0 + tx < K) ? A[(int64_t)(r0 + r) * K + k0 + tx] : 0;
-      Bs[r][tx] = (k0 + r < K && c0 + tx < N) ? B[(int64_t)(k0 + r) * N + c0 + tx] : 0;
-    }
+    for (int w = 0; w < 4; ++w)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int r = r0 + (tid >> 4) + 16 * w, k = k0 + 4 * (tid & 15) + u;
+        va[w][u] = r < M && k < K ? A[(int64_t)r * K + k] : 0;
+      }
+#pragma unroll
+    for (int w = 0; w < 2; ++w)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int c = c0 + lane, k = k0 + 4 * (warp + 8 * w) + u;
+        vb[w][u] = c < N && k < K ? B[(int64_t)k * N + c] : 0;
+      }
+    __syncthreads();  // the previous chunk's planes have been read
+#pragma unroll
+    for (int w = 0; w < 4; ++w)
+      mml::put_planes4<8>(pa + ((tid >> 4) + 16 * w) * kGStride + 4 * (tid & 15), kGM * kGStride, va[w]);
+#pragma unroll
+    for (int w = 0; w < 2; ++w)
+      mml::put_planes4<8>(pb + lane * kGStride + 4 * (warp + 8 * w), kGN * kGStride, vb[w]);
     __syncthreads();
-#pragma unroll 8
-    for (int kk = 0; kk < kGT; ++kk) {
-      const uint64_t b = Bs[kk][tx];
+    if (r0 + 16 * rg < M) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const u128 t = (u128)As[ty + 8 * q][kk] * b;  // < 2^122
-        const uint64_t lo = (uint64_t)t, hi = (uint64_t)(t >> 64);
-        acc[q] += (lo & kP) + ((lo >> 61) | (hi << 3));  // < 2^62 each, K of them < 2^126
+      for (int q = 0; q < 2; ++q) {
+        uint32_t acc[15][4];
+        mml::tile_k32<8, 2, kGStride>(acc, mml::saddr(pa) + 16 * rg * kGStride, kGM * kGStride,
+                                      mml::saddr(pb) + 8 * (cg0 + q) * kGStride, kGN * kGStride);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sum[q][e] = fold61(sum[q][e] + m61_fold15(acc, e));  // < 2^61 + 8
       }
     }
-    __syncthreads();
   }
-  const FpM61 f;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int r = r0 + ty + 8 * q;
-    if (r < M && c0 + tx < N) C[(int64_t)r * N + c0 + tx] = f.reduce(acc[q]);
-  }
+  for (int q = 0; q < 2; ++q)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int r = r0 + 16 * rg + (lane >> 2) + 8 * (e >> 1), c = c0 + 8 * (cg0 + q) + 2 * (lane & 3) + (e & 1);
+      const uint64_t v = fold61(sum[q][e]);
+      if (r < M && c < N) C[(int64_t)r * N + c] = v >= kP ? v - kP : v;
+    }
 }
 
 // ---- MIXMAX ---------------------------------------------------------------------
@@ -135,9 +161,17 @@ __device__ __forceinline__ uint64_t warp_excl_scan(uint64_t v, int lane) {
 
 // ROOT's iteration, run by one thread on the state s[0] = sumtot,
 // s[1..N-1] = v[1..N-1] (src/prng.rs:191-222).
-template <int N>
-__device__ void mix_iterate_exact(uint64_t* s, uint64_t special) {
+struct MixLinear {
+  __device__ __forceinline__ int operator()(int e) const { return e; }
+};
+template <int N, class At = MixLinear>
+__device__ void mix_iterate_exact(uint64_t* st, uint64_t special, At at = At()) {
   using T = MixTraits<N>;
+  struct Ref {
+    uint64_t* st;
+    At at;
+    __device__ uint64_t& operator[](int e) const { return st[at(e)]; }
+  } s{st, at};
   const uint64_t temp2 = s[1];
   uint64_t tv = s[0], acc = tv, ovf = 0, tp = 0;
   for (int i = 1; i < N; ++i) {
@@ -271,10 +305,118 @@ __device__ __forceinline__ void mix_iterate(uint64_t (&x)[MixTraits<N>::E], uint
   v0 = sum_old;
 }
 
+// ---- MIXMAX-256: a block of three iterations in lazily reduced sums ---------
+// No special multiplier here, so an iteration is two running sums and the
+// correction of v[2] and sumtot. In 64 bits there is room for sums of four
+// residues, and a third word takes the rest, so entries are reduced once per
+// iteration and running sums not at all. Only the third iteration's entries
+// are output: what ROOT leaves for a residue other than 0 does not depend on
+// the representation of its inputs (a folded sum lies in [0, p]), so the only
+// blocks to be run as ROOT runs them are those with an output entry, or a
+// sumtot, that is 0 mod p. Integer ALU bound: 2^28 outputs in 1715 us (3017
+// with every sum reduced and checked), 82 % of the ALU pipe.
+struct U96 {  // w2 2^64 + w1 2^32 + w0
+  uint32_t w0, w1, w2;
+  __device__ __forceinline__ void add(uint64_t v) {
+    asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, 0;"
+        : "+r"(w0), "+r"(w1), "+r"(w2)
+        : "r"((uint32_t)v), "r"((uint32_t)(v >> 32)));
+  }
+  __device__ __forceinline__ void add(const U96& v) {
+    asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
+        : "+r"(w0), "+r"(w1), "+r"(w2)
+        : "r"(v.w0), "r"(v.w1), "r"(v.w2));
+  }
+  // Congruent mod p and below 2^61 + 8 (w2 + 1).
+  __device__ __forceinline__ uint64_t fold() const {
+    return ((uint64_t)(w1 & 0x1fffffffu) << 32 | w0) + __funnelshift_l(w1, w2, 3);
+  }
+};
+__device__ __forceinline__ U96 u96(uint64_t v) { return U96{(uint32_t)v, (uint32_t)(v >> 32), 0}; }
+// y < 2^62: the canonical residue.
+__device__ __forceinline__ uint64_t canon(uint64_t y) { return (y + ((y + 1) >> 61)) & kP; }
+
+// Exclusive sum across the warp of values below 2^61 + 2^8, congruent mod p
+// and below 2^61 + 8.
+__device__ __forceinline__ uint64_t lazy_excl_scan(uint64_t v, int lane) {
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint64_t y = __shfl_up_sync(kFull, v, off);
+    if (lane >= off) v += y;
+    if (off == 2 || off == 8) v = fold61(v);  // sums of four so far, below 2^63 + 2^10
+  }
+  const uint64_t ex = __shfl_up_sync(kFull, v, 1);
+  return lane ? fold61(ex) : 0;
+}
+
+// One iteration on x (entry lane * 8 + k, below 2^61 + 2^8); kLast: canonical
+// results. zero: an entry or sumtot may be 0 mod p (sumtot in every iteration).
+template <bool kLast>
+__device__ __forceinline__ void mix256_iterate(uint64_t (&x)[8], uint64_t& v0, int lane, bool& zero) {
+  const uint64_t sum_old = __shfl_sync(kFull, x[0], 0);
+  const uint64_t temp2 = __shfl_sync(kFull, x[1], 0);
+  if (lane == 0) x[0] = 0;  // entry 0 is sumtot, not part of tp
+  // Lane totals: tp of the last entry, and the sum of the tp.
+  U96 tp = u96(x[0]), T = tp;
+#pragma unroll
+  for (int k = 1; k < 8; ++k) {
+    tp.add(x[k]);
+    T.add(tp);
+  }
+  const uint64_t ex1 = lazy_excl_scan(tp.fold(), lane);
+  if (lane == 0) T.add(sum_old);
+  T.add(ex1 << 2);  // 8 ex1 in two parts below 2^64
+  T.add(ex1 << 2);
+  const uint64_t ex2 = lazy_excl_scan(T.fold(), lane);
+  // tv: running sum of ex1 + tp from ex2.
+  U96 t = u96(ex1), r = u96(ex2);
+  uint64_t sum = 0;
+  U96 wide = u96(0);
+  uint32_t low = 0xffffffffu;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    t.add(x[k]);
+    r.add(t);
+    if (k == 0 && lane == 0) r.add(sum_old);
+    uint64_t y = r.fold();
+    if (k == 2 && lane == 0) y = fold61(y + 4 * kP - temp2);  // special = -1: v[2] -= the old v[1]
+    if (kLast) {
+      y = canon(y);
+      if (k > 0 || lane > 0) low = min(low, (uint32_t)y);
+      sum += y;  // 8 (p - 1) < 2^64
+    } else {
+      wide.add(y);
+    }
+    x[k] = y;
+  }
+  uint64_t tot = kLast ? fold61(sum) : wide.fold();
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    tot += __shfl_xor_sync(kFull, tot, off);
+    if (off == 2 || off == 8) tot = fold61(tot);
+  }
+  tot = canon(fold61(tot));
+  zero |= tot == 0 || (kLast && low == 0);  // low words: 2^-32 a false alarm
+  if (lane == 0) x[0] = tot;
+  v0 = sum_old;
+}
+
+// Entry e of a warp's state in shared memory: the 8 entries of a lane rotate
+// with it, so that lanes writing their k-th entries meet in few banks.
+struct MixSwizzle {
+  __device__ __forceinline__ int operator()(int e) const { return (e & ~7) | ((e ^ (e >> 3)) & 7); }
+};
+
+// The segment loop. kFast (MIXMAX-256): blocks by mix256_iterate, s holding
+// the state at the block's start for the exact run.
 template <int N, class R>
 __global__ void __launch_bounds__(kMixWarps * 32) mixmax_fill_kernel(MixFill a, R red) {
   using T = MixTraits<N>;
   constexpr int E = T::E;
+  constexpr bool kFast = N == 256;
+  static_assert(!kFast || (T::SM == 0 && T::SK == 1 && E == 8), "mix256_iterate");
+  using At = typename std::conditional<kFast, MixSwizzle, MixLinear>::type;
+  const At at;
   __shared__ uint64_t sh[kMixWarps][N];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t seg = a.seg_begin + (int64_t)blockIdx.x * kMixWarps + w;
@@ -282,32 +424,55 @@ __global__ void __launch_bounds__(kMixWarps * 32) mixmax_fill_kernel(MixFill a, 
   uint64_t* s = sh[w];
   uint64_t x[E];
   const uint64_t* st = a.starts + seg * N;
+  const auto put = [&]() {
+#pragma unroll
+    for (int k = 0; k < E; ++k)
+      if (lane * E + k < N) s[at(lane * E + k)] = x[k];
+    __syncwarp();
+  };
 #pragma unroll
   for (int k = 0; k < E; ++k) x[k] = lane * E + k < N ? st[lane * E + k] : 0;
   uint64_t v0 = 0;
+  if (kFast || (seg == 0 && a.h0 > 0)) put();
   if (seg == 0 && a.h0 > 0) {  // the rest of the starting block
-#pragma unroll
-    for (int k = 0; k < E; ++k)
-      if (lane * E + k < N) s[lane * E + k] = x[k];
-    __syncwarp();
-    for (int64_t j = lane; j < a.h0; j += 32) a.out[j] = red(s[a.c0 + j] << 3);
+    for (int64_t j = lane; j < a.h0; j += 32) a.out[j] = red(s[at((int)(a.c0 + j))] << 3);
     __syncwarp();
   }
   const int64_t b0 = seg * a.G + 1, b1 = (seg + 1) * a.G < a.nbk ? (seg + 1) * a.G : a.nbk;
   for (int64_t b = b0; b <= b1; ++b) {
+    if constexpr (kFast) {
+      bool zero = false;
 #pragma unroll 1
-    for (int it = 0; it <= T::SKIP; ++it) mix_iterate<N>(x, v0, s, lane, a.special);
+      for (int it = 0; it < T::SKIP; ++it) mix256_iterate<false>(x, v0, lane, zero);
+      mix256_iterate<true>(x, v0, lane, zero);
+      if (__any_sync(kFull, zero)) {
+        uint64_t v = 0;
+        if (lane == 0)
+          for (int it = 0; it <= T::SKIP; ++it) {
+            v = s[at(0)];
+            mix_iterate_exact<N>(s, a.special, at);
+          }
+        v0 = __shfl_sync(kFull, v, 0);
+        __syncwarp();
 #pragma unroll
-    for (int k = 0; k < E; ++k)
-      if (lane * E + k < N) s[lane * E + k] = x[k];
-    __syncwarp();
+        for (int k = 0; k < E; ++k) x[k] = s[at(lane * E + k)];
+        __syncwarp();
+      }
+    } else {
+#pragma unroll 1
+      for (int it = 0; it <= T::SKIP; ++it) mix_iterate<N>(x, v0, s, lane, a.special);
+    }
+    put();
     const int64_t base = a.h0 + (b - 1) * (N - 1) - 1;  // output index of v[e] is base + e
     if (base + N <= a.count) {
-      for (int e = lane; e < N; e += 32)
-        if (e >= 1) a.out[base + e] = red(s[e] << 3);
+#pragma unroll
+      for (int e0 = 0; e0 < N; e0 += 32) {
+        const int e = e0 + lane;
+        if (e >= 1 && e < N) a.out[base + e] = red(s[at(e)] << 3);
+      }
     } else {
       for (int e = lane; e < N; e += 32)
-        if (e >= 1 && base + e < a.count) a.out[base + e] = red(s[e] << 3);
+        if (e >= 1 && base + e < a.count) a.out[base + e] = red(s[at(e)] << 3);
     }
     __syncwarp();
   }
@@ -474,8 +639,11 @@ cudaError_t launch_xoro(const XoroFill& a, R red, cudaStream_t st) {
 
 cudaError_t m61_gemm(const uint64_t* A, const uint64_t* B, uint64_t* C, int M, int K, int N, cudaStream_t st) {
   if (M <= 0 || N <= 0 || K <= 0) return cudaSuccess;
-  const dim3 grid((N + kGT - 1) / kGT, (M + kGT - 1) / kGT);
-  m61_gemm_kernel<<<grid, 256, 0, st>>>(A, B, C, M, K, N);
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(m61_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
+  if (attr != cudaSuccess) return attr;
+  const dim3 grid((N + kGN - 1) / kGN, (M + kGM - 1) / kGM);
+  m61_gemm_kernel<<<grid, 256, kGemmSmem, st>>>(A, B, C, M, K, N);
   return cudaGetLastError();
 }
 
@@ -605,17 +773,22 @@ int mix_fill(PrngCache& c, int num_sms, modlin_prng_impl::MixMax& m, uint64_t p,
   const int64_t rest = (int64_t)count - h0;
   const int64_t nbk = rest > 0 ? (rest + N - 2) / (N - 1) : 0;
   int64_t S = 1, G = 1;
+  int bits = 0;
   if (nbk > 0) {
+    // Segments of 2^bits blocks, so that every jump between them is a cached
+    // power: the longest that leave three quarters of the resident warps busy
+    // (the kernel is bound by the ALUs, not by the warps in flight).
     const int64_t R = mixmax_resident_warps(N, num_sms);
-    G = (nbk + std::min<int64_t>(nbk, R) - 1) / std::min<int64_t>(nbk, R);
+    while (bits < 40 && ((nbk + ((int64_t)2 << bits) - 1) >> (bits + 1)) >= R * 3 / 4) ++bits;
+    G = (int64_t)1 << bits;
     S = (nbk + G - 1) / G;
   }
-  // workspace: starts S x N | ends S x (N+1) | 3 matrices | flags S + 1 ints
-  const size_t o_ends = (size_t)S * N, o_mat = o_ends + (size_t)S * (N + 1), o_flags = o_mat + 3 * mat;
+  // workspace: starts S x N | ends S x (N+1) | flags S + 1 ints
+  const size_t o_ends = (size_t)S * N, o_flags = o_ends + (size_t)S * (N + 1);
   int rc = ensure_ws(c, (o_flags + 1) * sizeof(uint64_t) + (size_t)(S + 1) * sizeof(int));
   if (rc) return rc;
   uint64_t* ws = static_cast<uint64_t*>(c.ws);
-  uint64_t *starts = ws, *ends = ws + o_ends, *J = ws + o_mat, *Jt = J + mat, *Jn = Jt + mat;
+  uint64_t *starts = ws, *ends = ws + o_ends;
   int* flags = reinterpret_cast<int*>(ws + o_flags);
   int* any = flags + S;
 
@@ -624,38 +797,20 @@ int mix_fill(PrngCache& c, int num_sms, modlin_prng_impl::MixMax& m, uint64_t p,
   x0[0] = m.sumtot;
   for (int i = 1; i < N; ++i) x0[i] = m.v[i];
   if (S > 1) {
-    int bits = 0;
-    while ((G >> bits) > 1) ++bits;  // floor(log2 G)
-    rc = ensure_pows(c, m, bits, st, launches);
+    int top = bits;
+    while (((int64_t)1 << (top - bits + 1)) < S) ++top;  // B^(2^bits) .. B^(2^top)
+    rc = ensure_pows(c, m, top, st, launches);
     if (rc) return rc;
-    // J = B^G from the cached powers (they commute).
-    bool first = true;
-    for (int k = 0; k <= bits; ++k) {
-      if (!((G >> k) & 1)) continue;
-      const uint64_t* P = c.pow[kind_slot(N)] + (size_t)k * mat;
-      if (first) {
-        PCK(cudaMemcpyAsync(J, P, mat * sizeof(uint64_t), cudaMemcpyDeviceToDevice, st));
-        first = false;
-      } else {
-        PCK(m61_gemm(J, P, Jn, N, N, N, st));
-        ++*launches;
-        std::swap(J, Jn);
-      }
-    }
     std::vector<uint64_t> xc(x0);
     for (auto& v : xc) v %= kM61;
     PCK(cudaMemcpyAsync(starts, xc.data(), N * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
     // Doubling: states [have, 2 have) = states [0, have) * B^(G have).
-    for (int64_t have = 1; have < S;) {
+    int k = bits;
+    for (int64_t have = 1; have < S; ++k) {
       const int64_t w = std::min(have, S - have);
-      PCK(m61_gemm(starts, J, starts + (size_t)have * N, (int)w, N, N, st));
+      PCK(m61_gemm(starts, c.pow[kind_slot(N)] + (size_t)k * mat, starts + (size_t)have * N, (int)w, N, N, st));
       ++*launches;
       have += w;
-      if (have < S) {
-        PCK(m61_gemm(J, J, Jt, N, N, N, st));
-        ++*launches;
-        std::swap(J, Jt);
-      }
     }
   }
   PCK(cudaMemcpyAsync(starts, x0.data(), N * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
