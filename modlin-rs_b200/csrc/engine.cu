@@ -62,7 +62,7 @@ struct DevBuf {
 // crossover, BM batch threads by the longest sequence.
 struct Tune {
   bool measured = false;
-  int tc_cross[4] = {512, 512, 512, 512};           // 1, 2, 4, 8 limbs
+  int tc_cross[4] = {64, 64, 64, 64};               // 1, 2, 4, 8 limbs
   int two_panel_min = 256;
   int bm_threads[4] = {256, 512, 512, 512};         // n < 1024, < 4096, < 16384, longer
   int bm_long_min = 1024;                           // one CTA below, many from here on

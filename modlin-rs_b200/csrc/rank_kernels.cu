@@ -20,12 +20,17 @@ namespace modlin {
 // alpha and its coefficients g against this round's new pivots, so that a
 // pivot row k satisfies  U_k = alpha_k * row_k - sum_{k2<k} G[k][k2] * U_k2.
 // ---------------------------------------------------------------------------
+// Issue-bound: 64 x 64 entries, two products and one reduction each, for every
+// pivot (ElimField::comb; 41 us over 2^61 - 1, 98 with two reduced products
+// per entry).
 template <class F>
 __global__ void __launch_bounds__(kWindowThreads) window_kernel(F f, const uint64_t* __restrict__ m, int64_t ld,
                                                                  int32_t n, int32_t r0, int32_t col, int32_t W,
                                                                  int32_t round, PanelState* ps, uint64_t* Upanel,
                                                                  uint64_t* G, const uint64_t* Lbuf,
                                                                  uint8_t* is_pivot) {
+  using W64 = typename ElimField<F>::W;
+  const ElimField<F> ef(f);
   extern __shared__ __align__(16) uint64_t smem_w[];
   uint64_t(*A)[kPanel] = reinterpret_cast<uint64_t(*)[kPanel]>(smem_w);                  // [64][64]
   uint64_t(*Gc)[kPanel] = reinterpret_cast<uint64_t(*)[kPanel]>(smem_w + kWindow * kPanel);  // [64][64]
@@ -48,7 +53,7 @@ __global__ void __launch_bounds__(kWindowThreads) window_kernel(F f, const uint6
   if (tid < kWindow) {
     rowidx[tid] = tid < nc ? (round == 0 ? r0 + tid : ps->cand[tid]) : -1;
     ispiv[tid] = 0;
-    alph[tid] = 1;
+    alph[tid] = ef.in(1);
   }
   for (int idx = tid; idx < kWindow * kPanel; idx += blockDim.x) {
     (&Gc[0][0])[idx] = 0;
@@ -57,7 +62,7 @@ __global__ void __launch_bounds__(kWindowThreads) window_kernel(F f, const uint6
   __syncthreads();
   for (int idx = tid; idx < nc * W; idx += blockDim.x) {
     const int i = idx / W, c = idx - (idx / W) * W;
-    A[i][c] = m[(int64_t)rowidx[i] * ld + col + c];
+    A[i][c] = ef.in(m[(int64_t)rowidx[i] * ld + col + c]);
   }
   __syncthreads();
 
@@ -67,7 +72,7 @@ __global__ void __launch_bounds__(kWindowThreads) window_kernel(F f, const uint6
   for (int c = 0; c < W; ++c) {
     if ((mask0 >> c) & 1ULL) continue;
     if (tid < kWindow) {
-      const bool nz = tid < nc && !ispiv[tid] && A[tid][c] != 0;
+      const bool nz = tid < nc && !ispiv[tid] && !ef.zero(A[tid][c]);
       const uint32_t bal = __ballot_sync(0xffffffffu, nz);
       if ((tid & 31) == 0) ballots[nb & 1][tid >> 5] = bal;
     }
@@ -78,15 +83,16 @@ __global__ void __launch_bounds__(kWindowThreads) window_kernel(F f, const uint6
     if (piv < 0) continue;
     const int t = npiv++;
     newmask |= 1ULL << c;
-    const uint64_t e = A[piv][c];
-    uint64_t h = 0;
+    const W64 e = A[piv][c];
+    W64 h = 0;
     if (j < nc && j != piv && !ispiv[j]) h = A[j][c];
     __syncwarp();
-    if (h != 0) {
-      for (int cc = c + 1 + sub; cc < W; cc += 8) A[j][cc] = f.sub(f.mul(e, A[j][cc]), f.mul(h, A[piv][cc]));
-      for (int t2 = sub; t2 < t; t2 += 8) Gc[j][t2] = f.mul(e, Gc[j][t2]);
+    if (!ef.zero(h)) {
+      const W64 nh = ef.neg(h);
+      for (int cc = c + 1 + sub; cc < W; cc += 8) A[j][cc] = ef.comb(e, A[j][cc], nh, A[piv][cc]);
+      for (int t2 = sub; t2 < t; t2 += 8) Gc[j][t2] = ef.comb(e, Gc[j][t2], ef.neg(0), 0);
       if (sub == 0) {
-        alph[j] = f.mul(e, alph[j]);
+        alph[j] = ef.comb(e, alph[j], ef.neg(0), 0);
         Gc[j][t] = h;
         A[j][c] = 0;
       }
@@ -105,21 +111,22 @@ __global__ void __launch_bounds__(kWindowThreads) window_kernel(F f, const uint6
     const int k = pb_old + t, i = pivcand[t];
     ps->prow[k] = rowidx[i];
     ps->pcol[k] = col + pivc[t];
-    ps->alpha[k] = alph[i];
-    ps->inv[k] = fp_inv(f, A[i][pivc[t]]);
+    ps->alpha[k] = ef.out(alph[i]);
+    const uint64_t pv = ef.out(A[i][pivc[t]]);
+    ps->inv[k] = std::is_same<F, FpM61>::value ? fp_inv_m61(pv) : fp_inv(f, pv);
     is_pivot[rowidx[i]] = 1;
   }
   for (int idx = tid; idx < npiv * kPanel; idx += blockDim.x) {
     const int t = idx / kPanel, cc = idx % kPanel;
-    Upanel[(int64_t)(pb_old + t) * kPanel + cc] = cc < W ? A[pivcand[t]][cc] : 0;
+    Upanel[(int64_t)(pb_old + t) * kPanel + cc] = cc < W ? ef.out(A[pivcand[t]][cc]) : 0;
   }
   for (int idx = tid; idx < npiv * kPanel; idx += blockDim.x) {
     const int t = idx / kPanel, k2 = idx % kPanel, k = pb_old + t, i = pivcand[t];
     uint64_t v = 0;
     if (k2 < pb_old)
-      v = f.mul(alph[i], Lbuf[(int64_t)(rowidx[i] - r0) * kPanel + k2]);
+      v = f.mul(ef.out(alph[i]), Lbuf[(int64_t)(rowidx[i] - r0) * kPanel + k2]);
     else if (k2 < k)
-      v = Gc[i][k2 - pb_old];
+      v = ef.out(Gc[i][k2 - pb_old]);
     G[(int64_t)k * kPanel + k2] = v;
   }
   if (tid == 0) {
@@ -135,47 +142,62 @@ __global__ void __launch_bounds__(kWindowThreads) window_kernel(F f, const uint6
 // (f = e * inv, row -= f * U_k; src/fp.rs:163-175), multipliers to Lbuf,
 // residual written back and, if nonzero, the row offered as a candidate.
 // ---------------------------------------------------------------------------
+// The pivot rows are normalised when they are loaded (U_k * inv_k), so a row's
+// dependent chain is one shuffle and one multiply-add per pivot; the
+// multipliers are formed afterwards (6 us for 436 rows and 64 pivots over
+// 2^61 - 1, 24 with the multiplier on the chain).
 template <class F>
 __global__ void __launch_bounds__(256) bulk_kernel(F f, uint64_t* __restrict__ m, int64_t ld, int32_t n, int32_t r0,
                                                     int32_t col, int32_t W, int32_t pb_lo, PanelState* ps,
                                                     const uint64_t* __restrict__ Upanel, uint64_t* Lbuf,
                                                     const uint8_t* __restrict__ is_pivot) {
-  __shared__ uint64_t Us[kPanel][kPanel];
+  using W64 = typename ElimField<F>::W;
+  const ElimField<F> ef(f);
+  __shared__ W64 Us[kPanel][kPanel];
   __shared__ uint64_t invs[kPanel];
   __shared__ int32_t pcs[kPanel];
   const int pb_hi = ps->pb;
   const int nk = pb_hi - pb_lo;
-  for (int idx = threadIdx.x; idx < nk * kPanel; idx += blockDim.x) {
-    const int t = idx / kPanel, c = idx % kPanel;
-    Us[t][c] = c < W ? Upanel[(int64_t)(pb_lo + t) * kPanel + c] : 0;
-  }
   for (int t = threadIdx.x; t < nk; t += blockDim.x) {
     invs[t] = ps->inv[pb_lo + t];
     pcs[t] = ps->pcol[pb_lo + t] - col;
   }
   __syncthreads();
+  for (int idx = threadIdx.x; idx < nk * kPanel; idx += blockDim.x) {
+    const int t = idx / kPanel, c = idx % kPanel;
+    Us[t][c] = ef.in(c < W ? f.mul(Upanel[(int64_t)(pb_lo + t) * kPanel + c], invs[t]) : 0);
+  }
+  __syncthreads();
   const int lane = threadIdx.x & 31;
   const int warps_total = gridDim.x * (blockDim.x >> 5);
+  const W64 one = ef.in(1);
   for (int r = r0 + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < n; r += warps_total) {
     if (is_pivot[r]) continue;
     uint64_t* row = m + (int64_t)r * ld + col;
-    uint64_t x0 = lane < W ? row[lane] : 0;
-    uint64_t x1 = lane + 32 < W ? row[lane + 32] : 0;
+    W64 x0 = ef.in(lane < W ? row[lane] : 0);
+    W64 x1 = ef.in(lane + 32 < W ? row[lane + 32] : 0);
+    W64 e0 = 0, e1 = 0;  // entries eliminated by pivots lane and lane + 32
     for (int t = 0; t < nk; ++t) {
       const int pc = pcs[t];
-      const uint64_t e = __shfl_sync(0xffffffffu, pc < 32 ? x0 : x1, pc & 31);
-      const uint64_t fm = e ? f.mul(e, invs[t]) : 0;
-      if (lane == 0) Lbuf[(int64_t)(r - r0) * kPanel + pb_lo + t] = fm;
-      if (fm) {
-        if (lane < W) x0 = f.sub(x0, f.mul(fm, Us[t][lane]));
-        if (lane + 32 < W) x1 = f.sub(x1, f.mul(fm, Us[t][lane + 32]));
+      const W64 e = __shfl_sync(0xffffffffu, pc < 32 ? x0 : x1, pc & 31);
+      if (t < 32) {
+        if (lane == t) e0 = e;
+      } else if (lane == t - 32) {
+        e1 = e;
       }
+      const W64 ne = ef.neg(e);
+      x0 = ef.comb(one, x0, ne, Us[t][lane]);
+      x1 = ef.comb(one, x1, ne, Us[t][lane + 32]);
     }
+    uint64_t* L = Lbuf + (int64_t)(r - r0) * kPanel + pb_lo;
+    if (lane < nk) L[lane] = f.mul(ef.out(e0), invs[lane]);
+    if (lane + 32 < nk) L[lane + 32] = f.mul(ef.out(e1), invs[lane + 32]);
+    const uint64_t y0 = ef.out(x0), y1 = ef.out(x1);
     if (nk > 0) {
-      if (lane < W) row[lane] = x0;
-      if (lane + 32 < W) row[lane + 32] = x1;
+      if (lane < W) row[lane] = y0;
+      if (lane + 32 < W) row[lane + 32] = y1;
     }
-    const bool nz = __any_sync(0xffffffffu, (x0 | x1) != 0);
+    const bool nz = __any_sync(0xffffffffu, (y0 | y1) != 0);
     if (nz && lane == 0) {
       const int s = atomicAdd(&ps->ncand, 1);
       if (s < kWindow) ps->cand[s] = r;
@@ -186,45 +208,51 @@ __global__ void __launch_bounds__(256) bulk_kernel(F f, uint64_t* __restrict__ m
 // ---------------------------------------------------------------------------
 // couple_kernel — U block (src/fp.rs:184-200): for every trailing column c,
 // U_k[c] = alpha_k * row_{prow_k}[c] - sum_{k2<k} G[k][k2] * U_k2[c],
-// sequential in k, a thread per column; the column's coupled values stay in
-// registers (fully unrolled triangular loop), u128 lazy accumulation.
+// sequential in k. Eight threads share a column's sum (a CTA takes 32
+// columns), lazy accumulation and a shuffle reduction per k: the chain of 64
+// steps of up to 8 products each binds it (11 us for 436 columns over
+// 2^61 - 1, 118 with a thread per column).
 // ---------------------------------------------------------------------------
+constexpr int kCoupleCols = 32, kCoupleSplit = 8;
 template <class F>
-__global__ void __launch_bounds__(128) couple_kernel(F f, const uint64_t* __restrict__ m, int64_t ld, int32_t n,
+__global__ void __launch_bounds__(256) couple_kernel(F f, const uint64_t* __restrict__ m, int64_t ld, int32_t n,
                                                       int32_t jend, const PanelState* __restrict__ ps,
                                                       const uint64_t* __restrict__ G, uint64_t* Ubuf, int64_t ldU) {
   extern __shared__ __align__(16) uint64_t smem_c[];
-  uint64_t(*Us)[128] = reinterpret_cast<uint64_t(*)[128]>(smem_c);            // [64][128]: my column's U_k
-  uint64_t(*Gs)[kPanel] = reinterpret_cast<uint64_t(*)[kPanel]>(smem_c + kPanel * 128);  // [64][64]
-  __shared__ uint64_t al[kPanel];
-  __shared__ int32_t prs[kPanel];
+  uint64_t(*Us)[kCoupleCols] = reinterpret_cast<uint64_t(*)[kCoupleCols]>(smem_c);  // alpha_k row_k, then U_k
+  uint64_t(*Gs)[kPanel] = reinterpret_cast<uint64_t(*)[kPanel]>(smem_c + kPanel * kCoupleCols);
   const int pb = ps->pb;
+  const int64_t c0 = (int64_t)jend + (int64_t)blockIdx.x * kCoupleCols;
   for (int idx = threadIdx.x; idx < pb * kPanel; idx += blockDim.x) Gs[idx / kPanel][idx % kPanel] = G[idx];
-  for (int k = threadIdx.x; k < pb; k += blockDim.x) {
-    al[k] = ps->alpha[k];
-    prs[k] = ps->prow[k];
+  for (int idx = threadIdx.x; idx < pb * kCoupleCols; idx += blockDim.x) {
+    const int k = idx / kCoupleCols;
+    const int64_t c = c0 + idx % kCoupleCols;
+    Us[k][idx % kCoupleCols] = c < n ? f.mul(ps->alpha[k], m[(int64_t)ps->prow[k] * ld + c]) : 0;
   }
   __syncthreads();
-  const int t = threadIdx.x;
-  const int64_t c = (int64_t)jend + (int64_t)blockIdx.x * blockDim.x + t;
-  const bool valid = c < n;
+  // A column's threads are neighbours in a warp.
+  const int t = threadIdx.x / kCoupleSplit, q = threadIdx.x % kCoupleSplit;
   const uint64_t sb = f.safe_batch();
-  for (int k = 0; k < pb; ++k) {
-    const uint64_t v = valid ? f.mul(al[k], m[(int64_t)prs[k] * ld + c]) : 0;
+  for (int k = 1; k < pb; ++k) {
     u128 acc = 0;
-    uint64_t tot = 0, cnt = 0;
-#pragma unroll 8
-    for (int k2 = 0; k2 < k; ++k2) {
+    uint64_t cnt = 0;
+    for (int k2 = q; k2 < k; k2 += kCoupleSplit) {  // at most 8 products
       acc += f.prod(Gs[k][k2], Us[k2][t]);
       if (++cnt == sb) {
-        tot = f.add(tot, f.reduce(acc));
-        acc = 0;
-        cnt = 0;
+        acc = f.reduce(acc);  // counts as one product
+        cnt = 1;
       }
     }
-    const uint64_t u = f.sub(v, f.add(tot, f.reduce(acc)));
-    Us[k][t] = u;
-    if (valid) Ubuf[(int64_t)k * ldU + c] = u;
+    uint64_t part = f.reduce(acc);
+#pragma unroll
+    for (int o = 1; o < kCoupleSplit; o <<= 1) part = f.add(part, __shfl_xor_sync(0xffffffffu, part, o));
+    if (q == 0) Us[k][t] = f.sub(Us[k][t], part);
+    __syncwarp();
+  }
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < pb * kCoupleCols; idx += blockDim.x) {
+    const int64_t c = c0 + idx % kCoupleCols;
+    if (c < n) Ubuf[(int64_t)(idx / kCoupleCols) * ldU + c] = Us[idx / kCoupleCols][idx % kCoupleCols];
   }
 }
 
@@ -704,13 +732,13 @@ template <class F>
 void launch_couple(const F& f, const uint64_t* m, int64_t ld, int n, int jend, const PanelState* ps,
                    const uint64_t* G, uint64_t* Ubuf, int64_t ldU, cudaStream_t st) {
   const int cols = n - jend;
-  const size_t smem = (size_t)(kPanel * 128 + kPanel * kPanel) * sizeof(uint64_t);
+  const size_t smem = (size_t)(kPanel * kCoupleCols + kPanel * kPanel) * sizeof(uint64_t);
   static bool attr_set = false;
   if (!attr_set) {
     cudaFuncSetAttribute(couple_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     attr_set = true;
   }
-  couple_kernel<F><<<(cols + 127) / 128, 128, smem, st>>>(f, m, ld, n, jend, ps, G, Ubuf, ldU);
+  couple_kernel<F><<<(cols + kCoupleCols - 1) / kCoupleCols, 256, smem, st>>>(f, m, ld, n, jend, ps, G, Ubuf, ldU);
 }
 
 void launch_moves(uint64_t* m, int64_t ld, int n, int jend, const int2* moves, int nmoves, uint64_t* Lbuf, int r0,
