@@ -20,9 +20,9 @@
 // depends on the first 32 entries of A and B only, so one warp runs them on
 // that window (bm_base), collecting the 2 x 2 polynomial matrix
 //     A' = P A + Q B,  B' = U A + V B   (degree <= 32, about 16 as a rule)
-// which the other threads then apply to the rest of A and B (bm_tile): 2 x 2
-// products per entry and coefficient, about 2 per entry and step, summed
-// without reduction and reduced once per 32 steps.
+// which the other warps then apply to the rest of A and B (bm_apply): 2 x 2
+// products per entry and coefficient, about 2 per entry and step, as 8-bit limb
+// products on the tensor cores, reduced once per 32 steps.
 //
 // Kernels:
 //  * bm_block_kernel / bm_batch_kernel — one CTA per sequence, A and B in its
@@ -39,120 +39,61 @@
 
 #include "bm_kernels.cuh"
 #include "field.cuh"
+#include "mma_limbs.cuh"
 
 namespace modlin {
 
 namespace {
 
-constexpr int kBmK = 32;          // steps per block, window entries
+constexpr int kBmK = 32;             // steps per block, window entries
 constexpr int kCoefRows = kBmK + 1;  // offsets 0 .. 32
-constexpr int kBmPad = 2 * kBmK;  // entries past the end that a window may read
 constexpr unsigned kAll = 0xffffffffu;
 
 // ---------------------------------------------------------------------------
-// Field policies. R: a canonical residue. S: what the arrays and matrices
-// hold; pack(R). W: what bm_base works on; load(S), store(W) -> S.
-// comb = (bb a + nd b) / r mod p on W, nd = neg(d). Dot: a sum of up to
-// 2 * kCoefRows = 66 products of S, reduced once by value(), / r^2. r = 1, or
-// the Montgomery radix 2^32 or 2^64: a common factor of all of A (or of all of
-// B) changes no zero and so no complexity, and Montgomery's reduction is a
-// third of Barrett's dependent chain. A Dot that can overflow is folded every
-// kFold offsets (two products each), and after kFoldHigh of those again.
+// Field policies. W: what bm_base works on; load and store convert canonical
+// residues. comb = (bb a + nd b) / r mod p, nd = neg(d), with r = 1 or the
+// Montgomery radix 2^32 or 2^64: a common factor of all of A (or of all of B)
+// changes no zero and so no complexity, and Montgomery's reduction is a third
+// of Barrett's dependent chain. Red, L: the reductions of limb products
+// (limb_sums.cuh) and the limbs of a residue.
 // ---------------------------------------------------------------------------
-
-// p = 2^61 - 1. S and W are two 31-bit halves (M61Halves); S is balanced (|lo|
-// <= 2^30, |hi| <= 2^29 + 1), so that a Dot takes more products.
-struct BmM61 : M61Halves {
-  using S = uint64_t;
-  using R = uint64_t;
+// Values up to p + 6 on W: bb a + nd b < 2^122.1 + 2^123.1.
+struct BmM61 {
+  using F = FpM61;
+  using W = uint64_t;
+  static constexpr int L = 8;
   __device__ explicit BmM61(const FieldParams&) {}
-  __device__ __forceinline__ S pack(R x) const {
-    const int64_t y = (int64_t)x - (x >= (1ULL << 60) ? (int64_t)kM61 : 0);  // in [-2^60, 2^60]
-    const int32_t l = (int32_t)((uint32_t)y << 1) >> 1;
-    return words(l, (int32_t)((y - l) >> 31));
-  }
-  __device__ __forceinline__ W load(S x) const {
-    int64_t v = ((int64_t)hi(x) << 31) + lo(x);
-    if (v < 0) v += (int64_t)kM61;
-    return split((uint64_t)v);
-  }
-  __device__ __forceinline__ S store(W x) const { return pack(M61Halves::value(x)); }
-  __device__ __forceinline__ R add(R a, R b) const {
-    const uint64_t s = a + b;
-    return s >= kM61 ? s - kM61 : s;
-  }
-  // Three offsets: |ll| <= 6 * 2^60, |mid| <= 12 * 2^59 (1 + 2^-28), then fold
-  // moves ll's high part into mid and mid's into hh. Nine offsets: |hh| <=
-  // 18 * 2^58 + 2^61, then fold_high takes it mod p below 2^61 + 4.
-  struct Dot {
-    int64_t ll = 0, mid = 0, hh = 0;
-    __device__ __forceinline__ void mac(S a, S b) {
-      ll = mad(lo(a), lo(b), ll);
-      mid = mad(lo(a), hi(b), mid);
-      hh = mad(hi(a), hi(b), hh);
-      mid = mad(hi(a), lo(b), mid);
-    }
-  };
-  static constexpr int kFold = 3, kFoldHigh = 3;
-  __device__ __forceinline__ void fold_high(Dot& d) const { d.hh = (d.hh & (int64_t)kM61) + (d.hh >> 61); }
-  __device__ __forceinline__ void fold(Dot& d) const {
-    d.mid += d.ll >> 31;
-    d.ll &= 0x7fffffff;
-    d.hh += d.mid >> 31;
-    d.mid &= 0x7fffffff;
-  }
-  __device__ __forceinline__ R value(const Dot& d) const {
-    // As in comb; ll and mid are below 2^63 in absolute value, hh may use all
-    // 64 bits: 2 hh = 2 (hh mod 2^60) + (hh >> 60) mod p.
-    const uint64_t t0 = ((uint64_t)d.ll & kM61) + 8 + (uint64_t)(d.ll >> 61);
-    const uint64_t t1 = ((uint64_t)((uint32_t)d.mid & 0x3fffffffu) << 31) + (1ULL << 34) + (uint64_t)(d.mid >> 30);
-    const uint64_t t2 = (((uint64_t)d.hh & ((1ULL << 60) - 1)) << 1) + 16 + (uint64_t)(d.hh >> 60);
-    uint64_t x = t0 + t1 + t2;  // each below 2^61 + 2^35; too large by c
-    constexpr uint64_t c = 8 + (1ULL << 34) + 16;
-    x = (x & kM61) + (x >> 61) + (kM61 - c);
-    x = (x & kM61) + (x >> 61);
-    return x >= kM61 ? x - kM61 : x;
+  __device__ __forceinline__ W load(uint64_t x) const { return x; }
+  __device__ __forceinline__ uint64_t store(W x) const { return x >= kM61 ? x - kM61 : x; }
+  __device__ __forceinline__ W neg(W d) const { return 2 * kM61 - d; }
+  __device__ __forceinline__ bool zero(W d) const { return d == 0 || d == kM61; }
+  __device__ __forceinline__ W comb(W bb, W a, W nd, W b) const {
+    const u128 t = (u128)bb * a + (u128)nd * b;
+    const uint64_t lo = (uint64_t)t, hi = (uint64_t)(t >> 64);  // hi < 2^60
+    return FpM61::fold((lo & kM61) + ((hi << 3) | (lo >> 61)));
   }
 };
 
 // Even p (p = 2): Barrett reduction.
+template <class G, int LIMBS>
 struct BmBarrett {
-  using S = uint64_t;
-  using W = S;
-  using R = S;
-  FpBarrett f;
-  uint64_t r128;  // 2^128 mod p
-  __device__ explicit BmBarrett(const FieldParams& p) : f(p) {
-    const uint64_t m = f.reduce(~(u128)0);
-    r128 = m + 1 == f.p ? 0 : m + 1;
-  }
-  __device__ __forceinline__ S pack(S x) const { return x; }
-  __device__ __forceinline__ S load(S x) const { return x; }
-  __device__ __forceinline__ S store(S x) const { return x; }
-  __device__ __forceinline__ S neg(S d) const { return f.p - d; }
-  __device__ __forceinline__ bool zero(S d) const { return d == 0; }
-  __device__ __forceinline__ S comb(S bb, S a, S nd, S b) const { return f.reduce((u128)bb * a + (u128)nd * b); }
-  __device__ __forceinline__ S add(S a, S b) const { return f.add(a, b); }
-  struct Dot {
-    u128 v = 0;
-    uint32_t c = 0;
-    __device__ __forceinline__ void mac(S a, S b) {
-      const u128 t = (u128)a * b;
-      v += t;
-      c += v < t;
-    }
-  };
-  static constexpr int kFold = kCoefRows, kFoldHigh = 0;
-  __device__ __forceinline__ void fold_high(Dot&) const {}
-  __device__ __forceinline__ void fold(Dot&) const {}
-  __device__ __forceinline__ S value(const Dot& d) const { return f.add(f.reduce(d.v), f.mul(r128, d.c % f.p)); }
+  using F = G;
+  using W = uint64_t;
+  static constexpr int L = LIMBS;
+  F f;
+  __device__ explicit BmBarrett(const FieldParams& p) : f(p) {}
+  __device__ __forceinline__ W load(uint64_t x) const { return x; }
+  __device__ __forceinline__ uint64_t store(W x) const { return x; }
+  __device__ __forceinline__ W neg(W d) const { return f.modulus() - d; }
+  __device__ __forceinline__ bool zero(W d) const { return d == 0; }
+  __device__ __forceinline__ W comb(W bb, W a, W nd, W b) const { return f.reduce2(f.prod(bb, a) + f.prod(nd, b)); }
 };
 
-// Odd p < 2^63, R = 2^64: t < 2 p^2 reduces to (t + m p) / R < 2 p < 2^64.
+// Odd p < 2^63, r = 2^64: t < 2 p^2 reduces to (t + m p) / r < 2 p < 2^64.
 struct BmMont64 {
-  using S = uint64_t;
-  using W = S;
-  using R = S;
+  using F = FpBarrett;
+  using W = uint64_t;
+  static constexpr int L = 8;
   uint64_t p, np;  // np = -1/p mod 2^64
   __device__ explicit BmMont64(const FieldParams& f) : p(f.p) {
     uint64_t x = p;  // p x = 1 mod 8, doubled in precision each time
@@ -160,49 +101,24 @@ struct BmMont64 {
     for (int i = 0; i < 5; ++i) x *= 2 - p * x;
     np = 0 - x;
   }
-  // (t + m p) / 2^64 for t = hi 2^64 + lo: the low words cancel, with a carry
-  // unless lo is 0.
-  __device__ __forceinline__ u128 redc(uint64_t lo, u128 hi) const {
-    return hi + __umul64hi(lo * np, p) + (lo != 0);
-  }
-  __device__ __forceinline__ S last(uint64_t u) const { return u >= p ? u - p : u; }
-  __device__ __forceinline__ S pack(S x) const { return x; }
-  __device__ __forceinline__ S load(S x) const { return x; }
-  __device__ __forceinline__ S store(S x) const { return x; }
-  __device__ __forceinline__ S neg(S d) const { return p - d; }
-  __device__ __forceinline__ bool zero(S d) const { return d == 0; }
-  __device__ __forceinline__ S comb(S bb, S a, S nd, S b) const {
+  __device__ __forceinline__ W load(uint64_t x) const { return x; }
+  __device__ __forceinline__ uint64_t store(W x) const { return x; }
+  __device__ __forceinline__ W neg(W d) const { return p - d; }
+  __device__ __forceinline__ bool zero(W d) const { return d == 0; }
+  __device__ __forceinline__ W comb(W bb, W a, W nd, W b) const {
     const u128 t = (u128)bb * a + (u128)nd * b;
-    return last((uint64_t)(t >> 64) + __umul64hi((uint64_t)t * np, p) + ((uint64_t)t != 0));
-  }
-  __device__ __forceinline__ S add(S a, S b) const { return a >= p - b ? a - (p - b) : a + b; }
-  struct Dot {
-    u128 v = 0;
-    uint32_t c = 0;
-    __device__ __forceinline__ void mac(S a, S b) {
-      const u128 t = (u128)a * b;
-      v += t;
-      c += v < t;
-    }
-  };
-  static constexpr int kFold = kCoefRows, kFoldHigh = 0;
-  __device__ __forceinline__ void fold_high(Dot&) const {}
-  __device__ __forceinline__ void fold(Dot&) const {}
-  __device__ __forceinline__ S value(const Dot& d) const {  // t < 66 p^2: 34 p after one step, 2 p after two
-    const u128 u = redc((uint64_t)d.v, (u128)(uint64_t)(d.v >> 64) + ((u128)d.c << 64));
-    return last((uint64_t)redc((uint64_t)u, (u128)(uint64_t)(u >> 64)));
+    // The low words cancel, with a carry unless they are 0.
+    const uint64_t u = (uint64_t)(t >> 64) + __umul64hi((uint64_t)t * np, p) + ((uint64_t)t != 0);
+    return u >= p ? u - p : u;
   }
 };
 
-// Odd p < 2^31, residues stored in 32 bits, radix 2^32: t < 2 p^2 < 2^63
-// reduces to (t + m p) / 2^32 < 2 p < 2^32. kWide (p >= 2^28, where 66
-// products may pass 2^63): S is balanced, |x| <= 2^30, so that three offsets
-// fit in 63 bits, and the high words are moved aside after them.
-template <bool kWide>
+// Odd p < 2^31, r = 2^32: t < 2 p^2 < 2^63 reduces to (t + m p) / r < 2 p < 2^32.
+template <int LIMBS>
 struct BmMont32 {
-  using S = int32_t;
+  using F = FpSmall;
   using W = uint32_t;
-  using R = uint32_t;
+  static constexpr int L = LIMBS;
   uint32_t p, np;  // np = -1/p mod 2^32
   __device__ explicit BmMont32(const FieldParams& f) : p((uint32_t)f.p) {
     uint32_t x = p;
@@ -210,72 +126,47 @@ struct BmMont32 {
     for (int i = 0; i < 4; ++i) x *= 2 - p * x;
     np = 0 - x;
   }
-  __device__ __forceinline__ uint32_t last(uint32_t u) const { return min(u, u - p); }  // u < 2 p
-  __device__ __forceinline__ S pack(R x) const { return kWide && x > p / 2 ? (S)(x - p) : (S)x; }
-  __device__ __forceinline__ W load(S x) const { return kWide && x < 0 ? (W)x + p : (W)x; }
-  __device__ __forceinline__ S store(W x) const { return pack(x); }
+  __device__ __forceinline__ W load(uint64_t x) const { return (W)x; }
+  __device__ __forceinline__ uint64_t store(W x) const { return x; }
   __device__ __forceinline__ W neg(W d) const { return p - d; }
   __device__ __forceinline__ bool zero(W d) const { return d == 0; }
   __device__ __forceinline__ W comb(W bb, W a, W nd, W b) const {
     const uint64_t t = (uint64_t)bb * a + (uint64_t)nd * b;
-    return last((uint32_t)((t + (uint64_t)((uint32_t)t * np) * p) >> 32));
-  }
-  __device__ __forceinline__ R add(R a, R b) const { return last(a + b); }
-  struct Dot {
-    int64_t v = 0;
-    int64_t h = 0;  // high words of earlier offsets
-    __device__ __forceinline__ void mac(S a, S b) { v += (int64_t)a * b; }
-  };
-  static constexpr int kFold = kWide ? 3 : kCoefRows, kFoldHigh = 0;
-  __device__ __forceinline__ void fold_high(Dot&) const {}
-  __device__ __forceinline__ void fold(Dot& d) const {
-    if (!kWide) return;
-    d.h += d.v >> 32;
-    d.v = (uint32_t)d.v;
-  }
-  __device__ __forceinline__ R value(const Dot& d) const {
-    // t = 2^32 h + v: one step leaves the high part, |u| < 2^36, plus m p /
-    // 2^32 and a carry unless the low word is 0; 2^37 / p multiples of p make
-    // it positive; the second step leaves less than p + 2^7.
-    const uint32_t lo = (uint32_t)d.v;
-    int64_t u = (d.v >> 32) + __umulhi(lo * np, p) + (lo != 0);
-    if (kWide) u += d.h + ((int64_t)p << 9);
-    return last((uint32_t)(((uint64_t)u + (uint64_t)((uint32_t)u * np) * p) >> 32));
+    const uint32_t u = (uint32_t)((t + (uint64_t)((uint32_t)t * np) * p) >> 32);
+    return min(u, u - p);
   }
 };
 
-// The matrix of one block by offset: A'[j] = sum_o P[o] A[j+o] + Q[o] B[j+o],
-// B'[j] = sum_o U[o] A[j+o] + V[o] B[j+o], o = omin .. 32.
-template <class S>
-struct alignas(4 * sizeof(S)) Coef {
-  S c[4];  // P, Q, U, V
-};
-
-template <class S>
-struct BmMatrix {
-  Coef<S> row[kCoefRows];
+// The matrix of one block by offset: A'[j] = sum_o c[0][o] A[j+o] + c[1][o]
+// B[j+o], B'[j] = sum_o c[2][o] A[j+o] + c[3][o] B[j+o], o = omin .. 32 (P, Q, U,
+// V; canonical residues).
+struct alignas(16) BmMatrix {
+  uint64_t c[4][kCoefRows];
   int omin;
 };
+static_assert(sizeof(BmMatrix) % 16 == 0, "published as 16-byte words");
 
 // ---------------------------------------------------------------------------
 // bm_base — one warp runs steps i .. min(i + 32, n) on the windows a, b (lane
-// j: A[j], B[j]) and writes their matrix. In the frame of the block's start,
-// after k steps, A_k = P A + Q B is divisible by x^k and B_k = x^sb (U A + V B)
-// with deg P, Q < max(k, 1) and sb + deg U, V <= k; so window entry j and
-// coefficient j never need the same lane at once, and x holds P in lanes
-// below k and A_k's entries from lane k on, y holds U and the unshifted B_k's
-// entries likewise (entry k - sb, the pivot, is kept in bb).
-// Latency-bound chain of 32 x (shuffle, two products, reduction).
+// j: A[j], B[j], canonical) and writes their matrix. In the frame of the
+// block's start, after k steps, A_k = P A + Q B is divisible by x^k and B_k =
+// x^sb (U A + V B) with deg P, Q < max(k, 1) and sb + deg U, V <= k; so window
+// entry j and coefficient j never need the same lane at once, and x holds P in
+// lanes below k and A_k's entries from lane k on, y holds U and the unshifted
+// B_k's entries likewise (entry k - sb, the pivot, is kept in bb).
+// A dependent chain of 32 x (shuffle, two products, reduction): 190 cycles a
+// step over 2^61 - 1, 90 with 32-bit Montgomery. (A second warp for Q and V
+// measured 203 and 120: the chain, not the issue, is the bound.)
 // ---------------------------------------------------------------------------
-template <class F>
-__device__ __forceinline__ void bm_base(const F& f, typename F::S a, typename F::S b, int64_t i, int64_t n,
-                                        int64_t& l_io, BmMatrix<typename F::S>* M) {
-  using W = typename F::W;
+template <class P>
+__device__ __forceinline__ void bm_base(const P& f, uint64_t a, uint64_t b, int64_t i, int64_t n, int64_t& l_io,
+                                        BmMatrix* M) {
+  using W = typename P::W;
   const int lane = threadIdx.x & 31;
-  W x = f.load(a), y = lane == 0 ? 0 : f.load(b), Q = 0, V = lane == 0;
+  W x = f.load(a), y = lane == 0 ? 0 : f.load(b), Q = 0, V = lane == 0 ? f.load(1) : 0;
   W bb = __shfl_sync(kAll, f.load(b), 0);
   int sb = 0, da = 0, db = 0;
-  int64_t l = l_io;
+  const int64_t l = l_io;
   const int steps = n - i < kBmK ? (int)(n - i) : kBmK;
   int slack = (int)(i - 2 * l);  // 2 l <= i + k exactly when slack + k >= 0
   int dl = 0;                    // change of l
@@ -284,7 +175,7 @@ __device__ __forceinline__ void bm_base(const F& f, typename F::S a, typename F:
     const W d = __shfl_sync(kAll, x, k);
     W ys = __shfl_sync(kAll, y, lane - sb), vs = __shfl_sync(kAll, V, lane - sb);
     if (lane < sb) ys = vs = 0;
-    if (lane == k) x = k == 0;
+    if (lane == k) x = k == 0 ? f.load(1) : 0;
     // d == 0 takes the same update: A <- bb A, a nonzero multiple.
     const W nd = f.neg(d);
     const W nx = f.comb(bb, x, nd, ys), nq = f.comb(bb, Q, nd, vs);
@@ -311,235 +202,295 @@ __device__ __forceinline__ void bm_base(const F& f, typename F::S a, typename F:
   if (steps < kBmK) return;  // the sequence ends here: nothing is applied
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    M->row[lane].c[q] = 0;
-    if (lane == 0) M->row[kBmK].c[q] = 0;
+    M->c[q][lane] = 0;
+    if (lane == 0) M->c[q][kBmK] = 0;
   }
   __syncwarp();
-  M->row[kBmK - lane].c[0] = f.store(x);
-  M->row[kBmK - lane].c[1] = f.store(Q);
+  M->c[0][kBmK - lane] = f.store(x);
+  M->c[1][kBmK - lane] = f.store(Q);
   if (lane <= db) {
-    M->row[kBmK - sb - lane].c[2] = f.store(y);
-    M->row[kBmK - sb - lane].c[3] = f.store(V);
+    M->c[2][kBmK - sb - lane] = f.store(y);
+    M->c[3][kBmK - sb - lane] = f.store(V);
   }
   if (lane == 0) M->omin = kBmK - (da > sb + db ? da : sb + db);
   __syncwarp();
 }
 
 // ---------------------------------------------------------------------------
-// bm_front — kFront warps compute the next window, outputs 0 .. 31: warp w
-// sums every (kFront / 4)-th offset of coefficient w & 3 (P, Q, U, V); warp 0
-// adds the parts and returns the window. Barrier 3 joins the warps. On the
-// critical path of the steps, so spread thin: latency of ~5 dependent
-// products at 8 warps.
+// Applying a matrix: limb products on the tensor cores (mma_limbs.cuh). A and
+// B are kept as L byte planes each (plane q at q * pitch; A's, then B's). A tile
+// is 64 consecutive outputs j = base + 4 m + r (m < 16, r < 4) of both A' and
+// B': the left operand of the m16n8k32 product has row m = plane bytes from
+// base + wb + 4 m on (32 window positions, read as words from shared memory),
+// the right one column 2 r + type with the coefficients shifted by r. With the
+// usual 17 offsets (16 .. 32) one window of 32 positions covers all; below
+// offset 4 it takes two. 2 L^2 instructions per tile: 128 over 2^61 - 1, i.e. 256
+// cycles of an SM per 64 outputs, against 1150 on the integer pipes (18 x 4
+// multiply-adds at 4 cycles a warp for each of four half products).
 // ---------------------------------------------------------------------------
-template <int kFront, class F>
-__device__ __forceinline__ void bm_front(const F& f, const typename F::S* A, const typename F::S* B,
-                                         const BmMatrix<typename F::S>& M, typename F::R (*fr)[32], int w,
-                                         typename F::S& a, typename F::S& b) {
-  using S = typename F::S;
-  using R = typename F::R;
-  constexpr int kStep = kFront / 4;
+template <int L>
+struct BmFrag {
+  uint32_t b[2][L][2];  // [source A or B][limb][k half]
+};
+
+template <int L>
+__device__ __forceinline__ void bm_frag(BmFrag<L>& fr, const BmMatrix& M, int wb) {
+  const int lane = threadIdx.x & 31, n = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int src = 0; src < 2; ++src)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint64_t* c = M.c[(n & 1) * 2 + src];
+      const int o = wb + 4 * t + 16 * h - (n >> 1);
+      uint64_t v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = (unsigned)(o + q) < (unsigned)kCoefRows ? c[o + q] : 0;
+      uint32_t w[L];
+      mml::limb_words<L>(w, v);
+#pragma unroll
+      for (int i = 0; i < L; ++i) fr.b[src][i][h] = w[i];
+    }
+}
+
+// Adds the products of the tile at `base` (a multiple of 4) to acc.
+template <int L>
+__device__ __forceinline__ void bm_tile(uint32_t (&acc)[2 * L - 1][4], const BmFrag<L>& fr, const uint8_t* planes,
+                                        int pitch, int pos) {
   const int lane = threadIdx.x & 31;
-  const S* X = ((w & 1) ? B : A) + lane;
-  const S* c = &M.row[0].c[w & 3];
-  typename F::Dot acc[2];
-  int o = M.omin + (w >> 2);
-#pragma unroll 1
-  for (; o + 3 * kStep < kCoefRows; o += 4 * kStep) {
-    S xv[4], cv[4];
+  const uint8_t* p0 = planes + pos + 4 * ((lane >> 2) + (lane & 3));
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      xv[u] = X[o + u * kStep];
-      cv[u] = c[4 * (o + u * kStep)];
+  for (int src = 0; src < 2; ++src)
+#pragma unroll
+    for (int i = 0; i < L; ++i) {
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(p0 + (src * L + i) * pitch);
+      const uint32_t a[4] = {w[0], w[8], w[4], w[12]};
+#pragma unroll
+      for (int j = 0; j < L; ++j) mml::mma_k32(acc[i + j], a, fr.b[src][j][0], fr.b[src][j][1]);
     }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) acc[u & 1].mac(cv[u], xv[u]);
-    f.fold(acc[0]);
-    f.fold(acc[1]);
-  }
-#pragma unroll
-  for (int u = 0; u < 3; ++u)
-    if (o + u * kStep < kCoefRows) acc[u & 1].mac(c[4 * (o + u * kStep)], X[o + u * kStep]);
-  const R v = f.add(f.value(acc[0]), f.value(acc[1]));
-  if (w != 0) {
-    fr[w][lane] = v;
-    asm volatile("bar.arrive 3, %0;" ::"n"(32 * kFront) : "memory");
-    return;
-  }
-  asm volatile("bar.sync 3, %0;" ::"n"(32 * kFront) : "memory");
-  R ra = f.add(v, fr[1][lane]), rb = f.add(fr[2][lane], fr[3][lane]);
-#pragma unroll
-  for (int q = 4; q < kFront; q += 4) {
-    ra = f.add(ra, f.add(fr[q][lane], fr[q + 1][lane]));
-    rb = f.add(rb, f.add(fr[q + 2][lane], fr[q + 3][lane]));
-  }
-  a = f.pack(ra);
-  b = f.pack(rb);
 }
 
-// ---------------------------------------------------------------------------
-// bm_dots — entries j[q] (q < N) of A' and B' by one thread. Bound by the
-// integer multiply pipe: four products per entry pair and offset.
-// ---------------------------------------------------------------------------
-template <int N, class F>
-__device__ __forceinline__ void bm_dots(const F& f, const typename F::S* A, const typename F::S* B,
-                                        const BmMatrix<typename F::S>& M, int j0, int T, int lim,
-                                        typename F::R (&va)[4], typename F::R (&vb)[4]) {
-  using S = typename F::S;
-  typename F::Dot da[N], db[N];
-  const S *pa[N], *pb[N];
-#pragma unroll
-  for (int q = 0; q < N; ++q) {
-    const int j = min(j0 + q * T, lim - 1);
-    pa[q] = A + j;
-    pb[q] = B + j;
+// The fragments of a matrix as a warp keeps them, and one tile's residues: v =
+// A'(j0), B'(j0), A'(j0 + 32), B'(j0 + 32) with j0 = base + lane.
+template <class P>
+struct BmApply {
+  static constexpr int L = P::L;
+  const LimbRed<typename P::F, L>& red;
+  const BmMatrix& M;
+  BmFrag<L> fr;
+  int wb;
+  bool two;
+  __device__ __forceinline__ BmApply(const LimbRed<typename P::F, L>& r, const BmMatrix& m) : red(r), M(m) {
+    wb = M.omin & ~3;
+    two = wb == 0;
+    bm_frag(fr, M, wb);
   }
-  const auto at = [&](int o) {
-    const Coef<S> c = M.row[o];
-    S av[N], bv[N];
+  __device__ __forceinline__ void tile(const uint8_t* planes, int pitch, int base, uint64_t (&v)[4]) {
+    uint32_t acc[2 * L - 1][4];
 #pragma unroll
-    for (int q = 0; q < N; ++q) {
-      av[q] = pa[q][o];
-      bv[q] = pb[q][o];
+    for (int d = 0; d < 2 * L - 1; ++d)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[d][q] = 0;
+    bm_tile<L>(acc, fr, planes, pitch, base + wb);
+    if (two) {
+      bm_frag(fr, M, 32);
+      bm_tile<L>(acc, fr, planes, pitch, base + 32);
+      bm_frag(fr, M, 0);
     }
 #pragma unroll
-    for (int q = 0; q < N; ++q) da[q].mac(c.c[0], av[q]);
-#pragma unroll
-    for (int q = 0; q < N; ++q) db[q].mac(c.c[2], av[q]);
-#pragma unroll
-    for (int q = 0; q < N; ++q) da[q].mac(c.c[1], bv[q]);
-#pragma unroll
-    for (int q = 0; q < N; ++q) db[q].mac(c.c[3], bv[q]);
-  };
-  constexpr int kU = F::kFold < 4 ? F::kFold : 4;
-  int o = M.omin, high = 0;
-#pragma unroll 1
-  for (; o + kU <= kCoefRows; o += kU) {
-#pragma unroll
-    for (int u = 0; u < kU; ++u) at(o + u);
-    if (F::kFold < kCoefRows) {
-#pragma unroll
-      for (int q = 0; q < N; ++q) {
-        f.fold(da[q]);
-        f.fold(db[q]);
-      }
-    }
-    if (F::kFoldHigh && ++high == F::kFoldHigh) {
-      high = 0;
-#pragma unroll
-      for (int q = 0; q < N; ++q) {
-        f.fold_high(da[q]);
-        f.fold_high(db[q]);
-      }
-    }
+    for (int q = 0; q < 4; ++q) v[q] = red.residue(acc, q);
   }
-#pragma unroll 1
-  for (; o < kCoefRows; ++o) at(o);
-#pragma unroll
-  for (int q = 0; q < N; ++q) {
-    va[q] = f.value(da[q]);
-    vb[q] = f.value(db[q]);
-  }
+};
+
+template <int L>
+__device__ __forceinline__ void bm_put(uint8_t* planes, int pitch, int j, uint64_t a, uint64_t b) {
+  mml::put_planes1<L>(planes + j, pitch, a);
+  mml::put_planes1<L>(planes + L * pitch + j, pitch, b);
 }
 
-// ---------------------------------------------------------------------------
-// bm_apply — entries t0 .. lim of A' and B' in place by a group of T threads
-// (t: this thread's number), up to four entries per thread and tile. Output j
-// is stored at j and reads reach from j to j + 32, so bar(k), the barrier of
-// tile k, separates the group's reads from its writes. A warp computes only as
-// many entries as it has (a tile's last entries leave the other warps free).
-// ---------------------------------------------------------------------------
-template <class F, class Bar>
-__device__ __forceinline__ void bm_apply(const F& f, typename F::S* A, typename F::S* B,
-                                         const BmMatrix<typename F::S>& M, int t0, int T, int t, int lim, bool& nz,
-                                         Bar&& bar) {
-  for (int k = 0; t0 < lim; ++k, t0 += 4 * T) {
-    typename F::R va[4], vb[4];
-    const int left = lim - t0 - (t & ~31);  // from this warp's first entry
-    const int mine = left <= 0 ? 0 : (left + T - 1) / T;
-    if (mine >= 3)
-      bm_dots<4>(f, A, B, M, t0 + t, T, lim, va, vb);
-    else if (mine == 2)
-      bm_dots<2>(f, A, B, M, t0 + t, T, lim, va, vb);
-    else if (mine == 1)
-      bm_dots<1>(f, A, B, M, t0 + t, T, lim, va, vb);
+// Outputs t0 .. lim in place by the `warps` warps of a group (this one: w),
+// two tiles per warp and pass: output j is stored at j and reads reach past it
+// only, so bar(k), the barrier of pass k, separates the reads from the writes.
+template <class P, class Bar>
+__device__ __forceinline__ void bm_apply(const LimbRed<typename P::F, P::L>& red, uint8_t* planes, int pitch,
+                                         const BmMatrix& M, int t0, int warps, int w, int lim, bool& nz, Bar&& bar) {
+  constexpr int kPer = 2;
+  const int lane = threadIdx.x & 31;
+  if (t0 >= lim) return;
+  BmApply<P> ap(red, M);
+  for (int k = 0; t0 < lim; ++k, t0 += 64 * kPer * warps) {
+    uint64_t v[kPer][4];
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      const int base = t0 + 64 * (q * warps + w);
+      if (base < lim) ap.tile(planes, pitch, base, v[q]);
+    }
     bar(k);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int j = t0 + q * T + t;
-      if (q < mine && j < lim) {
-        A[j] = f.pack(va[q]);
-        B[j] = f.pack(vb[q]);
-        nz |= va[q] != 0;
+    for (int q = 0; q < kPer; ++q)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int j = t0 + 64 * (q * warps + w) + 32 * h + lane;
+        if (j < lim) {
+          bm_put<P::L>(planes, pitch, j, v[q][2 * h], v[q][2 * h + 1]);
+          nz |= v[q][2 * h] != 0;
+        }
       }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// bm_front — the next window and the 32 entries after it (the tile at 0), on
+// the chain of the steps. With 8 limbs warps 0 .. 3 share it: warp w takes
+// source w & 1 and half of A's or B's limbs, and warp 0 adds the four parts
+// (barrier 3; 1300 cycles against 1830 in one warp). With up to 4 limbs warp 0
+// does it alone (700 to 1000 cycles; 1400 to 1600 in four). v is warp 0's.
+// ---------------------------------------------------------------------------
+template <class P>
+__device__ __forceinline__ void bm_front(const LimbRed<typename P::F, P::L>& red, const uint8_t* planes, int pitch,
+                                         const BmMatrix& M, uint64_t (*fr)[4][32], int w, uint64_t (&v)[4]) {
+  constexpr int L = P::L, H = L / 2;  // limbs of a warp
+  if constexpr (L <= 4) {
+    if (w == 0) {
+      BmApply<P> ap(red, M);
+      ap.tile(planes, pitch, 0, v);
+      __syncwarp();
+    }
+    return;
+  }
+  const int lane = threadIdx.x & 31, src = w & 1, hi = w >> 1;
+  const typename P::F& f = red.field();
+  uint32_t acc[2 * L - 1][4];
+#pragma unroll
+  for (int d = 0; d < 2 * L - 1; ++d)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) acc[d][q] = 0;
+  {
+    const int n = lane >> 2, t = lane & 3;
+    const uint64_t* c = M.c[(n & 1) * 2 + src];
+    for (int wb = M.omin & ~3; wb <= kBmK; wb += 32) {
+      uint32_t b[2][L];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int o = wb + 4 * t + 16 * h - (n >> 1);
+        uint64_t x[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) x[q] = (unsigned)(o + q) < (unsigned)kCoefRows ? c[o + q] : 0;
+        mml::limb_words<L>(b[h], x);
+      }
+      const uint8_t* p0 = planes + (src * L + hi * H) * pitch + wb + 4 * (n + t);
+#pragma unroll
+      for (int i = 0; i < H; ++i) {
+        const uint32_t* x = reinterpret_cast<const uint32_t*>(p0 + i * pitch);
+        const uint32_t a[4] = {x[0], x[8], x[4], x[12]};
+#pragma unroll
+        for (int j = 0; j < L; ++j) mml::mma_k32(acc[i + j], a, b[0][j], b[1][j]);
+      }
+      if (wb >= 4) break;  // this window covers all offsets
     }
   }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint64_t x = red.residue(acc, q);
+    if (hi) x = red.template shifted<8 * H>(x);
+    v[q] = x;
+  }
+  if (w != 0) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) fr[w - 1][q][lane] = v[q];
+    asm volatile("bar.arrive 3, 128;" ::: "memory");
+    return;
+  }
+  asm volatile("bar.sync 3, 128;" ::: "memory");
+#pragma unroll
+  for (int q = 0; q < 4; ++q) v[q] = f.add(f.add(v[q], fr[0][q][lane]), f.add(fr[1][q][lane], fr[2][q][lane]));
+}
+
+// Entry j from its byte planes.
+template <int L>
+__device__ __forceinline__ uint64_t bm_get(const uint8_t* planes, int pitch, int j) {
+  uint64_t v = 0;
+#pragma unroll
+  for (int i = 0; i < L; ++i) v |= (uint64_t)planes[i * pitch + j] << (8 * i);
+  return v;
 }
 
 // Entries of A and B of the start: c = b = 1, bb = 1 (src/fp.rs:262-268), so
 // A = s and B = 1 + x s.
 __device__ __forceinline__ uint64_t bm_b0(const uint64_t* s, int64_t j) { return j ? s[j - 1] : 1; }
 
+// Byte planes of a sequence's residuals: pitch bytes each, past the end as much
+// as a tile may read.
+constexpr int kBmPad = 160;
+__host__ __device__ constexpr int64_t bm_pitch(int64_t n) { return (n + kBmPad + 15) / 16 * 16; }
+
 struct BmShared {
-  BmMatrix<uint64_t> M[2];
-  alignas(16) uint64_t fr[8][32];
+  BmMatrix M[2];
+  uint64_t fr[3][4][32];  // parts of the front tile
   int64_t l;
   long long job;
   int flag;
 };
 
-// ---------------------------------------------------------------------------
-// One sequence with the whole CTA (blockDim a multiple of 32, at least 128).
-// A, B: n + kBmPad entries each, owned by this CTA. Per block of 32 steps one
-// barrier of the whole CTA, and one among the applying warps per tile.
-// ---------------------------------------------------------------------------
-template <class F>
-__device__ __forceinline__ int64_t bm_run(const F& f, const uint64_t* __restrict__ s, int64_t n64, typename F::S* A,
-                                          typename F::S* B, BmShared& sh) {
-  using S = typename F::S;
-  using R = typename F::R;
-  const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5;
-  const int n = (int)n64;
-  BmMatrix<S>* M = reinterpret_cast<BmMatrix<S>*>(sh.M);
-  typename F::R(*fr)[32] = reinterpret_cast<typename F::R(*)[32]>(sh.fr);
+// Entries [0, n) of the start and zeros behind them, n rounded up to a word.
+template <int L>
+__device__ __forceinline__ bool bm_start(const uint64_t* __restrict__ s, int n, uint8_t* planes, int pitch) {
   bool nz = false;
-  for (int j = tid; j < n + kBmPad; j += T) {
-    const S v = j < n ? f.pack((R)s[j]) : 0;
-    A[j] = v;
-    B[j] = j < n ? f.pack((R)bm_b0(s, j)) : 0;
-    nz |= v != 0;
+  for (int j = 4 * threadIdx.x; j < pitch; j += 4 * blockDim.x) {
+    uint64_t a[4], b[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      a[q] = j + q < n ? s[j + q] : 0;
+      b[q] = j + q < n ? bm_b0(s, j + q) : 0;
+      nz |= a[q] != 0;
+    }
+    mml::put_planes4<L>(planes + j, pitch, a);
+    mml::put_planes4<L>(planes + L * pitch + j, pitch, b);
   }
+  return nz;
+}
+
+// ---------------------------------------------------------------------------
+// One sequence with the whole CTA (blockDim a multiple of 32, at least 128):
+// warps 0 .. 3 compute the next window, then warp 0 runs the next 32 steps
+// while the others apply the matrix. Per block of 32 steps one barrier of the
+// whole CTA, and one among the applying warps per pass. planes: 2 L of
+// bm_pitch(n) bytes, owned by this CTA.
+// ---------------------------------------------------------------------------
+template <class P>
+__device__ __forceinline__ int64_t bm_run(const P& f, const LimbRed<typename P::F, P::L>& red,
+                                          const uint64_t* __restrict__ s, int64_t n64, uint8_t* planes,
+                                          BmShared& sh) {
+  constexpr int L = P::L;
+  const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5;
+  const int n = (int)n64, pitch = (int)bm_pitch(n64);
+  bool nz = bm_start<L>(s, n, planes, pitch);
   int64_t l = 0;
   __syncthreads();
-  S a = 0, b = 0;
-  if (warp == 0) {
-    a = A[lane];
-    b = B[lane];
-    bm_base(f, a, b, 0, n, l, &M[0]);
-  }
+  if (warp == 0)
+    bm_base(f, bm_get<L>(planes, pitch, lane), bm_get<L>(planes + L * pitch, pitch, lane), 0, n, l, &sh.M[0]);
   for (int i = 0;; i += kBmK) {
     // Every thread's part of A (steps i on) has been written and tested, and
     // the block's matrix is there.
     const bool any = __syncthreads_or(nz);
     if (!any || i + kBmK >= n) break;
     nz = false;
-    const BmMatrix<S>& m = M[(i / kBmK) & 1];
+    const int par = (i / kBmK) & 1;
+    const BmMatrix& m = sh.M[par];
     const int lim = n - i - kBmK;  // outputs
-    if (T >= 512) {
-      if (warp < 8) bm_front<8>(f, A, B, m, fr, warp, a, b);
-    } else if (warp < 4) {
-      bm_front<4>(f, A, B, m, fr, warp, a, b);
-    }
+    uint64_t v[4];
+    if (warp < 4) bm_front<P>(red, planes, pitch, m, sh.fr, warp, v);
     if (warp == 0) {
-      // The first tile's writes wait until the front has read its inputs.
-      if (lim > kBmK) asm volatile("bar.arrive 1, %0;" ::"r"(T) : "memory");
-      if (lane >= lim) a = b = 0;
-      nz = a != 0;
-      A[lane] = a;  // read by no thread until the next barrier of the CTA
-      B[lane] = b;
-      bm_base(f, a, b, i + kBmK, n, l, &M[((i / kBmK) & 1) ^ 1]);
+      // The first pass's writes wait until the front tile has read its inputs.
+      if (lim > 64) asm volatile("bar.arrive 1, %0;" ::"r"(T) : "memory");
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (lane + 32 * h >= lim) v[2 * h] = v[2 * h + 1] = 0;
+        nz |= v[2 * h] != 0;
+        bm_put<L>(planes, pitch, lane + 32 * h, v[2 * h], v[2 * h + 1]);  // read by no other warp before the barrier
+      }
+      bm_base(f, v[0], v[1], i + kBmK, n, l, &sh.M[par ^ 1]);
     } else {
-      bm_apply(f, A, B, m, kBmK, T - 32, tid - 32, lim, nz, [&](int k) {
+      bm_apply<P>(red, planes, pitch, m, 64, T / 32 - 1, warp - 1, lim, nz, [&](int k) {
         if (k == 0)
           asm volatile("bar.sync 1, %0;" ::"r"(T) : "memory");
         else
@@ -552,37 +503,35 @@ __device__ __forceinline__ int64_t bm_run(const F& f, const uint64_t* __restrict
   return sh.l;
 }
 
-template <class F>
-__device__ __forceinline__ int64_t bm_any(const BmJob& job, const FieldParams& fp, uint64_t* smem, uint64_t* gws,
-                                          int64_t smem_words, BmShared& sh) {
-  using S = typename F::S;
-  const F f(fp);
-  const int64_t m = job.n + kBmPad;
-  if (bm_words<S>(job.n) <= smem_words) {
-    S* A = reinterpret_cast<S*>(smem);
-    return bm_run(f, job.s, job.n, A, A + m, sh);
-  }
-  S* A = reinterpret_cast<S*>(gws);
-  return bm_run(f, job.s, job.n, A, A + m, sh);
+template <class P>
+__device__ __noinline__ int64_t bm_any(const BmJob& job, uint64_t* gws, int64_t smem_words, BmShared& sh) {
+  extern __shared__ __align__(16) uint64_t bm_smem[];
+  const FieldParams fp{job.p, job.mu_lo, job.mu_hi, job.safe_batch};
+  const P f(fp);
+  const LimbRed<typename P::F, P::L> red{typename P::F(fp)};
+  const bool fits = bm_words(P::L, job.n) <= smem_words;
+  if (fits) return bm_run(f, red, job.s, job.n, reinterpret_cast<uint8_t*>(bm_smem), sh);
+  return bm_run(f, red, job.s, job.n, reinterpret_cast<uint8_t*>(gws), sh);
 }
 
-__device__ __forceinline__ int64_t bm_dispatch(const BmJob& job, uint64_t* smem, uint64_t* gws, int64_t smem_words,
-                                               BmShared& sh) {
+__device__ __forceinline__ int64_t bm_dispatch(const BmJob& job, uint64_t* gws, int64_t smem_words, BmShared& sh) {
   if (job.n <= 0) return 0;
-  const FieldParams fp{job.p, job.mu_lo, job.mu_hi, job.safe_batch};
-  if (job.p == kM61) return bm_any<BmM61>(job, fp, smem, gws, smem_words, sh);
-  if (!(job.p & 1)) return bm_any<BmBarrett>(job, fp, smem, gws, smem_words, sh);
-  if (job.p < (1ULL << 28)) return bm_any<BmMont32<false>>(job, fp, smem, gws, smem_words, sh);
-  if (job.p < (1ULL << 31)) return bm_any<BmMont32<true>>(job, fp, smem, gws, smem_words, sh);
-  return bm_any<BmMont64>(job, fp, smem, gws, smem_words, sh);
+  const uint64_t p = job.p;
+  if (p == kM61) return bm_any<BmM61>(job, gws, smem_words, sh);
+  if (!(p & 1) || (p >> 31 == 1))
+    return p < (1ULL << 32) ? bm_any<BmBarrett<FpSmall, 4>>(job, gws, smem_words, sh)
+                            : bm_any<BmBarrett<FpBarrett, 8>>(job, gws, smem_words, sh);
+  if (p < (1ULL << 8)) return bm_any<BmMont32<1>>(job, gws, smem_words, sh);
+  if (p < (1ULL << 16)) return bm_any<BmMont32<2>>(job, gws, smem_words, sh);
+  if (p < (1ULL << 31)) return bm_any<BmMont32<4>>(job, gws, smem_words, sh);
+  return bm_any<BmMont64>(job, gws, smem_words, sh);
 }
 
 // Plain form: one CTA runs one sequence, A and B in dynamic shared memory when
 // they fit, else in the global workspace.
 __global__ void __launch_bounds__(512) bm_block_kernel(BmJob job, uint64_t* gws, int64_t smem_words, int64_t* out) {
-  extern __shared__ __align__(16) uint64_t bm_smem[];
   __shared__ BmShared sh;
-  const int64_t l = bm_dispatch(job, bm_smem, gws, smem_words, sh);
+  const int64_t l = bm_dispatch(job, gws, smem_words, sh);
   if (threadIdx.x == 0) *out = l;
 }
 
@@ -592,7 +541,6 @@ __global__ void __launch_bounds__(512) bm_block_kernel(BmJob job, uint64_t* gws,
 __global__ void __launch_bounds__(512)
     bm_batch_kernel(const BmJob* __restrict__ jobs, int64_t count, unsigned long long* next, uint64_t* gws,
                     int64_t gws_words, int64_t smem_words, int64_t* out) {
-  extern __shared__ __align__(16) uint64_t bm_smem[];
   __shared__ BmShared sh;
   for (;;) {
     if (threadIdx.x == 0) sh.job = (long long)atomicAdd(next, 1ULL);
@@ -601,7 +549,7 @@ __global__ void __launch_bounds__(512)
     __syncthreads();
     if (q >= count) break;
     const BmJob job = jobs[q];
-    const int64_t l = bm_dispatch(job, bm_smem, gws + (int64_t)blockIdx.x * gws_words, smem_words, sh);
+    const int64_t l = bm_dispatch(job, gws + (int64_t)blockIdx.x * gws_words, smem_words, sh);
     if (threadIdx.x == 0) out[job.slot] = l;
     __syncthreads();
   }
@@ -642,8 +590,8 @@ struct LongSync {
 struct LongArgs {
   const uint64_t* s;
   int64_t n;
-  void* buf;        // [2][2][n + kBmPad] entries: parity, A or B
-  void* ring;       // [2 kBmH] matrices
+  uint8_t* buf;     // [2][2 L][bm_pitch(n)] bytes: parity, A's and B's limb planes
+  BmMatrix* ring;   // [2 kBmH]
   unsigned int* nz;  // per superblock: some output is nonzero
   LongSync* gs;
   int64_t* out;
@@ -695,30 +643,53 @@ __device__ __forceinline__ bool long_wait(const unsigned int* p, unsigned int wa
   return true;
 }
 
-template <class F>
+template <class P>
 __global__ void __launch_bounds__(kLongThreads, 1) bm_long_kernel(FieldParams fp, LongArgs g) {
-  using S = typename F::S;
+  constexpr int L = P::L;
   extern __shared__ __align__(16) uint64_t bm_smem[];
   __shared__ BmShared sh;
-  const F f(fp);
+  const P f(fp);
+  const LimbRed<typename P::F, L> red{typename P::F(fp)};
   const int tid = threadIdx.x, T = kLongThreads, lane = tid & 31, warp = tid >> 5;
   const int G = gridDim.x;
-  const int64_t n = g.n, pitch = n + kBmPad;
-  S* buf = static_cast<S*>(g.buf);
-  BmMatrix<S>* ring = static_cast<BmMatrix<S>*>(g.ring);
-  BmMatrix<S>* M = reinterpret_cast<BmMatrix<S>*>(sh.M);
-  S* A = reinterpret_cast<S*>(bm_smem);
-  // Entry j of A (which = 0) or B (1) at the start of superblock s.
-  const auto entry = [&](int64_t s, int which, int64_t j) -> S {
-    if (j >= n - s * kBmT) return 0;
-    if (s == 0) return f.pack((typename F::R)(which ? bm_b0(g.s, j) : g.s[j]));
-    return __ldcg(buf + ((s & 1) * 2 + which) * pitch + j);
+  const int64_t n = g.n, gpitch = bm_pitch(n);
+  uint8_t* planes = reinterpret_cast<uint8_t*>(bm_smem);
+  // Entries lo .. lo + len (len a multiple of 4, as is lo) of A and B at the
+  // start of superblock s into the planes; whether an A entry is nonzero.
+  const auto load = [&](int64_t s, int64_t lo, int len, int pitch) {
+    const int64_t left = n - s * kBmT - lo;  // valid entries
+    bool nz = false;
+    if (s == 0) {
+      for (int j = 4 * tid; j < len; j += 4 * T) {
+        uint64_t a[4], b[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          a[q] = j + q < left ? g.s[lo + j + q] : 0;
+          b[q] = j + q < left ? bm_b0(g.s, lo + j + q) : 0;
+          nz |= a[q] != 0;
+        }
+        mml::put_planes4<L>(planes + j, pitch, a);
+        mml::put_planes4<L>(planes + L * pitch + j, pitch, b);
+      }
+    } else {
+      const uint8_t* src = g.buf + (s & 1) * 2 * L * gpitch + lo;
+      for (int j = 4 * tid; j < len; j += 4 * T) {
+        // Bytes past the valid entries are zeroed (the buffer holds older ones).
+        const uint32_t mask = j + 4 <= left ? 0xffffffffu : j >= left ? 0u : (1u << (8 * (int)(left - j))) - 1;
+#pragma unroll
+        for (int q = 0; q < 2 * L; ++q) {
+          const uint32_t v = mask ? __ldcg(reinterpret_cast<const unsigned int*>(src + q * gpitch + j)) & mask : 0;
+          *reinterpret_cast<uint32_t*>(planes + q * pitch + j) = v;
+          if (q < L) nz |= v != 0;
+        }
+      }
+    }
+    return nz;
   };
 
   if (blockIdx.x == 0) {
     // ---------------- the steps -------------------------------------------
-    S* B = A + kBmT + kBmPad;
-    typename F::R(*fr)[32] = reinterpret_cast<typename F::R(*)[32]>(sh.fr);
+    const int pitch = (int)bm_pitch(kBmT);
     int64_t l = 0;
     unsigned int want_front = 0, want_done = 0;
     bool ok = true;
@@ -732,14 +703,7 @@ __global__ void __launch_bounds__(kLongThreads, 1) bm_long_kernel(FieldParams fp
         ok = sh.flag;
         if (!ok) break;
       }
-      bool nz = false;
-      for (int j = tid; j < kBmT + kBmPad; j += T) {
-        const S v = j < kBmT ? entry(s, 0, j) : 0;
-        A[j] = v;
-        B[j] = j < kBmT ? entry(s, 1, j) : 0;
-        nz |= v != 0;
-      }
-      const bool any = __syncthreads_or(nz);
+      const bool any = __syncthreads_or(load(s, 0, kBmT, pitch));
       if (s > 0 && !any) {
         // The window is zero: if all of A is, the sequence is done.
         if (tid == 0) {
@@ -752,41 +716,38 @@ __global__ void __launch_bounds__(kLongThreads, 1) bm_long_kernel(FieldParams fp
           break;
         }
       }
-      S a = 0, b = 0;
       const int64_t i0 = s * kBmT;
       const bool feeds = n - i0 > kBmT;  // later steps need the matrices
-      if (warp == 0) {
-        a = A[lane];
-        b = B[lane];
-        bm_base(f, a, b, i0, n, l, &M[0]);
-      }
+      if (warp == 0)
+        bm_base(f, bm_get<L>(planes, pitch, lane), bm_get<L>(planes + L * pitch, pitch, lane), i0, n, l, &sh.M[0]);
       for (int h = 0; h < kBmH && i0 + h * kBmK < n; ++h) {
         __syncthreads();
-        const BmMatrix<S>& m = M[h & 1];
+        const BmMatrix& m = sh.M[h & 1];
         const int lim = kBmT - (h + 1) * kBmK;  // outputs inside the window
         const bool more = lim > 0 && i0 + (h + 1) * kBmK < n;
-        if (more && warp < 8) bm_front<8>(f, A, B, m, fr, warp, a, b);
+        uint64_t v[4];
+        if (more && warp < 4) bm_front<P>(red, planes, pitch, m, sh.fr, warp, v);
         if (warp == 0) {
           if (more) {
-            if (lim > kBmK) asm volatile("bar.arrive 1, %0;" ::"r"(T - 32) : "memory");
-            A[lane] = a;
-            B[lane] = b;
-            bm_base(f, a, b, i0 + (h + 1) * kBmK, n, l, &M[(h & 1) ^ 1]);
+            if (lim > 64) asm volatile("bar.arrive 1, %0;" ::"r"(T - 32) : "memory");
+            bm_put<L>(planes, pitch, lane, v[0], v[1]);
+            if (lim > 32) bm_put<L>(planes, pitch, lane + 32, v[2], v[3]);
+            bm_base(f, v[0], v[1], i0 + (h + 1) * kBmK, n, l, &sh.M[(h & 1) ^ 1]);
           }
         } else if (warp == T / 32 - 1) {
           if (feeds) {
             // The last warp publishes: 16-byte words of the matrix, then the count.
             const int64_t q = s * kBmH + h;
             const uint4* src = reinterpret_cast<const uint4*>(&m);
-            uint4* dst = reinterpret_cast<uint4*>(ring + q % (2 * kBmH));
-            for (int w = lane; w < (int)(sizeof(BmMatrix<S>) / 16); w += 32) __stcg(dst + w, src[w]);
+            uint4* dst = reinterpret_cast<uint4*>(g.ring + q % (2 * kBmH));
+            for (int w = lane; w < (int)(sizeof(BmMatrix) / 16); w += 32) __stcg(dst + w, src[w]);
             __threadfence();
             __syncwarp();
             if (lane == 0 && !(q == 0 && g.skip_cta == 0)) atomicAdd(&g.gs->pub, 1u);
           }
         } else if (more) {
           bool unused = false;
-          bm_apply(f, A, B, m, kBmK, T - 64, tid - 32, lim, unused, [&](int k) {
+          bm_apply<P>(red, planes, pitch, m, 64, T / 32 - 2, warp - 1, lim, unused, [&](int k) {
             if (k == 0)
               asm volatile("bar.sync 1, %0;" ::"r"(T - 32) : "memory");
             else
@@ -806,51 +767,56 @@ __global__ void __launch_bounds__(kLongThreads, 1) bm_long_kernel(FieldParams fp
 
   // ---------------- the chunks ----------------------------------------------
   const int wk = blockIdx.x - 1;
-  S* B = A + g.cap + kBmT + kBmPad;
+  const int pitch = (int)bm_pitch(g.cap + kBmT);
   unsigned int want_done = 0;
   for (int64_t s = 0;; ++s) {
-    const LongPlan P(n, s, G, g.cap);
-    if (P.nout == 0) return;
-    for (int c = wk; c < P.chunks; c += G - 1) {
+    const LongPlan plan(n, s, G, g.cap);
+    if (plan.nout == 0) return;
+    for (int c = wk; c < plan.chunks; c += G - 1) {
       if (tid == 0) sh.flag = long_wait(&g.gs->done, want_done, g.gs, g.spin);
       __syncthreads();
       if (!sh.flag) return;
       int64_t lo, hi;
-      P.range(c, lo, hi);
+      plan.range(c, lo, hi);
       const int len = (int)(hi - lo);
-      for (int j = tid; j < len + kBmT; j += T) {
-        A[j] = entry(s, 0, lo + j);
-        B[j] = entry(s, 1, lo + j);
-      }
+      load(s, lo, (len + kBmT + 3) / 4 * 4, pitch);
       bool nz = false;
       for (int h = 0; h < kBmH; ++h) {
         const int64_t q = s * kBmH + h;
         if (tid == 0) sh.flag = long_wait(&g.gs->pub, (unsigned)(q + 1), g.gs, g.spin);
         __syncthreads();  // also: the previous matrix has been applied
         if (!sh.flag) return;
-        const uint4* src = reinterpret_cast<const uint4*>(ring + q % (2 * kBmH));
-        uint4* dst = reinterpret_cast<uint4*>(&M[0]);
-        for (int w = tid; w < (int)(sizeof(BmMatrix<S>) / 16); w += T) dst[w] = __ldcg(src + w);
+        const uint4* src = reinterpret_cast<const uint4*>(g.ring + q % (2 * kBmH));
+        uint4* dst = reinterpret_cast<uint4*>(&sh.M[0]);
+        for (int w = tid; w < (int)(sizeof(BmMatrix) / 16); w += T) dst[w] = __ldcg(src + w);
         __syncthreads();
         nz = false;
-        bm_apply(f, A, B, M[0], 0, T, tid, len + kBmT - (h + 1) * kBmK, nz, [](int) { __syncthreads(); });
+        bm_apply<P>(red, planes, pitch, sh.M[0], 0, T / 32, warp, len + kBmT - (h + 1) * kBmK, nz,
+                    [](int) { __syncthreads(); });
       }
       __syncthreads();
-      S* oa = buf + ((s + 1) & 1) * 2 * pitch + lo;
-      for (int j = tid; j < len; j += T) {
-        __stcg(oa + j, A[j]);
-        __stcg(oa + pitch + j, B[j]);
-      }
+      uint8_t* dst = g.buf + ((s + 1) & 1) * 2 * L * gpitch + lo;
+      for (int j = 4 * tid; j < len; j += 4 * T)
+#pragma unroll
+        for (int q = 0; q < 2 * L; ++q) {
+          // A chunk's last word may reach into the next chunk's.
+          const uint8_t* w = planes + q * pitch + j;
+          uint8_t* d = dst + q * gpitch + j;
+          if (j + 4 <= len)
+            __stcg(reinterpret_cast<unsigned int*>(d), *reinterpret_cast<const unsigned int*>(w));
+          else
+            for (int e = 0; j + e < len; ++e) d[e] = w[e];
+        }
       __threadfence();
       const bool any = __syncthreads_or(nz);
       if (tid == 0 && !(s == 0 && (int)blockIdx.x == g.skip_cta)) {
         if (any) atomicOr(g.nz + s + 1, 1u);
         __threadfence();
-        if (c < P.front) atomicAdd(&g.gs->front, 1u);
+        if (c < plan.front) atomicAdd(&g.gs->front, 1u);
         atomicAdd(&g.gs->done, 1u);
       }
     }
-    want_done += P.chunks;
+    want_done += plan.chunks;
   }
 }
 
@@ -859,8 +825,13 @@ __global__ void __launch_bounds__(kLongThreads, 1) bm_long_kernel(FieldParams fp
 // ---------------------------------------------------------------------------
 // Host launchers.
 // ---------------------------------------------------------------------------
-int64_t bm_smem_words(uint64_t p, int64_t n) { return (p & 1) && p < (1ULL << 31) ? bm_words<uint32_t>(n) : bm_words<uint64_t>(n); }
-int64_t bm_workspace_words(int64_t n) { return bm_words<uint64_t>(n); }
+static int bm_limbs(uint64_t p) {
+  if (p >= (1ULL << 32)) return 8;
+  if (!(p & 1) || p >= (1ULL << 16)) return 4;
+  return p < (1ULL << 8) ? 1 : 2;
+}
+int64_t bm_smem_words(uint64_t p, int64_t n) { return bm_words(bm_limbs(p), n); }
+int64_t bm_workspace_words(int64_t n) { return bm_words(8, n); }
 
 cudaError_t launch_bm_block(const BmJob& job, uint64_t* gws, int64_t smem_words, int threads, int64_t* d_out,
                             cudaStream_t st) {
@@ -907,25 +878,24 @@ int bm_batch_max_blocks_per_sm(int threads, int64_t smem_words) {
 // Layout of the long kernel's workspace: sync words, nonzero flags per
 // superblock, the ring, the two buffers.
 static size_t long_flags(int64_t n) { return ((size_t)(n / kBmT + 3) * sizeof(unsigned int) + 255) / 256 * 256; }
-static size_t long_ring() { return (2 * kBmH * sizeof(BmMatrix<uint64_t>) + 255) / 256 * 256; }
+static size_t long_ring() { return (2 * kBmH * sizeof(BmMatrix) + 255) / 256 * 256; }
 
 size_t bm_long_bytes(int64_t n) {
-  return 256 + long_flags(n) + long_ring() + (size_t)4 * (n + kBmPad) * sizeof(uint64_t);
+  return 256 + long_flags(n) + long_ring() + (size_t)4 * bm_pitch(n) * sizeof(uint64_t);
 }
 int bm_long_err_offset() { return (int)offsetof(LongSync, err); }
 
-template <class F>
+template <class P>
 static cudaError_t launch_long_t(const FieldParams& fp, const uint64_t* s, int64_t n, int ctas, bool cluster,
                                  void* ws, long long spin, int skip_cta, int64_t* d_out, cudaStream_t st) {
-  using S = typename F::S;
   char* w = static_cast<char*>(ws);
   LongArgs a{};
   a.s = s;
   a.n = n;
   a.gs = reinterpret_cast<LongSync*>(w);
   a.nz = reinterpret_cast<unsigned int*>(w + 256);
-  a.ring = w + 256 + long_flags(n);
-  a.buf = w + 256 + long_flags(n) + long_ring();
+  a.ring = reinterpret_cast<BmMatrix*>(w + 256 + long_flags(n));
+  a.buf = reinterpret_cast<uint8_t*>(w + 256 + long_flags(n) + long_ring());
   a.out = d_out;
   a.spin = spin;
   a.skip_cta = skip_cta;
@@ -934,22 +904,22 @@ static cudaError_t launch_long_t(const FieldParams& fp, const uint64_t* s, int64
   const int64_t fchunks = (front + kBmFront - 1) / kBmFront;
   const int64_t rest = std::max<int64_t>(n - 2 * kBmT, 0);
   const int64_t share = std::max<int64_t>(ctas - 1 - fchunks, 1);
-  const int64_t room = kLongSmem / (2 * (int64_t)sizeof(S)) - kBmT - kBmPad;
+  const int64_t room = kLongSmem / (2 * P::L) - kBmT - kBmPad - 16;
   int64_t cap = ((rest + share - 1) / share + 31) / 32 * 32;
   cap = std::max<int64_t>(std::min(cap, room / 32 * 32), kBmFront);
   a.cap = (int)cap;
-  const size_t smem = (size_t)2 * (cap + kBmT + kBmPad) * sizeof(S);
-  cudaError_t e = cudaFuncSetAttribute(bm_long_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const size_t smem = (size_t)2 * P::L * bm_pitch(cap + kBmT);
+  cudaError_t e = cudaFuncSetAttribute(bm_long_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(ws, 0, 256 + long_flags(n), st);
   if (e != cudaSuccess) return e;
   if (!cluster) {
     FieldParams f = fp;
     void* args[] = {&f, &a};
-    return cudaLaunchCooperativeKernel((void*)bm_long_kernel<F>, dim3(ctas), dim3(kLongThreads), args, smem, st);
+    return cudaLaunchCooperativeKernel((void*)bm_long_kernel<P>, dim3(ctas), dim3(kLongThreads), args, smem, st);
   }
   if (ctas > 8) {
-    e = cudaFuncSetAttribute(bm_long_kernel<F>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    e = cudaFuncSetAttribute(bm_long_kernel<P>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
   }
   cudaLaunchConfig_t cfg = {};
@@ -965,21 +935,25 @@ static cudaError_t launch_long_t(const FieldParams& fp, const uint64_t* s, int64
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int nclusters = 0;
-  e = cudaOccupancyMaxActiveClusters(&nclusters, bm_long_kernel<F>, &cfg);
+  e = cudaOccupancyMaxActiveClusters(&nclusters, bm_long_kernel<P>, &cfg);
   if (e != cudaSuccess) return e;
   if (nclusters < 1) return cudaErrorInvalidConfiguration;
-  return cudaLaunchKernelEx(&cfg, bm_long_kernel<F>, fp, a);
+  return cudaLaunchKernelEx(&cfg, bm_long_kernel<P>, fp, a);
 }
 
 static cudaError_t launch_long(const FieldParams& fp, const uint64_t* s, int64_t n, int ctas, bool cluster, void* ws,
                                long long spin, int skip_cta, int64_t* d_out, cudaStream_t st) {
-  if (fp.p == kM61) return launch_long_t<BmM61>(fp, s, n, ctas, cluster, ws, spin, skip_cta, d_out, st);
-  if (!(fp.p & 1)) return launch_long_t<BmBarrett>(fp, s, n, ctas, cluster, ws, spin, skip_cta, d_out, st);
-  if (fp.p < (1ULL << 28))
-    return launch_long_t<BmMont32<false>>(fp, s, n, ctas, cluster, ws, spin, skip_cta, d_out, st);
-  if (fp.p < (1ULL << 31))
-    return launch_long_t<BmMont32<true>>(fp, s, n, ctas, cluster, ws, spin, skip_cta, d_out, st);
-  return launch_long_t<BmMont64>(fp, s, n, ctas, cluster, ws, spin, skip_cta, d_out, st);
+  const uint64_t p = fp.p;
+#define MODLIN_LONG(P) launch_long_t<P>(fp, s, n, ctas, cluster, ws, spin, skip_cta, d_out, st)
+  using Even32 = BmBarrett<FpSmall, 4>;
+  using Even64 = BmBarrett<FpBarrett, 8>;
+  if (p == kM61) return MODLIN_LONG(BmM61);
+  if (!(p & 1) || (p >> 31 == 1)) return p < (1ULL << 32) ? MODLIN_LONG(Even32) : MODLIN_LONG(Even64);
+  if (p < (1ULL << 8)) return MODLIN_LONG(BmMont32<1>);
+  if (p < (1ULL << 16)) return MODLIN_LONG(BmMont32<2>);
+  if (p < (1ULL << 31)) return MODLIN_LONG(BmMont32<4>);
+  return MODLIN_LONG(BmMont64);
+#undef MODLIN_LONG
 }
 
 cudaError_t launch_bm_long(const FieldParams& fp, const uint64_t* s, int64_t n, int ctas, int num_sms, void* ws,

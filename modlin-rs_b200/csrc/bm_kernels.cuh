@@ -17,13 +17,10 @@ struct BmJob {
   int64_t slot;       // output index
 };
 
-// 64-bit words of the two residual arrays of an n-residue sequence, stored as
-// S (32-bit entries for p < 2^31).
-template <class S>
-MODLIN_HD int64_t bm_words(int64_t n) {
-  return (2 * (n + 64) * (int64_t)sizeof(S) + 7) / 8;
-}
-int64_t bm_smem_words(uint64_t p, int64_t n);  // for the storage type of p
+// 64-bit words of the two residual arrays of an n-residue sequence as byte
+// planes, `limbs` each.
+MODLIN_HD int64_t bm_words(int limbs, int64_t n) { return 2 * limbs * ((n + 160 + 15) / 16 * 16) / 8; }
+int64_t bm_smem_words(uint64_t p, int64_t n);  // for p's limbs
 int64_t bm_workspace_words(int64_t n);         // for any p
 
 constexpr int64_t kBmMaxN = int64_t(1) << 30;  // longest sequence of the one-CTA kernels (32-bit indices)

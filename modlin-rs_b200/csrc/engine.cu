@@ -65,9 +65,9 @@ struct Tune {
   int tc_cross[4] = {64, 64, 64, 64};               // 1, 2, 4, 8 limbs
   int two_panel_min = 256;
   int bm_threads[4] = {256, 512, 512, 512};         // n < 1024, < 4096, < 16384, longer
-  int bm_long_min = 1024;                           // one CTA below, many from here on
+  int bm_long_min = 1300;                           // one CTA below, many from here on
   int bm_cluster_min = 4096;                        // from here on one cluster beats one CTA (not a rule of AUTO)
-  int bm_batch_threads[3] = {128, 256, 512};        // longest < 512, < 2048, longer
+  int bm_batch_threads[3] = {256, 256, 512};        // longest < 512, < 2048, longer
   // Shared memory per batch CTA (KiB), by the same classes: a sequence whose
   // residuals (16 bytes an entry, 8 for p < 2^31) do not fit runs from the
   // CTA's global workspace; smaller caps put more CTAs on an SM.

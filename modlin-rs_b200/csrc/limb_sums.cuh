@@ -56,6 +56,12 @@ struct LimbRed;
 template <>
 struct LimbRed<FpM61, 8> {
   __device__ explicit LimbRed(const FpM61&) {}
+  __device__ __forceinline__ FpM61 field() const { return FpM61(); }
+  // 2^S x mod p for a canonical x.
+  template <int S>
+  __device__ __forceinline__ uint64_t shifted(uint64_t x) const {
+    return ((x << S) & kM61) | (x >> (61 - S));
+  }
   static __device__ __forceinline__ uint64_t last(uint64_t y) {
     const uint64_t x = FpM61::fold(y);
     return x >= kM61 ? x - kM61 : x;
@@ -91,6 +97,11 @@ struct LimbRed<FpSmall, LIMBS> {
     w[1] = (uint32_t)f.reduce64(1ULL << 40);
     w[2] = (uint32_t)f.reduce64(1ULL << 48);
   }
+  __device__ __forceinline__ const FpSmall& field() const { return f; }
+  template <int S>
+  __device__ __forceinline__ uint64_t shifted(uint64_t x) const {
+    return f.reduce64(x << S);  // x < 2^32, S <= 32
+  }
   __device__ __forceinline__ uint64_t lazy(const uint32_t (&a)[2 * LIMBS - 1][4], int c) const { return sum(a, c); }
   __device__ __forceinline__ uint64_t minus(uint64_t v, uint64_t t) const { return f.reduce64(v + kp - t); }
   __device__ __forceinline__ uint64_t sum(const uint32_t (&a)[2 * LIMBS - 1][4], int c) const {
@@ -121,6 +132,11 @@ struct LimbRed<FpBarrett, 8> {
   FpBarrett f;
   uint64_t r64;  // 2^64 mod p
   __device__ explicit LimbRed(const FpBarrett& g) : f(g), r64(g.reduce((u128)1 << 64)) {}
+  __device__ __forceinline__ const FpBarrett& field() const { return f; }
+  template <int S>
+  __device__ __forceinline__ uint64_t shifted(uint64_t x) const {
+    return f.reduce((u128)x << S);
+  }
   __device__ __forceinline__ uint64_t residue(const uint32_t (&a)[15][4], int c) const {
     return finish_wide(f, a, c, r64);
   }

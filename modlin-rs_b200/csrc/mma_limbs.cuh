@@ -112,24 +112,30 @@ __device__ __forceinline__ void tile_k16(uint32_t (&acc)[2 * LIMBS - 1][4], uint
   }
 }
 
-// Bytes i of four residues as one word per limb i: dst[i * plane] (4-byte
-// aligned) for i < LIMBS.
+// Bytes i of four residues as one word per limb i.
 template <int LIMBS>
-__device__ __forceinline__ void put_planes4(uint8_t* dst, int plane, const uint64_t (&v)[4]) {
+__device__ __forceinline__ void limb_words(uint32_t (&w)[LIMBS], const uint64_t (&v)[4]) {
 #pragma unroll
   for (int h = 0; h < (LIMBS > 4 ? 2 : 1); ++h) {
     const uint32_t x0 = (uint32_t)(v[0] >> (32 * h)), x1 = (uint32_t)(v[1] >> (32 * h)),
                    x2 = (uint32_t)(v[2] >> (32 * h)), x3 = (uint32_t)(v[3] >> (32 * h));
     const uint32_t p = __byte_perm(x0, x1, 0x5140), q = __byte_perm(x2, x3, 0x5140);
-    uint8_t* d = dst + 4 * h * plane;
-    *reinterpret_cast<uint32_t*>(d) = __byte_perm(p, q, 0x5410);
-    if (LIMBS > 1) *reinterpret_cast<uint32_t*>(d + plane) = __byte_perm(p, q, 0x7632);
-    if (LIMBS > 2) {
+    w[4 * h] = __byte_perm(p, q, 0x5410);
+    if constexpr (LIMBS > 1) w[4 * h + 1] = __byte_perm(p, q, 0x7632);
+    if constexpr (LIMBS > 2) {
       const uint32_t r = __byte_perm(x0, x1, 0x7362), s = __byte_perm(x2, x3, 0x7362);
-      *reinterpret_cast<uint32_t*>(d + 2 * plane) = __byte_perm(r, s, 0x5410);
-      *reinterpret_cast<uint32_t*>(d + 3 * plane) = __byte_perm(r, s, 0x7632);
+      w[4 * h + 2] = __byte_perm(r, s, 0x5410);
+      w[4 * h + 3] = __byte_perm(r, s, 0x7632);
     }
   }
+}
+// The same, word i to dst[i * plane] (4-byte aligned).
+template <int LIMBS>
+__device__ __forceinline__ void put_planes4(uint8_t* dst, int plane, const uint64_t (&v)[4]) {
+  uint32_t w[LIMBS];
+  limb_words<LIMBS>(w, v);
+#pragma unroll
+  for (int i = 0; i < LIMBS; ++i) *reinterpret_cast<uint32_t*>(dst + i * plane) = w[i];
 }
 
 // The limbs of one residue as single bytes.
