@@ -339,35 +339,34 @@ __device__ __forceinline__ void bm_apply(const LimbRed<typename P::F, P::L>& red
 }
 
 // ---------------------------------------------------------------------------
-// bm_front — the next window and the 32 entries after it (the tile at 0), on
-// the chain of the steps. With 8 limbs warps 0 .. 3 share it: warp w takes
-// source w & 1 and half of A's or B's limbs, and warp 0 adds the four parts
-// (barrier 3; 1300 cycles against 1830 in one warp). With up to 4 limbs warp 0
-// does it alone (700 to 1000 cycles; 1400 to 1600 in four). v is warp 0's.
+// bm_front — the next window (outputs 0 .. 31 as v[0], v[1] of warp 0), on the
+// chain of the steps: kParts warps take a source each, with 8 limbs also half
+// of its limbs each, and warp 0 adds the parts (barrier 3). Cycles in one warp
+// and as it is: 1830 and 980 (8 limbs), 1070 and 805 (4 limbs); with fewer
+// limbs one warp is enough.
 // ---------------------------------------------------------------------------
+template <int L>
+constexpr int bm_front_parts() {
+  return L == 8 ? 4 : L == 4 ? 2 : 1;
+}
 template <class P>
 __device__ __forceinline__ void bm_front(const LimbRed<typename P::F, P::L>& red, const uint8_t* planes, int pitch,
-                                         const BmMatrix& M, uint64_t (*fr)[4][32], int w, uint64_t (&v)[4]) {
-  constexpr int L = P::L, H = L / 2;  // limbs of a warp
-  if constexpr (L <= 4) {
-    if (w == 0) {
-      BmApply<P> ap(red, M);
-      ap.tile(planes, pitch, 0, v);
-      __syncwarp();
-    }
-    return;
-  }
-  const int lane = threadIdx.x & 31, src = w & 1, hi = w >> 1;
+                                         const BmMatrix& M, uint64_t (*fr)[2][32], int w, uint64_t (&v)[2]) {
+  constexpr int L = P::L, kParts = bm_front_parts<L>();
+  constexpr int H = kParts == 4 ? L / 2 : L, kSrc = kParts == 1 ? 2 : 1;  // limbs and sources of a warp
+  const int lane = threadIdx.x & 31, n = lane >> 2, t = lane & 3;
+  const int src0 = w & 1, hi = w >> 1;
   const typename P::F& f = red.field();
   uint32_t acc[2 * L - 1][4];
 #pragma unroll
   for (int d = 0; d < 2 * L - 1; ++d)
 #pragma unroll
     for (int q = 0; q < 4; ++q) acc[d][q] = 0;
-  {
-    const int n = lane >> 2, t = lane & 3;
-    const uint64_t* c = M.c[(n & 1) * 2 + src];
-    for (int wb = M.omin & ~3; wb <= kBmK; wb += 32) {
+  for (int wb = M.omin & ~3; wb <= kBmK; wb += 32) {
+#pragma unroll
+    for (int k = 0; k < kSrc; ++k) {
+      const int src = src0 + k;
+      const uint64_t* c = M.c[(n & 1) * 2 + src];
       uint32_t b[2][L];
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -385,24 +384,33 @@ __device__ __forceinline__ void bm_front(const LimbRed<typename P::F, P::L>& red
 #pragma unroll
         for (int j = 0; j < L; ++j) mml::mma_k32(acc[i + j], a, b[0][j], b[1][j]);
       }
-      if (wb >= 4) break;  // this window covers all offsets
     }
+    if (wb >= 4) break;  // this window covers all offsets
   }
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
+  for (int q = 0; q < 2; ++q) {
     uint64_t x = red.residue(acc, q);
-    if (hi) x = red.template shifted<8 * H>(x);
+    if (kParts == 4 && hi) x = red.template shifted<8 * (L / 2)>(x);
     v[q] = x;
   }
-  if (w != 0) {
+  if constexpr (kParts == 1) {
+    __syncwarp();
+  } else {
+    if (w != 0) {
+      fr[w - 1][0][lane] = v[0];
+      fr[w - 1][1][lane] = v[1];
+      asm volatile("bar.arrive 3, %0;" ::"n"(32 * kParts) : "memory");
+      return;
+    }
+    asm volatile("bar.sync 3, %0;" ::"n"(32 * kParts) : "memory");
 #pragma unroll
-    for (int q = 0; q < 4; ++q) fr[w - 1][q][lane] = v[q];
-    asm volatile("bar.arrive 3, 128;" ::: "memory");
-    return;
+    for (int q = 0; q < 2; ++q) {
+      if constexpr (kParts == 4)
+        v[q] = f.add(f.add(v[q], fr[0][q][lane]), f.add(fr[1][q][lane], fr[2][q][lane]));
+      else
+        v[q] = f.add(v[q], fr[0][q][lane]);
+    }
   }
-  asm volatile("bar.sync 3, 128;" ::: "memory");
-#pragma unroll
-  for (int q = 0; q < 4; ++q) v[q] = f.add(f.add(v[q], fr[0][q][lane]), f.add(fr[1][q][lane], fr[2][q][lane]));
 }
 
 // Entry j from its byte planes.
@@ -425,7 +433,7 @@ __host__ __device__ constexpr int64_t bm_pitch(int64_t n) { return (n + kBmPad +
 
 struct BmShared {
   BmMatrix M[2];
-  uint64_t fr[3][4][32];  // parts of the front tile
+  uint64_t fr[3][2][32];  // parts of the next window
   int64_t l;
   long long job;
   int flag;
@@ -451,7 +459,7 @@ __device__ __forceinline__ bool bm_start(const uint64_t* __restrict__ s, int n, 
 
 // ---------------------------------------------------------------------------
 // One sequence with the whole CTA (blockDim a multiple of 32, at least 128):
-// warps 0 .. 3 compute the next window, then warp 0 runs the next 32 steps
+// the first warps compute the next window, then warp 0 runs the next 32 steps
 // while the others apply the matrix. Per block of 32 steps one barrier of the
 // whole CTA, and one among the applying warps per pass. planes: 2 L of
 // bm_pitch(n) bytes, owned by this CTA.
@@ -477,20 +485,17 @@ __device__ __forceinline__ int64_t bm_run(const P& f, const LimbRed<typename P::
     const int par = (i / kBmK) & 1;
     const BmMatrix& m = sh.M[par];
     const int lim = n - i - kBmK;  // outputs
-    uint64_t v[4];
-    if (warp < 4) bm_front<P>(red, planes, pitch, m, sh.fr, warp, v);
+    uint64_t v[2];
+    if (warp < bm_front_parts<L>()) bm_front<P>(red, planes, pitch, m, sh.fr, warp, v);
     if (warp == 0) {
-      // The first pass's writes wait until the front tile has read its inputs.
-      if (lim > 64) asm volatile("bar.arrive 1, %0;" ::"r"(T) : "memory");
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (lane + 32 * h >= lim) v[2 * h] = v[2 * h + 1] = 0;
-        nz |= v[2 * h] != 0;
-        bm_put<L>(planes, pitch, lane + 32 * h, v[2 * h], v[2 * h + 1]);  // read by no other warp before the barrier
-      }
+      // The first pass's writes wait until the front has read its inputs.
+      if (lim > kBmK) asm volatile("bar.arrive 1, %0;" ::"r"(T) : "memory");
+      if (lane >= lim) v[0] = v[1] = 0;
+      nz |= v[0] != 0;
+      bm_put<L>(planes, pitch, lane, v[0], v[1]);  // read by no other warp before the barrier
       bm_base(f, v[0], v[1], i + kBmK, n, l, &sh.M[par ^ 1]);
     } else {
-      bm_apply<P>(red, planes, pitch, m, 64, T / 32 - 1, warp - 1, lim, nz, [&](int k) {
+      bm_apply<P>(red, planes, pitch, m, kBmK, T / 32 - 1, warp - 1, lim, nz, [&](int k) {
         if (k == 0)
           asm volatile("bar.sync 1, %0;" ::"r"(T) : "memory");
         else
@@ -725,13 +730,12 @@ __global__ void __launch_bounds__(kLongThreads, 1) bm_long_kernel(FieldParams fp
         const BmMatrix& m = sh.M[h & 1];
         const int lim = kBmT - (h + 1) * kBmK;  // outputs inside the window
         const bool more = lim > 0 && i0 + (h + 1) * kBmK < n;
-        uint64_t v[4];
-        if (more && warp < 4) bm_front<P>(red, planes, pitch, m, sh.fr, warp, v);
+        uint64_t v[2];
+        if (more && warp < bm_front_parts<L>()) bm_front<P>(red, planes, pitch, m, sh.fr, warp, v);
         if (warp == 0) {
           if (more) {
-            if (lim > 64) asm volatile("bar.arrive 1, %0;" ::"r"(T - 32) : "memory");
+            if (lim > kBmK) asm volatile("bar.arrive 1, %0;" ::"r"(T - 32) : "memory");
             bm_put<L>(planes, pitch, lane, v[0], v[1]);
-            if (lim > 32) bm_put<L>(planes, pitch, lane + 32, v[2], v[3]);
             bm_base(f, v[0], v[1], i0 + (h + 1) * kBmK, n, l, &sh.M[(h & 1) ^ 1]);
           }
         } else if (warp == T / 32 - 1) {
@@ -747,7 +751,7 @@ __global__ void __launch_bounds__(kLongThreads, 1) bm_long_kernel(FieldParams fp
           }
         } else if (more) {
           bool unused = false;
-          bm_apply<P>(red, planes, pitch, m, 64, T / 32 - 2, warp - 1, lim, unused, [&](int k) {
+          bm_apply<P>(red, planes, pitch, m, kBmK, T / 32 - 2, warp - 1, lim, unused, [&](int k) {
             if (k == 0)
               asm volatile("bar.sync 1, %0;" ::"r"(T - 32) : "memory");
             else
