@@ -100,7 +100,7 @@ struct Ctx {
   DevBuf tcBp[2];   // limb planes of -P^-1 (B operand of the multipliers H = X P^-1), alternating steps
   DevBuf tcX[2];    // limb planes of the block steps' X panels (alternating steps)
   cudaStream_t aux = nullptr;  // look-ahead stream: the next block's inverse
-  cudaEvent_t ev_narrow = nullptr, ev_inv[2] = {nullptr, nullptr};
+  cudaEvent_t ev_narrow = nullptr, ev_diag = nullptr, ev_inv[2] = {nullptr, nullptr};
   PanelState* h_ps = nullptr;
   int2* h_moves = nullptr;
   // linear-complexity workspaces
@@ -257,11 +257,11 @@ static int rank_impl(const RankRun& R, size_t* rank_out) {
   //   W = P^-1 U_next (the next step's wn columns; w x wn, 64 x 64 products),
   //   narrow update A[r0+w .., next columns] -= X W (K = w),
   //   H = X P^-1 (one n x w x w product), wide update A[.., rest] -= H U.
-  // On the second stream, after the narrow update, the chain of step t+1
-  // computes -P^-1 of the next block (one block inverse, or for w = 128 two
-  // inverses and six 64 x 64 products) while the wide update runs. The
-  // critical path per step is chain -> W -> narrow -> next chain; the
-  // multipliers H and the wide update are off it.
+  // On the second stream, after W, the next step's block alone, A - X W, and
+  // from it the chain of step t+1: -P^-1 of that block (one block inverse, or
+  // for w = 128 two inverses and six 64 x 64 products), while the narrow and
+  // wide updates run. The critical path per step is chain -> W -> next block ->
+  // next chain; the updates and the multipliers H are off it.
   // The host queues step t before it knows whether step t's block is
   // invertible: every kernel of step t carries Guard{gbad, t} and does
   // nothing once a chain has recorded a failure at or before t. The host then
@@ -273,12 +273,13 @@ static int rank_impl(const RankRun& R, size_t* rank_out) {
   uint64_t *V11n = nullptr, *Yb = nullptr, *Sb = nullptr, *VSn = nullptr, *Zb = nullptr;
   uint64_t* Pn[2] = {nullptr, nullptr};  // -P^-1 of alternating steps (row stride w)
   uint64_t* Wbuf = Ubuf;                 // W = P^-1 U_next: w rows, row stride n, absolute columns
+  uint64_t* Nb = nullptr;                // the next step's block (row stride wn)
   int* gbad = nullptr;                   // first failed step of the pipeline (0x7f7f7f7f: none)
   int* h_bad = reinterpret_cast<int*>(C->h_out) + 4;  // its value after each step's chain
   uint8_t *tA = nullptr, *tB = nullptr, *tBn = nullptr, *tBp[2] = {nullptr, nullptr}, *tX[2] = {nullptr, nullptr};
   int* terr = C->tcerr.as<int>();
   if (tc) {
-    CK(C->binv.ensure(256 + 14 * blk * 8));
+    CK(C->binv.ensure(256 + 18 * blk * 8));
     CK(C->lbuf.ensure((size_t)n * 2 * kPanel * 8));
     CK(C->ubuf.ensure((size_t)2 * kPanel * n * 8));
     CK(C->tcBn.ensure(tc_b_bytes(2 * kPanel)));
@@ -296,6 +297,7 @@ static int rank_impl(const RankRun& R, size_t* rank_out) {
     Zb = VSn + blk;
     Pn[0] = Zb + blk;   // 128 x 128
     Pn[1] = Pn[0] + 4 * blk;
+    Nb = Pn[1] + 4 * blk;
     tA = C->tcA.as<uint8_t>();
     tB = C->tcB.as<uint8_t>();
     tBn = C->tcBn.as<uint8_t>();
@@ -306,30 +308,30 @@ static int rank_impl(const RankRun& R, size_t* rank_out) {
     if (!C->aux) {
       CK(cudaStreamCreateWithFlags(&C->aux, cudaStreamNonBlocking));
       CK(cudaEventCreateWithFlags(&C->ev_narrow, cudaEventDisableTiming));
+      CK(cudaEventCreateWithFlags(&C->ev_diag, cudaEventDisableTiming));
       CK(cudaEventCreateWithFlags(&C->ev_inv[0], cudaEventDisableTiming));
       CK(cudaEventCreateWithFlags(&C->ev_inv[1], cudaEventDisableTiming));
     }
   }
 
-  // -P^-1 of the 128 x 128 block at (rr, cc) into Pout (row stride 128) on
-  // `s`: P = [[P11, P12], [P21, P22]] in 64 x 64 blocks, V11 = P11^-1,
+  // -P^-1 of the 128 x 128 block at P11 (row stride ldp) into Pout (row stride
+  // 128) on `s`: P = [[P11, P12], [P21, P22]] in 64 x 64 blocks, V11 = P11^-1,
   // S = P22 - P21 V11 P12, and
   // -P^-1 = [[-V11 - Z S^-1 Y, Z S^-1], [S^-1 Y, -S^-1]] with Y = P21 V11,
   // Z = V11 P12: six kernels (programmatic dependent launches chain them).
-  auto prep128 = [&](int rr, int cc, cudaStream_t s, uint64_t* Pout, const Guard& g) -> cudaError_t {
-    const uint64_t* P11 = R.m + (int64_t)rr * ld + cc;
+  auto prep128 = [&](const uint64_t* P11, int64_t ldp, cudaStream_t s, uint64_t* Pout, const Guard& g) -> cudaError_t {
     const uint64_t* P12 = P11 + kPanel;
-    const uint64_t* P21 = P11 + (int64_t)kPanel * ld;
+    const uint64_t* P21 = P11 + (int64_t)kPanel * ldp;
     const uint64_t* P22 = P21 + kPanel;
     uint64_t* const TL = Pout;
     uint64_t* const TR = Pout + kPanel;
     uint64_t* const BL = Pout + 2 * blk;
     uint64_t* const BR = BL + kPanel;
-    launch_block_inverse<F>(f, R.m, ld, rr, cc, V11n, nullptr, s, false, g);
-    const SgProb yz[2] = {{P21, V11n, nullptr, Yb, ld, kPanel, 0, kPanel, 1, kPanel},    // Y = P21 V11
-                          {V11n, P12, nullptr, Zb, kPanel, ld, 0, kPanel, 1, kPanel}};  // Z = V11 P12
+    launch_block_inverse<F>(f, P11, ldp, 0, 0, V11n, nullptr, s, false, g);
+    const SgProb yz[2] = {{P21, V11n, nullptr, Yb, ldp, kPanel, 0, kPanel, 1, kPanel},    // Y = P21 V11
+                          {V11n, P12, nullptr, Zb, kPanel, ldp, 0, kPanel, 1, kPanel}};  // Z = V11 P12
     launch_small_gemm64_batch<F>(f, yz, 2, s, g);
-    launch_small_gemm64<F>(f, Yb, kPanel, P12, ld, P22, ld, Sb, kPanel, true, s, g);  // S = P22 - Y P12
+    launch_small_gemm64<F>(f, Yb, kPanel, P12, ldp, P22, ldp, Sb, kPanel, true, s, g);  // S = P22 - Y P12
     launch_block_inverse<F>(f, Sb, kPanel, 0, 0, VSn, nullptr, s, false, g);
     const SgProb tb[3] = {{Zb, VSn, nullptr, TR, kPanel, kPanel, 0, 2 * kPanel, 1, kPanel},     // Z S^-1
                           {VSn, Yb, nullptr, BL, kPanel, kPanel, 0, 2 * kPanel, 1, kPanel},     // S^-1 Y
@@ -340,17 +342,17 @@ static int rank_impl(const RankRun& R, size_t* rank_out) {
     return cudaGetLastError();
   };
 
-  // Chain of step t on the second stream: -P^-1 of the w x w block at (r, c)
-  // into Pn[t & 1] and its limb planes into tBp[t & 1]; a singular block
-  // records t in gbad. Its kernels are skipped once an earlier step has
+  // Chain of step t on the second stream: -P^-1 of the w x w block at P (row
+  // stride ldp) into Pn[t & 1] and its limb planes into tBp[t & 1]; a singular
+  // block records t in gbad. Its kernels are skipped once an earlier step has
   // failed (Guard step t - 1). The host learns the result from h_bad[t & 1]
   // after ev_inv[t & 1].
-  auto chain = [&](int t, int r, int c, int w) -> int {
+  auto chain = [&](int t, const uint64_t* P, int64_t ldp, int w) -> int {
     const Guard gc{gbad, t - 1};
     if (w == 2 * kPanel) {
-      CK(prep128(r, c, C->aux, Pn[t & 1], gc));
+      CK(prep128(P, ldp, C->aux, Pn[t & 1], gc));
     } else {
-      launch_block_inverse<F>(f, R.m, ld, r, c, Pn[t & 1], nullptr, C->aux, false, gc);
+      launch_block_inverse<F>(f, P, ldp, 0, 0, Pn[t & 1], nullptr, C->aux, false, gc);
       g_launches++;
       CK(cudaGetLastError());
     }
@@ -394,7 +396,7 @@ static int rank_impl(const RankRun& R, size_t* rank_out) {
     CK(cudaEventRecord(C->ev_narrow, st));
     CK(cudaStreamWaitEvent(C->aux, C->ev_narrow, 0));
     int t = 0, r0 = rank_io, c0 = col_io, w = width(r0, c0);
-    if (int rc = chain(0, r0, c0, w)) return rc;
+    if (int rc = chain(0, R.m + (int64_t)r0 * ld + c0, ld, w)) return rc;
     CK(tc_split_a(*R.fp, R.m + c0, ld, 0, r0 + w, n, w, tX[0], st));
     g_launches++;
     for (;;) {
@@ -406,28 +408,46 @@ static int rank_impl(const RankRun& R, size_t* rank_out) {
       CK(cudaStreamWaitEvent(st, C->ev_inv[t & 1], 0));
       if (wn > 0) {
         if (int rc = make_w(Pt, r0, w, c1, wn, g)) return rc;
+        // The next block alone, A - X W for its wn x wn entries, starts the next
+        // chain; the narrow update below computes them again in place.
+        CK(cudaEventRecord(C->ev_narrow, st));
+        CK(cudaStreamWaitEvent(C->aux, C->ev_narrow, 0));
+        {
+          SgProb pr[4];
+          int np = 0;
+          for (int i = 0; i < wn / kPanel; ++i)
+            for (int j = 0; j < wn / kPanel; ++j) {
+              const int rr = r1 + i * kPanel, cc = c1 + j * kPanel;
+              pr[np++] = {R.m + (int64_t)rr * ld + c0, Wbuf + cc, R.m + (int64_t)rr * ld + cc,
+                          Nb + ((int64_t)i * wn + j) * kPanel, ld, n, ld, wn, 1, w};
+            }
+          launch_small_gemm64_batch<F>(f, pr, np, C->aux, g);
+          CK(cudaGetLastError());
+        }
+        CK(cudaEventRecord(C->ev_diag, C->aux));
+        if (int rc = chain(t + 1, Nb, wn, wn)) return rc;
         CK(tc_split_b(*R.fp, Wbuf, n, c1, cw, w, tBn, st, g));
+        // The narrow update writes the block's entries in A, which the product
+        // above reads.
+        CK(cudaStreamWaitEvent(st, C->ev_diag, 0));
         // Over 2^61 - 1 the narrow update also writes the next step's X
         // (its rows from r1 + wn) as limb planes.
         LimbOut lx;
         if (fused) lx = LimbOut{tX[(t + 1) & 1], r1 + wn, wn > kPanel ? 2 * kPanel : kPanel, 0};
-        CK(tc_update(*R.fp, R.m, ld, r1, n, c1, cw, w, tX[t & 1], tBn, C->num_sms, terr, st, g, lx));
-        CK(cudaEventRecord(C->ev_narrow, st));
-        CK(cudaStreamWaitEvent(C->aux, C->ev_narrow, 0));
-        if (int rc = chain(t + 1, r1, c1, wn)) return rc;
+        // One SM stays free for the chain, here and below (a CTA waiting for that
+        // SM would hold up the whole product).
+        CK(tc_update(*R.fp, R.m, ld, r1, n, c1, cw, w, tX[t & 1], tBn, C->num_sms - 1, terr, st, g, lx));
         if (!fused) {
           CK(tc_split_a(*R.fp, R.m + c1, ld, 0, r1 + wn, n, wn, tX[(t + 1) & 1], st, g));
           g_launches++;
         }
-        g_launches += 2;
+        g_launches += 3;
       }
       if (r1 < n && cw < n) {
         // H = X P^-1 = 0 - X (-P^-1) for the rows r1 .. n (relative rows
         // w .. n - r0), as the wide update's A operand. Over 2^61 - 1 the
         // product writes H's limb planes directly; otherwise H goes through
         // Hb and a split.
-        // With a chain running, one SM stays free for it (a CTA waiting for
-        // that SM would hold up the whole product).
         const int ctas = wn > 0 ? C->num_sms - 1 : C->num_sms;
         if (fused) {
           const LimbOut lh{tA, w, w > kPanel ? 2 * kPanel : kPanel, 1};
