@@ -493,7 +493,7 @@ static int rank_impl(const RankRun& R, size_t* rank_out) {
 
   int rank = 0, col = 0;
   bool general_next = false;  // the panel at col had a singular block
-  int empty_left = 1, empty_gap = 1;  // panels without a pivot until the rest is looked at
+  int short_left = 1, short_gap = 1;  // panels with dependent columns until the rest is looked at
   while (col < n && rank < n) {
     if (!general_next && width(rank, col) > 0) {
       if (int rc = run_pipeline(rank, col, general_next)) return rc;
@@ -566,16 +566,18 @@ static int rank_impl(const RankRun& R, size_t* rank_out) {
     }
     rank += pb;
     col = jend;
-    if (pb == 0 && rank < n && col < n && --empty_left == 0) {
-      // A panel without a pivot: when all that is left is zero, so are all
-      // later panels. Looked at after 1, 2, 4, ... such panels.
+    if (pb < W && rank < n && col < n && --short_left == 0) {
+      // A panel with dependent columns: when all that is left is zero, there
+      // are no more pivots. Looked at after 1, 2, 4, ... such panels, so a
+      // matrix with many of them pays a few looks. 3001 x 3001 of rank 1100
+      // over 2^61 - 1: 2068 us waiting for a panel without a pivot, 1947 here.
       int* h_nz = reinterpret_cast<int*>(C->h_out);
       CK(launch_any_nonzero(R.m, ld, rank, col, n, C->tcerr.as<int>() + 2, C->num_sms, st));
       g_launches += 2;
       CK(cudaMemcpyAsync(h_nz, C->tcerr.as<int>() + 2, sizeof(int), cudaMemcpyDeviceToHost, st));
       CK(cudaStreamSynchronize(st));
       if (!*h_nz) col = n;
-      empty_left = empty_gap *= 2;
+      short_left = short_gap *= 2;
     }
     if (R.cb) R.cb(R.cb_ctx, (size_t)col, (size_t)n);
   }
