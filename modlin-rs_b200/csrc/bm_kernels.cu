@@ -253,9 +253,9 @@ __device__ __forceinline__ void bm_frag(BmFrag<L>& fr, const BmMatrix& M, int wb
 }
 
 // Adds the products of the tile at `base` (a multiple of 4) to acc.
-template <int L>
+template <int L, class I>
 __device__ __forceinline__ void bm_tile(uint32_t (&acc)[2 * L - 1][4], const BmFrag<L>& fr, const uint8_t* planes,
-                                        int pitch, int pos) {
+                                        I pitch, I pos) {
   const int lane = threadIdx.x & 31;
   const uint8_t* p0 = planes + pos + 4 * ((lane >> 2) + (lane & 3));
 #pragma unroll
@@ -284,16 +284,17 @@ struct BmApply {
     two = wb == 0;
     bm_frag(fr, M, wb);
   }
-  __device__ __forceinline__ void tile(const uint8_t* planes, int pitch, int base, uint64_t (&v)[4]) {
+  template <class I>
+  __device__ __forceinline__ void tile(const uint8_t* planes, I pitch, I base, uint64_t (&v)[4]) {
     uint32_t acc[2 * L - 1][4];
 #pragma unroll
     for (int d = 0; d < 2 * L - 1; ++d)
 #pragma unroll
       for (int q = 0; q < 4; ++q) acc[d][q] = 0;
-    bm_tile<L>(acc, fr, planes, pitch, base + wb);
+    bm_tile<L, I>(acc, fr, planes, pitch, base + wb);
     if (two) {
       bm_frag(fr, M, 32);
-      bm_tile<L>(acc, fr, planes, pitch, base + 32);
+      bm_tile<L, I>(acc, fr, planes, pitch, base + 32);
       bm_frag(fr, M, 0);
     }
 #pragma unroll
@@ -301,8 +302,8 @@ struct BmApply {
   }
 };
 
-template <int L>
-__device__ __forceinline__ void bm_put(uint8_t* planes, int pitch, int j, uint64_t a, uint64_t b) {
+template <int L, class I>
+__device__ __forceinline__ void bm_put(uint8_t* planes, I pitch, I j, uint64_t a, uint64_t b) {
   mml::put_planes1<L>(planes + j, pitch, a);
   mml::put_planes1<L>(planes + L * pitch + j, pitch, b);
 }
@@ -310,9 +311,9 @@ __device__ __forceinline__ void bm_put(uint8_t* planes, int pitch, int j, uint64
 // Outputs t0 .. lim in place by the `warps` warps of a group (this one: w),
 // two tiles per warp and pass: output j is stored at j and reads reach past it
 // only, so bar(k), the barrier of pass k, separates the reads from the writes.
-template <class P, class Bar>
-__device__ __forceinline__ void bm_apply(const LimbRed<typename P::F, P::L>& red, uint8_t* planes, int pitch,
-                                         const BmMatrix& M, int t0, int warps, int w, int lim, bool& nz, Bar&& bar) {
+template <class P, class I, class Bar>
+__device__ __forceinline__ void bm_apply(const LimbRed<typename P::F, P::L>& red, uint8_t* planes, I pitch,
+                                         const BmMatrix& M, I t0, int warps, int w, I lim, bool& nz, Bar&& bar) {
   constexpr int kPer = 2;
   const int lane = threadIdx.x & 31;
   if (t0 >= lim) return;
@@ -321,7 +322,7 @@ __device__ __forceinline__ void bm_apply(const LimbRed<typename P::F, P::L>& red
     uint64_t v[kPer][4];
 #pragma unroll
     for (int q = 0; q < kPer; ++q) {
-      const int base = t0 + 64 * (q * warps + w);
+      const I base = t0 + 64 * (q * warps + w);
       if (base < lim) ap.tile(planes, pitch, base, v[q]);
     }
     bar(k);
@@ -329,9 +330,9 @@ __device__ __forceinline__ void bm_apply(const LimbRed<typename P::F, P::L>& red
     for (int q = 0; q < kPer; ++q)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int j = t0 + 64 * (q * warps + w) + 32 * h + lane;
+        const I j = t0 + 64 * (q * warps + w) + 32 * h + lane;
         if (j < lim) {
-          bm_put<P::L>(planes, pitch, j, v[q][2 * h], v[q][2 * h + 1]);
+          bm_put<P::L, I>(planes, pitch, j, v[q][2 * h], v[q][2 * h + 1]);
           nz |= v[q][2 * h] != 0;
         }
       }
@@ -349,8 +350,8 @@ template <int L>
 constexpr int bm_front_parts() {
   return L == 8 ? 4 : L == 4 ? 2 : 1;
 }
-template <class P>
-__device__ __forceinline__ void bm_front(const LimbRed<typename P::F, P::L>& red, const uint8_t* planes, int pitch,
+template <class P, class I>
+__device__ __forceinline__ void bm_front(const LimbRed<typename P::F, P::L>& red, const uint8_t* planes, I pitch,
                                          const BmMatrix& M, uint64_t (*fr)[2][32], int w, uint64_t (&v)[2]) {
   constexpr int L = P::L, kParts = bm_front_parts<L>();
   constexpr int H = kParts == 4 ? L / 2 : L, kSrc = kParts == 1 ? 2 : 1;  // limbs and sources of a warp
@@ -414,8 +415,8 @@ __device__ __forceinline__ void bm_front(const LimbRed<typename P::F, P::L>& red
 }
 
 // Entry j from its byte planes.
-template <int L>
-__device__ __forceinline__ uint64_t bm_get(const uint8_t* planes, int pitch, int j) {
+template <int L, class I>
+__device__ __forceinline__ uint64_t bm_get(const uint8_t* planes, I pitch, int j) {
   uint64_t v = 0;
 #pragma unroll
   for (int i = 0; i < L; ++i) v |= (uint64_t)planes[i * pitch + j] << (8 * i);
@@ -440,10 +441,10 @@ struct BmShared {
 };
 
 // Entries [0, n) of the start and zeros behind them, n rounded up to a word.
-template <int L>
-__device__ __forceinline__ bool bm_start(const uint64_t* __restrict__ s, int n, uint8_t* planes, int pitch) {
+template <int L, class I>
+__device__ __forceinline__ bool bm_start(const uint64_t* __restrict__ s, I n, uint8_t* planes, I pitch) {
   bool nz = false;
-  for (int j = 4 * threadIdx.x; j < pitch; j += 4 * blockDim.x) {
+  for (I j = 4 * threadIdx.x; j < pitch; j += 4 * blockDim.x) {
     uint64_t a[4], b[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -462,40 +463,41 @@ __device__ __forceinline__ bool bm_start(const uint64_t* __restrict__ s, int n, 
 // the first warps compute the next window, then warp 0 runs the next 32 steps
 // while the others apply the matrix. Per block of 32 steps one barrier of the
 // whole CTA, and one among the applying warps per pass. planes: 2 L of
-// bm_pitch(n) bytes, owned by this CTA.
+// bm_pitch(n) bytes, owned by this CTA. I: int for planes in shared memory,
+// int64_t for the workspace, where 8 planes of a sequence of 2^28 pass 2^31.
 // ---------------------------------------------------------------------------
-template <class P>
+template <class I, class P>
 __device__ __forceinline__ int64_t bm_run(const P& f, const LimbRed<typename P::F, P::L>& red,
                                           const uint64_t* __restrict__ s, int64_t n64, uint8_t* planes,
                                           BmShared& sh) {
   constexpr int L = P::L;
   const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5;
-  const int n = (int)n64, pitch = (int)bm_pitch(n64);
+  const I n = (I)n64, pitch = (I)bm_pitch(n64);
   bool nz = bm_start<L>(s, n, planes, pitch);
   int64_t l = 0;
   __syncthreads();
   if (warp == 0)
-    bm_base(f, bm_get<L>(planes, pitch, lane), bm_get<L>(planes + L * pitch, pitch, lane), 0, n, l, &sh.M[0]);
-  for (int i = 0;; i += kBmK) {
+    bm_base(f, bm_get<L, I>(planes, pitch, lane), bm_get<L, I>(planes + L * pitch, pitch, lane), 0, n, l, &sh.M[0]);
+  for (I i = 0;; i += kBmK) {
     // Every thread's part of A (steps i on) has been written and tested, and
     // the block's matrix is there.
     const bool any = __syncthreads_or(nz);
     if (!any || i + kBmK >= n) break;
     nz = false;
-    const int par = (i / kBmK) & 1;
+    const int par = (int)(i / kBmK) & 1;
     const BmMatrix& m = sh.M[par];
-    const int lim = n - i - kBmK;  // outputs
+    const I lim = n - i - kBmK;  // outputs
     uint64_t v[2];
-    if (warp < bm_front_parts<L>()) bm_front<P>(red, planes, pitch, m, sh.fr, warp, v);
+    if (warp < bm_front_parts<L>()) bm_front<P, I>(red, planes, pitch, m, sh.fr, warp, v);
     if (warp == 0) {
       // The first pass's writes wait until the front has read its inputs.
       if (lim > kBmK) asm volatile("bar.arrive 1, %0;" ::"r"(T) : "memory");
       if (lane >= lim) v[0] = v[1] = 0;
       nz |= v[0] != 0;
-      bm_put<L>(planes, pitch, lane, v[0], v[1]);  // read by no other warp before the barrier
+      bm_put<L, I>(planes, pitch, lane, v[0], v[1]);  // read by no other warp before the barrier
       bm_base(f, v[0], v[1], i + kBmK, n, l, &sh.M[par ^ 1]);
     } else {
-      bm_apply<P>(red, planes, pitch, m, kBmK, T / 32 - 1, warp - 1, lim, nz, [&](int k) {
+      bm_apply<P, I>(red, planes, pitch, m, kBmK, T / 32 - 1, warp - 1, lim, nz, [&](int k) {
         if (k == 0)
           asm volatile("bar.sync 1, %0;" ::"r"(T) : "memory");
         else
@@ -515,8 +517,8 @@ __device__ __noinline__ int64_t bm_any(const BmJob& job, uint64_t* gws, int64_t 
   const P f(fp);
   const LimbRed<typename P::F, P::L> red{typename P::F(fp)};
   const bool fits = bm_words(P::L, job.n) <= smem_words;
-  if (fits) return bm_run(f, red, job.s, job.n, reinterpret_cast<uint8_t*>(bm_smem), sh);
-  return bm_run(f, red, job.s, job.n, reinterpret_cast<uint8_t*>(gws), sh);
+  if (fits) return bm_run<int>(f, red, job.s, job.n, reinterpret_cast<uint8_t*>(bm_smem), sh);
+  return bm_run<int64_t>(f, red, job.s, job.n, reinterpret_cast<uint8_t*>(gws), sh);
 }
 
 __device__ __forceinline__ int64_t bm_dispatch(const BmJob& job, uint64_t* gws, int64_t smem_words, BmShared& sh) {
@@ -724,18 +726,18 @@ __global__ void __launch_bounds__(kLongThreads, 1) bm_long_kernel(FieldParams fp
       const int64_t i0 = s * kBmT;
       const bool feeds = n - i0 > kBmT;  // later steps need the matrices
       if (warp == 0)
-        bm_base(f, bm_get<L>(planes, pitch, lane), bm_get<L>(planes + L * pitch, pitch, lane), i0, n, l, &sh.M[0]);
+        bm_base(f, bm_get<L, int>(planes, pitch, lane), bm_get<L, int>(planes + L * pitch, pitch, lane), i0, n, l, &sh.M[0]);
       for (int h = 0; h < kBmH && i0 + h * kBmK < n; ++h) {
         __syncthreads();
         const BmMatrix& m = sh.M[h & 1];
         const int lim = kBmT - (h + 1) * kBmK;  // outputs inside the window
         const bool more = lim > 0 && i0 + (h + 1) * kBmK < n;
         uint64_t v[2];
-        if (more && warp < bm_front_parts<L>()) bm_front<P>(red, planes, pitch, m, sh.fr, warp, v);
+        if (more && warp < bm_front_parts<L>()) bm_front<P, int>(red, planes, pitch, m, sh.fr, warp, v);
         if (warp == 0) {
           if (more) {
             if (lim > kBmK) asm volatile("bar.arrive 1, %0;" ::"r"(T - 32) : "memory");
-            bm_put<L>(planes, pitch, lane, v[0], v[1]);
+            bm_put<L, int>(planes, pitch, lane, v[0], v[1]);
             bm_base(f, v[0], v[1], i0 + (h + 1) * kBmK, n, l, &sh.M[(h & 1) ^ 1]);
           }
         } else if (warp == T / 32 - 1) {
@@ -751,7 +753,7 @@ __global__ void __launch_bounds__(kLongThreads, 1) bm_long_kernel(FieldParams fp
           }
         } else if (more) {
           bool unused = false;
-          bm_apply<P>(red, planes, pitch, m, kBmK, T / 32 - 2, warp - 1, lim, unused, [&](int k) {
+          bm_apply<P, int>(red, planes, pitch, m, kBmK, T / 32 - 2, warp - 1, lim, unused, [&](int k) {
             if (k == 0)
               asm volatile("bar.sync 1, %0;" ::"r"(T - 32) : "memory");
             else
@@ -795,7 +797,7 @@ __global__ void __launch_bounds__(kLongThreads, 1) bm_long_kernel(FieldParams fp
         for (int w = tid; w < (int)(sizeof(BmMatrix) / 16); w += T) dst[w] = __ldcg(src + w);
         __syncthreads();
         nz = false;
-        bm_apply<P>(red, planes, pitch, sh.M[0], 0, T / 32, warp, len + kBmT - (h + 1) * kBmK, nz,
+        bm_apply<P, int>(red, planes, pitch, sh.M[0], 0, T / 32, warp, len + kBmT - (h + 1) * kBmK, nz,
                     [](int) { __syncthreads(); });
       }
       __syncthreads();

@@ -19,11 +19,9 @@ struct BmJob {
 
 // 64-bit words of the two residual arrays of an n-residue sequence as byte
 // planes, `limbs` each.
-MODLIN_HD int64_t bm_words(int limbs, int64_t n) { return 2 * limbs * ((n + 160 + 15) / 16 * 16) / 8; }
+MODLIN_HD constexpr int64_t bm_words(int limbs, int64_t n) { return 2 * limbs * ((n + 160 + 15) / 16 * 16) / 8; }
 int64_t bm_smem_words(uint64_t p, int64_t n);  // for p's limbs
 int64_t bm_workspace_words(int64_t n);         // for any p
-
-constexpr int64_t kBmMaxN = int64_t(1) << 30;  // longest sequence of the one-CTA kernels (32-bit indices)
 
 // threads: a multiple of 32 from 128 to 512. gws: workspace of
 // bm_smem_words(p, n) words when that is more than smem_words.

@@ -10,9 +10,9 @@
 // sequence and the result slot, both in device memory.
 //
 // Limits and sharing:
-//  * at most kNoAllocMaxN residues per call (the array holds two arrays of
-//    kNoAllocMaxN words, 4 MiB, which every GPU that loads the library keeps
-//    until exit);
+//  * at most kNoAllocMaxN residues per call (the array holds the byte
+//    planes of two arrays of that many 8-limb residues, 4 MiB, which every
+//    GPU that loads the library keeps until exit);
 //  * every call uses the same array, so calls that overlap on the GPU race:
 //    issue them on one stream (or otherwise order them);
 //  * the array keeps the previous call's contents; the kernel initialises
@@ -40,7 +40,7 @@ namespace modlin {
 constexpr int64_t kNoAllocMaxN = int64_t(1) << 18;
 constexpr int64_t kNoAllocSmemWords = (200 * 1024) / 8;  // shared memory used when the residuals fit
 
-static __device__ __align__(256) uint64_t g_noalloc_scratch[2 * (kNoAllocMaxN + 64)];
+static __device__ __align__(256) uint64_t g_noalloc_scratch[bm_words(8, kNoAllocMaxN)];
 
 static std::mutex g_noalloc_mu;
 static uint64_t* g_noalloc_addr[64];  // device address of the array, per device

@@ -643,7 +643,6 @@ static int lc_device_locked(Ctx* C, uint64_t p, const uint64_t* d_s, size_t n, c
   CK(C->bmout.ensure(sizeof(int64_t) * 4));
   int64_t* d_out = C->bmout.as<int64_t>();
   if (kernel == MODLIN_LC_BLOCK) {
-    if ((int64_t)n > kBmMaxN) return MODLIN_EINVAL_N;
     const int64_t smem_words = (200 * 1024) / 8;
     const int64_t words = bm_smem_words(p, (int64_t)n);
     if (words > smem_words) CK(C->bmws.ensure((size_t)words * 8));
@@ -762,7 +761,6 @@ static int lc_batch_locked(Ctx* C, const uint64_t* p, const uint64_t* const* d_d
   for (size_t i = 0; i < count; ++i) {
     FieldParams fp;
     if (!make_field_params(p[i], &fp)) return MODLIN_EINVAL_P;
-    if ((int64_t)n[i] > kBmMaxN) return MODLIN_EINVAL_N;
     jobs[i] = BmJob{fp.p, fp.mu_lo, fp.mu_hi, fp.safe_batch, d_data[i], (int64_t)n[i], (int64_t)i};
   }
   // Longest first: the persistent CTAs then finish close together (LPT).

@@ -130,8 +130,8 @@ __device__ __forceinline__ void limb_words(uint32_t (&w)[LIMBS], const uint64_t 
   }
 }
 // The same, word i to dst[i * plane] (4-byte aligned).
-template <int LIMBS>
-__device__ __forceinline__ void put_planes4(uint8_t* dst, int plane, const uint64_t (&v)[4]) {
+template <int LIMBS, class I>
+__device__ __forceinline__ void put_planes4(uint8_t* dst, I plane, const uint64_t (&v)[4]) {
   uint32_t w[LIMBS];
   limb_words<LIMBS>(w, v);
 #pragma unroll
@@ -139,8 +139,8 @@ __device__ __forceinline__ void put_planes4(uint8_t* dst, int plane, const uint6
 }
 
 // The limbs of one residue as single bytes.
-template <int LIMBS>
-__device__ __forceinline__ void put_planes1(uint8_t* dst, int plane, uint64_t v) {
+template <int LIMBS, class I>
+__device__ __forceinline__ void put_planes1(uint8_t* dst, I plane, uint64_t v) {
 #pragma unroll
   for (int i = 0; i < LIMBS; ++i) dst[i * plane] = (uint8_t)(v >> (8 * i));
 }
