@@ -196,9 +196,9 @@ int modlin_rank_batch(const modlin_job *jobs, size_t count, size_t *ranks_out);
  * into one persistent launch; larger ones run one after another. */
 int modlin_rank_batch_device(const uint64_t *p, uint64_t *const *d_m, const size_t *n, size_t count,
                              size_t *ranks_out, void *stream);
-/* modlin_rank_batch_device with options: kernel MODLIN_RANK_TC puts every job
- * of side up to 8192 on the tensor-core batch kernel, MODLIN_RANK_PLAIN on the
- * integer-pipe one, MODLIN_RANK_AUTO splits them at the tuned side. */
+/* modlin_rank_batch_device with options (MODLIN_RANK_*): every job
+ * of side up to 8192 is ranked by the one batch kernel whatever the choice;
+ * larger ones run one after another with it. */
 int modlin_rank_batch_device_ex(const uint64_t *p, uint64_t *const *d_m, const size_t *n, size_t count,
                                 const modlin_rank_opts *opts, size_t *ranks_out, void *stream);
 /* Linear complexities of `count` sequences in one persistent launch. */
@@ -300,7 +300,9 @@ int modlin_reduce_device(uint64_t p, uint64_t *d_x, size_t count, void *stream);
  * the limb count itself is the smallest exact one); the remaining-block size
  * below which one-panel block steps replace two-panel ones (timed on a
  * 16384 x 16384 rank); Berlekamp-Massey threads per CTA by length, the
- * block/cluster crossover, and batch threads per CTA by the longest sequence.
+ * lengths from which many CTAs and one cluster beat one CTA (the second is
+ * only reported), and batch threads and shared memory per CTA by the longest
+ * sequence.
  * Takes a few seconds; the choices hold for this process and device. `report`
  * (may be NULL) receives them and the timings as JSON, truncated to cap - 1
  * characters. Before any call, fixed defaults apply. */
@@ -328,7 +330,7 @@ int modlin_set_tc_pairs(int enable);
  * no device waits): the next MODLIN_LC_GRID launch in this process bounds
  * each grid-barrier wait by spin_cycles (1 .. 4e9) instead of ~1 s, and its
  * CTA skip_cta (a CTA the launch has: 0 always is) does not arrive at the
- * first step's barrier, so every wait expires, the kernel returns early and
+ * first exchange, so every wait expires, the kernel returns early and
  * the call reports MODLIN_ETIMEOUT. Nothing faults or hangs. */
 int modlin_testing_grid_timeout_once(long long spin_cycles, int skip_cta);
 /* Milliseconds spent in the trailing-update kernels of the last rank call,

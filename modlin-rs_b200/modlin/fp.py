@@ -159,8 +159,9 @@ def rank_batch(items) -> list[int]:
 
 def rank_batch_device(ps, ptrs, ns, stream: int = 0, kernel: str = "auto") -> list[int]:
     """Device-resident batch: ``ptrs[i]`` points at an ``ns[i]`` x ``ns[i]``
-    matrix mod ``ps[i]`` (clobbered). ``kernel``: "auto" (tuned split),
-    "tc" (tensor-core batch kernel) or "plain"."""
+    matrix mod ``ps[i]`` (clobbered). ``kernel`` ("auto", "tc" or
+    "plain") is the choice for sides above 8192; smaller ones share one
+    batch kernel."""
     k = len(ptrs)
     P = (ctypes.c_uint64 * max(k, 1))(*ps)
     D = (ctypes.c_void_p * max(k, 1))(*ptrs)
