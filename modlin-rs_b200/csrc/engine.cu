@@ -691,7 +691,6 @@ static int rank_batch_locked(Ctx* C, const uint64_t* p, uint64_t* const* d_m, co
   if (count == 0) return MODLIN_OK;
   std::vector<RankJob> jobs;
   std::vector<size_t> big;
-  int64_t maxn = 0;
   for (size_t i = 0; i < count; ++i) {
     if (n[i] == 0) {
       ranks_out[i] = 0;
@@ -704,17 +703,16 @@ static int rank_batch_locked(Ctx* C, const uint64_t* p, uint64_t* const* d_m, co
     FieldParams fp;
     make_field_params(p[i], &fp);
     jobs.push_back(RankJob{fp.p, fp.mu_lo, fp.mu_hi, fp.safe_batch, d_m[i], (int64_t)n[i], (int64_t)i});
-    maxn = std::max<int64_t>(maxn, (int64_t)n[i]);
   }
   if (!jobs.empty()) {
     sort_rank_jobs(jobs);
-    const RankBatchShape B = rank_batch_shape((int64_t)jobs.size(), maxn, C->num_sms);
+    const RankBatchShape B = rank_batch_shape(jobs, C->num_sms);
     if (B.blocks < 1) return MODLIN_ECUDA;
     CK(C->rbjobs.ensure(sizeof(RankJob) * jobs.size()));
-    CK(C->bmnext.ensure(sizeof(unsigned long long)));
+    CK(C->bmnext.ensure(kRankBatchCounters * sizeof(unsigned long long)));
     CK(C->rbout.ensure(sizeof(int64_t) * count));
     CK(cudaMemcpyAsync(C->rbjobs.p, jobs.data(), sizeof(RankJob) * jobs.size(), cudaMemcpyHostToDevice, st));
-    CK(launch_rank_batch(C->rbjobs.as<RankJob>(), (int64_t)jobs.size(), C->bmnext.as<unsigned long long>(), maxn, B,
+    CK(launch_rank_batch(C->rbjobs.as<RankJob>(), (int64_t)jobs.size(), C->bmnext.as<unsigned long long>(), B,
                          C->rbout.as<int64_t>(), st));
     g_launches += 2;
     std::vector<int64_t> out(count);
@@ -1738,7 +1736,7 @@ int modlin_plain_mac_peak(uint64_t p, double* modmac_per_s) {
 
 struct modlin_rank_batch_plan {
   int device;
-  int64_t count, max_n;
+  int64_t count;
   modlin::RankBatchShape shape;
   int64_t* out;  // caller's device array
   modlin::DevBuf jobs, next;
@@ -1761,25 +1759,22 @@ int modlin_rank_batch_plan_new(const uint64_t* p, uint64_t* const* d_m, const si
   int rc = get_ctx(&C);
   if (rc) return rc;
   std::vector<RankJob> jobs;
-  int64_t maxn = 1;
   for (size_t i = 0; i < count; ++i) {
     FieldParams fp;
     if (!make_field_params(p[i], &fp)) return MODLIN_EINVAL_P;
     if ((int64_t)n[i] > kRankBatchMaxN) return MODLIN_EINVAL_N;
     if (n[i] && !d_m[i]) return MODLIN_EINVAL_ARG;
     jobs.push_back(RankJob{fp.p, fp.mu_lo, fp.mu_hi, fp.safe_batch, d_m[i], (int64_t)n[i], (int64_t)i});
-    maxn = std::max<int64_t>(maxn, (int64_t)n[i]);
   }
   sort_rank_jobs(jobs);
   std::unique_ptr<modlin_rank_batch_plan> P(new modlin_rank_batch_plan());
   P->device = C->device;
   P->count = (int64_t)count;
-  P->max_n = maxn;
   P->out = d_ranks_out;
-  P->shape = rank_batch_shape((int64_t)count, maxn, C->num_sms);
+  P->shape = rank_batch_shape(jobs, C->num_sms);
   if (count && P->shape.blocks < 1) return MODLIN_ECUDA;
   CK(P->jobs.ensure(std::max<size_t>(jobs.size(), 1) * sizeof(RankJob)));
-  CK(P->next.ensure(sizeof(unsigned long long)));
+  CK(P->next.ensure(kRankBatchCounters * sizeof(unsigned long long)));
   if (count) CK(cudaMemcpy(P->jobs.p, jobs.data(), jobs.size() * sizeof(RankJob), cudaMemcpyHostToDevice));
   *plan_out = P.release();
   return MODLIN_OK;
@@ -1789,8 +1784,7 @@ int modlin_rank_batch_plan_launch(modlin_rank_batch_plan* P, void* stream) {
   if (!P) return MODLIN_EINVAL_ARG;
   if (P->count == 0) return MODLIN_OK;
   cudaStream_t st = user_stream(stream);
-  CK(launch_rank_batch(P->jobs.as<RankJob>(), P->count, P->next.as<unsigned long long>(), P->max_n, P->shape, P->out,
-                       st));
+  CK(launch_rank_batch(P->jobs.as<RankJob>(), P->count, P->next.as<unsigned long long>(), P->shape, P->out, st));
   g_launches += 2;
   return MODLIN_OK;
 }

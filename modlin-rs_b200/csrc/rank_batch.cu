@@ -19,70 +19,17 @@
 // Every residue is exact, so the rank is the reference's.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <climits>
+#include <functional>
+#include <queue>
+#include <vector>
 
-#include "block_inv.cuh"
-#include "field.cuh"
-#include "mma_limbs.cuh"
-#include "rank_batch.cuh"
+#include "rank_batch_dev.cuh"
 
 namespace modlin {
 
 namespace {
-
-constexpr int kP = 64;  // panel width
-constexpr int kG = 8;   // rows per warp in flight during the in-panel elimination
-constexpr int kStride = 80;                // bytes per row of a 64-deep limb plane
-constexpr int kPlane = kP * kStride;       // one limb plane of a 64 x 64 tile
-constexpr int kRegion = 8 * kPlane;        // 8 limb planes: 40 KiB
-
-// Lazy accumulation of products of residues: u128 sums reduced once per
-// safe_batch products in general; for p < 2^32 a product fits in 32 x 32 ->
-// 64 bits, so the sums stay in a u64 and are reduced once per
-// floor((2^64 - 1) / (p - 1)^2) products (at least 1; p < 2^31 gives >= 4).
-// A reduced sum (< p) counts as one product.
-template <class F>
-struct Acc {
-  using T = u128;
-  __device__ static T prod(const F& f, uint64_t a, uint64_t b) { return f.prod(a, b); }
-  __device__ static uint64_t reduce(const F& f, T x) { return f.reduce(x); }
-  __device__ static uint64_t batch(const F& f) { return f.safe_batch(); }
-};
-template <>
-struct Acc<FpSmall> {
-  using T = uint64_t;
-  __device__ static T prod(const FpSmall&, uint64_t a, uint64_t b) { return (uint64_t)(uint32_t)a * (uint32_t)b; }
-  __device__ static uint64_t reduce(const FpSmall& f, T x) { return f.reduce64(x); }
-  __device__ static uint64_t batch(const FpSmall& f) {
-    const uint64_t q = f.modulus() - 1;
-    return q <= 1 ? UINT64_MAX : UINT64_MAX / (q * q);
-  }
-};
-
-// Regions of shared memory: `a` holds the block being inverted, then the left
-// operand's planes, or LF on the panel path; `b` the inverse's scratch, then
-// the right operand's planes, or Us; `a2` (one CTA an SM) the left operand's
-// second buffer.
-struct BatchSmem {
-  alignas(16) uint8_t b[kRegion];
-  alignas(16) uint8_t a[kRegion];
-  uint64_t prow[kP];  // pivot row's panel segment
-  int pcol[kP];
-  int red[16];
-  uint64_t inv;
-  int found;
-  long long job;
-};
-static_assert(sizeof(InvScratch<8>) <= kRegion && kP * kInvLd * 8 <= kRegion && kP * (kP + 1) * 8 <= kRegion, "");
-
-// Diagonal sums of the 16 x 8 tile (row group rg, column group cg) of the
-// 64 x 64 product of the planes at A and B.
-template <int LIMBS>
-__device__ __forceinline__ void block_tile(uint32_t (&acc)[2 * LIMBS - 1][4], const uint8_t* A, const uint8_t* B,
-                                           int rg, int cg) {
-  mml::tile_k32<LIMBS, 2, kStride>(acc, mml::saddr(A) + rg * 16 * kStride, kPlane, mml::saddr(B) + cg * 8 * kStride,
-                                   kPlane);
-}
 
 // One block step at (r0, c0); false when P is not invertible (nothing has
 // changed but the order of the 64 rows). any: something right of and below
@@ -508,23 +455,94 @@ static int batch_threads(int64_t count, int64_t max_n, int num_sms) {
   return count <= num_sms || max_n >= kRankBatchWideN ? 512 : 256;
 }
 
-RankBatchShape rank_batch_shape(int64_t count, int64_t max_n, int num_sms) {
-  RankBatchShape B{0, 0};
-  if (rank_batch_attr() != cudaSuccess) return B;
-  B.threads = batch_threads(count, max_n, num_sms);
-  const size_t smem = rank_batch_smem_bytes(B.threads, max_n);
+// Running time of a job on a team of `size`, relative to one CTA: the block
+// inverses are not shared. Their part measured 0.22 and 0.53 at sides 1024 and
+// 512 of 16 bits, 0.17 and 0.44 of 31, 0.12 and 0.32 over 2^61 - 1.
+static double team_time(const RankJob& j, int size) {
+  const double k = j.p < (1ULL << 16) ? 240 : j.p < (1ULL << 32) ? 200 : 150;
+  const double fixed = std::min(1.0, k / (double)j.n);
+  return fixed + (1 - fixed) / size;
+}
+
+// About the end of a batch (jobs longest first, costs `cost`) whose first
+// `shared` jobs go to `teams` teams of `size` CTAs and the others, `rest` in
+// all, to the CTAs as they become free. Above `best`: a lower bound of it.
+static double batch_end(const std::vector<RankJob>& jobs, const std::vector<double>& cost, size_t shared, int size,
+                        int teams, double rest, double best) {
+  double sum = 0;
+  for (size_t i = 0; i < shared; ++i) sum += cost[i] * team_time(jobs[i], size);
+  const double area = (sum * size + rest) / (teams * size);
+  if (area >= best) return area;
+  std::priority_queue<double, std::vector<double>, std::greater<double>> t(std::greater<double>(),
+                                                                           std::vector<double>(teams, 0.0));
+  double last = area;
+  for (size_t i = 0; i < shared; ++i) {
+    const double e = t.top() + cost[i] * team_time(jobs[i], size);
+    t.pop();
+    t.push(e);
+    last = std::max(last, e);
+  }
+  if (shared < cost.size()) last = std::max(last, t.top() + cost[shared]);
+  return last;
+}
+
+RankBatchShape rank_batch_shape(const std::vector<RankJob>& jobs, int num_sms) {
+  RankBatchShape B{};
+  const int64_t count = (int64_t)jobs.size();
+  if (count == 0 || rank_batch_attr() != cudaSuccess) return B;
+  B.max_n = 1;
+  double total = 0, longest = 0;
+  for (const RankJob& j : jobs) {
+    B.max_n = std::max(B.max_n, j.n);
+    const double c = rank_batch_cost(j.p, j.n);
+    total += c;
+    longest = std::max(longest, c);
+  }
+  B.threads = batch_threads(count, B.max_n, num_sms);
+  B.cluster = 1;
+  const size_t smem = rank_batch_smem_bytes(B.threads, B.max_n);
   int nb = 0;
   if (B.threads == 512)
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rank_batch_kernel<512>, 512, smem);
   else
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rank_batch_kernel<256>, 256, smem);
-  B.blocks = (int)(count < (int64_t)nb * num_sms ? count : (int64_t)nb * num_sms);
+  B.blocks = (int)std::min<int64_t>(count, (int64_t)nb * num_sms);
+  // Teams when the longest job is more than an SM's share of the batch (it
+  // would be the batch's end): of the candidates, the one with the earliest
+  // end, when that is 15 % before the end without. 512 matrices of sides 64 to
+  // 1024 over four primes: 12.9 ms without, 9.4 with; 40 of side 1024 over
+  // 2^61 - 1: 11.0 and 6.3; 100 of them stay without. Sides below 4 tiles gain
+  // nothing.
+  const double share = total / num_sms;
+  if (B.threads != 512 || nb < 1 || longest <= share) return B;
+  std::vector<double> cost(count);
+  for (int64_t i = 0; i < count; ++i) cost[i] = rank_batch_cost(jobs[i].p, jobs[i].n);
+  const int* teams = rank_team_resident(num_sms);
+  double best = 0.85 * longest;
+  for (int k = 0; k < 3; ++k) {
+    if (teams[k] < 1) continue;
+    int64_t shared = 0;
+    double rest = total;
+    for (const double over : {2.0, 1.5, 1.0, 0.75, 0.5}) {
+      const int64_t before = shared;
+      for (; shared < count && cost[shared] > over * share && jobs[shared].n >= 4 * kP; ++shared) rest -= cost[shared];
+      if (shared == before) continue;
+      const double end = batch_end(jobs, cost, (size_t)shared, 2 << k, teams[k], rest, best);
+      if (end < best) {
+        best = end;
+        B.cluster = 2 << k;
+        B.shared = shared;
+        B.blocks = teams[k] * B.cluster;
+      }
+    }
+  }
   return B;
 }
 
-cudaError_t launch_rank_batch(const RankJob* d_jobs, int64_t count, unsigned long long* d_next, int64_t max_n,
+cudaError_t launch_rank_batch(const RankJob* d_jobs, int64_t count, unsigned long long* d_next,
                               const RankBatchShape& B, int64_t* d_out, cudaStream_t st) {
-  const size_t smem = rank_batch_smem_bytes(B.threads, max_n);
+  if (B.shared) return launch_rank_team(d_jobs, count, d_next, B, d_out, st);
+  const size_t smem = rank_batch_smem_bytes(B.threads, B.max_n);
   cudaError_t e = rank_batch_attr();
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(d_next, 0, sizeof(unsigned long long), st);
@@ -539,7 +557,7 @@ cudaError_t launch_rank_batch(const RankJob* d_jobs, int64_t count, unsigned lon
 // Modular multiply-adds of a limb class relative to one-limb primes, roughly:
 // the batch takes its longest jobs first.
 double rank_batch_cost(uint64_t p, int64_t n) {
-  const double w = p < (1ULL << 16) ? 1.0 : p < (1ULL << 32) ? 1.3 : p == kM61 ? 2.2 : 5.0;
+  const double w = p < (1ULL << 16) ? 1.0 : p < (1ULL << 32) ? 1.45 : p == kM61 ? 2.65 : 5.0;
   return w * (double)n * n * (n + 200);
 }
 

@@ -4,6 +4,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <vector>
 
 namespace modlin {
 
@@ -23,12 +24,21 @@ constexpr int64_t kRankBatchWideN = 384;
 
 struct RankBatchShape {
   int threads, blocks;
+  int cluster;     // CTAs per team
+  int64_t shared;  // jobs (the first ones) that teams take
+  int64_t max_n;
 };
-// Launch shape for `count` jobs of sides up to max_n; blocks 0 on an error.
-RankBatchShape rank_batch_shape(int64_t count, int64_t max_n, int num_sms);
+// Launch shape for jobs sorted longest first; blocks 0 on an error.
+RankBatchShape rank_batch_shape(const std::vector<RankJob>& jobs, int num_sms);
 // Relative running time of a job.
 double rank_batch_cost(uint64_t p, int64_t n);
-cudaError_t launch_rank_batch(const RankJob* d_jobs, int64_t count, unsigned long long* d_next, int64_t max_n,
+constexpr int kRankBatchCounters = 2;  // job counters at d_next
+cudaError_t launch_rank_batch(const RankJob* d_jobs, int64_t count, unsigned long long* d_next,
                               const RankBatchShape& shape, int64_t* d_out, cudaStream_t st);
+// The same for a shape with teams, and the teams of 2, 4 and 8 CTAs that the
+// GPU holds at a time.
+cudaError_t launch_rank_team(const RankJob* d_jobs, int64_t count, unsigned long long* d_next,
+                             const RankBatchShape& shape, int64_t* d_out, cudaStream_t st);
+const int* rank_team_resident(int num_sms);
 
 }  // namespace modlin

@@ -1,0 +1,574 @@
+// Batched rank with teams: the longest matrices of a batch are each shared by
+// the CTAs of a thread-block cluster, which then take the other matrices one
+// by one. For batches whose longest matrix would be their end (the rule is
+// rank_batch_shape's).
+//
+// A team's CTAs each invert the step's block (the same work, no exchange) and
+// take every size-th tile of 64 rows of the panel and of the rest; one cluster
+// barrier a step orders their writes before the next step's reads. A panel
+// without a block step is eliminated by the first CTA alone, its update of the
+// rest is again the team's. The control flow is the same in all CTAs of a team:
+// they compute what decides it from the same data, which no CTA writes before
+// a cluster barrier, or get it from the first. 1016 x 1016 over 2^61 - 1: 11.55
+// ms on one CTA, 2.83 on eight.
+//
+// The steps are those of rank_batch.cu. That kernel stays for batches without
+// teams: it is up to 9 % faster there for p < 2^32 (148 of side 512 mod 65521:
+// 0.86 ms, 0.94 here).
+#include <cooperative_groups.h>
+#include <cuda_runtime.h>
+
+#include <climits>
+
+#include "rank_batch_dev.cuh"
+
+namespace modlin {
+
+namespace cg = cooperative_groups;
+
+namespace {
+
+constexpr int kT = 512;
+constexpr int kMaxCluster = 8;  // portable cluster size
+
+// The CTAs of a cluster that work on one matrix: how many (1: no exchange at
+// all) and which one this is.
+struct Team {
+  int size, rank;
+};
+
+struct TeamSmem : BatchSmem {
+  // Written by the cluster's CTAs: whether something nonzero is left (by
+  // parity of the exchange and CTA), and the panel path's pivots.
+  int nz[2][kMaxCluster];
+  int panel_pivots;
+  Team team;
+};
+
+// The CTA's shared memory: TeamSmem, the left operand's second buffer, the row
+// order.
+extern __shared__ __align__(16) unsigned char rb_smem[];
+__device__ __forceinline__ TeamSmem& batch_smem() { return *reinterpret_cast<TeamSmem*>(rb_smem); }
+__device__ __forceinline__ uint8_t* second_buffer() { return rb_smem + sizeof(TeamSmem); }
+__device__ __forceinline__ int* row_order() { return reinterpret_cast<int*>(second_buffer() + kRegion); }
+
+// A warp's tiles of a 64 x 64 output: rows 16 rg .. +16, kTiles groups of 8
+// columns from cg0; and a thread's share of a left operand (64 rows of 64).
+struct TileMap {
+  static constexpr int kTiles = 32 / (kT / 32), kRound = kT / 16, kN = kP / kRound;
+};
+
+// Left operand: rows rt .. rt + 63, columns c0 .. c0 + 63, through registers.
+__device__ __forceinline__ void load_rows(const uint64_t* __restrict__ m, int n, const int* perm, int c0, int rt,
+                                          uint64_t (&v)[TileMap::kN][4]) {
+  const int tid = threadIdx.x;
+#pragma unroll
+  for (int w = 0; w < TileMap::kN; ++w) {
+    const int i = (tid >> 4) + TileMap::kRound * w, k4 = 4 * (tid & 15);
+    const uint64_t* src = rt + i < n ? m + (int64_t)perm[rt + i] * n + c0 + k4 : nullptr;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[w][u] = src ? src[u] : 0;
+  }
+}
+template <int LIMBS>
+__device__ __forceinline__ void put_rows(uint8_t* dst, const uint64_t (&v)[TileMap::kN][4]) {
+  const int tid = threadIdx.x;
+#pragma unroll
+  for (int w = 0; w < TileMap::kN; ++w)
+    mml::put_planes4<LIMBS>(dst + ((tid >> 4) + TileMap::kRound * w) * kStride + 4 * (tid & 15), kPlane, v[w]);
+}
+
+// C += H U for the row tiles of 64 at rb, rb + stride, .. and the columns from
+// cb: H in columns c0 .. c0 + 63 of those rows, U the first pb of the rows at r0
+// (H's other columns are zero). Whether this thread wrote something nonzero.
+// A function of its own: its registers are the products'.
+template <class F, int LIMBS>
+__device__ __noinline__ bool update_rest(const F& fr, uint64_t* __restrict__ m, const int n, int r0, int pb, int rb,
+                                         int stride, int c0, int cb) {
+  TeamSmem& S = batch_smem();
+  uint8_t* const a2 = second_buffer();
+  int* const perm = row_order();
+  const F f = fr;
+  const LimbRed<F, LIMBS> red(f);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int kTiles = TileMap::kTiles, kN = TileMap::kN;
+  constexpr bool kEarly = LIMBS <= 4;
+  const int rg = warp & 3, cg0 = (warp >> 2) * kTiles;
+  const int g = lane >> 2, t2 = 2 * (lane & 3);
+  uint8_t* const bufs[2] = {S.a, a2};
+  uint32_t acc[2 * LIMBS - 1][4];
+  uint64_t lv[kN][4];
+  // Past the pivots H is zero: any of U's rows will do.
+  const auto row = [pb](int k) { return k < pb ? k : 0; };
+  // Trailing update by strips of kCols column tiles whose right operands fill
+  // region b: the left operand's load and the barriers are shared by them.
+  constexpr int kCols = LIMBS == 8 ? 1 : LIMBS == 4 ? 2 : 4;
+  bool nz = false;
+  for (int ct = cb; ct < n && rb < n; ct += kP * kCols) {
+    __syncthreads();
+    constexpr int kRows4 = kT / 64;
+#pragma unroll 1
+    for (int s = 0; s < kCols; ++s) {
+      uint64_t uv[kN][4];
+      const int col = ct + kP * s + (tid & 63);
+#pragma unroll
+      for (int w = 0; w < kN; ++w)  // U: plane row = column
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          uv[w][u] = col < n ? m[(int64_t)perm[r0 + row(4 * ((tid >> 6) + kRows4 * w) + u)] * n + col] : 0;
+#pragma unroll
+      for (int w = 0; w < kN; ++w)
+        mml::put_planes4<LIMBS>(S.b + s * LIMBS * kPlane + (tid & 63) * kStride + 4 * ((tid >> 6) + kRows4 * w),
+                                kPlane, uv[w]);
+    }
+    if (kEarly) load_rows(m, n, perm, c0, rb, lv);
+    for (int rt = rb, k = 0; rt < n; rt += stride, k ^= 1) {
+      const int ra = rt + 16 * rg + g, rz = ra + 8;
+      uint64_t* pa = ra < n ? m + (int64_t)perm[ra] * n : nullptr;
+      uint64_t* pz = rz < n ? m + (int64_t)perm[rz] * n : nullptr;
+      // C of this warp's tiles is loaded before the left operand where
+      // registers allow, else before each tile's products (which cover it).
+      constexpr bool kAhead = LIMBS <= 4;
+      constexpr int kAll = kTiles * kCols;
+      uint64_t cv[kAhead ? kAll : 1][4];
+      const auto column = [&](int q) { return ct + kP * (q / kTiles) + 8 * (cg0 + q % kTiles) + t2; };
+      const auto load_c = [&](int q, uint64_t (&x)[4]) {
+        const int c = column(q);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const uint64_t* src = e < 2 ? pa : pz;
+          x[e] = src && c + (e & 1) < n ? src[c + (e & 1)] : 0;
+        }
+      };
+      if (kAhead) {
+#pragma unroll
+        for (int q = 0; q < kAll; ++q) load_c(q, cv[q]);
+      }
+      if (!kEarly) load_rows(m, n, perm, c0, rt, lv);
+      put_rows<LIMBS>(bufs[k], lv);
+      __syncthreads();
+      if (kEarly && rt + stride < n) load_rows(m, n, perm, c0, rt + stride, lv);
+#pragma unroll(kAhead ? kAll : 1)
+      for (int q = 0; q < kAll; ++q) {
+        const int c = column(q);
+        uint64_t(&x)[4] = cv[kAhead ? q : 0];
+        if (!kAhead) load_c(q, x);
+        block_tile<LIMBS>(acc, bufs[k], S.b + q / kTiles * LIMBS * kPlane, rg, cg0 + q % kTiles);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          uint64_t* dst = e < 2 ? pa : pz;
+          const uint64_t v = red.plus(x[e], acc, e);
+          if (dst && c + (e & 1) < n) {
+            dst[c + (e & 1)] = v;
+            nz |= v != 0;
+          }
+        }
+      }
+    }
+  }
+  return nz;
+}
+
+// Whether any CTA of the team has something nonzero left.
+__device__ __forceinline__ bool team_any(TeamSmem& S, int c0, bool any) {
+  // Two buffers: the next step's writes come before every CTA has read these
+  // (other paths to an exchange have cluster barriers of their own).
+  const int parity = (c0 / kP) & 1;
+  cg::cluster_group cl = cg::this_cluster();
+  if (threadIdx.x < S.team.size) cl.map_shared_rank(&S, threadIdx.x)->nz[parity][S.team.rank] = any;
+  cl.sync();
+  for (int q = 0; q < S.team.size; ++q) any |= S.nz[parity][q] != 0;
+  return any;
+}
+
+// One block step at (r0, c0); false when P is not invertible (nothing has
+// changed but the order of the 64 rows). any: something right of and below
+// the block is nonzero afterwards.
+// Bound: 8 x 64 x 64 limb-product instructions per tile and 2^61 - 1 (8192 of
+// an SM's cycles), the epilogue and the conversions for fewer limbs.
+// A team's CTAs each invert P (the same work, no exchange) and take every
+// size-th tile of 64 rows: H over their rows of X, then their rows of C. One
+// cluster barrier a step orders their writes before the next step's reads.
+template <class F, int LIMBS, bool kTeam>
+__device__ __noinline__ bool block_step(const F& f, uint64_t* __restrict__ m, const int n, int r0, int c0, bool& any) {
+  TeamSmem& S = batch_smem();
+  uint8_t* const a2 = second_buffer();
+  int* const perm = row_order();
+  const int first = kTeam ? kP * S.team.rank : 0;  // of this CTA's row tiles, after the block
+  const int stride = kTeam ? kP * S.team.size : kP;
+  const LimbRed<F, LIMBS> red(f);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint64_t p = f.modulus();
+  uint64_t* M = reinterpret_cast<uint64_t*>(S.a);
+  InvScratch<LIMBS>& I = *reinterpret_cast<InvScratch<LIMBS>*>(S.b);
+  for (int q = tid; q < kP * kP; q += kT) M[(q >> 6) * kInvLd + (q & 63)] = m[(int64_t)perm[r0 + (q >> 6)] * n + c0 + (q & 63)];
+  __syncthreads();
+  if (!inv64<F, LIMBS, kT>(f, red, M, I)) return false;
+  uint64_t fac[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) fac[u] = I.fac[u];
+  const int moved = tid < kP ? perm[r0 + I.order[tid]] : 0;
+  __syncthreads();
+  if (tid < kP) perm[r0 + tid] = moved;
+  // Right operand: -P^-1, plane row = column of P^-1.
+  for (int q = tid; q < kP * 16; q += kT) {
+    const int i = q & 63, k4 = 4 * (q >> 6);
+    const uint64_t fk = k4 < 32 ? (k4 < 16 ? fac[0] : fac[1]) : (k4 < 48 ? fac[2] : fac[3]);
+    uint64_t v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      v[u] = f.mul(M[(k4 + u) * kInvLd + i], fk);
+      v[u] = v[u] ? p - v[u] : 0;
+    }
+    mml::put_planes4<LIMBS>(S.b + i * kStride + k4, kPlane, v);
+  }
+  const int rb = r0 + kP + first, cb = c0 + kP;  // this CTA's first row tile
+  // This warp's tiles: rows 16 rg .. +16, kTiles groups of 8 columns from cg0.
+  constexpr int kTiles = TileMap::kTiles;
+  const int rg = warp & 3, cg0 = (warp >> 2) * kTiles;
+  const int g = lane >> 2, t2 = 2 * (lane & 3);
+  constexpr int kN = TileMap::kN;
+  // The next tile's rows are loaded during this one's products where the
+  // registers allow; with two buffers one barrier a tile is enough.
+  constexpr bool kEarly = LIMBS <= 4;
+  uint8_t* const bufs[2] = {S.a, a2};
+  uint32_t acc[2 * LIMBS - 1][4];
+  uint64_t lv[kN][4];
+  if (cb < n && rb < n && kEarly) load_rows(m, n, perm, c0, rb, lv);
+  for (int rt = rb, k = 0; rt < n && cb < n; rt += stride, k ^= 1) {  // H over X
+    if (!kEarly) load_rows(m, n, perm, c0, rt, lv);
+    if (rt == rb) __syncthreads();  // the last product has read the buffer (or P^-1)
+    put_rows<LIMBS>(bufs[k], lv);
+    __syncthreads();
+    if (kEarly && rt + stride < n) load_rows(m, n, perm, c0, rt + stride, lv);
+    const int ra = rt + 16 * rg + g, rz = ra + 8;
+    uint64_t* pa = ra < n ? m + (int64_t)perm[ra] * n + c0 : nullptr;
+    uint64_t* pz = rz < n ? m + (int64_t)perm[rz] * n + c0 : nullptr;
+#pragma unroll 1
+    for (int q = 0; q < kTiles; ++q) {
+      block_tile<LIMBS>(acc, bufs[k], S.b, rg, cg0 + q);
+      const int c = 8 * (cg0 + q) + t2;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        uint64_t* dst = e < 2 ? pa : pz;
+        const uint64_t v = red.residue(acc, e);
+        if (dst) dst[c + (e & 1)] = v;
+      }
+    }
+  }
+  const bool nz = rb < n && cb < n &&
+                  update_rest<F, LIMBS>(f, m, n, r0, kP, rb, stride, c0, cb);
+  any = __syncthreads_or(nz);
+  if constexpr (kTeam) any = team_any(S, c0, any);
+  return true;
+}
+
+template <class F, int LIMBS, bool kTeam>
+__device__ __noinline__ int rank_one(const F& f, uint64_t* __restrict__ m, const int n) {
+  TeamSmem& S = batch_smem();
+  int* const perm = row_order();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  using A = Acc<F>;
+  using AT = typename A::T;
+  const uint64_t p = f.modulus();
+  const uint64_t sb = A::batch(f);
+  uint64_t(*LF)[kP + 1] = reinterpret_cast<uint64_t(*)[kP + 1]>(S.a);  // multipliers of a row tile, or F[k][k2]
+  uint64_t(*Us)[kP] = reinterpret_cast<uint64_t(*)[kP]>(S.b);          // U block of one 64-column tile
+  for (int i = tid; i < n; i += kT) perm[i] = i;
+  __syncthreads();
+  int r0 = 0;
+  for (int c0 = 0; c0 < n && r0 < n; c0 += kP) {
+    const int W = min(kP, n - c0);
+    if (W == kP && n - r0 >= kP) {
+      // A block without a pivot (4 / p of the invertible ones, the dependent
+      // ones always) is tried again with the next 64 rows, and once more.
+      bool any = false, step = false;
+      for (int t = 1;; ++t) {
+        step = block_step<F, LIMBS, kTeam>(f, m, n, r0, c0, any);
+        if (step || t == 3 || n - r0 < (t + 1) * kP) break;
+        // The rows of the failed block are written by the next attempt's step.
+        if constexpr (kTeam) cg::this_cluster().sync();
+        if (tid < kP) {
+          const int o = perm[r0 + tid];
+          perm[r0 + tid] = perm[r0 + t * kP + tid];
+          perm[r0 + t * kP + tid] = o;
+        }
+        __syncthreads();
+      }
+      if (step) {
+        r0 += kP;
+        if (!any) break;
+        continue;
+      }
+      __syncthreads();
+    }
+    int pb = 0;
+    // The panel path is the team's first CTA's, which may write once no other
+    // reads the block it failed on.
+    const bool mine = !kTeam || S.team.rank == 0;
+    if constexpr (kTeam) cg::this_cluster().sync();
+    // ---- A. in-panel elimination ------------------------------------------
+    for (int kk = 0; mine && kk < W && r0 + pb < n; ++kk) {
+      const int c = c0 + kk, r = r0 + pb;
+      int best = INT_MAX;
+      for (int i = r + tid; i < n; i += kT)
+        if (m[(int64_t)perm[i] * n + c] != 0) {
+          best = i;
+          break;
+        }
+      best = __reduce_min_sync(0xffffffffu, best);
+      if (lane == 0) S.red[warp] = best;
+      __syncthreads();
+      if (tid == 0) {
+        int b = INT_MAX;
+        for (int w = 0; w < kT / 32; ++w) b = min(b, S.red[w]);
+        S.found = b != INT_MAX;
+        if (b != INT_MAX) {
+          const int t = perm[r];
+          perm[r] = perm[b];
+          perm[b] = t;
+          S.pcol[pb] = c;
+          const uint64_t e = m[(int64_t)perm[r] * n + c];
+          S.inv = std::is_same<F, FpM61>::value ? fp_inv_m61(e) : fp_inv_binary(e, p);
+        }
+      }
+      __syncthreads();
+      if (!S.found) continue;
+      const uint64_t* P = m + (int64_t)perm[r] * n + c0;
+      if (tid < W) S.prow[tid] = P[tid];
+      __syncthreads();
+      // Rows below, kG per warp at a time: lane l holds panel entries l and
+      // l + 32 of each of its rows (coalesced loads, all issued before any
+      // is used), so each group costs one memory round trip.
+      const uint64_t inv = S.inv;
+      const uint64_t pv0 = lane > kk && lane < W ? S.prow[lane] : 0;
+      const uint64_t pv1 = lane + 32 > kk && lane + 32 < W ? S.prow[lane + 32] : 0;
+      for (int base = r + 1 + warp; base < n; base += kT / 32 * kG) {
+        uint64_t* R[kG];
+        uint64_t x0[kG], x1[kG];
+#pragma unroll
+        for (int g = 0; g < kG; ++g) {
+          const int i = base + g * (kT / 32);
+          R[g] = i < n ? m + (int64_t)perm[i] * n + c0 : nullptr;
+          x0[g] = R[g] && lane < W ? R[g][lane] : 0;
+          x1[g] = R[g] && lane + 32 < W ? R[g][lane + 32] : 0;
+        }
+#pragma unroll
+        for (int g = 0; g < kG; ++g) {
+          const uint64_t e = __shfl_sync(0xffffffffu, kk < 32 ? x0[g] : x1[g], kk & 31);
+          if (e == 0) continue;  // uniform across the warp
+          const uint64_t fm = f.mul(e, inv);
+          if (lane > kk && lane < W) R[g][lane] = f.sub(x0[g], f.mul(fm, pv0));
+          if (lane + 32 > kk && lane + 32 < W) R[g][lane + 32] = f.sub(x1[g], f.mul(fm, pv1));
+          if (lane == (kk & 31)) R[g][kk] = fm;
+        }
+      }
+      __syncthreads();
+      ++pb;
+    }
+    const int jend = c0 + W;
+    if (mine && pb > 0 && jend < n && r0 + pb < n) {
+      // ---- B. U, in place, per 64-column tile ------------------------------
+      for (int idx = tid; idx < pb * pb; idx += kT) {  // pivot rows' multipliers F[k][k2] (k2 < k)
+        const int k = idx / pb, k2 = idx - k * pb;
+        LF[k][k2] = k2 < k ? m[(int64_t)perm[r0 + k] * n + S.pcol[k2]] : 0;
+      }
+      for (int ct = jend; ct < n; ct += kP) {
+        for (int idx = tid; idx < pb * kP; idx += kT) {
+          const int k = idx >> 6, ci = idx & 63;
+          const int cc = ct + ci;
+          Us[k][ci] = cc < n ? m[(int64_t)perm[r0 + k] * n + cc] : 0;
+        }
+        __syncthreads();
+        {
+          // U_k -= sum_{k2<k} F[k][k2] U_k2, kQ threads per column.
+          constexpr int kQ = kT / kP;
+          const int ci = tid / kQ, q = tid % kQ;
+          for (int k = 1; k < pb; ++k) {
+            AT acc = 0;
+            uint64_t tot = 0, cnt = 0;
+            for (int k2 = q; k2 < k; k2 += kQ) {
+              acc += A::prod(f, LF[k][k2], Us[k2][ci]);
+              if (++cnt >= sb) {
+                tot = f.add(tot, A::reduce(f, acc));
+                acc = 0;
+                cnt = 0;
+              }
+            }
+            uint64_t part = f.add(tot, A::reduce(f, acc));
+#pragma unroll
+            for (int o = 1; o < kQ; o <<= 1) part = f.add(part, __shfl_xor_sync(0xffffffffu, part, o));
+            if (q == 0) Us[k][ci] = f.sub(Us[k][ci], part);
+            __syncwarp();
+          }
+        }
+        __syncthreads();
+        for (int idx = tid; idx < pb * kP; idx += kT) {
+          const int k = idx >> 6, cc = ct + (idx & 63);
+          if (cc < n) m[(int64_t)perm[r0 + k] * n + cc] = Us[k][idx & 63];
+        }
+        __syncthreads();
+      }
+      // H: the multipliers negated, in the panel's first pb columns, zeros
+      // behind them. A warp per row.
+      for (int i = r0 + pb + warp; i < n; i += kT / 32) {
+        uint64_t* R = m + (int64_t)perm[i] * n;
+        uint64_t h0 = lane < pb ? R[S.pcol[lane]] : 0, h1 = lane + 32 < pb ? R[S.pcol[lane + 32]] : 0;
+        __syncwarp();
+        R[c0 + lane] = h0 ? p - h0 : 0;
+        R[c0 + lane + 32] = h1 ? p - h1 : 0;
+      }
+    }
+    __syncthreads();
+    if constexpr (kTeam) {
+      // The pivots and the row order for the others.
+      cg::cluster_group cl = cg::this_cluster();
+      if (mine && tid < S.team.size) cl.map_shared_rank(&S, tid)->panel_pivots = pb;
+      cl.sync();
+      if (!mine) {
+        const int* src = cl.map_shared_rank(perm, 0);
+        for (int i = tid; i < n; i += kT) perm[i] = src[i];
+      }
+      pb = S.panel_pivots;
+      cl.sync();
+    }
+    // ---- C. trailing rows, as in a block step --------------------------------
+    if (pb > 0) {
+      bool nz = false;
+      if (jend < n) {
+        const int rb = r0 + pb + (kTeam ? kP * S.team.rank : 0);
+        if (rb < n)
+          nz = update_rest<F, LIMBS>(f, m, n, r0, pb, rb, kTeam ? kP * S.team.size : kP, c0,
+                                         jend);
+        nz = __syncthreads_or(nz);
+        if constexpr (kTeam) nz = team_any(S, c0, nz);
+      }
+      r0 += pb;
+      if (!nz) break;
+    }
+  }
+  return r0;
+}
+
+template <bool kTeam>
+__device__ __forceinline__ int rank_any(const RankJob& J) {
+  const FieldParams fp{J.p, J.mu_lo, J.mu_hi, J.safe_batch};
+  const int n = (int)J.n;
+  if (J.p == kM61) return rank_one<FpM61, 8, kTeam>(FpM61(fp), J.m, n);
+  if (J.p < (1ULL << 32)) {
+    const FpSmall f(fp);
+    return J.p <= (1ULL << 8)    ? rank_one<FpSmall, 1, kTeam>(f, J.m, n)
+           : J.p <= (1ULL << 16) ? rank_one<FpSmall, 2, kTeam>(f, J.m, n)
+                                 : rank_one<FpSmall, 4, kTeam>(f, J.m, n);
+  }
+  return rank_one<FpBarrett, 8, kTeam>(FpBarrett(fp), J.m, n);
+}
+
+// The first `shared` jobs (the longest) go to the clusters; then each CTA takes
+// the others one by one, from a second counter.
+__global__ void __launch_bounds__(kT, 1)
+    rank_team_kernel(const RankJob* __restrict__ jobs, int64_t count, int64_t shared, unsigned long long* next,
+                      int64_t* out) {
+  TeamSmem& S = batch_smem();
+  const Team& team = S.team;
+  if (threadIdx.x == 0) {
+    S.team.size = (int)cg::this_cluster().num_blocks();
+    S.team.rank = (int)cg::this_cluster().block_rank();
+  }
+  __syncthreads();
+  for (;;) {
+    long long q;
+    if (team.size > 1) {
+      cg::cluster_group cl = cg::this_cluster();
+      if (team.rank == 0 && threadIdx.x == 0) {
+        const long long t = (long long)atomicAdd(next, 1ULL);
+        for (int c = 0; c < team.size; ++c) cl.map_shared_rank(&S, c)->job = t;
+      }
+      cl.sync();
+      q = S.job;
+      cl.sync();  // the next job's number, and the next matrix, come after
+      if (q >= shared) {
+        // No CTA touches another's shared memory from here on.
+        __syncthreads();
+        if (threadIdx.x == 0) S.team = Team{1, 0};
+        __syncthreads();
+        continue;
+      }
+    } else {
+      if (threadIdx.x == 0) S.job = shared + (long long)atomicAdd(next + 1, 1ULL);
+      __syncthreads();
+      q = S.job;
+      __syncthreads();
+      if (q >= count) break;
+    }
+    const RankJob J = jobs[q];
+    int r;
+    if (team.size > 1)
+      r = rank_any<true>(J);
+    else
+      r = rank_any<false>(J);
+    if (threadIdx.x == 0 && team.rank == 0) out[J.slot] = r;
+    __syncthreads();
+  }
+}
+
+}  // namespace
+
+static size_t team_smem_bytes(int64_t max_n) { return sizeof(TeamSmem) + kRegion + (size_t)max_n * sizeof(int); }
+
+static cudaError_t team_attr() {
+  static const cudaError_t e = cudaFuncSetAttribute(rank_team_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                    (int)team_smem_bytes(kRankBatchMaxN));
+  return e;
+}
+
+static cudaLaunchConfig_t team_config(int size, int blocks, size_t smem, cudaStream_t st, cudaLaunchAttribute* attr) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(512);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = size;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+// Teams of 2, 4 and 8 CTAs that the GPU holds at a time.
+const int* rank_team_resident(int num_sms) {
+  struct Teams {
+    int n[3] = {0, 0, 0};
+  };
+  static const Teams t = [num_sms] {
+    Teams q;
+    if (team_attr() != cudaSuccess) return q;
+    for (int k = 0; k < 3; ++k) {
+      cudaLaunchAttribute attr[1];
+      const int size = 2 << k;
+      const cudaLaunchConfig_t cfg =
+          team_config(size, num_sms / size * size, team_smem_bytes(kRankBatchMaxN), nullptr, attr);
+      if (cudaOccupancyMaxActiveClusters(&q.n[k], rank_team_kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        q.n[k] = 0;
+      }
+    }
+    return q;
+  }();
+  return t.n;
+}
+
+cudaError_t launch_rank_team(const RankJob* d_jobs, int64_t count, unsigned long long* d_next,
+                             const RankBatchShape& B, int64_t* d_out, cudaStream_t st) {
+  cudaError_t e = team_attr();
+  if (e != cudaSuccess) return e;
+  e = cudaMemsetAsync(d_next, 0, kRankBatchCounters * sizeof(unsigned long long), st);
+  if (e != cudaSuccess) return e;
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = team_config(B.cluster, B.blocks, team_smem_bytes(B.max_n), st, attr);
+  return cudaLaunchKernelEx(&cfg, rank_team_kernel, d_jobs, count, B.shared, d_next, d_out);
+}
+
+}  // namespace modlin
