@@ -475,7 +475,9 @@ __global__ void __launch_bounds__(kT, 1)
     S.team.size = (int)cg::this_cluster().num_blocks();
     S.team.rank = (int)cg::this_cluster().block_rank();
   }
-  __syncthreads();
+  // Every CTA of the cluster has started before the first write to another's
+  // shared memory, the job's number below.
+  cg::this_cluster().sync();
   for (;;) {
     long long q;
     if (team.size > 1) {
