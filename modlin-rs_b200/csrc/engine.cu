@@ -184,6 +184,13 @@ struct RankRun {
   int two_panel_min;  // smallest remaining block (rows) for two-panel steps (tensor-core path)
 };
 
+// Smallest prime with block steps. Below it most blocks have none: the four 16 x
+// 16 blocks that the inverse passes through are all invertible for 0.7 % of
+// uniform blocks mod 2 and 10 % mod 3, and each failure costs an inverse and a
+// host answer. 1000 x 1000 mod 2: 7.5 ms with attempts, 3.8 without; mod 3 6.0
+// and 3.8; mod 5 4.8 with, 3.8 on the plain path.
+constexpr uint64_t kBlockMinPrime = 5;
+
 static bool use_tc(const RankRun& R) {
   if (R.kernel == MODLIN_RANK_PLAIN) return false;
   if (R.kernel == MODLIN_RANK_TC) return true;
@@ -379,8 +386,9 @@ static int rank_impl(const RankRun& R, size_t* rank_out) {
   };
 
   const bool fused = tc && tc_limb_out_supported(R.fp->p);  // limb planes from the epilogues
+  const bool blocks = tc && R.fp->p >= kBlockMinPrime;
   auto width = [&](int r, int c) -> int {
-    if (!tc) return 0;
+    if (!blocks) return 0;
     if (n - r >= R.two_panel_min && n - c >= 2 * kPanel && n - r >= 2 * kPanel) return 2 * kPanel;
     if (n - c >= kPanel && n - r >= kPanel) return kPanel;
     return 0;
