@@ -689,9 +689,12 @@ static int lc_device_locked(Ctx* C, uint64_t p, const uint64_t* d_s, size_t n, c
 // (longest first), larger ones through the single-matrix engine afterwards.
 // Longest first: the persistent CTAs then finish close together (LPT).
 static void sort_rank_jobs(std::vector<RankJob>& jobs) {
-  std::stable_sort(jobs.begin(), jobs.end(), [](const RankJob& a, const RankJob& b) {
-    return rank_batch_cost(a.p, a.n) > rank_batch_cost(b.p, b.n);
-  });
+  std::vector<std::pair<double, size_t>> key(jobs.size());
+  for (size_t i = 0; i < jobs.size(); ++i) key[i] = {-rank_batch_cost(jobs[i].p, jobs[i].n), i};
+  std::sort(key.begin(), key.end());
+  std::vector<RankJob> sorted(jobs.size());
+  for (size_t i = 0; i < jobs.size(); ++i) sorted[i] = jobs[key[i].second];
+  jobs.swap(sorted);
 }
 
 static int rank_batch_locked(Ctx* C, const uint64_t* p, uint64_t* const* d_m, const size_t* n, size_t count,

@@ -37,8 +37,8 @@ namespace {
 // Bound: 8 x 64 x 64 limb-product instructions per tile and 2^61 - 1 (8192 of
 // an SM's cycles), the epilogue and the conversions for fewer limbs.
 template <class F, int LIMBS, int kT>
-__device__ bool block_step(const F& f, uint64_t* __restrict__ m, const int n, int* perm, BatchSmem& S, uint8_t* a2,
-                           int r0, int c0, bool& any) {
+__device__ __forceinline__ bool block_step_body(const F& f, uint64_t* __restrict__ m, const int n, int* perm,
+                                                BatchSmem& S, uint8_t* a2, int r0, int c0, bool& any) {
   const LimbRed<F, LIMBS> red(f);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint64_t p = f.modulus();
@@ -185,28 +185,51 @@ __device__ bool block_step(const F& f, uint64_t* __restrict__ m, const int n, in
   return true;
 }
 
+// As a function of its own its registers are the products' (148 matrices of side
+// 512 mod 65521: 795 -> 770 us); only four limbs on 512 threads are faster
+// within rank_one (979 us, 1027 on their own).
+template <class F, int LIMBS, int kT>
+__device__ __noinline__ bool block_step_call(const F& f, uint64_t* __restrict__ m, const int n, int* perm,
+                                             BatchSmem& S, uint8_t* a2, int r0, int c0, bool& any) {
+  return block_step_body<F, LIMBS, kT>(f, m, n, perm, S, a2, r0, c0, any);
+}
+template <class F, int LIMBS, int kT>
+__device__ __forceinline__ bool block_step(const F& f, uint64_t* __restrict__ m, const int n, int* perm, BatchSmem& S,
+                                           uint8_t* a2, int r0, int c0, bool& any) {
+  if constexpr (LIMBS == 4 && kT == 512)
+    return block_step_body<F, LIMBS, kT>(f, m, n, perm, S, a2, r0, c0, any);
+  else
+    return block_step_call<F, LIMBS, kT>(f, m, n, perm, S, a2, r0, c0, any);
+}
+
+// The CTA's shared memory: BatchSmem, the left operand's second buffer (one CTA
+// an SM), the row order.
+extern __shared__ __align__(16) unsigned char rb_smem[];
+template <int NT>
+struct OneCta {
+  static constexpr int kT = NT;
+  static __device__ __forceinline__ BatchSmem& smem() { return *reinterpret_cast<BatchSmem*>(rb_smem); }
+  static __device__ __forceinline__ uint8_t* a2() { return rb_smem + sizeof(BatchSmem); }
+  static __device__ __forceinline__ int* perm() { return reinterpret_cast<int*>(a2() + (NT == 512 ? kRegion : 0)); }
+};
+
 template <class F, int LIMBS, int kT>
 __device__ __noinline__ int rank_one(const F& f, uint64_t* __restrict__ m, const int n, int* perm, BatchSmem& S,
                                      uint8_t* a2) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  using A = Acc<F>;
-  using AT = typename A::T;
+  const int tid = threadIdx.x;
   const uint64_t p = f.modulus();
-  const uint64_t sb = A::batch(f);
-  uint64_t(*LF)[kP + 1] = reinterpret_cast<uint64_t(*)[kP + 1]>(S.a);  // multipliers of a row tile, or F[k][k2]
-  uint64_t(*Us)[kP] = reinterpret_cast<uint64_t(*)[kP]>(S.b);          // U block of one 64-column tile
   for (int i = tid; i < n; i += kT) perm[i] = i;
   __syncthreads();
   int r0 = 0;
   for (int c0 = 0; c0 < n && r0 < n; c0 += kP) {
     const int W = min(kP, n - c0);
-    if (W == kP && n - r0 >= kP) {
-      // A block without a pivot (4 / p of the invertible ones, the dependent
-      // ones always) is tried again with the next 64 rows, and once more.
+    const int tries = block_tries(p, n - r0);
+    if (W == kP && n - r0 >= kP && tries > 0) {
+      // A block without a pivot is tried again with the next 64 rows.
       bool any = false, step = false;
       for (int t = 1;; ++t) {
         step = block_step<F, LIMBS, kT>(f, m, n, perm, S, a2, r0, c0, any);
-        if (step || t == 3 || n - r0 < (t + 1) * kP) break;
+        if (step || t == tries || n - r0 < (t + 1) * kP) break;
         if (tid < kP) {
           const int o = perm[r0 + tid];
           perm[r0 + tid] = perm[r0 + t * kP + tid];
@@ -221,172 +244,13 @@ __device__ __noinline__ int rank_one(const F& f, uint64_t* __restrict__ m, const
       }
       __syncthreads();
     }
-    int pb = 0;
-    // ---- A. in-panel elimination ------------------------------------------
-    for (int kk = 0; kk < W && r0 + pb < n; ++kk) {
-      const int c = c0 + kk, r = r0 + pb;
-      int best = INT_MAX;
-      for (int i = r + tid; i < n; i += kT)
-        if (m[(int64_t)perm[i] * n + c] != 0) {
-          best = i;
-          break;
-        }
-      best = __reduce_min_sync(0xffffffffu, best);
-      if (lane == 0) S.red[warp] = best;
-      __syncthreads();
-      if (tid == 0) {
-        int b = INT_MAX;
-        for (int w = 0; w < kT / 32; ++w) b = min(b, S.red[w]);
-        S.found = b != INT_MAX;
-        if (b != INT_MAX) {
-          const int t = perm[r];
-          perm[r] = perm[b];
-          perm[b] = t;
-          S.pcol[pb] = c;
-          const uint64_t e = m[(int64_t)perm[r] * n + c];
-          S.inv = std::is_same<F, FpM61>::value ? fp_inv_m61(e) : fp_inv_binary(e, p);
-        }
-      }
-      __syncthreads();
-      if (!S.found) continue;
-      const uint64_t* P = m + (int64_t)perm[r] * n + c0;
-      if (tid < W) S.prow[tid] = P[tid];
-      __syncthreads();
-      // Rows below, kG per warp at a time: lane l holds panel entries l and
-      // l + 32 of each of its rows (coalesced loads, all issued before any
-      // is used), so each group costs one memory round trip.
-      const uint64_t inv = S.inv;
-      const uint64_t pv0 = lane > kk && lane < W ? S.prow[lane] : 0;
-      const uint64_t pv1 = lane + 32 > kk && lane + 32 < W ? S.prow[lane + 32] : 0;
-      for (int base = r + 1 + warp; base < n; base += kT / 32 * kG) {
-        uint64_t* R[kG];
-        uint64_t x0[kG], x1[kG];
-#pragma unroll
-        for (int g = 0; g < kG; ++g) {
-          const int i = base + g * (kT / 32);
-          R[g] = i < n ? m + (int64_t)perm[i] * n + c0 : nullptr;
-          x0[g] = R[g] && lane < W ? R[g][lane] : 0;
-          x1[g] = R[g] && lane + 32 < W ? R[g][lane + 32] : 0;
-        }
-#pragma unroll
-        for (int g = 0; g < kG; ++g) {
-          const uint64_t e = __shfl_sync(0xffffffffu, kk < 32 ? x0[g] : x1[g], kk & 31);
-          if (e == 0) continue;  // uniform across the warp
-          const uint64_t fm = f.mul(e, inv);
-          if (lane > kk && lane < W) R[g][lane] = f.sub(x0[g], f.mul(fm, pv0));
-          if (lane + 32 > kk && lane + 32 < W) R[g][lane + 32] = f.sub(x1[g], f.mul(fm, pv1));
-          if (lane == (kk & 31)) R[g][kk] = fm;
-        }
-      }
-      __syncthreads();
-      ++pb;
-    }
+    const int pb = eliminate_panel<F, LIMBS, OneCta<kT>>(f, m, n, r0, c0, W);
     if (pb == 0) continue;
     const int jend = c0 + W;
     bool nz = false;
     if (jend < n && r0 + pb < n) {
-      // ---- B + C. per 64-column tile: U block, then the trailing rows ------
-      const int tx = tid & 15, ty = tid >> 4;
-      for (int ct = jend; ct < n; ct += kP) {
-        // Pivot rows' multipliers F[k][k2] (k2 < k) and their tile of U.
-        for (int idx = tid; idx < pb * pb; idx += kT) {
-          const int k = idx / pb, k2 = idx - k * pb;
-          LF[k][k2] = k2 < k ? m[(int64_t)perm[r0 + k] * n + S.pcol[k2]] : 0;
-        }
-        for (int idx = tid; idx < pb * kP; idx += kT) {
-          const int k = idx >> 6, ci = idx & 63;
-          const int cc = ct + ci;
-          Us[k][ci] = cc < n ? m[(int64_t)perm[r0 + k] * n + cc] : 0;
-        }
-        __syncthreads();
-        {
-          // U_k -= sum_{k2<k} F[k][k2] U_k2, kQ threads per column.
-          constexpr int kQ = kT / kP;
-          const int ci = tid / kQ, q = tid % kQ;
-          for (int k = 1; k < pb; ++k) {
-            AT acc = 0;
-            uint64_t tot = 0, cnt = 0;
-            for (int k2 = q; k2 < k; k2 += kQ) {
-              acc += A::prod(f, LF[k][k2], Us[k2][ci]);
-              if (++cnt >= sb) {
-                tot = f.add(tot, A::reduce(f, acc));
-                acc = 0;
-                cnt = 0;
-              }
-            }
-            uint64_t part = f.add(tot, A::reduce(f, acc));
-#pragma unroll
-            for (int o = 1; o < kQ; o <<= 1) part = f.add(part, __shfl_xor_sync(0xffffffffu, part, o));
-            if (q == 0) Us[k][ci] = f.sub(Us[k][ci], part);
-            __syncwarp();
-          }
-        }
-        __syncthreads();
-        for (int rt = r0 + pb; rt < n; rt += kP) {
-          // Multipliers of the row tile: LF[k][ri] = m[row][pcol[k]].
-          for (int idx = tid; idx < pb * kP; idx += kT) {
-            const int ri = idx / pb, k = idx - ri * pb;
-            const int rr = rt + ri;
-            LF[k][ri] = rr < n ? m[(int64_t)perm[rr] * n + S.pcol[k]] : 0;
-          }
-          __syncthreads();
-          constexpr int kI = kP / (kT / 16);  // rows per thread
-          // A reduced accumulator (< p <= (p-1)^2 + 1) counts as one product,
-          // so sb terms never overflow the u128.
-          // The tile's C entries are loaded before the products so that
-          // their latency overlaps the arithmetic.
-          uint64_t cv[kI][4];
-#pragma unroll
-          for (int i = 0; i < kI; ++i) {
-            const int rr = rt + ty + kT / 16 * i;
-            const uint64_t* R = rr < n ? m + (int64_t)perm[rr] * n : nullptr;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const int cc = ct + tx + 16 * q;
-              cv[i][q] = R && cc < n ? R[cc] : 0;
-            }
-          }
-          AT acc[kI][4];
-#pragma unroll
-          for (int i = 0; i < kI; ++i)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) acc[i][q] = 0;
-          uint64_t cnt = 0;
-          for (int k = 0; k < pb; ++k) {
-            uint64_t a[kI], b[4];
-#pragma unroll
-            for (int i = 0; i < kI; ++i) a[i] = LF[k][ty + kT / 16 * i];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) b[q] = Us[k][tx + 16 * q];
-#pragma unroll
-            for (int i = 0; i < kI; ++i)
-#pragma unroll
-              for (int q = 0; q < 4; ++q) acc[i][q] += A::prod(f, a[i], b[q]);
-            if (++cnt >= sb) {
-#pragma unroll
-              for (int i = 0; i < kI; ++i)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) acc[i][q] = A::reduce(f, acc[i][q]);
-              cnt = 1;
-            }
-          }
-#pragma unroll
-          for (int i = 0; i < kI; ++i) {
-            const int rr = rt + ty + kT / 16 * i;
-            if (rr >= n) continue;
-            uint64_t* R = m + (int64_t)perm[rr] * n;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const int cc = ct + tx + 16 * q;
-              if (cc >= n) continue;
-              const uint64_t v = f.sub(cv[i][q], A::reduce(f, acc[i][q]));
-              R[cc] = v;
-              nz |= v != 0;
-            }
-          }
-          __syncthreads();
-        }
-      }
+      panel_rows<F, OneCta<kT>>(f, m, n, r0, pb, c0);
+      nz = update_rest<F, LIMBS, OneCta<kT>>(f, m, n, r0, pb, r0 + pb, kP, c0, jend);
     }
     r0 += pb;
     if (!__syncthreads_or(nz)) break;
@@ -398,11 +262,9 @@ __device__ __noinline__ int rank_one(const F& f, uint64_t* __restrict__ m, const
 template <int NT>
 __global__ void __launch_bounds__(NT, 512 / NT)
     rank_batch_kernel(const RankJob* __restrict__ jobs, int64_t count, unsigned long long* next, int64_t* out) {
-  extern __shared__ __align__(16) unsigned char rb_smem[];
-  BatchSmem& S = *reinterpret_cast<BatchSmem*>(rb_smem);
-  // One CTA an SM: the left operand's second buffer, then the row order.
-  uint8_t* a2 = rb_smem + sizeof(BatchSmem);
-  int* perm = reinterpret_cast<int*>(a2 + (NT == 512 ? kRegion : 0));
+  BatchSmem& S = OneCta<NT>::smem();
+  uint8_t* a2 = OneCta<NT>::a2();
+  int* perm = OneCta<NT>::perm();
   for (;;) {
     if (threadIdx.x == 0) S.job = (long long)atomicAdd(next, 1ULL);
     __syncthreads();

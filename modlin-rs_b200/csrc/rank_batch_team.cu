@@ -51,123 +51,13 @@ extern __shared__ __align__(16) unsigned char rb_smem[];
 __device__ __forceinline__ TeamSmem& batch_smem() { return *reinterpret_cast<TeamSmem*>(rb_smem); }
 __device__ __forceinline__ uint8_t* second_buffer() { return rb_smem + sizeof(TeamSmem); }
 __device__ __forceinline__ int* row_order() { return reinterpret_cast<int*>(second_buffer() + kRegion); }
-
-// A warp's tiles of a 64 x 64 output: rows 16 rg .. +16, kTiles groups of 8
-// columns from cg0; and a thread's share of a left operand (64 rows of 64).
-struct TileMap {
-  static constexpr int kTiles = 32 / (kT / 32), kRound = kT / 16, kN = kP / kRound;
+struct TeamCta {
+  static constexpr int kT = 512;
+  static __device__ __forceinline__ BatchSmem& smem() { return batch_smem(); }
+  static __device__ __forceinline__ uint8_t* a2() { return second_buffer(); }
+  static __device__ __forceinline__ int* perm() { return row_order(); }
 };
-
-// Left operand: rows rt .. rt + 63, columns c0 .. c0 + 63, through registers.
-__device__ __forceinline__ void load_rows(const uint64_t* __restrict__ m, int n, const int* perm, int c0, int rt,
-                                          uint64_t (&v)[TileMap::kN][4]) {
-  const int tid = threadIdx.x;
-#pragma unroll
-  for (int w = 0; w < TileMap::kN; ++w) {
-    const int i = (tid >> 4) + TileMap::kRound * w, k4 = 4 * (tid & 15);
-    const uint64_t* src = rt + i < n ? m + (int64_t)perm[rt + i] * n + c0 + k4 : nullptr;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) v[w][u] = src ? src[u] : 0;
-  }
-}
-template <int LIMBS>
-__device__ __forceinline__ void put_rows(uint8_t* dst, const uint64_t (&v)[TileMap::kN][4]) {
-  const int tid = threadIdx.x;
-#pragma unroll
-  for (int w = 0; w < TileMap::kN; ++w)
-    mml::put_planes4<LIMBS>(dst + ((tid >> 4) + TileMap::kRound * w) * kStride + 4 * (tid & 15), kPlane, v[w]);
-}
-
-// C += H U for the row tiles of 64 at rb, rb + stride, .. and the columns from
-// cb: H in columns c0 .. c0 + 63 of those rows, U the first pb of the rows at r0
-// (H's other columns are zero). Whether this thread wrote something nonzero.
-// A function of its own: its registers are the products'.
-template <class F, int LIMBS>
-__device__ __noinline__ bool update_rest(const F& fr, uint64_t* __restrict__ m, const int n, int r0, int pb, int rb,
-                                         int stride, int c0, int cb) {
-  TeamSmem& S = batch_smem();
-  uint8_t* const a2 = second_buffer();
-  int* const perm = row_order();
-  const F f = fr;
-  const LimbRed<F, LIMBS> red(f);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int kTiles = TileMap::kTiles, kN = TileMap::kN;
-  constexpr bool kEarly = LIMBS <= 4;
-  const int rg = warp & 3, cg0 = (warp >> 2) * kTiles;
-  const int g = lane >> 2, t2 = 2 * (lane & 3);
-  uint8_t* const bufs[2] = {S.a, a2};
-  uint32_t acc[2 * LIMBS - 1][4];
-  uint64_t lv[kN][4];
-  // Past the pivots H is zero: any of U's rows will do.
-  const auto row = [pb](int k) { return k < pb ? k : 0; };
-  // Trailing update by strips of kCols column tiles whose right operands fill
-  // region b: the left operand's load and the barriers are shared by them.
-  constexpr int kCols = LIMBS == 8 ? 1 : LIMBS == 4 ? 2 : 4;
-  bool nz = false;
-  for (int ct = cb; ct < n && rb < n; ct += kP * kCols) {
-    __syncthreads();
-    constexpr int kRows4 = kT / 64;
-#pragma unroll 1
-    for (int s = 0; s < kCols; ++s) {
-      uint64_t uv[kN][4];
-      const int col = ct + kP * s + (tid & 63);
-#pragma unroll
-      for (int w = 0; w < kN; ++w)  // U: plane row = column
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          uv[w][u] = col < n ? m[(int64_t)perm[r0 + row(4 * ((tid >> 6) + kRows4 * w) + u)] * n + col] : 0;
-#pragma unroll
-      for (int w = 0; w < kN; ++w)
-        mml::put_planes4<LIMBS>(S.b + s * LIMBS * kPlane + (tid & 63) * kStride + 4 * ((tid >> 6) + kRows4 * w),
-                                kPlane, uv[w]);
-    }
-    if (kEarly) load_rows(m, n, perm, c0, rb, lv);
-    for (int rt = rb, k = 0; rt < n; rt += stride, k ^= 1) {
-      const int ra = rt + 16 * rg + g, rz = ra + 8;
-      uint64_t* pa = ra < n ? m + (int64_t)perm[ra] * n : nullptr;
-      uint64_t* pz = rz < n ? m + (int64_t)perm[rz] * n : nullptr;
-      // C of this warp's tiles is loaded before the left operand where
-      // registers allow, else before each tile's products (which cover it).
-      constexpr bool kAhead = LIMBS <= 4;
-      constexpr int kAll = kTiles * kCols;
-      uint64_t cv[kAhead ? kAll : 1][4];
-      const auto column = [&](int q) { return ct + kP * (q / kTiles) + 8 * (cg0 + q % kTiles) + t2; };
-      const auto load_c = [&](int q, uint64_t (&x)[4]) {
-        const int c = column(q);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const uint64_t* src = e < 2 ? pa : pz;
-          x[e] = src && c + (e & 1) < n ? src[c + (e & 1)] : 0;
-        }
-      };
-      if (kAhead) {
-#pragma unroll
-        for (int q = 0; q < kAll; ++q) load_c(q, cv[q]);
-      }
-      if (!kEarly) load_rows(m, n, perm, c0, rt, lv);
-      put_rows<LIMBS>(bufs[k], lv);
-      __syncthreads();
-      if (kEarly && rt + stride < n) load_rows(m, n, perm, c0, rt + stride, lv);
-#pragma unroll(kAhead ? kAll : 1)
-      for (int q = 0; q < kAll; ++q) {
-        const int c = column(q);
-        uint64_t(&x)[4] = cv[kAhead ? q : 0];
-        if (!kAhead) load_c(q, x);
-        block_tile<LIMBS>(acc, bufs[k], S.b + q / kTiles * LIMBS * kPlane, rg, cg0 + q % kTiles);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          uint64_t* dst = e < 2 ? pa : pz;
-          const uint64_t v = red.plus(x[e], acc, e);
-          if (dst && c + (e & 1) < n) {
-            dst[c + (e & 1)] = v;
-            nz |= v != 0;
-          }
-        }
-      }
-    }
-  }
-  return nz;
-}
+using Map = TileMap<kT>;
 
 // Whether any CTA of the team has something nonzero left.
 __device__ __forceinline__ bool team_any(TeamSmem& S, int c0, bool any) {
@@ -224,23 +114,23 @@ __device__ __noinline__ bool block_step(const F& f, uint64_t* __restrict__ m, co
   }
   const int rb = r0 + kP + first, cb = c0 + kP;  // this CTA's first row tile
   // This warp's tiles: rows 16 rg .. +16, kTiles groups of 8 columns from cg0.
-  constexpr int kTiles = TileMap::kTiles;
+  constexpr int kTiles = Map::kTiles;
   const int rg = warp & 3, cg0 = (warp >> 2) * kTiles;
   const int g = lane >> 2, t2 = 2 * (lane & 3);
-  constexpr int kN = TileMap::kN;
+  constexpr int kN = Map::kN;
   // The next tile's rows are loaded during this one's products where the
   // registers allow; with two buffers one barrier a tile is enough.
   constexpr bool kEarly = LIMBS <= 4;
   uint8_t* const bufs[2] = {S.a, a2};
   uint32_t acc[2 * LIMBS - 1][4];
   uint64_t lv[kN][4];
-  if (cb < n && rb < n && kEarly) load_rows(m, n, perm, c0, rb, lv);
+  if (cb < n && rb < n && kEarly) load_rows<kT>(m, n, perm, c0, rb, lv);
   for (int rt = rb, k = 0; rt < n && cb < n; rt += stride, k ^= 1) {  // H over X
-    if (!kEarly) load_rows(m, n, perm, c0, rt, lv);
+    if (!kEarly) load_rows<kT>(m, n, perm, c0, rt, lv);
     if (rt == rb) __syncthreads();  // the last product has read the buffer (or P^-1)
-    put_rows<LIMBS>(bufs[k], lv);
+    put_rows<LIMBS, kT>(bufs[k], lv);
     __syncthreads();
-    if (kEarly && rt + stride < n) load_rows(m, n, perm, c0, rt + stride, lv);
+    if (kEarly && rt + stride < n) load_rows<kT>(m, n, perm, c0, rt + stride, lv);
     const int ra = rt + 16 * rg + g, rz = ra + 8;
     uint64_t* pa = ra < n ? m + (int64_t)perm[ra] * n + c0 : nullptr;
     uint64_t* pz = rz < n ? m + (int64_t)perm[rz] * n + c0 : nullptr;
@@ -257,7 +147,7 @@ __device__ __noinline__ bool block_step(const F& f, uint64_t* __restrict__ m, co
     }
   }
   const bool nz = rb < n && cb < n &&
-                  update_rest<F, LIMBS>(f, m, n, r0, kP, rb, stride, c0, cb);
+                  update_rest<F, LIMBS, TeamCta>(f, m, n, r0, kP, rb, stride, c0, cb);
   any = __syncthreads_or(nz);
   if constexpr (kTeam) any = team_any(S, c0, any);
   return true;
@@ -267,25 +157,19 @@ template <class F, int LIMBS, bool kTeam>
 __device__ __noinline__ int rank_one(const F& f, uint64_t* __restrict__ m, const int n) {
   TeamSmem& S = batch_smem();
   int* const perm = row_order();
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  using A = Acc<F>;
-  using AT = typename A::T;
-  const uint64_t p = f.modulus();
-  const uint64_t sb = A::batch(f);
-  uint64_t(*LF)[kP + 1] = reinterpret_cast<uint64_t(*)[kP + 1]>(S.a);  // multipliers of a row tile, or F[k][k2]
-  uint64_t(*Us)[kP] = reinterpret_cast<uint64_t(*)[kP]>(S.b);          // U block of one 64-column tile
+  const int tid = threadIdx.x;
   for (int i = tid; i < n; i += kT) perm[i] = i;
   __syncthreads();
   int r0 = 0;
   for (int c0 = 0; c0 < n && r0 < n; c0 += kP) {
     const int W = min(kP, n - c0);
-    if (W == kP && n - r0 >= kP) {
-      // A block without a pivot (4 / p of the invertible ones, the dependent
-      // ones always) is tried again with the next 64 rows, and once more.
+    const int tries = block_tries(f.modulus(), n - r0);
+    if (W == kP && n - r0 >= kP && tries > 0) {
+      // A block without a pivot is tried again with the next 64 rows.
       bool any = false, step = false;
       for (int t = 1;; ++t) {
         step = block_step<F, LIMBS, kTeam>(f, m, n, r0, c0, any);
-        if (step || t == 3 || n - r0 < (t + 1) * kP) break;
+        if (step || t == tries || n - r0 < (t + 1) * kP) break;
         // The rows of the failed block are written by the next attempt's step.
         if constexpr (kTeam) cg::this_cluster().sync();
         if (tid < kP) {
@@ -307,117 +191,10 @@ __device__ __noinline__ int rank_one(const F& f, uint64_t* __restrict__ m, const
     // reads the block it failed on.
     const bool mine = !kTeam || S.team.rank == 0;
     if constexpr (kTeam) cg::this_cluster().sync();
-    // ---- A. in-panel elimination ------------------------------------------
-    for (int kk = 0; mine && kk < W && r0 + pb < n; ++kk) {
-      const int c = c0 + kk, r = r0 + pb;
-      int best = INT_MAX;
-      for (int i = r + tid; i < n; i += kT)
-        if (m[(int64_t)perm[i] * n + c] != 0) {
-          best = i;
-          break;
-        }
-      best = __reduce_min_sync(0xffffffffu, best);
-      if (lane == 0) S.red[warp] = best;
-      __syncthreads();
-      if (tid == 0) {
-        int b = INT_MAX;
-        for (int w = 0; w < kT / 32; ++w) b = min(b, S.red[w]);
-        S.found = b != INT_MAX;
-        if (b != INT_MAX) {
-          const int t = perm[r];
-          perm[r] = perm[b];
-          perm[b] = t;
-          S.pcol[pb] = c;
-          const uint64_t e = m[(int64_t)perm[r] * n + c];
-          S.inv = std::is_same<F, FpM61>::value ? fp_inv_m61(e) : fp_inv_binary(e, p);
-        }
-      }
-      __syncthreads();
-      if (!S.found) continue;
-      const uint64_t* P = m + (int64_t)perm[r] * n + c0;
-      if (tid < W) S.prow[tid] = P[tid];
-      __syncthreads();
-      // Rows below, kG per warp at a time: lane l holds panel entries l and
-      // l + 32 of each of its rows (coalesced loads, all issued before any
-      // is used), so each group costs one memory round trip.
-      const uint64_t inv = S.inv;
-      const uint64_t pv0 = lane > kk && lane < W ? S.prow[lane] : 0;
-      const uint64_t pv1 = lane + 32 > kk && lane + 32 < W ? S.prow[lane + 32] : 0;
-      for (int base = r + 1 + warp; base < n; base += kT / 32 * kG) {
-        uint64_t* R[kG];
-        uint64_t x0[kG], x1[kG];
-#pragma unroll
-        for (int g = 0; g < kG; ++g) {
-          const int i = base + g * (kT / 32);
-          R[g] = i < n ? m + (int64_t)perm[i] * n + c0 : nullptr;
-          x0[g] = R[g] && lane < W ? R[g][lane] : 0;
-          x1[g] = R[g] && lane + 32 < W ? R[g][lane + 32] : 0;
-        }
-#pragma unroll
-        for (int g = 0; g < kG; ++g) {
-          const uint64_t e = __shfl_sync(0xffffffffu, kk < 32 ? x0[g] : x1[g], kk & 31);
-          if (e == 0) continue;  // uniform across the warp
-          const uint64_t fm = f.mul(e, inv);
-          if (lane > kk && lane < W) R[g][lane] = f.sub(x0[g], f.mul(fm, pv0));
-          if (lane + 32 > kk && lane + 32 < W) R[g][lane + 32] = f.sub(x1[g], f.mul(fm, pv1));
-          if (lane == (kk & 31)) R[g][kk] = fm;
-        }
-      }
-      __syncthreads();
-      ++pb;
-    }
     const int jend = c0 + W;
-    if (mine && pb > 0 && jend < n && r0 + pb < n) {
-      // ---- B. U, in place, per 64-column tile ------------------------------
-      for (int idx = tid; idx < pb * pb; idx += kT) {  // pivot rows' multipliers F[k][k2] (k2 < k)
-        const int k = idx / pb, k2 = idx - k * pb;
-        LF[k][k2] = k2 < k ? m[(int64_t)perm[r0 + k] * n + S.pcol[k2]] : 0;
-      }
-      for (int ct = jend; ct < n; ct += kP) {
-        for (int idx = tid; idx < pb * kP; idx += kT) {
-          const int k = idx >> 6, ci = idx & 63;
-          const int cc = ct + ci;
-          Us[k][ci] = cc < n ? m[(int64_t)perm[r0 + k] * n + cc] : 0;
-        }
-        __syncthreads();
-        {
-          // U_k -= sum_{k2<k} F[k][k2] U_k2, kQ threads per column.
-          constexpr int kQ = kT / kP;
-          const int ci = tid / kQ, q = tid % kQ;
-          for (int k = 1; k < pb; ++k) {
-            AT acc = 0;
-            uint64_t tot = 0, cnt = 0;
-            for (int k2 = q; k2 < k; k2 += kQ) {
-              acc += A::prod(f, LF[k][k2], Us[k2][ci]);
-              if (++cnt >= sb) {
-                tot = f.add(tot, A::reduce(f, acc));
-                acc = 0;
-                cnt = 0;
-              }
-            }
-            uint64_t part = f.add(tot, A::reduce(f, acc));
-#pragma unroll
-            for (int o = 1; o < kQ; o <<= 1) part = f.add(part, __shfl_xor_sync(0xffffffffu, part, o));
-            if (q == 0) Us[k][ci] = f.sub(Us[k][ci], part);
-            __syncwarp();
-          }
-        }
-        __syncthreads();
-        for (int idx = tid; idx < pb * kP; idx += kT) {
-          const int k = idx >> 6, cc = ct + (idx & 63);
-          if (cc < n) m[(int64_t)perm[r0 + k] * n + cc] = Us[k][idx & 63];
-        }
-        __syncthreads();
-      }
-      // H: the multipliers negated, in the panel's first pb columns, zeros
-      // behind them. A warp per row.
-      for (int i = r0 + pb + warp; i < n; i += kT / 32) {
-        uint64_t* R = m + (int64_t)perm[i] * n;
-        uint64_t h0 = lane < pb ? R[S.pcol[lane]] : 0, h1 = lane + 32 < pb ? R[S.pcol[lane + 32]] : 0;
-        __syncwarp();
-        R[c0 + lane] = h0 ? p - h0 : 0;
-        R[c0 + lane + 32] = h1 ? p - h1 : 0;
-      }
+    if (mine) {
+      pb = eliminate_panel<F, LIMBS, TeamCta>(f, m, n, r0, c0, W);
+      if (pb > 0 && jend < n && r0 + pb < n) panel_rows<F, TeamCta>(f, m, n, r0, pb, c0);
     }
     __syncthreads();
     if constexpr (kTeam) {
@@ -432,13 +209,13 @@ __device__ __noinline__ int rank_one(const F& f, uint64_t* __restrict__ m, const
       pb = S.panel_pivots;
       cl.sync();
     }
-    // ---- C. trailing rows, as in a block step --------------------------------
+    // The trailing rows, as in a block step.
     if (pb > 0) {
       bool nz = false;
       if (jend < n) {
         const int rb = r0 + pb + (kTeam ? kP * S.team.rank : 0);
         if (rb < n)
-          nz = update_rest<F, LIMBS>(f, m, n, r0, pb, rb, kTeam ? kP * S.team.size : kP, c0,
+          nz = update_rest<F, LIMBS, TeamCta>(f, m, n, r0, pb, rb, kTeam ? kP * S.team.size : kP, c0,
                                          jend);
         nz = __syncthreads_or(nz);
         if constexpr (kTeam) nz = team_any(S, c0, nz);
