@@ -39,6 +39,7 @@
 
 #include "bm_kernels.cuh"
 #include "field.cuh"
+#include "launch.cuh"
 #include "mma_limbs.cuh"
 
 namespace modlin {
@@ -854,13 +855,12 @@ cudaError_t bm_block_prepare() {
   return cudaFuncGetAttributes(&a, bm_block_kernel);
 }
 
-// The batch kernel's dynamic shared memory cap is set once to the largest
+// The batch kernel's dynamic shared memory cap is set once per device to the largest
 // size any batch asks for (200 KiB), so launches of any batch, graph-captured
 // ones included, need no attribute call.
 static cudaError_t bm_batch_attr() {
-  static cudaError_t e =
-      cudaFuncSetAttribute(bm_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  return e;
+  static PerDevice once;
+  return allow_smem(once, bm_batch_kernel, 200 * 1024);
 }
 
 cudaError_t launch_bm_batch(const BmJob* d_jobs, int64_t count, unsigned long long* d_next, uint64_t* gws,

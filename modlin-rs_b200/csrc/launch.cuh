@@ -15,6 +15,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
+#include <cstdint>
 #include <cstdlib>
 #include <utility>
 
@@ -44,6 +46,33 @@ inline bool pdl_enabled() {
     return !(v && v[0] == '0');
   }();
   return on;
+}
+
+// Set-up of a function that the runtime keeps per device (its opt-in to more
+// than 48 KiB of dynamic shared memory): run once for each device, the current
+// one of the calling thread, and again after a failure. A second thread may run
+// it at the same time, to the same effect.
+class PerDevice {
+ public:
+  template <class Fn>
+  cudaError_t operator()(Fn&& set_up) {
+    int dev = 0;
+    const cudaError_t d = cudaGetDevice(&dev);
+    if (d != cudaSuccess) return d;
+    const uint64_t bit = dev >= 0 && dev < 64 ? 1ULL << dev : 0;
+    if (done_.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    const cudaError_t e = set_up();
+    if (e == cudaSuccess) done_.fetch_or(bit, std::memory_order_release);
+    return e;
+  }
+
+ private:
+  std::atomic<uint64_t> done_{0};
+};
+// The opt-in of one kernel: `static PerDevice once; allow_smem(once, kernel, bytes);`
+template <class K>
+cudaError_t allow_smem(PerDevice& once, K kernel, size_t bytes) {
+  return once([&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); });
 }
 
 // kernel<<<grid, block, smem, st>>>(args...), with the PDL attribute when

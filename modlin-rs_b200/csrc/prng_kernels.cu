@@ -33,6 +33,7 @@
 #include <type_traits>
 
 #include "field.cuh"
+#include "launch.cuh"
 #include "mma_limbs.cuh"
 #include "prng_kernels.cuh"
 
@@ -639,8 +640,8 @@ cudaError_t launch_xoro(const XoroFill& a, R red, cudaStream_t st) {
 
 cudaError_t m61_gemm(const uint64_t* A, const uint64_t* B, uint64_t* C, int M, int K, int N, cudaStream_t st) {
   if (M <= 0 || N <= 0 || K <= 0) return cudaSuccess;
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(m61_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
+  static PerDevice once;
+  const cudaError_t attr = allow_smem(once, m61_gemm_kernel, kGemmSmem);
   if (attr != cudaSuccess) return attr;
   const dim3 grid((N + kGN - 1) / kGN, (M + kGM - 1) / kGM);
   m61_gemm_kernel<<<grid, 256, kGemmSmem, st>>>(A, B, C, M, K, N);

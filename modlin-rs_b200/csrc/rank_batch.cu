@@ -25,6 +25,7 @@
 #include <queue>
 #include <vector>
 
+#include "launch.cuh"
 #include "rank_batch_dev.cuh"
 
 namespace modlin {
@@ -296,19 +297,13 @@ static size_t rank_batch_smem_bytes(int threads, int64_t max_n) {
   return sizeof(BatchSmem) + (threads == 512 ? kRegion : 0) + (size_t)max_n * sizeof(int);
 }
 
-// The kernels' dynamic shared memory cap is set once to what the largest side
+// The kernels' dynamic shared memory cap is set once per device to what the largest side
 // needs, so launches of any batch (graph-captured ones included) need no
 // attribute call.
 static cudaError_t rank_batch_attr() {
-  static cudaError_t e = [] {
-    cudaError_t r = cudaFuncSetAttribute(rank_batch_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)rank_batch_smem_bytes(256, kRankBatchMaxN));
-    if (r == cudaSuccess)
-      r = cudaFuncSetAttribute(rank_batch_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)rank_batch_smem_bytes(512, kRankBatchMaxN));
-    return r;
-  }();
-  return e;
+  static PerDevice narrow, wide;
+  const cudaError_t e = allow_smem(narrow, rank_batch_kernel<256>, rank_batch_smem_bytes(256, kRankBatchMaxN));
+  return e != cudaSuccess ? e : allow_smem(wide, rank_batch_kernel<512>, rank_batch_smem_bytes(512, kRankBatchMaxN));
 }
 
 // Threads per CTA: 512 when every matrix has an SM to itself, or the largest
@@ -379,7 +374,8 @@ RankBatchShape rank_batch_shape(const std::vector<RankJob>& jobs, int num_sms) {
   if (B.threads != 512 || nb < 1 || longest <= share) return B;
   std::vector<double> cost(count);
   for (int64_t i = 0; i < count; ++i) cost[i] = rank_batch_cost(jobs[i].p, jobs[i].n);
-  const int* teams = rank_team_resident(num_sms);
+  const RankTeams resident = rank_team_resident(num_sms);
+  const int* teams = resident.n;
   double best = 0.85 * longest;
   for (int k = 0; k < 3; ++k) {
     if (teams[k] < 1) continue;

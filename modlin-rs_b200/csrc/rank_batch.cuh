@@ -36,9 +36,12 @@ constexpr int kRankBatchCounters = 2;  // job counters at d_next
 cudaError_t launch_rank_batch(const RankJob* d_jobs, int64_t count, unsigned long long* d_next,
                               const RankBatchShape& shape, int64_t* d_out, cudaStream_t st);
 // The same for a shape with teams, and the teams of 2, 4 and 8 CTAs that the
-// GPU holds at a time.
+// current device holds at a time.
+struct RankTeams {
+  int n[3];
+};
 cudaError_t launch_rank_team(const RankJob* d_jobs, int64_t count, unsigned long long* d_next,
                              const RankBatchShape& shape, int64_t* d_out, cudaStream_t st);
-const int* rank_team_resident(int num_sms);
+RankTeams rank_team_resident(int num_sms);
 
 }  // namespace modlin

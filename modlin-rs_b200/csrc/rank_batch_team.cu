@@ -19,7 +19,10 @@
 #include <cuda_runtime.h>
 
 #include <climits>
+#include <map>
+#include <mutex>
 
+#include "launch.cuh"
 #include "rank_batch_dev.cuh"
 
 namespace modlin {
@@ -296,9 +299,8 @@ __global__ void __launch_bounds__(kT, 1)
 static size_t team_smem_bytes(int64_t max_n) { return sizeof(TeamSmem) + kRegion + (size_t)max_n * sizeof(int); }
 
 static cudaError_t team_attr() {
-  static const cudaError_t e = cudaFuncSetAttribute(rank_team_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                    (int)team_smem_bytes(kRankBatchMaxN));
-  return e;
+  static PerDevice once;
+  return allow_smem(once, rank_team_kernel, team_smem_bytes(kRankBatchMaxN));
 }
 
 static cudaLaunchConfig_t team_config(int size, int blocks, size_t smem, cudaStream_t st, cudaLaunchAttribute* attr) {
@@ -316,27 +318,31 @@ static cudaLaunchConfig_t team_config(int size, int blocks, size_t smem, cudaStr
   return cfg;
 }
 
-// Teams of 2, 4 and 8 CTAs that the GPU holds at a time.
-const int* rank_team_resident(int num_sms) {
-  struct Teams {
-    int n[3] = {0, 0, 0};
-  };
-  static const Teams t = [num_sms] {
-    Teams q;
-    if (team_attr() != cudaSuccess) return q;
-    for (int k = 0; k < 3; ++k) {
-      cudaLaunchAttribute attr[1];
-      const int size = 2 << k;
-      const cudaLaunchConfig_t cfg =
-          team_config(size, num_sms / size * size, team_smem_bytes(kRankBatchMaxN), nullptr, attr);
-      if (cudaOccupancyMaxActiveClusters(&q.n[k], rank_team_kernel, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        q.n[k] = 0;
-      }
+// Teams of 2, 4 and 8 CTAs that the current device holds at a time (asked once
+// per device).
+RankTeams rank_team_resident(int num_sms) {
+  static std::mutex mu;
+  static std::map<int, RankTeams> known;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || team_attr() != cudaSuccess) {
+    cudaGetLastError();
+    return RankTeams{};
+  }
+  std::lock_guard<std::mutex> g(mu);
+  const auto it = known.find(dev);
+  if (it != known.end()) return it->second;
+  RankTeams t{};
+  for (int k = 0; k < 3; ++k) {
+    cudaLaunchAttribute attr[1];
+    const int size = 2 << k;
+    const cudaLaunchConfig_t cfg =
+        team_config(size, num_sms / size * size, team_smem_bytes(kRankBatchMaxN), nullptr, attr);
+    if (cudaOccupancyMaxActiveClusters(&t.n[k], rank_team_kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      t.n[k] = 0;
     }
-    return q;
-  }();
-  return t.n;
+  }
+  return known[dev] = t;
 }
 
 cudaError_t launch_rank_team(const RankJob* d_jobs, int64_t count, unsigned long long* d_next,

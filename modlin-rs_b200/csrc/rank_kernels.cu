@@ -730,11 +730,8 @@ void launch_window(const F& f, const uint64_t* m, int64_t ld, int n, int r0, int
                    PanelState* ps, uint64_t* Upanel, uint64_t* G, const uint64_t* Lbuf, uint8_t* is_pivot,
                    cudaStream_t st) {
   const size_t smem = 2 * kWindow * kPanel * sizeof(uint64_t);
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute(window_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    attr_set = true;
-  }
+  static PerDevice once;
+  allow_smem(once, window_kernel<F>, smem);
   window_kernel<F><<<1, kWindowThreads, smem, st>>>(f, m, ld, n, r0, col, W, round, ps, Upanel, G, Lbuf, is_pivot);
 }
 
@@ -754,11 +751,8 @@ void launch_couple(const F& f, const uint64_t* m, int64_t ld, int n, int jend, c
                    const uint64_t* G, uint64_t* Ubuf, int64_t ldU, cudaStream_t st) {
   const int cols = n - jend;
   const size_t smem = (size_t)(kPanel * kCoupleCols + kPanel * kPanel) * sizeof(uint64_t);
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute(couple_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    attr_set = true;
-  }
+  static PerDevice once;
+  allow_smem(once, couple_kernel<F>, smem);
   couple_kernel<F><<<(cols + kCoupleCols - 1) / kCoupleCols, 256, smem, st>>>(f, m, ld, n, jend, ps, G, Ubuf, ldU);
 }
 
@@ -781,11 +775,8 @@ void launch_trailing_plain(const F& f, uint64_t* m, int64_t ld, int rbeg, int re
                            const uint64_t* Lbuf, int r0, const uint64_t* Ubuf, int64_t ldU, int K, int* err,
                            cudaStream_t st) {
   if (rbeg >= rend || jend >= cend || K <= 0) return;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(trailing_plain_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPlainSmem);
-    attr = true;
-  }
+  static PerDevice once;
+  allow_smem(once, trailing_plain_kernel<F>, kPlainSmem);
   dim3 grid((cend - jend + 63) / 64, (rend - rbeg + 63) / 64);
   trailing_plain_kernel<F><<<grid, 256, kPlainSmem, st>>>(f, m, ld, rbeg, rend, jend, cend, Lbuf, r0, Ubuf, ldU, K,
                                                            err);
@@ -795,11 +786,8 @@ template <class F>
 void launch_block_inverse(const F& f, const uint64_t* m, int64_t ld, int r0, int col, uint64_t* Vneg, int* status,
                           cudaStream_t st, bool reset_status, const Guard& g) {
   const size_t smem = kPanel * kInvLd * 8 + sizeof(InvScratch<8>);  // more than the pivoting path's kPanel * (kPanel + 1) words
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute(block_inverse_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    attr_set = true;
-  }
+  static PerDevice once;
+  allow_smem(once, block_inverse_kernel<F>, smem);
   launch_k(block_inverse_kernel<F>, dim3(1), dim3(kInvThreads), smem, st, 1, f, m, ld, (int32_t)r0, (int32_t)col,
            Vneg, status, reset_status ? 1 : 0, g);
 }

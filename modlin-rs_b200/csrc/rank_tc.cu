@@ -43,6 +43,7 @@
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
+#include <atomic>
 #include <climits>
 #include <cstring>
 #include <cstdint>
@@ -1050,11 +1051,8 @@ void update_t(const F& f, uint64_t* m, int64_t ld, int rbeg, int rend, int jend,
   const int grid = total < max_ctas ? (int)total : max_ctas;  // one CTA per SM: it owns all 512 TMEM columns
   constexpr bool grouped = !std::is_same<F, FpBarrett>::value;
   constexpr int smem = grouped ? SH::SMEM_TMA : SH::SMEM;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(trailing_tc_kernel<F, LIMBS, KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    attr = true;
-  }
+  static PerDevice once;
+  allow_smem(once, trailing_tc_kernel<F, LIMBS, KK>, smem);
   // C through TMA (the grouped epilogue): 16-byte aligned rows and column offset.
   CUtensorMap cmap;
   std::memset(&cmap, 0, sizeof cmap);
@@ -1071,13 +1069,9 @@ template <int KK>
 cudaError_t update_pair_t(const uint8_t* Aw, const uint8_t* Bw, int rbeg, int rend, int jend, int cend, int max_ctas,
                           int* err, const CUtensorMap& cmap, cudaStream_t st, const Guard& g) {
   using SH = PairShape<KK>;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(trailing_tc_pair_kernel<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         SH::SMEM);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  static PerDevice once;
+  const cudaError_t e = allow_smem(once, trailing_tc_pair_kernel<KK>, SH::SMEM);
+  if (e != cudaSuccess) return e;
   Sched S;
   S.mtiles = (rend - rbeg + 255) / 256;
   S.nsub = (cend - jend + SH::NS - 1) / SH::NS;
@@ -1094,15 +1088,18 @@ cudaError_t update_pair_t(const uint8_t* Aw, const uint8_t* Bw, int rbeg, int re
   cfg.stream = st;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  static int fit = 0;  // clusters of two that can be resident at once
+  // Clusters of two that can be resident at once.
+  static std::atomic<int> fits[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  int fit = fits[dev].load();
   if (!fit) {
     cfg.gridDim = dim3(2 * pairs);
-    int c = 0;
-    if (cudaOccupancyMaxActiveClusters(&c, trailing_tc_pair_kernel<KK>, &cfg) != cudaSuccess || c < 1) {
+    if (cudaOccupancyMaxActiveClusters(&fit, trailing_tc_pair_kernel<KK>, &cfg) != cudaSuccess || fit < 1) {
       cudaGetLastError();
-      c = 1;
+      fit = 1;
     }
-    fit = c;
+    fits[dev].store(fit);
   }
   if (pairs > fit) pairs = fit;
   if (total < pairs) pairs = (int)total;
