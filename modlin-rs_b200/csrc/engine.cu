@@ -685,8 +685,6 @@ static int lc_device_locked(Ctx* C, uint64_t p, const uint64_t* d_s, size_t n, c
   return MODLIN_OK;
 }
 
-// Batched rank: jobs up to kRankBatchMaxN go into one persistent launch
-// (longest first), larger ones through the single-matrix engine afterwards.
 // Longest first: the persistent CTAs then finish close together (LPT).
 static void sort_rank_jobs(std::vector<RankJob>& jobs) {
   std::vector<std::pair<double, size_t>> key(jobs.size());
@@ -697,8 +695,11 @@ static void sort_rank_jobs(std::vector<RankJob>& jobs) {
   jobs.swap(sorted);
 }
 
+// Batched rank: jobs up to kRankBatchMaxN go into one persistent launch (longest
+// first), larger ones through the single-matrix engine afterwards, with `opts`.
 static int rank_batch_locked(Ctx* C, const uint64_t* p, uint64_t* const* d_m, const size_t* n, size_t count,
-                             size_t* ranks_out, cudaStream_t st, std::unique_lock<std::mutex>& g) {
+                             size_t* ranks_out, cudaStream_t st, std::unique_lock<std::mutex>& g,
+                             const modlin_rank_opts* opts = nullptr) {
   if (count == 0) return MODLIN_OK;
   std::vector<RankJob> jobs;
   std::vector<size_t> big;
@@ -734,7 +735,7 @@ static int rank_batch_locked(Ctx* C, const uint64_t* p, uint64_t* const* d_m, co
   if (!big.empty()) {
     g.unlock();
     for (size_t i : big) {
-      const int rc2 = modlin_rank_device(p[i], d_m[i], n[i], nullptr, &ranks_out[i], nullptr, st);
+      const int rc2 = modlin_rank_device(p[i], d_m[i], n[i], opts, &ranks_out[i], nullptr, st);
       if (rc2) return rc2;
     }
     g.lock();
@@ -1299,8 +1300,7 @@ int modlin_rank_batch_device_ex(const uint64_t* p, uint64_t* const* d_m, const s
   int rc = get_ctx(&C);
   if (rc) return rc;
   std::unique_lock<std::mutex> g(C->mu);
-  (void)opts;  // one kernel serves every choice
-  return rank_batch_locked(C, p, d_m, n, count, ranks_out, user_stream(stream), g);
+  return rank_batch_locked(C, p, d_m, n, count, ranks_out, user_stream(stream), g, opts);
 }
 
 int modlin_rank_batch_device(const uint64_t* p, uint64_t* const* d_m, const size_t* n, size_t count,
