@@ -891,6 +891,12 @@ size_t bm_long_bytes(int64_t n) {
 }
 int bm_long_err_offset() { return (int)offsetof(LongSync, err); }
 
+// Cycles that a wait may take beyond its base limit, per output of a working
+// CTA: a wait can span one sweep of all outputs, measured at 330 cycles an
+// output and CTA over 2^63 - 25 (180 over 2^61 - 1, 36 mod 65521), twice that
+// where a matrix takes two windows.
+constexpr long long kSweepCycles = 3000;
+
 template <class P>
 static cudaError_t launch_long_t(const FieldParams& fp, const uint64_t* s, int64_t n, int ctas, bool cluster,
                                  void* ws, long long spin, int skip_cta, int64_t* d_out, cudaStream_t st) {
@@ -903,7 +909,7 @@ static cudaError_t launch_long_t(const FieldParams& fp, const uint64_t* s, int64
   a.ring = reinterpret_cast<BmMatrix*>(w + 256 + long_flags(n));
   a.buf = reinterpret_cast<uint8_t*>(w + 256 + long_flags(n) + long_ring());
   a.out = d_out;
-  a.spin = spin;
+  a.spin = skip_cta >= 0 ? spin : spin + kSweepCycles * (n / (ctas - 1));
   a.skip_cta = skip_cta;
   // The largest chunk: the first superblock's share, within the shared memory.
   const int64_t front = std::min<int64_t>(std::max<int64_t>(n - kBmT, 0), kBmT);

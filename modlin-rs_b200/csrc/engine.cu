@@ -28,8 +28,8 @@ namespace modlin {
 
 std::atomic<uint64_t> g_launches{0};
 // Failure-detection test (modlin_testing_grid_timeout_once): the next grid
-// Berlekamp-Massey launch waits at most g_fault_spin cycles per barrier and
-// CTA g_fault_skip_cta skips its first step arrival; consumed by that launch.
+// Berlekamp-Massey launch waits at most g_fault_spin cycles at a time and CTA
+// g_fault_skip_cta does not signal; consumed by that launch.
 static std::atomic<long long> g_fault_spin{0};
 static std::atomic<int> g_fault_skip_cta{-1};
 static double g_last_trailing_ms = 0.0;
@@ -663,7 +663,8 @@ static int lc_device_locked(Ctx* C, uint64_t p, const uint64_t* d_s, size_t n, c
     return MODLIN_OK;
   }
   CK(C->bmws.ensure(bm_long_bytes((int64_t)n)));
-  // About one second of waiting at ~2 GHz before a wait is declared stuck.
+  // About one second of waiting at ~2 GHz, beyond a sweep's own time, before a
+  // wait is declared stuck.
   long long spin = 2000000000LL;
   if (kernel == MODLIN_LC_CLUSTER) {
     if ((int64_t)n > kBmClusterMaxN) return MODLIN_EINVAL_N;
