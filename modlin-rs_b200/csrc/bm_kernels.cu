@@ -886,8 +886,8 @@ int bm_batch_max_blocks_per_sm(int threads, int64_t smem_words) {
 static size_t long_flags(int64_t n) { return ((size_t)(n / kBmT + 3) * sizeof(unsigned int) + 255) / 256 * 256; }
 static size_t long_ring() { return (2 * kBmH * sizeof(BmMatrix) + 255) / 256 * 256; }
 
-size_t bm_long_bytes(int64_t n) {
-  return 256 + long_flags(n) + long_ring() + (size_t)4 * bm_pitch(n) * sizeof(uint64_t);
+size_t bm_long_bytes(uint64_t p, int64_t n) {
+  return 256 + long_flags(n) + long_ring() + (size_t)4 * bm_limbs(p) * bm_pitch(n);
 }
 int bm_long_err_offset() { return (int)offsetof(LongSync, err); }
 

@@ -38,11 +38,11 @@ cudaError_t bm_block_prepare();
 
 // One long sequence on up to `ctas` CTAs (cooperative launch; at least two),
 // or on one thread-block cluster of 16 CTAs (8 where 16 cannot be launched).
-// ws: bm_long_bytes(n) bytes. spin: cycles a CTA waits, beyond what a sweep of
+// ws: bm_long_bytes(p, n) bytes. spin: cycles a CTA waits, beyond what a sweep of
 // the sequence may take, before it gives up and sets the error word (at
 // bm_long_err_offset() in ws); skip_cta (>= 0, tests only): that CTA does not
 // signal, and spin is all that a CTA waits.
-size_t bm_long_bytes(int64_t n);
+size_t bm_long_bytes(uint64_t p, int64_t n);
 int bm_long_err_offset();
 cudaError_t launch_bm_long(const FieldParams& fp, const uint64_t* s, int64_t n, int ctas, int num_sms, void* ws,
                            long long spin, int skip_cta, int64_t* d_out, cudaStream_t st);

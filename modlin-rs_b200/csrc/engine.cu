@@ -645,9 +645,20 @@ static int lc_device_locked(Ctx* C, uint64_t p, const uint64_t* d_s, size_t n, c
     *lc_out = 0;
     return MODLIN_OK;
   }
-  int kernel = opts ? opts->kernel : MODLIN_LC_AUTO;
-  if (kernel == MODLIN_LC_AUTO)
-    kernel = (int64_t)n < C->tune.bm_long_min ? MODLIN_LC_BLOCK : MODLIN_LC_GRID;
+  const int choice = opts ? opts->kernel : MODLIN_LC_AUTO;
+  int kernel = choice;
+  if (choice == MODLIN_LC_AUTO) kernel = (int64_t)n < C->tune.bm_long_min ? MODLIN_LC_BLOCK : MODLIN_LC_GRID;
+  if (kernel == MODLIN_LC_CLUSTER && (int64_t)n > kBmClusterMaxN) return MODLIN_EINVAL_N;
+  if (kernel != MODLIN_LC_BLOCK) {
+    // 4 bytes a residue and limb; one CTA takes half of that, when memory is short.
+    const cudaError_t e = C->bmws.ensure(bm_long_bytes(p, (int64_t)n));
+    if (e == cudaErrorMemoryAllocation && choice == MODLIN_LC_AUTO) {
+      cudaGetLastError();
+      kernel = MODLIN_LC_BLOCK;
+    } else {
+      CK(e);
+    }
+  }
   CK(C->bmout.ensure(sizeof(int64_t) * 4));
   int64_t* d_out = C->bmout.as<int64_t>();
   if (kernel == MODLIN_LC_BLOCK) {
@@ -662,12 +673,10 @@ static int lc_device_locked(Ctx* C, uint64_t p, const uint64_t* d_s, size_t n, c
     *lc_out = (size_t)C->h_out[0];
     return MODLIN_OK;
   }
-  CK(C->bmws.ensure(bm_long_bytes((int64_t)n)));
   // About one second of waiting at ~2 GHz, beyond a sweep's own time, before a
   // wait is declared stuck.
   long long spin = 2000000000LL;
   if (kernel == MODLIN_LC_CLUSTER) {
-    if ((int64_t)n > kBmClusterMaxN) return MODLIN_EINVAL_N;
     CK(launch_bm_cluster(fp, d_s, (int64_t)n, C->bmws.p, spin, d_out, st));
   } else {
     const int ctas = opts && opts->grid_ctas > 0 ? opts->grid_ctas : C->num_sms;
@@ -928,7 +937,7 @@ static int autotune_locked(Ctx* C, std::string& rep) {
   const int thr[3] = {128, 256, 512};
   TK(C->seq.ensure((size_t)65536 * 8));
   TK(C->bmout.ensure(sizeof(int64_t) * 4));
-  TK(C->bmws.ensure(std::max<size_t>((size_t)bm_workspace_words(65536) * 8, bm_long_bytes(65536))));
+  TK(C->bmws.ensure(std::max<size_t>((size_t)bm_workspace_words(65536) * 8, bm_long_bytes(kM61, 65536))));
   uint64_t* seq = C->seq.as<uint64_t>();
   const int64_t smem_words = (200 * 1024) / 8;
   rep += ", \"bm_block_ms\": {";

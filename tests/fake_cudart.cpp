@@ -18,6 +18,7 @@ std::map<std::pair<int, const void*>, size_t> g_allowed;    // per device
 std::map<std::pair<int, std::string>, int> g_launched;      // per device
 std::string g_rejected;
 char g_symbol[8 << 20];
+size_t g_free = (size_t)-1;  // largest allocation that succeeds
 struct Call {
   dim3 grid, block;
   size_t smem;
@@ -46,6 +47,7 @@ cudaError_t launch(const void* f, size_t smem) {
 extern "C" {
 // For the test.
 void fake_set_device(int d) { g_dev = d; }
+void fake_set_free(size_t bytes) { g_free = bytes; }
 const char* fake_rejected() { return g_rejected.c_str(); }
 int fake_launches(const char* part) {
   int n = 0;
@@ -120,7 +122,7 @@ cudaError_t cudaGetLastError() {
 }
 const char* cudaGetErrorName(cudaError_t) { return "error"; }
 cudaError_t cudaMalloc(void** p, size_t n) {
-  *p = std::calloc(n ? n : 1, 1);
+  *p = n > g_free ? nullptr : std::calloc(n ? n : 1, 1);
   return *p ? cudaSuccess : set(cudaErrorMemoryAllocation);
 }
 cudaError_t cudaMallocHost(void** p, size_t n) { return cudaMalloc(p, n); }
