@@ -169,15 +169,10 @@ __global__ void split_b_kernel(const uint64_t* __restrict__ Ubuf, int64_t ldU, i
   }
 }
 
-// Exact residue of sum_d 2^(8d) S_d for one output column (S in registers
-// acc_lo/acc_hi = the two 128-bit halves prepared by the fold).
-template <class F>
-__device__ __forceinline__ uint64_t finish(const F& f, u128 lo, u128 hi, uint64_t r64) {
-  if constexpr (std::is_same<F, FpM61>::value) {
-    return f.reduce(lo);  // already folded into one 128-bit value
-  } else {
-    return f.add(f.reduce(lo), f.mul(f.reduce(hi), r64));
-  }
+// Exact residue of lo + 2^64 hi, the two halves of sum_d 2^(8d) S_d for one
+// output column (r64 = 2^64 mod p).
+__device__ __forceinline__ uint64_t finish(const FpBarrett& f, u128 lo, u128 hi, uint64_t r64) {
+  return f.add(f.reduce(lo), f.mul(f.reduce(hi), r64));
 }
 
 // In place 8 x 8 byte transpose: afterwards byte c of t[i] is the former
@@ -556,136 +551,135 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16) + qc * 4;
     int it = 0;
     bool ok = true;
-    if constexpr (LIMBS == 8) {
-      // C goes through shared memory so that global accesses are coalesced.
-      // The 4 warps of a TMEM lane quadrant form a group that owns rows
-      // 32*quad..+32 of the 128 x 16 tile: warp (quad, qc) copies rows
-      // 32*quad + 8*qc..+8 kCDepth - 1 subtiles ahead with cp.async, every
-      // thread then works on its own row in shared memory, and the results
-      // leave the same way. Each group synchronises on its own named barrier
-      // (1 + quad), so the four groups drift and their phases overlap.
-      constexpr int kRowsPerWarp = 8;
-      const int rbase_w = quad * 32 + qc * kRowsPerWarp;
-      const int rr = lane >> 4, cc = lane & 15, rr4 = lane >> 3, cc2 = (lane & 7) * 2;
-      auto epi_bar = [quad]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + quad) : "memory"); };
-      // 16-byte copies when every row start is 16-byte aligned and the
-      // subtile is complete, else 8-byte copies.
-      const bool vec_ld = (ld & 1) == 0 && ((uintptr_t)m & 15) == 0 && (jend & 1) == 0;
-      int64_t pg = g0;
-      int pmt = (int)(g0 / S.nsub), psb = (int)(g0 - (int64_t)pmt * S.nsub);
-      int pcount = 0;
-      auto pf_issue = [&]() {
-        if (pg < g1) {
-          const int mt = pmt, sb = psb;
-          const int64_t pbase = (int64_t)rbeg + (int64_t)mt * 128;
-          uint64_t* slot = sC + (size_t)(pcount % kCDepth) * 128 * kCStride;
-          const int64_t sc0 = (int64_t)jend + (int64_t)sb * NS;
-          if (vec_ld && sc0 + 16 <= cend) {
+    static_assert(LIMBS == 8, "the other primes' epilogue is grouped");
+    // C goes through shared memory so that global accesses are coalesced.
+    // The 4 warps of a TMEM lane quadrant form a group that owns rows
+    // 32*quad..+32 of the 128 x 16 tile: warp (quad, qc) copies rows
+    // 32*quad + 8*qc..+8 kCDepth - 1 subtiles ahead with cp.async, every
+    // thread then works on its own row in shared memory, and the results
+    // leave the same way. Each group synchronises on its own named barrier
+    // (1 + quad), so the four groups drift and their phases overlap.
+    constexpr int kRowsPerWarp = 8;
+    const int rbase_w = quad * 32 + qc * kRowsPerWarp;
+    const int rr = lane >> 4, cc = lane & 15, rr4 = lane >> 3, cc2 = (lane & 7) * 2;
+    auto epi_bar = [quad]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + quad) : "memory"); };
+    // 16-byte copies when every row start is 16-byte aligned and the
+    // subtile is complete, else 8-byte copies.
+    const bool vec_ld = (ld & 1) == 0 && ((uintptr_t)m & 15) == 0 && (jend & 1) == 0;
+    int64_t pg = g0;
+    int pmt = (int)(g0 / S.nsub), psb = (int)(g0 - (int64_t)pmt * S.nsub);
+    int pcount = 0;
+    auto pf_issue = [&]() {
+      if (pg < g1) {
+        const int mt = pmt, sb = psb;
+        const int64_t pbase = (int64_t)rbeg + (int64_t)mt * 128;
+        uint64_t* slot = sC + (size_t)(pcount % kCDepth) * 128 * kCStride;
+        const int64_t sc0 = (int64_t)jend + (int64_t)sb * NS;
+        if (vec_ld && sc0 + 16 <= cend) {
 #pragma unroll
-            for (int i = 0; i < kRowsPerWarp / 4; ++i) {
-              const int lr = rbase_w + 4 * i + rr4;
-              const int64_t gr = pbase + lr;
-              if (gr < rend) cp_async16(slot + lr * kCStride + cc2, m + gr * ld + sc0 + cc2);
-            }
-          } else {
-            const int64_t gc = sc0 + cc;
-#pragma unroll
-            for (int i = 0; i < kRowsPerWarp / 2; ++i) {
-              const int lr = rbase_w + 2 * i + rr;
-              const int64_t gr = pbase + lr;
-              if (gr < rend && gc < cend) cp_async8(slot + lr * kCStride + cc, m + gr * ld + gc);
-            }
+          for (int i = 0; i < kRowsPerWarp / 4; ++i) {
+            const int lr = rbase_w + 4 * i + rr4;
+            const int64_t gr = pbase + lr;
+            if (gr < rend) cp_async16(slot + lr * kCStride + cc2, m + gr * ld + sc0 + cc2);
           }
-          ++pg;
-          if (++psb == S.nsub) {
-            psb = 0;
-            ++pmt;
+        } else {
+          const int64_t gc = sc0 + cc;
+#pragma unroll
+          for (int i = 0; i < kRowsPerWarp / 2; ++i) {
+            const int lr = rbase_w + 2 * i + rr;
+            const int64_t gr = pbase + lr;
+            if (gr < rend && gc < cend) cp_async8(slot + lr * kCStride + cc, m + gr * ld + gc);
           }
         }
-        cp_async_commit();
-        ++pcount;
-      };
-      for (int k = 0; k < kCDepth - 1; ++k) pf_issue();
-      int mt = (int)(g0 / S.nsub), sb = (int)(g0 - (int64_t)mt * S.nsub);
-      for (int64_t g = g0; g < g1; ++g, ++it, sb = sb + 1 == S.nsub ? (++mt, 0) : sb + 1) {
-        const int64_t base = (int64_t)rbeg + (int64_t)mt * 128;
-        const bool row_ok = base + row < rend;
-        const int ab = it & 1;
-        const uint32_t lane_addr = lane_base + ab * 256;
-        cp_async_wait<kCDepth - 2>();
-        epi_bar();  // this subtile's C is in shared memory; the previous one has been stored
-        pf_issue();
-        uint64_t* slot = sC + (size_t)(it % kCDepth) * 128 * kCStride;
-        uint64_t* my = slot + row * kCStride + qc * 4;
-        const int64_t c0 = (int64_t)jend + (int64_t)sb * NS + qc * 4;
-        uint64_t cv[4];
+        ++pg;
+        if (++psb == S.nsub) {
+          psb = 0;
+          ++pmt;
+        }
+      }
+      cp_async_commit();
+      ++pcount;
+    };
+    for (int k = 0; k < kCDepth - 1; ++k) pf_issue();
+    int mt = (int)(g0 / S.nsub), sb = (int)(g0 - (int64_t)mt * S.nsub);
+    for (int64_t g = g0; g < g1; ++g, ++it, sb = sb + 1 == S.nsub ? (++mt, 0) : sb + 1) {
+      const int64_t base = (int64_t)rbeg + (int64_t)mt * 128;
+      const bool row_ok = base + row < rend;
+      const int ab = it & 1;
+      const uint32_t lane_addr = lane_base + ab * 256;
+      cp_async_wait<kCDepth - 2>();
+      epi_bar();  // this subtile's C is in shared memory; the previous one has been stored
+      pf_issue();
+      uint64_t* slot = sC + (size_t)(it % kCDepth) * 128 * kCStride;
+      uint64_t* my = slot + row * kCStride + qc * 4;
+      const int64_t c0 = (int64_t)jend + (int64_t)sb * NS + qc * 4;
+      uint64_t cv[4];
+      {
+        const ulonglong2 v0 = *reinterpret_cast<const ulonglong2*>(my);
+        const ulonglong2 v1 = *reinterpret_cast<const ulonglong2*>(my + 2);
+        cv[0] = v0.x;
+        cv[1] = v0.y;
+        cv[2] = v1.x;
+        cv[3] = v1.y;
+      }
+      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(acc_full + ab, (it >> 1) & 1, err));
+      if (ok) {
+        fence_after();
+        uint64_t res[4];
         {
-          const ulonglong2 v0 = *reinterpret_cast<const ulonglong2*>(my);
-          const ulonglong2 v1 = *reinterpret_cast<const ulonglong2*>(my + 2);
-          cv[0] = v0.x;
-          cv[1] = v0.y;
-          cv[2] = v1.x;
-          cv[3] = v1.y;
-        }
-        if (ok) ok = __all_sync(0xffffffffu, mbar_wait(acc_full + ab, (it >> 1) & 1, err));
-        if (ok) {
-          fence_after();
-          uint64_t res[4];
-          {
-            u128 lo[4], hi[4];
+          u128 lo[4], hi[4];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) lo[c] = hi[c] = 0;
+          for (int c = 0; c < 4; ++c) lo[c] = hi[c] = 0;
 #pragma unroll 1
-            for (int d = 0; d < SH::DIAG; ++d) {
-              uint32_t a[4];
-              tmem_ld4(lane_addr + d * NS, a);
-              tmem_wait_ld();
+          for (int d = 0; d < SH::DIAG; ++d) {
+            uint32_t a[4];
+            tmem_ld4(lane_addr + d * NS, a);
+            tmem_wait_ld();
 #pragma unroll
-              for (int c = 0; c < 4; ++c) {
-                asm volatile("" : "+r"(a[c]));
-                if (d < 8)
-                  lo[c] += (u128)a[c] << (8 * d);
-                else
-                  hi[c] += (u128)a[c] << (8 * (d - 8));
-              }
+            for (int c = 0; c < 4; ++c) {
+              asm volatile("" : "+r"(a[c]));
+              if (d < 8)
+                lo[c] += (u128)a[c] << (8 * d);
+              else
+                hi[c] += (u128)a[c] << (8 * (d - 8));
             }
-            fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(acc_empty + ab);
-#pragma unroll
-            for (int c = 0; c < 4; ++c) res[c] = f.sub(cv[c], finish(f, lo[c], hi[c], r64));
           }
-          if (row_ok) {
-            if (c0 + 4 <= cend) {
-              *reinterpret_cast<ulonglong2*>(my) = make_ulonglong2(res[0], res[1]);
-              *reinterpret_cast<ulonglong2*>(my + 2) = make_ulonglong2(res[2], res[3]);
-            } else {
+          fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(acc_empty + ab);
 #pragma unroll
-              for (int c = 0; c < 4; ++c)
-                if (c0 + c < cend) my[c] = res[c];
-            }
+          for (int c = 0; c < 4; ++c) res[c] = f.sub(cv[c], finish(f, lo[c], hi[c], r64));
+        }
+        if (row_ok) {
+          if (c0 + 4 <= cend) {
+            *reinterpret_cast<ulonglong2*>(my) = make_ulonglong2(res[0], res[1]);
+            *reinterpret_cast<ulonglong2*>(my + 2) = make_ulonglong2(res[2], res[3]);
+          } else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              if (c0 + c < cend) my[c] = res[c];
           }
         }
-        epi_bar();  // results of all rows in shared memory
-        if (ok) {
-          const int64_t sc0 = (int64_t)jend + (int64_t)sb * NS;
-          if (vec_ld && sc0 + 16 <= cend) {
+      }
+      epi_bar();  // results of all rows in shared memory
+      if (ok) {
+        const int64_t sc0 = (int64_t)jend + (int64_t)sb * NS;
+        if (vec_ld && sc0 + 16 <= cend) {
 #pragma unroll
-            for (int i = 0; i < kRowsPerWarp / 4; ++i) {
-              const int lr = rbase_w + 4 * i + rr4;
-              const int64_t gr = base + lr;
-              if (gr < rend)
-                *reinterpret_cast<ulonglong2*>(m + gr * ld + sc0 + cc2) =
-                    *reinterpret_cast<const ulonglong2*>(slot + lr * kCStride + cc2);
-            }
-          } else {
-            const int64_t gc = sc0 + cc;
+          for (int i = 0; i < kRowsPerWarp / 4; ++i) {
+            const int lr = rbase_w + 4 * i + rr4;
+            const int64_t gr = base + lr;
+            if (gr < rend)
+              *reinterpret_cast<ulonglong2*>(m + gr * ld + sc0 + cc2) =
+                  *reinterpret_cast<const ulonglong2*>(slot + lr * kCStride + cc2);
+          }
+        } else {
+          const int64_t gc = sc0 + cc;
 #pragma unroll
-            for (int i = 0; i < kRowsPerWarp / 2; ++i) {
-              const int lr = rbase_w + 2 * i + rr;
-              const int64_t gr = base + lr;
-              if (gr < rend && gc < cend) m[gr * ld + gc] = slot[lr * kCStride + cc];
-            }
+          for (int i = 0; i < kRowsPerWarp / 2; ++i) {
+            const int lr = rbase_w + 2 * i + rr;
+            const int64_t gr = base + lr;
+            if (gr < rend && gc < cend) m[gr * ld + gc] = slot[lr * kCStride + cc];
           }
         }
       }
@@ -1112,8 +1106,6 @@ cudaError_t update_pair_t(const uint8_t* Aw, const uint8_t* Bw, int rbeg, int re
 inline int limbs_of(uint64_t p) { return p == kM61 ? 8 : limbs_for(p); }
 
 }  // namespace tc
-
-int tc_crossover_n(uint64_t) { return 512; }
 
 // Whether updates over 2^61 - 1 run on CTA pairs (modlin_set_tc_pairs; off
 // by default: measured 1.5 % slower than single CTAs in the 16384^2 rank).

@@ -22,8 +22,6 @@ struct LimbOut {
   int32_t c_zero = 0;
 };
 
-// Smallest side for which MODLIN_RANK_AUTO uses the tensor-core update.
-int tc_crossover_n(uint64_t p);
 // Workspace bytes for the limb planes of L (rows x K) and U (K x cols), K <= 128.
 size_t tc_a_bytes(int rows);
 size_t tc_b_bytes(int cols);
