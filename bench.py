@@ -42,6 +42,19 @@ def algorithmic_work(n, pcols):
     return sum((n - 1 - k) * (n - 1 - j) for k, j in enumerate(pcols))
 
 
+def limb_ops(p):
+    """int8 operations of one multiply-add mod p as 8-bit limb products (1, 2, 4 or 8 limbs a residue)."""
+    limbs = 1 if p <= 1 << 8 else 2 if p <= 1 << 16 else 4 if p < 1 << 32 else 8
+    return 2 * limbs * limbs
+
+
+def residual_macs(n, lc):
+    """Multiply-adds of the residual form of Berlekamp-Massey: 2 (n - i) at step i, over the min(n, 2 lc) steps that
+    can change the complexity."""
+    t = min(n, 2 * lc)
+    return t * (2 * n - t + 1)
+
+
 def trailing_work(n, pcols, panel=64):
     """modMACs of the trailing-update launches: per panel with pb pivots,
     (rows below the panel's pivots) x (columns right of the panel) x pb."""
@@ -383,7 +396,8 @@ def bm_measure(torch, modlin, steps=2, warmup=1, long_n=200000, long_L=65280, ba
     assert not bad, bad[:5]
     iid_dev = max(abs(lcs[i] - (j[1] + 1) // 2) for i, j in enumerate(jobs) if not j[2])
     batch = {"sequences": len(jobs), "total_steps": total, "ms": ms, "steps_per_s": total / (ms * 1e-3),
-             "planted_exact": True, "iid_max_dev_from_half": iid_dev}
+             "planted_exact": True, "iid_max_dev_from_half": iid_dev,
+             "int8_ops": sum(limb_ops(p) * residual_macs(n, c) for p, n, c in zip(ps, ns, lcs))}
     g = gold.get(f"lc_batch_{len(jobs)}")
     cached = bool(g)
     if not g and len(jobs) <= 8192:  # no cached answers for this size: the live oracle
@@ -569,6 +583,7 @@ def rank_batch_measure(torch, modlin, steps=2, warmup=1, count=4096, single_samp
     want = [j[3] if j[2] else j[1] for j in jobs]
     res = {"matrices": len(jobs), "ms": ms, "matrices_per_s": len(jobs) / (ms * 1e-3), "work_modmac": work_mac,
            "modmac_per_s": work_mac / (ms * 1e-3),
+           "int8_ops": sum(limb_ops(p) * sum((n - 1 - k) ** 2 for k in range(r)) for p, n, r in zip(ps, ns, ranks)),
            "oracle": {"all_ranks_equal": True, "matrices_compared": len(jobs),
                       "answers": "cached, input digest equal" if cached else "live oracle",
                       "non_generic_ranks": sum(1 for i in range(len(jobs)) if ranks[i] != want[i])},
@@ -1105,31 +1120,29 @@ def main():
         extras["rank_batch"] = rank_batch_measure(torch, modlin, steps=1, warmup=1, single_sample=16)
         # The generators' device fill and the README's largest rank job.
         extras["prng_fill"] = prng_fill_measure(torch, modlin)
-        # Rooflines of the other workloads. Integer-pipe work against the
-        # measured u64 multiply-accumulate peak (the plain trailing update's
-        # inner loop alone, all SMs); tensor-core work against the int8 GEMM.
-        peak_int = extras["trailing_update"]["plain_mac_peak_modmac_per_s"]
+        # Rooflines of the other workloads: the batches' limb products against
+        # the int8 GEMM, the long sequences' dependent steps against one step's
+        # latency.
         int8 = int8_sustained_tops(torch) or int8_peak_tops(torch)
-        int_src = "measured: u64 x u64 -> u128 multiply-accumulate loop on operands in shared memory, all SMs " \
-                  "(modlin_plain_mac_peak)"
-        bm = extras["berlekamp_massey"]
-        if "mac_per_s" in bm["batch"]:
-            a = bm["batch"]["mac_per_s"]
-            bm["batch"]["roofline"] = {"bound": "tensor pipe and the chain of steps in one warp", "achieved": a,
-                                       "peak": peak_int, "unit": "modMAC/s", "frac": a / peak_int,
-                                       "peak_source": int_src}
+        bm, rb = extras["berlekamp_massey"], extras["rank_batch"]
+        for e, what in ((bm["batch"], "the residual form's multiply-adds"),
+                        (rb, "the elimination's multiply-adds")):
+            if int8:
+                a = e["int8_ops"] / (e["ms"] * 1e-3) / 1e12
+                e["roofline"] = {"bound": "tensor", "achieved": a, "peak": int8, "unit": "TFLOP/s", "frac": a / int8,
+                                 "peak_source": "measured, sustained: cuBLASLt int8 GEMM 8192^3 (torch._int_mm) back "
+                                                "to back for 2.5 s on this GPU",
+                                 "note": what + " x limb products x 2 ops / batch time; the kernels' mma.sync does "
+                                                "4096 of them per SM and cycle, about half of the GEMM's rate"}
         for key in ("long_planted", "long_iid"):
             e = bm[key]
-            if "mac_per_s" in e.get("grid", {}):
-                a, pk = e["grid"]["mac_per_s"], peak_int
-                e["roofline"] = {"bound": "latency: the chain of steps in one warp", "achieved": a, "peak": pk,
-                                 "unit": "modMAC/s", "frac": a / pk,
-                                 "peak_source": int_src}
-        rb = extras["rank_batch"]
-        rb["roofline"] = {"bound": "tensor pipe (limb products; the peak is the integer pipes')",
-                          "achieved": rb["modmac_per_s"],
-                          "peak": peak_int, "unit": "modMAC/s", "frac": rb["modmac_per_s"] / peak_int,
-                          "peak_source": int_src}
+            steps_needed = min(e["n"], 2 * e["lc"])
+            a, pk = steps_needed / (e["grid"]["ms"] * 1e-3), measured_peaks().get("sm_max_mhz", 1965.0) * 1e6 / 190
+            e["roofline"] = {"bound": "latency: the chain of steps in one warp", "achieved": a, "peak": pk,
+                             "unit": "steps/s", "frac": a / pk,
+                             "peak_source": "190 cycles a step over 2^61 - 1 (clock64, the step's chain alone) at the "
+                                            "card's maximum SM clock",
+                             "note": "steps: the min(n, 2 complexity) that can change the complexity"}
         rp = extras["rank_planted"]
         if int8:
             a = rp["tc"]["modmac_per_s"] * 128 / 1e12
