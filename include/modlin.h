@@ -142,9 +142,11 @@ int modlin_block_inverse_device(uint64_t p, const uint64_t *d_P, size_t ldp, uin
 
 /* ---- Linear complexity (src/fp.rs:257-308) ------------------------------ */
 
-#define MODLIN_LC_AUTO 0      /* block kernel for short sequences, grid from about 1000 on */
+#define MODLIN_LC_AUTO 0      /* block kernel for short sequences, grid from 1300 residues on (tunable);
+                                 block also when the grid's workspace cannot be allocated */
 #define MODLIN_LC_BLOCK 1     /* one CTA runs the whole sequence (plain form) */
-#define MODLIN_LC_GRID 2      /* persistent cooperative kernel, one CTA per SM */
+#define MODLIN_LC_GRID 2      /* persistent cooperative kernel, one CTA per SM; device workspace of 4
+                                 bytes a residue and limb (odd p below 2^8, 2^16, 2^32, 2^63: 1, 2, 4, 8; p = 2: 4) */
 #define MODLIN_LC_CLUSTER 3   /* the grid kernel on one 16-CTA thread-block cluster
                                  (n <= 409600; MODLIN_EINVAL_N beyond) */
 
@@ -196,9 +198,9 @@ int modlin_rank_batch(const modlin_job *jobs, size_t count, size_t *ranks_out);
  * into one persistent launch; larger ones run one after another. */
 int modlin_rank_batch_device(const uint64_t *p, uint64_t *const *d_m, const size_t *n, size_t count,
                              size_t *ranks_out, void *stream);
-/* modlin_rank_batch_device with options (MODLIN_RANK_*): every job
- * of side up to 8192 is ranked by the one batch kernel whatever the choice;
- * larger ones run one after another with it. */
+/* modlin_rank_batch_device with options (MODLIN_RANK_*): sides up to 8192 are
+ * ranked in the one batched launch whatever the choice; larger ones run one
+ * after another with it. */
 int modlin_rank_batch_device_ex(const uint64_t *p, uint64_t *const *d_m, const size_t *n, size_t count,
                                 const modlin_rank_opts *opts, size_t *ranks_out, void *stream);
 /* Linear complexities of `count` sequences in one persistent launch. */

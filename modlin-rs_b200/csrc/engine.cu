@@ -58,8 +58,8 @@ struct DevBuf {
 
 // Choices the autotuner measures (defaults until modlin_autotune runs on the
 // device): plain/tensor-core crossover per limb count, smallest side for
-// two-panel block steps, BM threads per CTA by length, BM block/cluster
-// crossover, BM batch threads by the longest sequence.
+// two-panel block steps, BM threads per CTA by length, the length from which
+// many CTAs beat one, BM batch threads by the longest sequence.
 struct Tune {
   bool measured = false;
   int tc_cross[4] = {64, 64, 64, 64};               // 1, 2, 4, 8 limbs
@@ -69,7 +69,7 @@ struct Tune {
   int bm_cluster_min = 4096;                        // from here on one cluster beats one CTA (not a rule of AUTO)
   int bm_batch_threads[3] = {256, 256, 512};        // longest < 512, < 2048, longer
   // Shared memory per batch CTA (KiB), by the same classes: a sequence whose
-  // residuals (16 bytes an entry, 8 for p < 2^31) do not fit runs from the
+  // residuals (2 bytes an entry and limb) do not fit runs from the
   // CTA's global workspace; smaller caps put more CTAs on an SM.
   int bm_batch_smem_kib[3] = {200, 200, 200};
 };

@@ -10,11 +10,9 @@
 //    Schur complement: H = -X P^-1 for the panel X below P (written over X),
 //    then C += H U tile by tile. P^-1 by inv64, the products as 64 x 64 x 64
 //    limb products on the tensor cores (mma_limbs.cuh).
-//  * Otherwise (dependent columns, the last ragged panel) the reference's panel
-//    (src/fp.rs:125-255): A. in-panel elimination with the first nonzero row as
-//    pivot (src/fp.rs:151-178); B. U block by forward substitution
-//    (src/fp.rs:181-200); C. trailing update on the integer pipes
-//    (src/fp.rs:202-248), one reduction per safe_batch products.
+//  * Otherwise (dependent columns, the last ragged panel, p = 2) the reference's
+//    panel (src/fp.rs:125-200) and the update of the rest as in a block step
+//    (rank_batch_dev.cuh).
 // When an update leaves nothing nonzero, the rank is what has been counted.
 // Every residue is exact, so the rank is the reference's.
 #include <cuda_runtime.h>

@@ -13,8 +13,8 @@
 // ms on one CTA, 2.83 on eight.
 //
 // The steps are those of rank_batch.cu. That kernel stays for batches without
-// teams: it is up to 9 % faster there for p < 2^32 (148 of side 512 mod 65521:
-// 0.86 ms, 0.94 here).
+// teams: it is up to 10 % faster there for p < 2^32 (148 of side 512 mod 65521:
+// 0.78 ms, 0.84 here).
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 

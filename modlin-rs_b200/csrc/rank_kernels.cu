@@ -21,8 +21,8 @@ namespace modlin {
 // pivot row k satisfies  U_k = alpha_k * row_k - sum_{k2<k} G[k][k2] * U_k2.
 // ---------------------------------------------------------------------------
 // Issue-bound: 64 x 64 entries, two products and one reduction each, for every
-// pivot (ElimField::comb; 41 us over 2^61 - 1, 98 with two reduced products
-// per entry).
+// pivot (ElimField::comb; 64 pivots over 2^61 - 1: 117 us, 127 with two reduced
+// products per entry).
 template <class F>
 __global__ void __launch_bounds__(kWindowThreads) window_kernel(F f, const uint64_t* __restrict__ m, int64_t ld,
                                                                  int32_t n, int32_t r0, int32_t col, int32_t W,
@@ -144,8 +144,8 @@ __global__ void __launch_bounds__(kWindowThreads) window_kernel(F f, const uint6
 // ---------------------------------------------------------------------------
 // The pivot rows are normalised when they are loaded (U_k * inv_k), so a row's
 // dependent chain is one shuffle and one multiply-add per pivot; the
-// multipliers are formed afterwards (6 us for 436 rows and 64 pivots over
-// 2^61 - 1, 24 with the multiplier on the chain).
+// multipliers are formed afterwards (64 pivots over 2^61 - 1: 6 us for 436 rows,
+// 24 with the multiplier on the chain; 60 and 79 us for 5950 rows).
 template <class F>
 __global__ void __launch_bounds__(256) bulk_kernel(F f, uint64_t* __restrict__ m, int64_t ld, int32_t n, int32_t r0,
                                                     int32_t col, int32_t W, int32_t pb_lo, PanelState* ps,
@@ -210,8 +210,8 @@ __global__ void __launch_bounds__(256) bulk_kernel(F f, uint64_t* __restrict__ m
 // U_k[c] = alpha_k * row_{prow_k}[c] - sum_{k2<k} G[k][k2] * U_k2[c],
 // sequential in k. Eight threads share a column's sum (a CTA takes 32
 // columns), lazy accumulation and a shuffle reduction per k: the chain of 64
-// steps of up to 8 products each binds it (11 us for 436 columns over
-// 2^61 - 1, 118 with a thread per column).
+// steps of up to 8 products each binds it (over 2^61 - 1 11 us for 436 columns,
+// 118 with a thread per column; 65 and 142 us for 5950 columns).
 // ---------------------------------------------------------------------------
 constexpr int kCoupleCols = 32, kCoupleSplit = 8;
 template <class F>
